@@ -332,16 +332,17 @@ typedef struct {
 } mclsgpu_domain_info;
 int mclsgpu_domain_query(mclsgpu_domain* dom, mclsgpu_domain_info* info);
 
-/* FP32 walk launch shape: histories carried per lane (1, 2, 4 or 8; 2
- * applies to fixed-length histories on records of at most 64 bytes, 4 and 8
- * to fixed-length histories on 32-byte records, others fall back to fewer) and
- * threads per block (128 or 256).  No counterpart in the reference. */
+/* FP32 walk launch shape: histories carried per lane (1, 2, 4 or 8) and threads
+ * per block (128 or 256).  Adjoint fixed-length histories use up to 2 per lane
+ * on records of at most 64 bytes and up to 4 on 32-byte records; forward
+ * histories and those ended by a weight cutoff walk one per lane (the latter
+ * in blocks of 256).  No counterpart in the reference. */
 int mclsgpu_domain_set_launch(mclsgpu_domain* dom, int histories_per_lane,
                               int block_size);
 /* Record loads of the FP32 walk allocated in L1 (1) or bypassing it (0, the
  * default).  No counterpart in the reference. */
 int mclsgpu_domain_set_record_cache(mclsgpu_domain* dom, int allocate_l1);
-/* Autotuner: times every launch shape on `reps` Monte Carlo solves of the
+/* Autotuner: times the domain's launch shapes on `reps` Monte Carlo solves of the
  * device vector rhs_dev (n entries), with the record loads bypassing and
  * allocated in L1, keeps the fastest walk and reports it.
  * The random stream position is restored afterwards.  No counterpart in the

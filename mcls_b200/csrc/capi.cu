@@ -52,6 +52,7 @@ int check_device_status(mclsgpu_context* ctx) {
 }
 
 void prepare_walk(mclsgpu_domain* dom);
+int prepare_walk_order(mclsgpu_domain* dom);
 int walk_agreement(mclsgpu_domain* dom, long long histories, uint64_t seed, long long* hist_diff,
                    long long* trans_diff);
 void prepare_source(mclsgpu_domain* dom);
@@ -152,6 +153,7 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->w);
     dfree(d->dt_h32);
     dfree(d->rec);
+    dfree(d->walk_order);
     dfree(d->d_jump);
     dfree(d->d_pos);
     dfree(d->hoff);
@@ -575,9 +577,10 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
     }
     if (!rc) {
         prepare_walk(dom);
+        rc = prepare_walk_order(dom);
         prepare_source(dom);
         e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "domain build");
+        if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "domain build");
     }
     if (rc) {
         release_domain(dom);

@@ -52,22 +52,25 @@ __global__ void k_domain_count(const int* rp, const int* ci, const double* v, in
 
 __global__ void k_domain_fill(const int* rp, const int* ci, const double* v, int n, int row0,
                               double relax, const int* drp, int* dcol, double* dh,
-                              double* dcdf, double* dw, int* status) {
+                              double* dcdf, double* dw, int* status, int* neg) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int o = drp[i];
         double c = 0.0;
+        bool neg_row = false;
         const int o0 = o;
         for (int k = rp[i]; k < rp[i + 1]; ++k) {
             double h = iteration_value(row0 + i, ci[k], v[k], relax);
             if (fabs(h) < DBL_EPSILON) continue;
             dcol[o] = ci[k];
             dh[o] = h;
+            neg_row |= !(h > 0.0);
             c = (o == o0) ? fabs(h) : __dadd_rn(fabs(h), c);  // :342-348
             dcdf[o] = c;
             ++o;
         }
         const double W = c;  // :353
         dw[i] = W;
+        if (neg_row) *neg = 1;
         if (!(W > 0.0) || !isfinite(W)) {
             atomicOr(status, DEV_ERR_DEGENERATE);
             continue;
@@ -202,6 +205,42 @@ int collect_offsets(mclsgpu_context* ctx, const DevCsr& D, int max_k, int* offse
     return MCLSGPU_OK;
 }
 
+// The grid behind a set of column offsets: the positive offsets fall into
+// clusters of consecutive integers; the first holds 1 (the x neighbours), the
+// second is centred on the line length X, and of the rest the middle one on
+// the plane X * Y.  Offsets that fit no such grid of n rows keep the identity.
+RowOrder row_order(int n, int K, const int* off, int rows) {
+    RowOrder o;
+    std::vector<long long> centre;
+    int first = 0;
+    for (int k = 0; k < K;) {
+        if (off[k] <= 0) {
+            ++k;
+            continue;
+        }
+        int e = k;
+        while (e + 1 < K && off[e + 1] == off[e] + 1) ++e;
+        if (centre.empty()) first = off[k];
+        centre.push_back(((long long)off[k] + off[e]) / 2);
+        k = e + 1;
+    }
+    if (centre.size() < 2 || first != 1) return o;
+    const long long X = centre[1];
+    const size_t rest = centre.size() - 2;
+    const long long plane = rest ? centre[2 + (rest - 1) / 2] : n;
+    if (X < 2 || plane % X || n % plane || plane / X < 2) return o;
+    o.X = unsigned(X);
+    o.Y = unsigned(plane / X);
+    o.Z = unsigned(n / plane);
+    // Four rows along x (one 32-byte sector of a vector), then as square as
+    // the row count allows.
+    o.bx = 4;
+    const unsigned lines = unsigned(rows) / 4;
+    o.bz = o.Z > 1 && lines >= 4 ? 2 : 1;
+    o.by = lines / o.bz;
+    return o;
+}
+
 // Build the FP64 domain arrays and FP32 records from the composite M.
 int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
                         mclsgpu_domain* dom, int row0) {
@@ -240,9 +279,14 @@ int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
     if ((e = dmalloc(&D.ci, tot + 1)) != cudaSuccess || (e = dmalloc(&D.v, tot + 1)) != cudaSuccess ||
         (e = dmalloc(&dom->cdf, tot + 1)) != cudaSuccess || (e = dmalloc(&dom->w, n + 1)) != cudaSuccess)
         return cuda_fail(ctx, e, "cudaMalloc");
+    int* d_neg = nullptr;
+    if ((e = dmalloc(&d_neg, 1)) != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
+    cudaMemsetAsync(d_neg, 0, sizeof(int), s);
     k_domain_fill<<<grid_for(n), 256, 0, s>>>(M.rp, M.ci, M.v, n, row0, relax, D.rp, D.ci, D.v,
-                                              dom->cdf, dom->w, ctx->d_status);
+                                              dom->cdf, dom->w, ctx->d_status, d_neg);
+    cudaMemcpyAsync(&dom->neg_h, d_neg, sizeof(int), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
+    dfree(d_neg);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "domain fill");
     if ((rc = check_device_status(ctx))) return rc;
 

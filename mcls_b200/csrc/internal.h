@@ -113,6 +113,38 @@ struct McsaState {
     int pad;
 };
 
+// Order in which the forward walk's threads take the rows of a domain on a
+// structured grid (X fastest, then Y, then Z): bricks of bx x by x bz rows, the
+// last ones narrower, x fastest inside a brick; bricks follow each other along
+// X, then Y, then Z.  A bijection of [0, n) for any X, Y, Z.  X = 1: none.
+struct RowOrder {
+    unsigned X = 1, Y = 1, Z = 1;
+    unsigned bx = 1, by = 1, bz = 1;
+};
+// The order for n rows whose columns sit at the K sorted offsets `off`, with
+// `rows` rows in a brick.
+RowOrder row_order(int n, int K, const int* off, int rows);
+
+// What a forward fixed-length FP32 walk does with a row's sum of `per`
+// histories: d = sum / per [+ source (expected value)], then out = d,
+// out + d, or xin + w rin + d.
+enum : int { kBaseNone = 0, kBaseOut = 1, kBaseSmoothed = 2 };
+struct RowFinish {
+    double* out = nullptr;
+    const double* src = nullptr;
+    const double* xin = nullptr;
+    const double* rin = nullptr;
+    double w = 0.0;
+    double omega = 0.0;
+    double inv_per = 1.0;
+    int has_omega = 0;
+    int per_pow2 = 0;
+    int ev = 0;
+    int base = kBaseNone;
+    int hlog = 0;               // log2 of the lanes that share a row
+    const int* order = nullptr; // position -> row (null: the identity)
+};
+
 }  // namespace mclsgpu
 
 struct mclsgpu_domain {
@@ -139,6 +171,11 @@ struct mclsgpu_domain {
     int walk_ilp = 1;
     int walk_block = 256;
     int walk_l1 = 0;               // record loads allocated in L1
+    // Forward fixed-length walks: log2 of the lanes that share a row, and the
+    // order the rows are taken in (null: ascending).
+    int walk_hlog = 0;
+    int* walk_order = nullptr;
+    int neg_h = 1;                 // some entry of H is negative
     // Stencil records (stencil_k > 0): row r's slot j is column r + stencil_off[j].
     int stencil_k = 0;
     int rec_q16 = 0;               // stencil records with 16-bit CDF thresholds
@@ -285,8 +322,8 @@ void anderson_drop_graph(mclsgpu_domain* dom);
 
 // FP32 forward walks: the tally source of v into the domain's records (H v
 // for the expected-value estimator, v for collision, with the Neumann
-// relaxation when has_omega) and the tallies y cleared.  row0: the global
-// index of the domain's first row (v is the whole vector, nv entries).
+// relaxation when has_omega) and the tallies y (may be null) cleared.  row0: the
+// global index of the domain's first row (v is the whole vector, nv entries).
 void launch_forward_records(mclsgpu_domain* dom, const double* v, int nv, double omega,
                             int has_omega, int row0, double* y);
 
@@ -337,6 +374,12 @@ void mc_correction(mclsgpu_domain* dom, const double* v, double* out);
 // Anderson loops run from the host instead of a captured graph.
 inline bool walk_needs_rounds(const mclsgpu_domain* dom) {
     return dom->p.rng_mode == MCLSGPU_RNG_REFERENCE && dom->p.weight_cutoff > 0.0;
+}
+// True when the walk kernel itself finishes the estimate (RowFinish): forward
+// fixed-length FP32 walks.  The others leave tallies in y64.
+inline bool walk_finishes(const mclsgpu_domain* dom) {
+    return dom->p.precision == MCLSGPU_FP32 && dom->p.direction == MCLSGPU_FORWARD &&
+           !(dom->p.weight_cutoff > 0.0);
 }
 // Walk statistics since the last reset (steps, histories, walk time).
 int mcsa_read_stats(mclsgpu_domain* dom, mclsgpu_stats* st);

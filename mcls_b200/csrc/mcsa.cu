@@ -23,6 +23,7 @@
 // CUDA graph: a WHILE conditional node whose body is one iteration and whose
 // condition is set on the device by the convergence check, so a solve makes
 // no host round trip per iteration.
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -38,8 +39,8 @@ void launch_forward_source(mclsgpu_domain* dom, const double* v, double omega, i
 void launch_forward_setup(mclsgpu_domain* dom);
 void launch_advance_walk_pos(mclsgpu_domain* dom);
 void prepare_walk(mclsgpu_domain* dom);
-void launch_walk(mclsgpu_domain* dom, long long max_trace, long long* tr_states, double* tr_w,
-                 int* tr_ev, long long* tr_start, bool fused);
+void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
+                 long long* tr_states, double* tr_w, int* tr_ev, long long* tr_start, bool fused);
 
 namespace {
 
@@ -152,9 +153,12 @@ struct FinalizeArgs {
     int n;
     int mode;            // 0 adjoint collision, 1 adjoint EV, 2 forward
     int ev;
-    int accumulate;      // 1: out += delta (MCSA), 0: out = delta
+    int base;            // kBase*: out = delta, out + delta, or xin + w rin + delta
     int fp32;
     double per;          // forward histories per state
+    const double* xin;
+    const double* rin;
+    double w;
     const double* sc;    // [2] = 1/nh
     const double* src;   // MC source vector before scaling
     double omega;
@@ -165,8 +169,6 @@ struct FinalizeArgs {
     const float* dth32;
     const double* dth64;
     double* out;
-    const int* d_nh;
-    unsigned long long* d_hist;
 };
 
 __global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
@@ -192,12 +194,33 @@ __global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
             d = __ddiv_rn(a.y64[i], a.per);
             if (a.ev) d = __dadd_rn(d, srci);
         }
-        a.out[i] = a.accumulate ? __dadd_rn(a.out[i], d) : d;
+        if (a.base == kBaseOut)
+            d = __dadd_rn(a.out[i], d);
+        else if (a.base == kBaseSmoothed)
+            d = __dadd_rn(__dadd_rn(a.xin[i], __dmul_rn(a.w, a.rin[i])), d);
+        a.out[i] = d;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.d_hist) *a.d_hist += (unsigned long long)(*a.d_nh);
 }
 
-__global__ void k_epoch_inc(unsigned long long* e) { *e += 1ULL; }
+// The duration of the last FP32 walk launch (first block start to last block
+// end) into t[2], the launch count in t[3].
+__device__ __forceinline__ void add_walk_time(unsigned long long* t) {
+    if (t[1] > t[0]) {
+        t[2] += t[1] - t[0];
+        t[3] += 1;
+    }
+    t[0] = ~0ULL;
+    t[1] = 0;
+}
+
+// End of a Monte Carlo solve: the stream epoch, the history count, the walk
+// timing.
+__global__ void k_mc_end(unsigned long long* epoch, unsigned long long* hist, const int* d_nh,
+                         unsigned long long* tim) {
+    *epoch += 1ULL;
+    *hist += (unsigned long long)(*d_nh);
+    add_walk_time(tim);
+}
 
 // Convergence check of one MCSA iteration (src/MCLS_MCSASolverManager_impl.hpp:380-394).
 __device__ __forceinline__ int mcsa_check(McsaState* st, const double* sumsq, double* hist,
@@ -250,18 +273,7 @@ struct ResidArgs {
     int n;
     const double* b;
     const double* dinv;       // null: no left preconditioner
-    const double* xin;        // x after smoothing
-    const double* rin;        // residual after smoothing (the MC source)
-    const double* y;          // tallies
-    const double* sc;         // [2] = 1/nh
-    double omega;
-    int has_omega;
-    double per;
-    double inv_per;
-    int per_pow2;
-    int ev;
-    int mode;                 // 0 adjoint collision, 1 forward, 2 x already corrected
-    double* xout;
+    const double* x;          // the corrected iterate
     double* rout;
     double* part;
     unsigned int* ticket;
@@ -277,28 +289,6 @@ struct ResidArgs {
     cudaGraphConditionalHandle handle;
     int use_cond;
 };
-
-// x + delta at state j: the MC correction of the estimator, rounded exactly
-// as the separate normalise-and-add kernel rounds it.
-__device__ __forceinline__ double corrected(const ResidArgs& a, int j, double inv) {
-    const double xj = a.xin[j];
-    if (a.mode == 0) return __dadd_rn(xj, __dmul_rn(a.y[j], inv));
-    if (a.mode == 1) {
-        // sum / count (ForwardTally::finalize); for a power-of-two count the
-        // product with its reciprocal is the same number and much cheaper.
-        double d = a.per_pow2 ? a.y[j] * a.inv_per : __ddiv_rn(a.y[j], a.per);
-        if (a.ev) d = __dadd_rn(d, a.has_omega ? a.rin[j] * a.omega : a.rin[j]);
-        return __dadd_rn(xj, d);
-    }
-    return xj;
-}
-
-// x = x2 + delta (the MC correction applied state by state).
-__global__ void __launch_bounds__(kFusedThreads) k_apply_correction(ResidArgs a) {
-    const double inv = a.sc[2];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x)
-        a.xout[i] = corrected(a, i, inv);
-}
 
 // rp = PL (b - A x), |rp|^2, then (last block) the MCSA convergence check,
 // the stream epoch, the walk timing, the work-queue reset and the loop
@@ -335,13 +325,7 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
         const int keep = mcsa_check(a.st, &sumsq, a.hist, a.hist_cap, a.status);
         *a.d_epoch += 1ULL;
         *a.d_hist += (unsigned long long)(*a.d_nh);
-        unsigned long long* tm = a.d_tim;
-        if (tm[1] > tm[0]) {
-            tm[2] += tm[1] - tm[0];
-            tm[3] += 1;
-        }
-        tm[0] = ~0ULL;
-        tm[1] = 0;
+        add_walk_time(a.d_tim);
         *a.d_counter = 0;
         if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
     }
@@ -349,7 +333,7 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
 
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_residual_norm(Op A, ResidArgs a) {
-    const double* x = a.xout;
+    const double* x = a.x;
     double acc = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         const double s = A.dot(i, [&](int j) { return x[j]; });
@@ -540,45 +524,63 @@ void composite_apply(mclsgpu_domain* dom, const double* x, double* y) {
 }
 
 // One MC solve of the source vector `v` (device, already left preconditioned
-// when required) into out (accumulate: out += delta).  `fused`: inside the
-// fused MCSA iteration the normalise-and-add of the collision and forward
-// estimators, the epoch increment and the walk bookkeeping are done by
-// k_update_residual; only the adjoint expected-value gather runs here.
-static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int accumulate,
+// when required) into out: out = delta, out + delta or x + w rp + delta
+// (`base`; w the smoother's relaxation).  Walks that finish their rows
+// themselves write out; the others' tallies are normalised and added by
+// k_finalize.  `fused`: inside the fused MCSA iteration the epoch increment
+// and the walk bookkeeping are done by k_residual_norm.
+static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int base, double w,
                        long long max_trace, long long* tr_states, double* tr_w, int* tr_ev,
                        long long* tr_start, bool fused = false) {
     const mclsgpu_mc_params& p = dom->p;
     const double omega = p.neumann_relaxation;
     const int has_omega = p.neumann_relaxation > 0.0;
+    const double per = p.sample_ratio > 0.0 ? std::ceil(p.sample_ratio) : 1.0;
+    const int ev = p.estimator == MCLSGPU_EXPECTED_VALUE;
+    RowFinish fin;
+    fin.out = out;
+    fin.src = v;
+    fin.xin = dom->x;
+    fin.rin = dom->rp;
+    fin.w = w;
+    fin.omega = omega;
+    fin.has_omega = has_omega;
+    int ex = 0;
+    fin.per_pow2 = std::frexp(per, &ex) == 0.5;  // per = 2^(ex-1)
+    fin.inv_per = 1.0 / per;
+    fin.ev = ev;
+    fin.base = base;
     if (p.direction == MCLSGPU_ADJOINT)
         launch_adjoint_source(dom, v, omega, has_omega);
     else
         launch_forward_source(dom, v, omega, has_omega, fused);
-    launch_walk(dom, max_trace, tr_states, tr_w, tr_ev, tr_start, fused);
+    launch_walk(dom, fin, max_trace, tr_states, tr_w, tr_ev, tr_start, fused);
     launch_advance_walk_pos(dom);
-    if (fused && !(p.direction == MCLSGPU_ADJOINT && p.estimator == MCLSGPU_EXPECTED_VALUE))
-        return;
-    FinalizeArgs f{};
-    f.n = dom->n;
-    f.mode = p.direction == MCLSGPU_FORWARD ? 2 : (p.estimator == MCLSGPU_EXPECTED_VALUE ? 1 : 0);
-    f.ev = p.estimator == MCLSGPU_EXPECTED_VALUE;
-    f.accumulate = accumulate;
-    f.fp32 = p.precision == MCLSGPU_FP32;
-    f.per = p.sample_ratio > 0.0 ? std::ceil(p.sample_ratio) : 1.0;
-    f.sc = dom->d_scalars;
-    f.src = v;
-    f.omega = omega;
-    f.has_omega = has_omega;
-    f.y64 = dom->y64;
-    f.dtrp = dom->DT.rp;
-    f.dtci = dom->DT.ci;
-    f.dth32 = dom->dt_h32;
-    f.dth64 = dom->DT.v;
-    f.out = out;
-    f.d_nh = dom->d_nh;
-    f.d_hist = fused ? nullptr : dom->d_hist;
-    k_finalize<<<grid_for(dom->n, 256, 148 * 8), 256, 0, dom->ctx->stream>>>(f);
-    if (!fused) k_epoch_inc<<<1, 1, 0, dom->ctx->stream>>>(dom->d_epoch);
+    cudaStream_t s = dom->ctx->stream;
+    if (!walk_finishes(dom)) {
+        FinalizeArgs f{};
+        f.n = dom->n;
+        f.mode = p.direction == MCLSGPU_FORWARD ? 2 : (ev ? 1 : 0);
+        f.ev = ev;
+        f.base = base;
+        f.xin = dom->x;
+        f.rin = dom->rp;
+        f.w = w;
+        f.fp32 = p.precision == MCLSGPU_FP32;
+        f.per = per;
+        f.sc = dom->d_scalars;
+        f.src = v;
+        f.omega = omega;
+        f.has_omega = has_omega;
+        f.y64 = dom->y64;
+        f.dtrp = dom->DT.rp;
+        f.dtci = dom->DT.ci;
+        f.dth32 = dom->dt_h32;
+        f.dth64 = dom->DT.v;
+        f.out = out;
+        k_finalize<<<grid_for(dom->n, 256, 148 * 8), 256, 0, s>>>(f);
+    }
+    if (!fused) k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_hist, dom->d_nh, dom->d_tim);
 }
 
 static int read_stats(mclsgpu_domain* dom, mclsgpu_stats* st) {
@@ -622,10 +624,10 @@ static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x
     cudaEventRecord(e0, s);
     if (dom->right && !internal) {
         // v is rhs_dev or tmp, so tmp2 is free for the unrecovered result.
-        enqueue_mc(dom, v, dom->tmp2, 0, max_trace, tr_states, tr_w, tr_ev, tr_start);
+        enqueue_mc(dom, v, dom->tmp2, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start);
         spmv(s, dom->right->P, dom->tmp2, x_dev);
     } else {
-        enqueue_mc(dom, v, x_dev, 0, max_trace, tr_states, tr_w, tr_ev, tr_start);
+        enqueue_mc(dom, v, x_dev, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start);
     }
     cudaEventRecord(e1, s);
     cudaError_t e = cudaStreamSynchronize(s);
@@ -655,7 +657,7 @@ int mcsa_read_stats(mclsgpu_domain* dom, mclsgpu_stats* st) { return read_stats(
 void mcsa_reset_counters(mclsgpu_domain* dom) { reset_counters(dom); }
 
 void mc_correction(mclsgpu_domain* dom, const double* v, double* out) {
-    enqueue_mc(dom, v, out, 0, 0, nullptr, nullptr, nullptr, nullptr);
+    enqueue_mc(dom, v, out, kBaseNone, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
 }
 
 // The fused iteration covers one smoothing step, no right preconditioner and
@@ -667,8 +669,8 @@ static bool fused_iteration(const mclsgpu_domain* dom, const mclsgpu_mcsa_params
             (dom->left->mdia && dom->op->dia_k > 0));
 }
 
-// At most 8 blocks per SM: the per-block partial sums of k_apply_correction
-// and k_residual_norm go to dom->part, sized for that many blocks.
+// At most 8 blocks per SM: the per-block partial sums of k_residual_norm go to
+// dom->part, sized for that many blocks.
 static int fused_grid(const mclsgpu_domain* dom) {
     return grid_for(dom->n, kFusedThreads, dom->ctx->num_sms * 8);
 }
@@ -704,7 +706,7 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     if (!fused_iteration(dom, mp)) {
         for (int l = 0; l < mp->smoother_steps; ++l)
             enqueue_fixed_point_step(dom, mp->fixed_point_type, mp->richardson_omega);
-        enqueue_mc(dom, dom->rp, dom->x, 1, 0, nullptr, nullptr, nullptr, nullptr);
+        enqueue_mc(dom, dom->rp, dom->x, kBaseOut, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
         update_prec_residual(dom, dom->x, dom->b, dom->rp);
         sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
         if (use_cond)
@@ -729,28 +731,15 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dom->b, dinv, dom->x,
                           dom->rp, mp->richardson_omega, dom->x2, dom->rp2);
     }
-    const mclsgpu_mc_params& p = dom->p;
-    const bool adj_ev = p.direction == MCLSGPU_ADJOINT && p.estimator == MCLSGPU_EXPECTED_VALUE;
-    enqueue_mc(dom, dom->rp2, dom->x2, 1, 0, nullptr, nullptr, nullptr, nullptr, true);
+    // x = x + w rp + delta: the smoothing step's iterate is formed where the
+    // correction is added.
+    enqueue_mc(dom, dom->rp2, dom->x, kBaseSmoothed, mp->richardson_omega, 0, nullptr, nullptr,
+               nullptr, nullptr, true);
     ResidArgs a{};
     a.n = n;
     a.b = dom->b;
     a.dinv = dinv;
-    a.xin = dom->x2;
-    a.rin = dom->rp2;
-    a.y = dom->y64;
-    a.sc = dom->d_scalars;
-    a.omega = p.neumann_relaxation;
-    a.has_omega = p.neumann_relaxation > 0.0;
-    a.per = p.sample_ratio > 0.0 ? std::ceil(p.sample_ratio) : 1.0;
-    {
-        int ex = 0;
-        a.per_pow2 = std::frexp(a.per, &ex) == 0.5;  // per = 2^(ex-1)
-        a.inv_per = 1.0 / a.per;
-    }
-    a.ev = p.estimator == MCLSGPU_EXPECTED_VALUE;
-    a.mode = p.direction == MCLSGPU_FORWARD ? 1 : (adj_ev ? 2 : 0);
-    a.xout = dom->x;
+    a.x = dom->x;
     a.rout = dom->rp;
     a.part = dom->part;
     a.ticket = dom->d_ticket;
@@ -765,7 +754,6 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     a.d_nh = dom->d_nh;
     a.handle = handle;
     a.use_cond = use_cond;
-    k_apply_correction<<<grid, kFusedThreads, 0, s>>>(a);
     if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x, dom->b, nullptr,
                           dom->tmp);
@@ -1208,7 +1196,7 @@ int mclsgpu_mcsa_correction(mclsgpu_domain* dom, double* delta_dev) {
     for (int l = 0; l < p.smoother_steps; ++l)
         enqueue_fixed_point_step(dom, p.fixed_point_type, p.richardson_omega);
     // The residual problem's source is already left preconditioned.
-    enqueue_mc(dom, dom->rp, delta_dev, 0, 0, nullptr, nullptr, nullptr, nullptr);
+    enqueue_mc(dom, dom->rp, delta_dev, kBaseNone, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa correction");
     return check_device_status(ctx);
@@ -1299,18 +1287,22 @@ int mclsgpu_domain_autotune(mclsgpu_domain* dom, const double* rhs_dev, int reps
     cudaMemcpyAsync(&saved[1], dom->d_pos, sizeof(saved[1]), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "autotune");
-    // Four or eight histories per lane apply to fixed-length histories on
-    // 32-byte records only.
-    const bool four = dom->slots == 4 && !(dom->p.weight_cutoff > 0.0);
-    // Each shape with the record loads bypassing L1 and allocated in it.
-    const int shapes[16][3] = {{1, 256, 0}, {2, 256, 0}, {1, 128, 0}, {2, 128, 0},
-                               {4, 256, 0}, {4, 128, 0}, {8, 256, 0}, {8, 128, 0},
-                               {1, 256, 1}, {2, 256, 1}, {1, 128, 1}, {2, 128, 1},
-                               {4, 256, 1}, {4, 128, 1}, {8, 256, 1}, {8, 128, 1}};
+    // The shapes that differ for this domain: forward fixed-length histories
+    // walk one per lane, those ended by a cutoff have one shape, and four per
+    // lane apply to 32-byte records only.  Each with the record loads
+    // bypassing L1 and allocated in it.
+    const bool fixed = !(dom->p.weight_cutoff > 0.0);
+    const bool adjoint = dom->p.direction == MCLSGPU_ADJOINT;
+    const int most = !fixed || !adjoint ? 1 : dom->slots == 4 ? 4 : dom->slots == 8 ? 2 : 1;
+    std::vector<std::array<int, 3>> shapes;
+    for (int l1 = 0; l1 < (fixed ? 2 : 1); ++l1)
+        for (int h = 1; h <= most; h *= 2) {
+            shapes.push_back({h, 256, l1});
+            if (fixed) shapes.push_back({h, 128, l1});
+        }
     double best = 1e300;
     int bh = 1, bb = 256, bl = 0;
     for (const auto& sh : shapes) {
-        if (sh[0] >= 4 && !four) continue;
         int rc = mclsgpu_domain_set_launch(dom, sh[0], sh[1]);
         if (!rc) rc = mclsgpu_domain_set_record_cache(dom, sh[2]);
         if (rc) return rc;

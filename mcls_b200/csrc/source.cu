@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) k_forward_rec(const double* v, int n, int
                 c = fma(h[o + 32 * k], load_src(v, col[o + 32 * k], omega, has), c);
         }
         rec[size_t(i) * slots].y = __float_as_uint(__double2float_rn(c));
-        y[i] = 0.0;
+        if (y) y[i] = 0.0;
     }
 }
 
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) k_forward_rec_stencil(const double* v, in
             rec_stencil16_source<WORDS>(r, g, nv, v, omega, has, K, so);
         else
             rec_stencil_source<WORDS>(r, g, nv, v, omega, has, K, so);
-        y[i] = 0.0;
+        if (y) y[i] = 0.0;
     }
 }
 
@@ -654,7 +654,9 @@ void launch_forward_source(mclsgpu_domain* dom, const double* v, double omega, i
     const int ev = p.estimator == MCLSGPU_EXPECTED_VALUE;
     if (!fused) k_forward_nh<<<1, 1, 0, s>>>(dom->d_nh, n * per, dom->d_scalars);
     if (p.precision == MCLSGPU_FP32) {
-        launch_forward_records(dom, v, n, omega, has_omega, 0, dom->y64);
+        // Walks that finish their rows themselves read no tallies.
+        launch_forward_records(dom, v, n, omega, has_omega, 0,
+                               walk_finishes(dom) ? nullptr : dom->y64);
     } else {
         k_forward_c<double><<<grid_for(n), 256, 0, s>>>(v, n, omega, has_omega, ev, dom->D.rp,
                                                         dom->D.ci, dom->D.v, dom->c64);

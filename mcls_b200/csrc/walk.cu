@@ -8,16 +8,16 @@
 // termination once the history has taken "History Length" steps
 // (:135-136) or, with the legacy "Weight Cutoff", once |w| < cutoff * |w0|.
 //
-// walk32: the production kernel.  Persistent warps pull histories from a
-// work-queue counter and refill lanes as histories terminate.  A step reads
-// one packed FP32 record (slots * 8 bytes, 16-byte vector loads), selects the
-// first entry whose CDF value is >= u with predicated compares (the records'
-// padding entries hold 2.0 and are never selected) and carries the weight in
-// FP32.  Tallies reduce into FP64: the adjoint collision tally with a
-// fire-and-forget FP64 reduction per step, the forward history sum
-// Kahan-compensated in FP32 and reduced into FP64 once per history.  The
-// adjoint step-0 tally is made by the source build (counts * w0), so walks
-// tally from step 1.
+// walk32_*: the production kernels.  A step reads one packed FP32 record
+// (slots * 8 bytes, 32-byte vector loads), selects the first entry whose CDF
+// value is >= u with predicated compares (the records' padding entries hold
+// 2.0 and are never selected) and carries the weight in FP32; tallies reduce
+// into FP64.  Forward histories of fixed length (walk32_rows) keep a Kahan-
+// compensated FP32 sum each and the lanes of a row finish its estimate;
+// adjoint histories (walk32_adjoint) tally with a fire-and-forget FP64
+// reduction per step, the step-0 tally being made by the source build (counts
+// * w0), so walks tally from step 1; histories ended by a weight cutoff
+// (walk32_cutoff) are pulled from a work queue.
 //
 // walk64: the parity kernel.  FP64 CSR domain, binary search with
 // std::lower_bound semantics, FP64 weights and tallies, optional trajectory
@@ -60,7 +60,6 @@ struct WalkArgs {
     unsigned long long* d_steps;
     unsigned long long* d_tim;  // [0] first warp start, [1] last warp end (ns)
     int* status;
-    int row0;                   // global index of the first record / tally row
     int l1;                     // record loads allocate in L1
     int stoff[32];              // stencil records: column offset of each slot
     // variable-length histories on the reference stream (FP64 only): history
@@ -137,52 +136,51 @@ constexpr int kPacked = 0, kStencil = 1, kStencil16 = 2;
 // x: the first entry whose CDF value is >= u (sampleDiscreteCDF's
 // lower_bound) with u the draw's 24-bit uniform, or for stencil16 the first
 // slot with u16 < t_j, u16 = min(top 16 bits, 65534).  s becomes the selected
-// column; neg is the sign bit of the selected h.
-template <int S, int ST>
-__device__ __forceinline__ void select32(const WalkArgs& a, const uint32_t* q, uint64_t x, int& s,
+// column; neg is the sign bit of the selected h.  The slots are scanned from
+// the last to the first, each match overwriting the one before, so a slot
+// costs a compare and a predicated move and no "found" flag.  POS: the domain
+// has no negative h, so the sign is not read.  soff: the column offsets of the
+// stencil slots in shared memory, soff[kNoSlot] = 0 (no slot matched: a NaN
+// record, reported by the residual check).
+constexpr int kNoSlot = 31;
+template <int S, int ST, bool POS = false>
+__device__ __forceinline__ void select32(const int* soff, const uint32_t* q, uint64_t x, int& s,
                                          unsigned& neg) {
     if constexpr (ST == kPacked) {
         const float u = canonical32(x);
-        unsigned sel = q[3];  // slot 1 (first entry)
-        bool found = __uint_as_float(q[2]) >= u;
+        unsigned sel = 0u;
 #pragma unroll
-        for (int t = 2; t < S; ++t) {
-            const bool c = !found && __uint_as_float(q[2 * t]) >= u;
-            sel = c ? q[2 * t + 1] : sel;
-            found = found || c;
-        }
+        for (int t = S - 1; t >= 1; --t)
+            if (__uint_as_float(q[2 * t]) >= u) sel = q[2 * t + 1];
         neg = sel & 0x80000000u;
         s = int(sel & 0x7fffffffu);
     } else if constexpr (ST == kStencil) {
         // Stencil slots: first |cdf_j| >= u (NaN slots never match); the next
         // state is s + offset_j, the sign of h_j is the sign bit of the slot.
         const float u = canonical32(x);
-        int dsel = 0;
+        int jsel = kNoSlot;
         unsigned ng = 0u;
-        bool found = false;
 #pragma unroll
-        for (int j = 0; j < 2 * S - 2; ++j) {
-            const bool c = !found && fabsf(__uint_as_float(q[2 + j])) >= u;
-            dsel = c ? a.stoff[j] : dsel;
-            ng = c ? (q[2 + j] & 0x80000000u) : ng;
-            found = found || c;
-        }
-        neg = ng;
-        s += dsel;
+        for (int j = 2 * S - 3; j >= 0; --j)
+            if (fabsf(__uint_as_float(q[2 + j])) >= u) {
+                jsel = j;
+                if constexpr (!POS) ng = q[2 + j];
+            }
+        neg = ng & 0x80000000u;
+        s += soff[jsel];
     } else {
+        // A slot's threshold is compared inside its word: the high half
+        // against (u16 << 16 | 0xffff), the low half after a shift.
         const unsigned u16 = min(unsigned(x >> 48), 65534u);
-        int dsel = 0, jsel = 0;
-        bool found = false;
+        const unsigned top = (u16 << 16) | 0xffffu;
+        int jsel = kNoSlot;
 #pragma unroll
-        for (int j = 0; j < 2 * (2 * S - 3); ++j) {
-            const unsigned t = (q[3 + j / 2] >> (16 * (j & 1))) & 0xffffu;
-            const bool c = !found && u16 < t;
-            dsel = c ? a.stoff[j] : dsel;
-            jsel = c ? j : jsel;
-            found = found || c;
+        for (int j = 2 * (2 * S - 3) - 1; j >= 0; --j) {
+            const unsigned word = q[3 + j / 2];
+            if ((j & 1) ? word > top : (word << 16) > top) jsel = j;
         }
-        neg = ((q[2] >> jsel) & 1u) << 31;
-        s += dsel;
+        neg = POS ? 0u : ((q[2] >> jsel) & 1u) << 31;
+        s += soff[jsel];
     }
 }
 
@@ -204,23 +202,22 @@ __device__ __forceinline__ int select64(const WalkArgs& a, int s, double u, int&
 // loop body): tally at the pre-transition state, read the state's record,
 // draw u, select the first entry whose CDF value is >= u, update the state
 // and the weight.
-template <int S, int DIR, int ST>
-__device__ __forceinline__ void walk_step(const WalkArgs& a, const char* rec, int& s, float& w,
-                                          uint64_t& x, float& acc, float& comp, int k) {
-    // One record: S/4 256-bit loads, bypassing L1 (each step touches exactly
-    // the record's own sectors) or allocated in it (the launch shape says).
-    const char* r = rec + size_t(s - a.row0) * (S * 8);
+//
+// L1: the record loads allocate in L1 or bypass it.
+template <int S, int DIR, int ST, bool L1, bool POS = false>
+__device__ __forceinline__ void walk_step(const char* rec, double* y, const int* soff, int& s,
+                                          float& w, uint64_t& x, float& acc, float& comp, int k) {
+    // One record: S/4 256-bit loads.  rec and y point at global row 0.
+    const char* r = rec + size_t(unsigned(s)) * (S * 8);
     uint32_t q[2 * S];
-    if (a.l1) {
 #pragma unroll
-        for (int t = 0; t < S / 4; ++t) ld_record256_l1(r + 32 * t, q + 8 * t);
-    } else {
-#pragma unroll
-        for (int t = 0; t < S / 4; ++t) ld_record256(r + 32 * t, q + 8 * t);
+    for (int t = 0; t < S / 4; ++t) {
+        if constexpr (L1) ld_record256_l1(r + 32 * t, q + 8 * t);
+        else ld_record256(r + 32 * t, q + 8 * t);
     }
     if (DIR == MCLSGPU_ADJOINT) {
         // FP32 weight, FP64 reduction (fire-and-forget RED.ADD.F64).
-        if (k > 0) atomicAdd(&a.y64[s - a.row0], double(w));
+        if (k > 0) atomicAdd(&y[s], double(w));
     } else {
         // Kahan-compensated FP32 history sum; the tally source of the state
         // rides in the record header (slot 0, second word).
@@ -232,8 +229,8 @@ __device__ __forceinline__ void walk_step(const WalkArgs& a, const char* rec, in
     x = xs_step(x);
     const float Wt = __uint_as_float(q[0]);
     unsigned neg;
-    select32<S, ST>(a, q, x, s, neg);
-    w = neg ? -(w * Wt) : w * Wt;
+    select32<S, ST, POS>(soff, q, x, s, neg);
+    w = __uint_as_float(__float_as_uint(w * Wt) ^ neg);
 }
 
 // Starting state, weight and stream of history e.
@@ -251,126 +248,218 @@ __device__ __forceinline__ void walk_start(const WalkArgs& a, int e, uint64_t ek
     x = history_state(a, ekey, e);
 }
 
-// FIXED: every history takes exactly History Length steps (no weight
-// cutoff), so the lanes of a warp start and finish their histories together:
-// the warp takes 32 histories at a time and runs them without per-step
-// termination checks.  Otherwise lanes refill one by one from the queue as
-// their histories terminate.
-template <int S, int DIR, int ST, bool FIXED, int ILP = 1>
-__global__ void __launch_bounds__(256, ILP == 1   ? WalkOccupancy<S>::kMinBlocks
-                                      : ILP == 2 ? 5
-                                      : ILP == 4 ? 4
-                                                 : 3)
-    walk32(WalkArgs a) {
+// The column offsets of the record's slots in shared memory.
+__device__ __forceinline__ void stage_offsets(const int* stoff, int* soff) {
+    if (threadIdx.x < 32) soff[threadIdx.x] = threadIdx.x < kNoSlot ? stoff[threadIdx.x] : 0;
+}
+
+// First block start and last block end of a walk launch (d_tim): one atomic
+// each per block, not per warp, because they all meet at the same address.
+__device__ __forceinline__ void walk_begin_time(const WalkArgs& a) {
+    if (threadIdx.x == 0) atomicMin(&a.d_tim[0], global_ns());
+}
+__device__ __forceinline__ void walk_end_time(const WalkArgs& a) {
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(&a.d_tim[1], global_ns());
+}
+
+// What bounds it: 8,850 warp steps per SM for 41.9M steps (128^3, two
+// histories per row), and the loads' L1TEX cycles -- a warp's 32 records lie in
+// up to 32 different lines, one request to L2 each.  So the lanes of a warp
+// start in a brick of neighbouring rows (RowOrder) and the two histories of a
+// row sit in the same warp, which keeps them in fewer lines for longer: 26.8
+// lines per request for 32 rows along x, 20.3 for 4 x 2 x 2 rows with two
+// histories each, and 124 against 114 us for the launch.  Loads that allocate
+// in L1 hit 80 % of the time and are slower (139 us): their data-stage
+// wavefronts then bind.  Further histories per lane add no speed (137 us with
+// one, 145 with two and four before the bricks): 64 resident warps already
+// cover the latency.  With the work queue, the per-warp timing atomics and
+// the tallies in memory the launch took 145 us at its tuned shape (213 us at
+// the default one), and 15 us instead of 4.8 for a 20^3 grid.
+//
+// Forward histories of fixed length, one per thread at a time.  2^f.hlog
+// neighbouring lanes share a row and split its `per` histories; they add
+// their sums with shuffles and the first of them finishes the row's estimate,
+// out = [base +] sum / per [+ source], so a row's sum needs no atomics, no
+// cleared tally and no pass of its own.  The histories are assigned
+// statically: they all take the same number of steps, and a work queue costs
+// one contended atomic per warp.
+template <int S, int ST, bool POS, bool L1>
+__device__ __forceinline__ double row_histories(const WalkArgs& a, const RowFinish& f,
+                                                const int* soff, uint64_t ekey, int row) {
+    const char* rec = reinterpret_cast<const char*>(a.rec);
+    const int L = a.L, H = 1 << f.hlog;
+    double sum = 0.0;
+    for (int m = threadIdx.x & (H - 1); m < a.per; m += H) {
+        int s = row;
+        float w = 1.f, acc = 0.f, comp = 0.f;
+        uint64_t x = history_state(a, ekey, (long long)row * a.per + m);
+        for (int k = 0; k < L; ++k)
+            walk_step<S, MCLSGPU_FORWARD, ST, L1, POS>(rec, nullptr, soff, s, w, x, acc, comp, k);
+        sum += double(acc) - double(comp);
+    }
+    return sum;
+}
+
+template <int S, int ST, bool POS>
+__global__ void __launch_bounds__(256, WalkOccupancy<S>::kMinBlocks)
+    walk32_rows(WalkArgs a, RowFinish f) {
     static_assert(S % 4 == 0, "records are whole 32-byte halves");
+    __shared__ uint64_t s_ekey;
+    __shared__ int s_off[32];
+    stage_offsets(a.stoff, s_off);
+    if (threadIdx.x == 0) s_ekey = epoch_key(a.seed, *a.d_epoch);
+    walk_begin_time(a);
+    __syncthreads();
+    const unsigned pos = (blockIdx.x * blockDim.x + threadIdx.x) >> f.hlog;
+    // A position past the end walks the last row's histories and drops the
+    // result, so every lane takes part in the shuffles.
+    const bool live = pos < unsigned(a.n);
+    const unsigned p = live ? pos : unsigned(a.n) - 1u;
+    const int i = f.order ? f.order[p] : int(p);
+    double sum = a.l1 ? row_histories<S, ST, POS, true>(a, f, s_off, s_ekey, i)
+                      : row_histories<S, ST, POS, false>(a, f, s_off, s_ekey, i);
+    for (int d = 1; d < (1 << f.hlog); d <<= 1) sum += __shfl_xor_sync(kFull, sum, d);
+    if (live && (threadIdx.x & ((1 << f.hlog) - 1)) == 0) {
+        // sum / count (ForwardTally::finalize, src/MCLS_ForwardTally_impl.hpp:
+        // 194-208); for a power-of-two count the product with its reciprocal
+        // is the same number.
+        double d = f.per_pow2 ? sum * f.inv_per : __ddiv_rn(sum, double(a.per));
+        if (f.ev) d = __dadd_rn(d, f.has_omega ? f.src[i] * f.omega : f.src[i]);
+        if (f.base == kBaseOut)
+            d = __dadd_rn(f.out[i], d);
+        else if (f.base == kBaseSmoothed)
+            d = __dadd_rn(__dadd_rn(f.xin[i], __dmul_rn(f.w, f.rin[i])), d);
+        f.out[i] = d;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(a.d_steps, (unsigned long long)(a.n) * a.per * a.L);
+    walk_end_time(a);
+}
+
+// Adjoint histories of fixed length, ILP per lane, assigned statically (see
+// walk32_rows); they tally where they stand.
+template <int S, int ST, bool POS, bool L1, int ILP>
+__device__ __forceinline__ void adjoint_histories(const WalkArgs& a, const int* soff,
+                                                  uint64_t ekey, float wnorm, long long e0,
+                                                  int nh) {
+    const char* rec = reinterpret_cast<const char*>(a.rec);
+    const int L = a.L;
+    int s[ILP];
+    float w[ILP];
+    uint64_t x[ILP];
+#pragma unroll
+    for (int m = 0; m < ILP; ++m) {
+        const long long e = e0 + (long long)m * blockDim.x;
+        s[m] = 0;
+        w[m] = 0.f;
+        x[m] = 0;
+        if (e < nh) walk_start<MCLSGPU_ADJOINT>(a, int(e), ekey, wnorm, s[m], w[m], x[m]);
+    }
+    for (int k = 0; k < L; ++k) {
+#pragma unroll
+        for (int m = 0; m < ILP; ++m) {
+            float acc = 0.f, comp = 0.f;
+            if (e0 + (long long)m * blockDim.x < nh)
+                walk_step<S, MCLSGPU_ADJOINT, ST, L1, POS>(rec, a.y64, soff, s[m], w[m], x[m],
+                                                           acc, comp, k);
+        }
+    }
+}
+
+template <int S, int ST, bool POS, int ILP>
+__global__ void __launch_bounds__(256, ILP == 1 ? WalkOccupancy<S>::kMinBlocks
+                                       : ILP == 2 ? 5
+                                                  : 4)
+    walk32_adjoint(WalkArgs a) {
     __shared__ uint64_t s_ekey;
     __shared__ int s_nh;
     __shared__ float s_wnorm;
-    const int lane = threadIdx.x & 31;
+    __shared__ int s_off[32];
+    stage_offsets(a.stoff, s_off);
     if (threadIdx.x == 0) {
         s_ekey = epoch_key(a.seed, *a.d_epoch);
         s_nh = *a.d_nh;
         s_wnorm = float(a.sc[0]);
     }
+    walk_begin_time(a);
+    __syncthreads();
+    // The launch has a thread for every history the domain was sized for.
+    const long long e0 = (long long)blockIdx.x * (blockDim.x * ILP) + threadIdx.x;
+    if (e0 < s_nh) {
+        if (a.l1)
+            adjoint_histories<S, ST, POS, true, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh);
+        else
+            adjoint_histories<S, ST, POS, false, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(a.d_steps, (unsigned long long)s_nh * a.L);
+    walk_end_time(a);
+}
+
+// Histories ended by the weight cutoff: persistent warps whose lanes refill
+// one by one from the work queue as their histories terminate.
+template <int S, int DIR, int ST>
+__global__ void __launch_bounds__(256, WalkOccupancy<S>::kMinBlocks) walk32_cutoff(WalkArgs a) {
+    static_assert(S % 4 == 0, "records are whole 32-byte halves");
+    __shared__ uint64_t s_ekey;
+    __shared__ int s_nh;
+    __shared__ float s_wnorm;
+    __shared__ int s_off[32];
+    const int lane = threadIdx.x & 31;
+    stage_offsets(a.stoff, s_off);
+    if (threadIdx.x == 0) {
+        s_ekey = epoch_key(a.seed, *a.d_epoch);
+        s_nh = *a.d_nh;
+        s_wnorm = float(a.sc[0]);
+    }
+    walk_begin_time(a);
     __syncthreads();
     const char* rec = reinterpret_cast<const char*>(a.rec);
-    if (lane == 0) atomicMin(&a.d_tim[0], global_ns());
     unsigned steps = 0;
-    if constexpr (FIXED) {
-        // ILP histories per lane, interleaved step by step so that each lane
-        // has ILP independent record loads in flight.
-        const int L = a.L;
-        while (true) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(a.d_counter, 32 * ILP);
-            base = __shfl_sync(kFull, base, 0);
+    int s = 0, s0 = 0, k = 0;
+    float w = 0.f, wcut = 0.f, acc = 0.f, comp = 0.f;
+    uint64_t x = 0;
+    bool alive = false, drained = false;
+    while (true) {
+        const unsigned need = __ballot_sync(kFull, !alive);
+        if (need && !drained) {
+            const int leader = __ffs(need) - 1;
+            const int cnt = __popc(need);
             const int nh = s_nh;
-            if (base >= nh) break;
-            int s[ILP], s0[ILP];
-            float w[ILP], acc[ILP], comp[ILP];
-            uint64_t x[ILP];
-            bool alive[ILP];
-#pragma unroll
-            for (int m = 0; m < ILP; ++m) {
-                const int e = base + lane + 32 * m;
-                alive[m] = e < nh;
-                s[m] = 0;
-                w[m] = acc[m] = comp[m] = 0.f;
-                x[m] = 0;
-                if (alive[m]) walk_start<DIR>(a, e, s_ekey, s_wnorm, s[m], w[m], x[m]);
-                s0[m] = s[m];
-            }
-            for (int k = 0; k < L; ++k) {
-#pragma unroll
-                for (int m = 0; m < ILP; ++m)
-                    if (alive[m]) walk_step<S, DIR, ST>(a, rec, s[m], w[m], x[m], acc[m], comp[m], k);
-            }
-#pragma unroll
-            for (int m = 0; m < ILP; ++m) {
-                if (alive[m]) {
-                    steps += L;
-                    if (DIR == MCLSGPU_FORWARD)
-                        atomicAdd(&a.y64[s0[m]], double(acc[m]) - double(comp[m]));
+            int base = 0;
+            if (lane == leader) base = atomicAdd(a.d_counter, cnt);
+            base = __shfl_sync(kFull, base, leader);
+            if (base + cnt >= nh) drained = true;
+            if (!alive) {
+                const int e = base + __popc(need & ((1u << lane) - 1));
+                if (e < nh) {
+                    walk_start<DIR>(a, e, s_ekey, s_wnorm, s, w, x);
+                    acc = 0.f;
+                    comp = 0.f;
+                    s0 = s;
+                    wcut = a.cutoff * fabsf(w);
+                    k = 0;
+                    alive = true;
                 }
             }
         }
-    } else {
-        int s = 0, s0 = 0, k = 0;
-        float w = 0.f, wcut = 0.f, acc = 0.f, comp = 0.f;
-        uint64_t x = 0;
-        bool alive = false, drained = false;
-        while (true) {
-            const unsigned need = __ballot_sync(kFull, !alive);
-            if (need && !drained) {
-                const int leader = __ffs(need) - 1;
-                const int cnt = __popc(need);
-                const int nh = s_nh;
-                int base = 0;
-                if (lane == leader) base = atomicAdd(a.d_counter, cnt);
-                base = __shfl_sync(kFull, base, leader);
-                if (base + cnt >= nh) drained = true;
-                if (!alive) {
-                    const int e = base + __popc(need & ((1u << lane) - 1));
-                    if (e < nh) {
-                        walk_start<DIR>(a, e, s_ekey, s_wnorm, s, w, x);
-                        acc = 0.f;
-                        comp = 0.f;
-                        s0 = s;
-                        wcut = a.cutoff * fabsf(w);
-                        k = 0;
-                        alive = true;
-                    }
-                }
-            }
-            if (!__any_sync(kFull, alive)) break;
-            if (alive) {
-                walk_step<S, DIR, ST>(a, rec, s, w, x, acc, comp, k);
-                ++k;
-                ++steps;
-                if (k >= a.L || fabsf(w) < wcut) {
-                    alive = false;
-                    if (DIR == MCLSGPU_FORWARD)
-                        atomicAdd(&a.y64[s0], double(acc) - double(comp));
-                }
+        if (!__any_sync(kFull, alive)) break;
+        if (alive) {
+            walk_step<S, DIR, ST, false>(rec, a.y64, s_off, s, w, x, acc, comp, k);
+            ++k;
+            ++steps;
+            if (k >= a.L || fabsf(w) < wcut) {
+                alive = false;
+                if (DIR == MCLSGPU_FORWARD) atomicAdd(&a.y64[s0], double(acc) - double(comp));
             }
         }
     }
     // Step count: one reduction per warp.
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) steps += __shfl_down_sync(kFull, steps, d);
-    if (lane == 0) {
-        if (steps) atomicAdd(a.d_steps, (unsigned long long)steps);
-        atomicMax(&a.d_tim[1], global_ns());
-    }
-}
-
-// Device-side duration of the last walk launch (first warp start to last warp
-// end), accumulated into d_tim[2] with the launch count in d_tim[3].
-__global__ void k_walk_time_acc(unsigned long long* t) {
-    if (t[1] > t[0]) t[2] += t[1] - t[0];
-    t[3] += 1;
-    t[0] = ~0ULL;
-    t[1] = 0;
+    if (lane == 0 && steps) atomicAdd(a.d_steps, (unsigned long long)steps);
+    walk_end_time(a);
 }
 
 template <int DIR>
@@ -440,103 +529,154 @@ __global__ void __launch_bounds__(128) walk64(WalkArgs a) {
     if ((threadIdx.x & 31) == 0 && steps) atomicAdd(a.d_steps, steps);
 }
 
-template <int S, int DIR, int ST, bool FX, int ILP>
-int blocks_per_sm(int block) {
-    static int cached[5] = {0, 0, 0, 0, 0};  // block sizes 128..1024 by log2
-    const int slot = block <= 128 ? 0 : block <= 256 ? 1 : block <= 512 ? 2 : 3;
-    if (!cached[slot]) {
+// Resident 256-thread blocks per SM of a cutoff walk (a persistent grid).
+template <int S, int DIR, int ST>
+int cutoff_blocks_per_sm() {
+    static int cached = 0;
+    if (!cached) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32<S, DIR, ST, FX, ILP>, block, 0);
-        cached[slot] = b > 0 ? b : 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32_cutoff<S, DIR, ST>, 256, 0);
+        cached = b > 0 ? b : 1;
     }
-    return cached[slot];
+    return cached;
 }
 
-// Dispatch on the record stride; `launch` false only caches the occupancy.
-// Persistent grid: as many blocks as fit on every SM at once.
-template <int DIR, int ST, bool FX, int ILP>
-void launch32_slots(int slots, const WalkArgs& a, int sms, int block, cudaStream_t st,
-                    bool launch) {
-#define MCLSGPU_WALK_CASE(SL)                                                             \
-    case SL:                                                                              \
-        if (launch)                                                                       \
-            walk32<SL, DIR, ST, FX, ILP>                                                  \
-                <<<sms * blocks_per_sm<SL, DIR, ST, FX, ILP>(block), block, 0, st>>>(a);  \
-        else                                                                              \
-            blocks_per_sm<SL, DIR, ST, FX, ILP>(block);                                   \
-        break;
-    if constexpr (ILP >= 4) {
-        // four or eight histories per lane: 32-byte records only
-        switch (slots) {
-            default:
-                MCLSGPU_WALK_CASE(4)
-        }
-    } else if constexpr (ILP > 1 || ST == kStencil16) {
-        switch (slots) {
-            MCLSGPU_WALK_CASE(4)
-            default:
-                MCLSGPU_WALK_CASE(8)
-        }
-    } else if constexpr (ST == kStencil) {
-        switch (slots) {
-            MCLSGPU_WALK_CASE(4)
-            MCLSGPU_WALK_CASE(8)
-            default:
-                MCLSGPU_WALK_CASE(16)
-        }
-    } else {
-        switch (slots) {
-            MCLSGPU_WALK_CASE(4)
-            MCLSGPU_WALK_CASE(8)
-            MCLSGPU_WALK_CASE(12)
-            MCLSGPU_WALK_CASE(16)
-            MCLSGPU_WALK_CASE(24)
-            default:
-                MCLSGPU_WALK_CASE(32)
-        }
-    }
-#undef MCLSGPU_WALK_CASE
+struct WalkLaunch {
+    const mclsgpu_domain* dom;
+    WalkArgs a;
+    RowFinish fin;
+    bool launch;   // false: only cache the occupancy
+};
+
+template <int S, int ST, bool POS>
+void launch_rows(const WalkLaunch& l) {
+    const mclsgpu_domain* d = l.dom;
+    const int T = d->walk_block;
+    const long long threads = (long long)d->n << l.fin.hlog;
+    walk32_rows<S, ST, POS><<<int((threads + T - 1) / T), T, 0, d->ctx->stream>>>(l.a, l.fin);
 }
 
-void dispatch_walk32(const mclsgpu_domain* dom, const WalkArgs& a, bool launch) {
-    const int sms = dom->ctx->num_sms;
-    cudaStream_t st = dom->ctx->stream;
-    const bool adj = dom->p.direction == MCLSGPU_ADJOINT;
-    const bool fixed = !(dom->p.weight_cutoff > 0.0);
-    // Several histories per lane only for fixed-length histories: two on
-    // records of at most 8 slots (the register budget of 5 blocks per SM),
-    // four or eight on 32-byte records (4 or 3 blocks per SM).
-    const bool ilp8 = fixed && dom->walk_ilp == 8 && dom->slots == 4;
-    const bool ilp4 = fixed && dom->walk_ilp >= 4 && dom->slots == 4 && !ilp8;
-    const bool ilp2 = fixed && dom->walk_ilp >= 2 && dom->slots <= 8 && !ilp4 && !ilp8;
-    const int block = dom->walk_block;
-#define MCLSGPU_WALK_DIR(DIRV, STV)                                                           \
-    (ilp8   ? launch32_slots<DIRV, STV, true, 8>(dom->slots, a, sms, block, st, launch)       \
-     : ilp4 ? launch32_slots<DIRV, STV, true, 4>(dom->slots, a, sms, block, st, launch)       \
-     : ilp2 ? launch32_slots<DIRV, STV, true, 2>(dom->slots, a, sms, block, st, launch)       \
-     : fixed ? launch32_slots<DIRV, STV, true, 1>(dom->slots, a, sms, block, st, launch)      \
-             : launch32_slots<DIRV, STV, false, 1>(dom->slots, a, sms, block, st, launch))
-    if (dom->stencil_k && dom->rec_q16) {
-        if (adj) MCLSGPU_WALK_DIR(MCLSGPU_ADJOINT, kStencil16);
-        else MCLSGPU_WALK_DIR(MCLSGPU_FORWARD, kStencil16);
-    } else if (dom->stencil_k) {
-        if (adj) MCLSGPU_WALK_DIR(MCLSGPU_ADJOINT, kStencil);
-        else MCLSGPU_WALK_DIR(MCLSGPU_FORWARD, kStencil);
-    } else {
-        if (adj) MCLSGPU_WALK_DIR(MCLSGPU_ADJOINT, kPacked);
-        else MCLSGPU_WALK_DIR(MCLSGPU_FORWARD, kPacked);
+template <int S, int ST, bool POS, int ILP>
+void launch_adj(const WalkLaunch& l) {
+    const mclsgpu_domain* d = l.dom;
+    const long long per_block = (long long)d->walk_block * ILP;
+    long long grid = (d->nh_cap + per_block - 1) / per_block;
+    if (grid < 1) grid = 1;
+    walk32_adjoint<S, ST, POS, ILP><<<int(grid), d->walk_block, 0, d->ctx->stream>>>(l.a);
+}
+
+template <int S, int ST, bool POS>
+void launch32_fixed(const WalkLaunch& l) {
+    if (!l.launch) return;
+    const mclsgpu_domain* d = l.dom;
+    if (d->p.direction == MCLSGPU_ADJOINT) {
+        // Several histories per lane: two on records of at most 64 bytes,
+        // four on 32-byte records (the register budget).
+        const int ilp = d->walk_ilp;
+        if constexpr (S == 4)
+            if (ilp >= 4) return launch_adj<S, ST, POS, 4>(l);
+        if constexpr (S <= 8)
+            if (ilp >= 2) return launch_adj<S, ST, POS, 2>(l);
+        return launch_adj<S, ST, POS, 1>(l);
     }
-#undef MCLSGPU_WALK_DIR
+    launch_rows<S, ST, POS>(l);
+}
+
+template <int S, int ST>
+void launch32_case(const WalkLaunch& l) {
+    const mclsgpu_domain* d = l.dom;
+    if (d->p.weight_cutoff > 0.0) {
+        // No more blocks than the histories need, at most what fits at once.
+        long long need = (d->nh_cap + 255) / 256;
+        if (need < 1) need = 1;
+        const bool adj = d->p.direction == MCLSGPU_ADJOINT;
+        const long long fit = (long long)d->ctx->num_sms *
+                              (adj ? cutoff_blocks_per_sm<S, MCLSGPU_ADJOINT, ST>()
+                                   : cutoff_blocks_per_sm<S, MCLSGPU_FORWARD, ST>());
+        if (!l.launch) return;
+        const int grid = int(need < fit ? need : fit);
+        if (adj)
+            walk32_cutoff<S, MCLSGPU_ADJOINT, ST><<<grid, 256, 0, d->ctx->stream>>>(l.a);
+        else
+            walk32_cutoff<S, MCLSGPU_FORWARD, ST><<<grid, 256, 0, d->ctx->stream>>>(l.a);
+        return;
+    }
+    if constexpr (ST == kStencil)
+        if (!d->neg_h) return launch32_fixed<S, ST, true>(l);
+    launch32_fixed<S, ST, false>(l);
+}
+
+// Dispatch on the record layout; `launch` false only caches the occupancy.
+void dispatch_walk32(const WalkLaunch& l) {
+    const int slots = l.dom->slots;
+    if (l.dom->stencil_k && l.dom->rec_q16) {
+        if (slots == 4) launch32_case<4, kStencil16>(l);
+        else launch32_case<8, kStencil16>(l);
+    } else if (l.dom->stencil_k) {
+        if (slots == 4) launch32_case<4, kStencil>(l);
+        else if (slots == 8) launch32_case<8, kStencil>(l);
+        else launch32_case<16, kStencil>(l);
+    } else {
+        switch (slots) {
+            case 4: launch32_case<4, kPacked>(l); break;
+            case 8: launch32_case<8, kPacked>(l); break;
+            case 12: launch32_case<12, kPacked>(l); break;
+            case 16: launch32_case<16, kPacked>(l); break;
+            case 24: launch32_case<24, kPacked>(l); break;
+            default: launch32_case<32, kPacked>(l);
+        }
+    }
 }
 
 }  // namespace
+
+namespace {
+
+__device__ __forceinline__ unsigned fdiv(unsigned x, unsigned d, unsigned& rem) {
+    const unsigned q = x / d;
+    rem = x - q * d;
+    return q;
+}
+
+// order[pos] = the row at position pos of a RowOrder.
+__global__ void k_fill_order(RowOrder o, int n, int* order) {
+    for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n;
+         pos += gridDim.x * blockDim.x) {
+        unsigned r, x, y, line;
+        const unsigned zg = fdiv(pos, o.bz * o.X * o.Y, r);
+        const unsigned nz = min(o.bz, o.Z - zg * o.bz);
+        const unsigned yg = fdiv(r, o.by * o.X * nz, r);
+        const unsigned ny = min(o.by, o.Y - yg * o.by);
+        const unsigned strip = fdiv(r, o.bx * nz * ny, r);
+        const unsigned wx = min(o.bx, o.X - strip * o.bx);
+        line = fdiv(r, wx, x);
+        const unsigned z = fdiv(line, ny, y);
+        order[pos] = int(x + strip * o.bx + o.X * (y + yg * o.by + o.Y * (z + zg * o.bz)));
+    }
+}
+
+}  // namespace
+
+// The row order of the forward walk (set-up time).
+int prepare_walk_order(mclsgpu_domain* dom) {
+    if (!walk_finishes(dom)) return MCLSGPU_OK;
+    const int per = dom->p.sample_ratio > 0.0 ? int(ceil(dom->p.sample_ratio)) : 1;
+    dom->walk_hlog = per % 4 == 0 ? 2 : per % 2 == 0 ? 1 : 0;
+    const RowOrder o = row_order(dom->n, dom->op->dia_k, dom->op->dia_off, 32 >> dom->walk_hlog);
+    if (o.X <= 1) return MCLSGPU_OK;
+    cudaError_t e = dmalloc(&dom->walk_order, size_t(dom->n));
+    if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "cudaMalloc walk order");
+    const int grid = (dom->n + 255) / 256;
+    k_fill_order<<<grid < 2368 ? grid : 2368, 256, 0, dom->ctx->stream>>>(o, dom->n,
+                                                                        dom->walk_order);
+    return MCLSGPU_OK;
+}
 
 // Cache the occupancy of the walk kernel this domain will launch (set-up time,
 // outside any stream capture).
 void prepare_walk(mclsgpu_domain* dom) {
     if (dom->p.precision != MCLSGPU_FP32) return;
-    WalkArgs a{};
-    dispatch_walk32(dom, a, false);
+    dispatch_walk32(WalkLaunch{dom, WalkArgs{}, RowFinish{}, false});
 }
 
 namespace {
@@ -591,8 +731,8 @@ __device__ __forceinline__ void load_source_row(const float* p, float (&c)[W]) {
 // One history of a row of class C (2^C columns), returns its steps.
 template <int S, bool ST, int C>
 __device__ __forceinline__ unsigned batch_history(const WalkArgs& a, const char* rec,
-                                                  const BatchWalk& m, int s, float w,
-                                                  uint64_t x) {
+                                                  const int* soff, const BatchWalk& m, int s,
+                                                  float w, uint64_t x) {
     constexpr int W = 1 << C;
     const int r0 = m.cls.crow[C];
     const float* cbase = m.cR + m.cls.cel[C];
@@ -612,7 +752,8 @@ __device__ __forceinline__ unsigned batch_history(const WalkArgs& a, const char*
             acc[r] = t;
         }
         float da = 0.f, dc = 0.f;  // the record header's own tally is unused here
-        walk_step<S, MCLSGPU_FORWARD, ST ? kStencil : kPacked>(a, rec, s, w, x, da, dc, k);
+        walk_step<S, MCLSGPU_FORWARD, ST ? kStencil : kPacked, false>(rec, nullptr, soff, s, w, x, da, dc,
+                                                                 k);
     }
     double* y = m.Y + m.cls.cel[C] + size_t(s0 - r0) * W;
 #pragma unroll
@@ -626,6 +767,8 @@ __global__ void __launch_bounds__(256, 3) walk32_batch(WalkArgs a, BatchWalk m) 
     static_assert(S % 4 == 0, "records are whole 32-byte halves");
     __shared__ uint64_t s_ekey;
     __shared__ int s_nh, s_count;
+    __shared__ int s_off[32];
+    stage_offsets(a.stoff, s_off);
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         s_ekey = epoch_key(a.seed, *a.d_epoch);
@@ -663,11 +806,11 @@ __global__ void __launch_bounds__(256, 3) walk32_batch(WalkArgs a, BatchWalk m) 
             int c = 0;
             while (c < 4 && s >= m.cls.crow[c + 1]) ++c;
             switch (c) {
-                case 0: steps += batch_history<S, ST, 0>(a, rec, m, s, w, x); break;
-                case 1: steps += batch_history<S, ST, 1>(a, rec, m, s, w, x); break;
-                case 2: steps += batch_history<S, ST, 2>(a, rec, m, s, w, x); break;
-                case 3: steps += batch_history<S, ST, 3>(a, rec, m, s, w, x); break;
-                default: steps += batch_history<S, ST, 4>(a, rec, m, s, w, x); break;
+                case 0: steps += batch_history<S, ST, 0>(a, rec, s_off, m, s, w, x); break;
+                case 1: steps += batch_history<S, ST, 1>(a, rec, s_off, m, s, w, x); break;
+                case 2: steps += batch_history<S, ST, 2>(a, rec, s_off, m, s, w, x); break;
+                case 3: steps += batch_history<S, ST, 3>(a, rec, s_off, m, s, w, x); break;
+                default: steps += batch_history<S, ST, 4>(a, rec, s_off, m, s, w, x); break;
             }
         }
     }
@@ -826,10 +969,11 @@ static void walk_reference_rounds(mclsgpu_domain* dom, WalkArgs a, int grid) {
 }
 
 // Launch the walks of the current source.  Trace arrays only with FP64.
-// `fused`: the work-queue counter reset and the timing accumulation are done
-// by the fused residual kernel that follows the walk (MCSA loop).
-void launch_walk(mclsgpu_domain* dom, long long max_trace, long long* tr_states, double* tr_w,
-                 int* tr_ev, long long* tr_start, bool fused) {
+// `fused`: the work-queue counter is reset by the fused residual kernel that
+// follows the walk (MCSA loop).
+// `fin`: how forward fixed-length FP32 walks finish each row (walk_finishes).
+void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
+                 long long* tr_states, double* tr_w, int* tr_ev, long long* tr_start, bool fused) {
     mclsgpu_context* ctx = dom->ctx;
     const mclsgpu_mc_params& p = dom->p;
     WalkArgs a{};
@@ -851,9 +995,12 @@ void launch_walk(mclsgpu_domain* dom, long long max_trace, long long* tr_states,
     a.tr_start = tr_start;
     cudaStream_t st = ctx->stream;
     if (p.precision == MCLSGPU_FP32) {
-        if (!fused) cudaMemsetAsync(dom->d_counter, 0, sizeof(int), st);
-        dispatch_walk32(dom, a, true);
-        if (!fused) k_walk_time_acc<<<1, 1, 0, st>>>(dom->d_tim);
+        if (!fused && p.weight_cutoff > 0.0)
+            cudaMemsetAsync(dom->d_counter, 0, sizeof(int), st);
+        WalkLaunch l{dom, a, fin, true};
+        l.fin.hlog = dom->walk_hlog;
+        l.fin.order = dom->walk_order;
+        dispatch_walk32(l);
     } else {
         // One thread per history up to 8 blocks per SM (the kernel strides
         // beyond that); no more blocks than the history capacity needs.
@@ -904,20 +1051,17 @@ __device__ __forceinline__ void part_send(const PartWalk& p, int q, const Histor
 template <int S, int DIR, int ST>
 __global__ void __launch_bounds__(256) walk32_part(PartWalk p) {
     __shared__ int sb[kMaxParts + 1];
+    __shared__ int s_off[32];
     for (int t = threadIdx.x; t <= p.nparts; t += blockDim.x) sb[t] = p.bounds[t];
+    stage_offsets(p.stoff, s_off);
     __syncthreads();
-    WalkArgs a{};
-    a.y64 = p.y;
-    a.row0 = p.row0;
-    if constexpr (ST != kPacked) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) a.stoff[j] = p.stoff[j];
-    }
     const uint64_t ekey = epoch_key(p.seed, *p.d_epoch);
     const float wnorm = DIR == MCLSGPU_ADJOINT ? float(p.sc[0]) : 1.f;
     const float wcut = p.cutoff * wnorm;
     const long long nwork = p.in ? p.n_in : p.e_end - p.e_begin;
-    const char* rec = reinterpret_cast<const char*>(p.rec);
+    // walk_step indexes records and tallies by the global state.
+    const char* rec = reinterpret_cast<const char*>(p.rec) - ptrdiff_t(p.row0) * (S * 8);
+    double* y = p.y - p.row0;
     const int hi = p.row0 + p.n;
     unsigned steps = 0;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nwork;
@@ -961,7 +1105,7 @@ __global__ void __launch_bounds__(256) walk32_part(PartWalk p) {
             continue;
         }
         while (true) {
-            walk_step<S, DIR, ST>(a, rec, s, w, x, acc, comp, k);
+            walk_step<S, DIR, ST, false>(rec, y, s_off, s, w, x, acc, comp, k);
             ++k;
             ++steps;
             if (k >= p.L || fabsf(w) < wcut) {
@@ -1012,6 +1156,9 @@ __global__ void __launch_bounds__(256) walk32_part(PartWalk p) {
 template <int S, int ST>
 __global__ void __launch_bounds__(256) k_walk_agreement(WalkArgs a, long long nh, uint64_t ekey,
                                                         unsigned long long* out) {
+    __shared__ int s_off[32];
+    stage_offsets(a.stoff, s_off);
+    __syncthreads();
     const char* rec = reinterpret_cast<const char*>(a.rec);
     unsigned long long hd = 0, td = 0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nh;
@@ -1027,7 +1174,7 @@ __global__ void __launch_bounds__(256) k_walk_agreement(WalkArgs a, long long nh
             x = xs_step(x);
             int s32 = s;
             unsigned neg32;
-            select32<S, ST>(a, q, x, s32, neg32);
+            select32<S, ST>(s_off, q, x, s32, neg32);
             int r0, len;
             int j = select64(a, s, canonical64(x), r0, len);
             if (j >= len) {
