@@ -362,8 +362,9 @@ int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchL
 void prec_residual(mclsgpu_domain* dom, const double* x, const double* b, double* rp_out);
 // y = PL A PR x   (LinearProblem::apply); uses dom->tmp and dom->tmp2.
 void composite_apply(mclsgpu_domain* dom, const double* x, double* y);
-// x2 = x + w r; r2 = PL (b - A PR x2): one fused pass when PL is I, point
-// Jacobi or held on A's diagonals and there is no PR (x2 != x, r2 != r).
+// x2 = x + w r; r2 = PL (b - A PR x2) for r = PL (b - A PR x): one fused pass,
+// from r alone, when PL is I, point Jacobi or held on A's diagonals and there
+// is no PR (x2 != x, r2 != r); x2 may then be null.
 void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, double w,
                          double* x2, double* r2);
 // out = the Monte Carlo estimate for the source v (already left

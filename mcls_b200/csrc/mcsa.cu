@@ -223,17 +223,20 @@ __global__ void k_mc_end(unsigned long long* epoch, unsigned long long* hist, co
 }
 
 // Convergence check of one MCSA iteration (src/MCLS_MCSASolverManager_impl.hpp:380-394).
-__device__ __forceinline__ int mcsa_check(McsaState* st, const double* sumsq, double* hist,
-                                          int hist_cap, int* status) {
-    McsaState s = *st;
+// s: the loop state and `status` the device error word, as loaded.
+__device__ __forceinline__ int mcsa_check(McsaState s, int status, McsaState* st, double sumsq,
+                                          double* hist, int hist_cap, int* d_status) {
     s.iter += 1;
-    s.rnorm = sqrt(*sumsq);
+    s.rnorm = sqrt(sumsq);
     if (hist && s.iter <= hist_cap) hist[s.iter - 1] = s.rnorm;
     int keep = 1;
     if (s.iter % s.check_freq == 0) keep = (s.rnorm > s.crit) && (s.iter < s.max_iters);
     // A non-finite residual norm ends the loop as a divergence.
-    if (!isfinite(s.rnorm)) atomicOr(status, DEV_ERR_NONFINITE);
-    if (*status) keep = 0;
+    if (!isfinite(s.rnorm)) {
+        atomicOr(d_status, DEV_ERR_NONFINITE);
+        keep = 0;
+    }
+    if (status) keep = 0;
     s.done = !keep;
     s.converged = s.rnorm <= s.crit;
     *st = s;
@@ -242,30 +245,33 @@ __device__ __forceinline__ int mcsa_check(McsaState* st, const double* sumsq, do
 
 __global__ void k_mcsa_check(McsaState* st, const double* sumsq, double* hist, int hist_cap,
                              int* status, cudaGraphConditionalHandle handle) {
-    const int keep = mcsa_check(st, sumsq, hist, hist_cap, status);
+    const int keep = mcsa_check(*st, *status, st, *sumsq, hist, hist_cap, status);
     cudaGraphSetConditional(handle, keep ? 1u : 0u);
 }
 
 __global__ void k_mcsa_check_host(McsaState* st, const double* sumsq, double* hist, int hist_cap,
                                   int* status) {
-    mcsa_check(st, sumsq, hist, hist_cap, status);
+    mcsa_check(*st, *status, st, *sumsq, hist, hist_cap, status);
 }
 
 // ---- fused iteration kernels (smoother_steps == 1, PL in {I, point Jacobi}) ----
 constexpr int kFusedThreads = 256;
 
-// Richardson smoothing fused with the residual: x2 = x + w rp (rounded as the
-// separate update would be) and rp2 = PL (b - A x2), reading x + w rp at the
-// neighbours on the fly.
+// The residual after one Richardson step x2 = x + w rp, from rp alone:
+// rp2 = PL (b - A x2) = rp - w PL A rp (PL = I or a diagonal).  Against the
+// form that subtracts A x2 from b it reads neither x nor b and gathers one
+// vector at the neighbours instead of two: 56 instead of 88 bytes per row of
+// a symmetric 7-point operator, at 128^3 22 instead of 32 us.  x2 is written
+// when the caller needs it (not null).
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_richardson_residual(
-    Op A, const double* b, const double* dinv, const double* x, const double* r, double w,
-    double* x2, double* r2) {
+    Op A, const double* dinv, const double* x, const double* r, double w, double* x2,
+    double* r2) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
-        const double s = A.dot(i, [&](int j) { return __dadd_rn(x[j], __dmul_rn(w, r[j])); });
-        const double res = b[i] - s;
-        r2[i] = dinv ? dinv[i] * res : res;
-        x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
+        const double s = A.dot(i, [&](int j) { return r[j]; });
+        const double ri = r[i];
+        r2[i] = ri - w * (dinv ? dinv[i] * s : s);
+        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
     }
 }
 
@@ -312,6 +318,19 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     __syncthreads();
     if (!last) return;
     __threadfence();
+    // The bookkeeping's words are loaded together, before the sum they wait
+    // for: one after the other they cost 2 us of a small system's iteration.
+    McsaState st;
+    int status = 0, nh = 0;
+    unsigned long long epoch = 0, histories = 0, tim[4] = {0, 0, 0, 0};
+    if (threadIdx.x == 0) {
+        st = *a.st;
+        status = *a.status;
+        nh = *a.d_nh;
+        epoch = *a.d_epoch;
+        histories = *a.d_hist;
+        for (int k = 0; k < 4; ++k) tim[k] = a.d_tim[k];
+    }
     double t = 0.0;
     for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) t += a.part[i];
     for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
@@ -321,11 +340,13 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     if (threadIdx.x == 0) {
         double sumsq = 0.0;
         for (int w = 0; w < kFusedThreads / 32; ++w) sumsq += warp_sum[w];
+        const int keep =
+            mcsa_check(st, status, a.st, sumsq, a.hist, a.hist_cap, a.status);
         *a.ticket = 0u;
-        const int keep = mcsa_check(a.st, &sumsq, a.hist, a.hist_cap, a.status);
-        *a.d_epoch += 1ULL;
-        *a.d_hist += (unsigned long long)(*a.d_nh);
-        add_walk_time(a.d_tim);
+        *a.d_epoch = epoch + 1ULL;
+        *a.d_hist = histories + (unsigned long long)nh;
+        add_walk_time(tim);
+        for (int k = 0; k < 4; ++k) a.d_tim[k] = tim[k];
         *a.d_counter = 0;
         if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
     }
@@ -345,11 +366,18 @@ __global__ void __launch_bounds__(kFusedThreads) k_residual_norm(Op A, ResidArgs
     norm_and_check(a, acc);
 }
 
-// A left preconditioner M stored on A's diagonals (learned SPAI): out = M v.
+// The same step with a left preconditioner M stored on A's diagonals (learned
+// SPAI): rp2 = rp - w M v with v = A rp.
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_dia_apply(Op M, const double* v, double* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x)
-        out[i] = M.dot(i, [&](int j) { return v[j]; });
+__global__ void __launch_bounds__(kFusedThreads) k_dia_richardson(Op M, const double* v,
+                                                                 const double* x, const double* r,
+                                                                 double w, double* x2,
+                                                                 double* r2) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
+        const double ri = r[i];
+        r2[i] = ri - w * M.dot(i, [&](int j) { return v[j]; });
+        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
+    }
 }
 
 // rp = M (b - A x) from the raw residual, its norm and the convergence check.
@@ -682,22 +710,22 @@ void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, 
     const int grid = fused_grid(dom);
     const mclsgpu_precond* L = dom->left;
     if (!dom->right && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI)) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dom->b,
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual,
                           L ? L->diag : nullptr, x, r, w, x2, r2);
     } else if (!dom->right && L->mdia && op->dia_k > 0) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dom->b, nullptr, x,
-                          r, w, x2, dom->tmp);
-        MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, r2);
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_matvec, r, nullptr, dom->tmp);
+        MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_richardson, dom->tmp, x, r, w,
+                         x2, r2);
     } else {
         k_axpy_to<<<grid, kFusedThreads, 0, s>>>(x, r, w, x2, dom->n);
         update_prec_residual(dom, x2, dom->b, r2);
     }
 }
 
-// One MCSA iteration including its convergence check.  The fused form is
-// three kernels around the walk: Richardson + residual, the source build
-// (forward: tally sources into the records), the walk, and correction +
-// residual + norm + check.
+// One MCSA iteration including its convergence check.  The fused form: the
+// residual after the Richardson step, the source build (forward: tally
+// sources into the records), the walk, which adds the step and the correction
+// to x (or k_finalize does), and residual + norm + check.
 static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp,
                               cudaGraphConditionalHandle handle, int use_cond) {
     mclsgpu_context* ctx = dom->ctx;
@@ -723,14 +751,7 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     // goes to tmp and a second pass applies M.
     const double* mdia = dom->left ? dom->left->mdia : nullptr;
     const int grid = fused_grid(dom);
-    if (mdia) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dom->b, nullptr,
-                          dom->x, dom->rp, mp->richardson_omega, dom->x2, dom->tmp);
-        MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, dom->rp2);
-    } else {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dom->b, dinv, dom->x,
-                          dom->rp, mp->richardson_omega, dom->x2, dom->rp2);
-    }
+    richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, nullptr, dom->rp2);
     // x = x + w rp + delta: the smoothing step's iterate is formed where the
     // correction is added.
     enqueue_mc(dom, dom->rp2, dom->x, kBaseSmoothed, mp->richardson_omega, 0, nullptr, nullptr,
