@@ -33,6 +33,7 @@
 #include <mutex>
 #include <cstring>
 #include <random>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -151,8 +152,9 @@ __device__ __forceinline__ bool mbar_wait_n(uint32_t mbar, uint32_t parity, int 
     }
     return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    return mbar_wait_n(mbar, parity, *reinterpret_cast<volatile int*>(&g_wait_polls));
+// The bound in force, read once per kernel (a load per wait is on the chain).
+__device__ __forceinline__ int wait_polls() {
+    return *reinterpret_cast<volatile int*>(&g_wait_polls);
 }
 // After a wait gave up, the MMAs of the phase it waited for may still be
 // writing tensor memory.  The thread that issued them waits for that phase
@@ -187,6 +189,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// 32 consecutive columns.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
+}
+
 __device__ __forceinline__ float bf16_round(float x) {
     return __bfloat162float(__float2bfloat16_rn(x));
 }
@@ -216,23 +237,40 @@ struct SlotTable {
 };
 
 // Features of row i from the diagonal-offset storage of A (FP64 values,
-// features formed in FP32: the network reads them in BF16).
+// features formed in FP32: the network reads them in BF16).  KT slots when
+// KT > 0, t.K otherwise.  Every load is issued before the first division, so
+// a row costs one memory round trip, not one per slot.
+template <int KT>
 __device__ __forceinline__ void row_features(const double* dia, int n, const SlotTable& t, int i,
                                              float* f) {
+    constexpr int kMax = KT > 0 ? KT : kMaxSlots;
+    const int K = KT > 0 ? KT : t.K;
 #pragma unroll
     for (int k = 0; k < kF; ++k) f[k] = 0.f;
     if (i >= n) return;
-    const float aii = float(dia[size_t(t.centre) * n + i]);
-    int q = 0;
-    for (int s = 0; s < t.K; ++s) {
-        if (s == t.centre) continue;
-        const double a = dia[size_t(s) * n + i];
-        const int j = i + t.off[s];
-        if (a != 0.0 && j >= 0 && j < n) {
-            f[2 * q] = float(a) / aii;
-            f[2 * q + 1] = logf(float(dia[size_t(t.centre) * n + j]) / aii);
+    const double* centre = dia + size_t(t.centre) * n;
+    double a[kMax], d[kMax];
+    const float aii = float(centre[i]);
+#pragma unroll
+    for (int s = 0; s < kMax; ++s) {
+        a[s] = 0.0;
+        d[s] = 1.0;
+        if (s < K) {
+            const int j = i + t.off[s];
+            a[s] = dia[size_t(s) * n + i];
+            if (j >= 0 && j < n) d[s] = centre[j];
+            else a[s] = 0.0;
         }
-        ++q;
+    }
+    // Pair q: the q-th slot without the centre.
+#pragma unroll
+    for (int q = 0; q < kMax - 1; ++q) {
+        const double av = q < t.centre ? a[q] : a[q + 1];
+        const double dv = q < t.centre ? d[q] : d[q + 1];
+        if (av != 0.0) {
+            f[2 * q] = float(av) / aii;
+            f[2 * q + 1] = logf(float(dv) / aii);
+        }
     }
 }
 
@@ -255,7 +293,10 @@ struct SpaiFwdArgs {
     SlotTable slots;
     int n;
     double* mval;          // M values on A's pattern (may be null)
+    double* mdia;          // M by diagonal offsets, 0 off the pattern (may be null)
+    unsigned short* mask;  // with mdia: bit s = slot s is on the pattern
     float* out;            // raw outputs [n][16] (may be null)
+    int out_align32;       // out is 32-byte aligned
     int* status;
 };
 
@@ -264,27 +305,129 @@ constexpr int kFwdW1 = 0;                          // 64 x 16
 constexpr int kFwdW2 = kFwdW1 + kH * kF * 2;       // 64 x 64
 constexpr int kFwdW3 = kFwdW2 + kH * kH * 2;       // 16 x 64
 constexpr int kFwdX = kFwdW3 + kO * kH * 2;        // 128 x 16
-constexpr int kFwdH = kFwdX + kTileRows * kF * 2;  // 128 x 64
-constexpr int kFwdBar = kFwdH + kTileRows * kH * 2;
-// Requested dynamic shared memory: at most 4 CTAs per SM, so that their
-// 4 x 128 tensor-memory columns fit the SM's 512.
-constexpr int kFwdSmem = 56 * 1024;
-static_assert(kFwdBar + 64 <= kFwdSmem, "forward shared memory");
+constexpr int kFwdH = kFwdX + kTileRows * kF * 2;  // 128 x 64, then the tile's M values
+constexpr int kFwdBias = kFwdH + kTileRows * kH * 2;  // b1, b2, b3 (FP32)
+constexpr int kFwdBar = kFwdBias + (2 * kH + kO) * 4;
+constexpr int kFwdSmem = kFwdBar + 64;
+// CTAs per SM: the registers' and shared memory's limit; their tensor-memory
+// columns (64 each) are within the SM's 512.
+constexpr int kFwdCtas = 6;
+constexpr int kFwdCols = 64;
+static_assert(kTileRows * kMaxSlots * 8 <= kTileRows * kH * 2, "the tile's M values fit H");
+static_assert(kFwdCtas * (kFwdSmem + 1024) <= 227 * 1024 && kFwdCtas * kFwdCols <= 512,
+              "forward kernel residency");
+
+// One hidden layer's epilogue for this thread's row: 64 accumulator columns
+// plus bias, ReLU, to BF16 as the next layer's K-major operand.
+__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float* bias,
+                                                unsigned char* H, int row) {
+#pragma unroll 1
+    for (int c = 0; c < kH; c += 32) {
+        float z[32];
+        tmem_ld32(taddr + c, z);
+#pragma unroll
+        for (int k = 0; k < 32; k += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + c + k);
+            z[k] = fmaxf(z[k] + b.x, 0.f);
+            z[k + 1] = fmaxf(z[k + 1] + b.y, 0.f);
+            z[k + 2] = fmaxf(z[k + 2] + b.z, 0.f);
+            z[k + 3] = fmaxf(z[k + 3] + b.w, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) store8(H, row, c + k, kTileRows, z + k);
+    }
+}
+
+// The backward epilogue: dZ = dH where the activation is positive, to BF16.
+__device__ __forceinline__ void masked_epilogue(uint32_t taddr, const unsigned char* H,
+                                                unsigned char* dZ, int row) {
+#pragma unroll 1
+    for (int c = 0; c < kH; c += 32) {
+        float d[32];
+        tmem_ld32(taddr + c, d);
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+            float h[8];
+            load8(H, row, c + k, kTileRows, h);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d[k + j] = h[j] > 0.f ? d[k + j] : 0.f;
+            store8(dZ, row, c + k, kTileRows, d + k);
+        }
+    }
+}
+
+// Row `row` of M from its outputs: on A's pattern into `stage` (the tile's
+// entries in order, from tile entry e0) and/or by diagonal offset.
+template <int KT>
+__device__ __forceinline__ void emit_m(const SpaiFwdArgs& a, int row, const float* o,
+                                       double* stage, int e0) {
+    constexpr int kMax = KT > 0 ? KT : kMaxSlots;
+    const int K = KT > 0 ? KT : a.slots.K;
+    const int p0 = a.rp[row], len = a.rp[row + 1] - p0;
+    const double inv = 1.0 / a.dia[size_t(a.slots.centre) * a.n + row];
+    double m[kMax];
+#pragma unroll
+    for (int s = 0; s < kMax; ++s)
+        m[s] = ((s == a.slots.centre ? 1.0 : 0.0) + double(o[s])) * inv;
+    // A full row's entries are its slots in order (columns are sorted).
+    unsigned mask = (1u << K) - 1u;
+    if (len == K) {
+        if (stage) {
+#pragma unroll
+            for (int s = 0; s < kMax; ++s)
+                if (s < K) stage[p0 - e0 + s] = m[s];
+        }
+    } else {
+        mask = 0u;
+        for (int p = p0; p < p0 + len; ++p) {
+            const int d = a.ci[p] - row;
+            double v = 0.0;
+#pragma unroll
+            for (int s = 0; s < kMax; ++s)
+                if (s < K && a.slots.off[s] == d) {
+                    v = m[s];
+                    mask |= 1u << s;
+                }
+            if (stage) stage[p - e0] = v;
+        }
+    }
+    if (a.mdia) {
+#pragma unroll
+        for (int s = 0; s < kMax; ++s)
+            if (s < K) a.mdia[size_t(s) * a.n + row] = (mask >> s) & 1u ? m[s] : 0.0;
+        a.mask[row] = (unsigned short)mask;
+    }
+}
 
 // Forward pass: one CTA (4 warps, one row per thread) per 128-row tile,
-// persistent over tiles.  TMEM: columns 0-63 layer-1 and layer-3
-// accumulators, 64-127 layer 2.
-__global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
+// persistent over tiles; every layer accumulates in the same 64 TMEM columns.
+//
+// What bounds it: the chain of one tile (features, MMA, TMEM load, ReLU to
+// BF16, next MMA, ...), hidden by running six CTAs per SM.  At 128^3 (16,384
+// tiles, 376 MB in and out, 58 us at the copy rate) it took 804 us with three
+// CTAs of 162 registers, dependent loads slot by slot in the features, biases
+// read from global memory and M stored entry by entry; those are now one batch
+// of loads, shared memory, and a tile's M values staged in shared memory and
+// written in order.
+template <int KT>
+__global__ void __launch_bounds__(kThreads, kFwdCtas) k_spai_forward(SpaiFwdArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kFwdBar);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kFwdBar + 16);
+    float* bias = reinterpret_cast<float*>(smem + kFwdBias);
     const uint32_t mbar = smem_u32(bar);
     stage_weights(smem + kFwdW1, a.params + kW1, kH, kF);
     stage_weights(smem + kFwdW2, a.params + kW2, kH, kH);
     stage_weights(smem + kFwdW3, a.params + kW3, kO, kH);
+    if (tid < kH) {
+        bias[tid] = a.params[kB1 + tid];
+        bias[kH + tid] = a.params[kB2 + tid];
+    }
+    if (tid < kO) bias[2 * kH + tid] = a.params[kB3 + tid];
     if (tid == 0) mbar_init(mbar);
-    if (warp == 0) tmem_alloc(smem_u32(tslot), 128);
+    if (warp == 0) tmem_alloc(smem_u32(tslot), kFwdCols);
+    const int polls = wait_polls();
     fence_async_smem();
     fence_before_sync();
     __syncthreads();
@@ -294,9 +437,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
     const uint32_t sX = smem_u32(smem + kFwdX), sH = smem_u32(smem + kFwdH);
     const uint32_t sW1 = smem_u32(smem + kFwdW1), sW2 = smem_u32(smem + kFwdW2),
                    sW3 = smem_u32(smem + kFwdW3);
-    const float* b1 = a.params + kB1;
-    const float* b2 = a.params + kB2;
-    const float* b3 = a.params + kB3;
     uint32_t phase = 0;
     bool ok = true;
     // Thread 0 issues the MMAs, and only while its own waits succeed, so at
@@ -304,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
     bool pend = false;
     uint32_t pend_parity = 0;
     auto wait_mma = [&]() {
-        const bool got = ok && mbar_wait(mbar, phase);
+        const bool got = ok && mbar_wait_n(mbar, phase, polls);
         if (ok && !got) {
             pend = true;
             pend_parity = phase;
@@ -313,18 +453,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
         phase ^= 1;
         fence_after_sync();
     };
+    auto stage_sync = [&]() {
+        fence_async_smem();
+        fence_before_sync();
+        __syncthreads();
+    };
     const int ntiles = (a.n + kTileRows - 1) / kTileRows;
     for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
         const int row = tile * kTileRows + tid;
         {
             float f[kF];
-            row_features(a.dia, a.n, a.slots, row, f);
+            row_features<KT>(a.dia, a.n, a.slots, row, f);
             store8(smem + kFwdX, tid, 0, kTileRows, f);
             store8(smem + kFwdX, tid, 8, kTileRows, f + 8);
         }
-        fence_async_smem();
-        fence_before_sync();
-        __syncthreads();
+        stage_sync();
         // Layer 1: Z1 = X W1^T  (M 128, N 64, K 16).
         if (tid == 0 && ok) {
             fence_after_sync();
@@ -333,39 +476,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
             mma_commit(mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 16) {
-            float z[16];
-            tmem_ld16(lane_base + c, z);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) z[k] = fmaxf(z[k] + b1[c + k], 0.f);
-            store8(smem + kFwdH, tid, c, kTileRows, z);
-            store8(smem + kFwdH, tid, c + 8, kTileRows, z + 8);
-        }
-        fence_async_smem();
-        fence_before_sync();
-        __syncthreads();
-        // Layer 2: Z2 = H1 W2^T  (M 128, N 64, K 64).
+        hidden_epilogue(lane_base, bias, smem + kFwdH, tid);
+        stage_sync();
+        // Layer 2: Z2 = H1 W2^T  (M 128, N 64, K 64), over Z1, which every
+        // thread has read before the barrier above.
         if (tid == 0 && ok) {
             fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                mma_bf16(tmem + 64, desc_kmajor(sH, kTileRows, ks), desc_kmajor(sW2, kH, ks),
+                mma_bf16(tmem, desc_kmajor(sH, kTileRows, ks), desc_kmajor(sW2, kH, ks),
                          idesc_bf16(128, kH, 0, 0), ks > 0);
             mma_commit(mbar);
         }
         wait_mma();
         // H2 overwrites H1: layer 2's operands are consumed (its MMAs are
         // complete once the barrier phase has flipped).
-        float h2[kH];
-#pragma unroll
-        for (int c = 0; c < kH; c += 16) tmem_ld16(lane_base + 64 + c, h2 + c);
-#pragma unroll
-        for (int k = 0; k < kH; ++k) h2[k] = fmaxf(h2[k] + b2[k], 0.f);
-#pragma unroll
-        for (int c = 0; c < kH; c += 8) store8(smem + kFwdH, tid, c, kTileRows, h2 + c);
-        fence_async_smem();
-        fence_before_sync();
-        __syncthreads();
+        hidden_epilogue(lane_base, bias + kH, smem + kFwdH, tid);
+        stage_sync();
         // Layer 3: out = H2 W3^T  (M 128, N 16, K 64).
         if (tid == 0 && ok) {
             fence_after_sync();
@@ -381,24 +507,35 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
         // The next tile's layer 1 reuses these columns; a timed-out wait on
         // any thread ends the loop on all of them.
         ok = __syncthreads_and(ok);
-        if (ok && row < a.n) {
+        if (!ok) break;
 #pragma unroll
-            for (int k = 0; k < kO; ++k) o[k] += b3[k];
-            if (a.out) {
-                float4* dst = reinterpret_cast<float4*>(a.out + size_t(row) * kO);
+        for (int k = 0; k < kO; ++k) o[k] += bias[2 * kH + k];
+        if (a.out && row < a.n) {
+            float* dst = a.out + size_t(row) * kO;
+            if (a.out_align32) {
 #pragma unroll
-                for (int k = 0; k < kO; k += 4) dst[k / 4] = make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+                for (int k = 0; k < kO; k += 8)
+                    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + k),
+                                 "f"(o[k]), "f"(o[k + 1]), "f"(o[k + 2]), "f"(o[k + 3]),
+                                 "f"(o[k + 4]), "f"(o[k + 5]), "f"(o[k + 6]), "f"(o[k + 7])
+                                 : "memory");
+            } else {
+#pragma unroll
+                for (int k = 0; k < kO; k += 4)
+                    *reinterpret_cast<float4*>(dst + k) =
+                        make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
             }
-            if (a.mval) {
-                const double inv = 1.0 / a.dia[size_t(a.slots.centre) * a.n + row];
-                for (int p = a.rp[row]; p < a.rp[row + 1]; ++p) {
-                    const int d = a.ci[p] - row;
-                    double v = 0.0;
-                    for (int s = 0; s < a.slots.K; ++s)
-                        if (a.slots.off[s] == d) v = ((d == 0 ? 1.0 : 0.0) + double(o[s])) * inv;
-                    a.mval[p] = v;
-                }
-            }
+        }
+        if (a.mval) {
+            // Layer 3 has read H: the tile's M entries take its place.
+            double* stage = reinterpret_cast<double*>(smem + kFwdH);
+            const int last = min(a.n, (tile + 1) * kTileRows);
+            const int e0 = a.rp[tile * kTileRows], e1 = a.rp[last];
+            if (row < a.n) emit_m<KT>(a, row, o, stage, e0);
+            __syncthreads();
+            for (int e = tid; e < e1 - e0; e += kThreads) a.mval[e0 + e] = stage[e];
+        } else if (a.mdia && row < a.n) {
+            emit_m<KT>(a, row, o, nullptr, 0);
         }
     }
     if (!ok && tid == 0) atomicExch(a.status, MCLSGPU_ERR_TIMEOUT);
@@ -407,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_forward(SpaiFwdArgs a) {
     __syncthreads();
     if (warp == 0) {
         fence_after_sync();
-        tmem_dealloc(tmem, 128);
+        tmem_dealloc(tmem, kFwdCols);
     }
 }
 
@@ -437,33 +574,44 @@ constexpr int kBwG = kBwH2 + kTileRows * kH * 2;        // 128 x 16
 constexpr int kBwDZ2 = kBwG + kTileRows * kO * 2;       // 128 x 64
 constexpr int kBwDZ1 = kBwDZ2 + kTileRows * kH * 2;     // 128 x 64
 constexpr int kBwB3 = kBwDZ1 + kTileRows * kH * 2;      // 16 floats
-constexpr int kBwBar = kBwB3 + 64;
-// Requested dynamic shared memory: one CTA per SM, which allocates all 512
-// tensor-memory columns.
-constexpr int kBwSmem = 120 * 1024;
-static_assert(kBwBar + 64 <= kBwSmem, "backward shared memory");
-// TMEM columns of the backward kernel (512 allocated).
-constexpr uint32_t kTA = 0;      // Z1, then dH2 (M 128 x 64)
-constexpr uint32_t kTB = 64;     // Z2, then dH1 (M 128 x 64)
-constexpr uint32_t kTdW3 = 256;  // dW3^T: rows h2, cols o     (M 64 x 16)
-constexpr uint32_t kTdW2 = 288;  // dW2: rows h2, cols h1 | db2 (M 64 x 72)
-constexpr uint32_t kTdW1 = 384;  // dW1: rows h1, cols in | db1 (M 64 x 24)
+constexpr int kBwBias = kBwB3 + 64;                     // b1, b2 (FP32)
+constexpr int kBwBar = kBwBias + 2 * kH * 4;
+constexpr int kBwSmem = kBwBar + 64;
+// Two CTAs per SM, 256 tensor-memory columns each: a training sample of 32^3
+// rows (256 tiles) is then one tile per CTA instead of two in sequence.
+constexpr int kBwCtas = 2;
+constexpr int kBwCols = 256;
+static_assert(kBwCtas * (kBwSmem + 1024) <= 227 * 1024 && kBwCtas * kBwCols <= 512,
+              "backward kernel residency");
+// TMEM columns of the backward kernel.  One 64-column buffer serves Z1, Z2,
+// dH2 and dH1 in turn: each is read before the barrier that precedes the
+// MMAs of the next.
+constexpr uint32_t kTA = 0;      // Z1, Z2, dH2, dH1 (M 128 x 64)
+constexpr uint32_t kTdW3 = 64;   // dW3^T: rows h2, cols o     (M 64 x 16)
+constexpr uint32_t kTdW2 = 96;   // dW2: rows h2, cols h1 | db2 (M 64 x 72, read as 80)
+constexpr uint32_t kTdW1 = 192;  // dW1: rows h1, cols in | db1 (M 64 x 24, read as 32)
 
 // Backward pass: the forward activations of each tile are recomputed, the
 // output gradient G is propagated to dZ2 and dZ1, and the weight and bias
 // gradients accumulate in TMEM across the CTA's tiles; at the end each CTA
 // adds its sums into `grad`.
-__global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
+template <int KT>
+__global__ void __launch_bounds__(kThreads, kBwCtas) k_spai_backward(SpaiBwdArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kBwBar);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kBwBar + 16);
     float* db3 = reinterpret_cast<float*>(smem + kBwB3);
+    float* bias = reinterpret_cast<float*>(smem + kBwBias);
     const uint32_t mbar = smem_u32(bar);
     stage_weights(smem + kBwW1, a.params + kW1, kH, kF);
     stage_weights(smem + kBwW2, a.params + kW2, kH, kH);
     stage_weights(smem + kBwW3, a.params + kW3, kO, kH);
     if (tid < kO) db3[tid] = 0.f;
+    if (tid < kH) {
+        bias[tid] = a.params[kB1 + tid];
+        bias[kH + tid] = a.params[kB2 + tid];
+    }
     {
         // Ones groups (column 16 of X, column 64 of H1) for every row.
         float one[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -471,7 +619,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
         store8(smem + kBwH1, tid, 64, kTileRows, one);
     }
     if (tid == 0) mbar_init(mbar);
-    if (warp == 0) tmem_alloc(smem_u32(tslot), 512);
+    if (warp == 0) tmem_alloc(smem_u32(tslot), kBwCols);
+    const int polls = wait_polls();
     fence_async_smem();
     fence_before_sync();
     __syncthreads();
@@ -483,8 +632,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
                    sH1 = smem_u32(smem + kBwH1), sH2 = smem_u32(smem + kBwH2),
                    sG = smem_u32(smem + kBwG), sDZ2 = smem_u32(smem + kBwDZ2),
                    sDZ1 = smem_u32(smem + kBwDZ1);
-    const float* b1 = a.params + kB1;
-    const float* b2 = a.params + kB2;
     uint32_t phase = 0;
     bool ok = true;
     int done = 0;
@@ -499,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
         __syncthreads();
     };
     auto wait_mma = [&]() {
-        const bool got = ok && mbar_wait(mbar, phase);
+        const bool got = ok && mbar_wait_n(mbar, phase, polls);
         if (ok && !got) {
             pend = true;
             pend_parity = phase;
@@ -512,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
         const int row = tile * kTileRows + tid;
         {
             float f[kF];
-            row_features(a.dia, a.n, a.slots, row, f);
+            row_features<KT>(a.dia, a.n, a.slots, row, f);
             store8(smem + kBwX, tid, 0, kTileRows, f);
             store8(smem + kBwX, tid, 8, kTileRows, f + 8);
         }
@@ -524,33 +671,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
             mma_commit(mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 16) {
-            float z[16];
-            tmem_ld16(lane_base + kTA + c, z);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) z[k] = fmaxf(z[k] + b1[c + k], 0.f);
-            store8(smem + kBwH1, tid, c, kTileRows, z);
-            store8(smem + kBwH1, tid, c + 8, kTileRows, z + 8);
-        }
+        hidden_epilogue(lane_base + kTA, bias, smem + kBwH1, tid);
         stage_sync();
         if (tid == 0 && ok) {
             fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                mma_bf16(tmem + kTB, desc_kmajor(sH1, kTileRows, ks), desc_kmajor(sW2, kH, ks),
+                mma_bf16(tmem + kTA, desc_kmajor(sH1, kTileRows, ks), desc_kmajor(sW2, kH, ks),
                          idesc_bf16(128, kH, 0, 0), ks > 0);
             mma_commit(mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 16) {
-            float z[16];
-            tmem_ld16(lane_base + kTB + c, z);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) z[k] = fmaxf(z[k] + b2[c + k], 0.f);
-            store8(smem + kBwH2, tid, c, kTileRows, z);
-            store8(smem + kBwH2, tid, c + 8, kTileRows, z + 8);
-        }
+        hidden_epilogue(lane_base + kTA, bias + kH, smem + kBwH2, tid);
         {
             float g[kO];
 #pragma unroll
@@ -591,24 +722,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
             mma_commit(mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 16) {
-            float d[16], h[16];
-            tmem_ld16(lane_base + kTA + c, d);
-            load8(smem + kBwH2, tid, c, kTileRows, h);
-            load8(smem + kBwH2, tid, c + 8, kTileRows, h + 8);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) d[k] = h[k] > 0.f ? d[k] : 0.f;
-            store8(smem + kBwDZ2, tid, c, kTileRows, d);
-            store8(smem + kBwDZ2, tid, c + 8, kTileRows, d + 8);
-        }
+        masked_epilogue(lane_base + kTA, smem + kBwH2, smem + kBwDZ2, tid);
         stage_sync();
         // dH1 = dZ2 W2 (B = W2 MN-major: N 64 = h1, K 64 = h2) and
         // [dW2 | db2] += dZ2^T [H1 | 1] (K = 128 rows).
         if (tid == 0 && ok) {
             fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                mma_bf16(tmem + kTB, desc_kmajor(sDZ2, kTileRows, ks), desc_mnmajor(sW2, kH, ks),
+                mma_bf16(tmem + kTA, desc_kmajor(sDZ2, kTileRows, ks), desc_mnmajor(sW2, kH, ks),
                          idesc_bf16(128, kH, 0, 1), ks > 0);
             for (int ks = 0; ks < kTileRows / 16; ++ks)
                 mma_bf16(tmem + kTdW2, desc_mnmajor(sDZ2, kTileRows, ks),
@@ -617,17 +738,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
             mma_commit(mbar);
         }
         wait_mma();
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 16) {
-            float d[16], h[16];
-            tmem_ld16(lane_base + kTB + c, d);
-            load8(smem + kBwH1, tid, c, kTileRows, h);
-            load8(smem + kBwH1, tid, c + 8, kTileRows, h + 8);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) d[k] = h[k] > 0.f ? d[k] : 0.f;
-            store8(smem + kBwDZ1, tid, c, kTileRows, d);
-            store8(smem + kBwDZ1, tid, c + 8, kTileRows, d + 8);
-        }
+        masked_epilogue(lane_base + kTA, smem + kBwH1, smem + kBwDZ1, tid);
         stage_sync();
         // [dW1 | db1] += dZ1^T [X | 1] (K = 128 rows).
         if (tid == 0 && ok) {
@@ -678,95 +789,167 @@ __global__ void __launch_bounds__(kThreads, 1) k_spai_backward(SpaiBwdArgs a) {
     __syncthreads();
     if (warp == 0) {
         fence_after_sync();
-        tmem_dealloc(tmem, 512);
+        tmem_dealloc(tmem, kBwCols);
     }
 }
 
-// e_v = v - M (A v) per row; loss and the output gradient G.  With
-// pen_w > 0 the loss adds pen_w/n * sum_i max(0, W_i - pen_c)^2, W_i the
-// row sum of |H| for H = I - M A (the factor by which a forward walk's
-// weight grows at state i), computed from row i of M and the rows of A at
-// its neighbours.
-__global__ void k_spai_loss_grad(int n, int nvec, const int* rp, const int* ci, const double* mval,
-                                 const double* dia, SlotTable slots, const double* V,
-                                 const double* Z, const double* wv, double pen_w, double pen_c,
-                                 float* G, double* loss) {
-    double part = 0.0;
+// z_v = A v for every training vector (blockIdx.y) and, in the vector's block
+// that finishes last, wv[v] = 1 / (nvec |v|^2) (block sums in block order).
+template <int KT>
+__global__ void __launch_bounds__(256) k_spai_vectors(int n, int nvec, const double* dia,
+                                                      SlotTable slots, const double* V, double* Z,
+                                                      double* part, unsigned* tickets,
+                                                      double* wv) {
+    constexpr int kMax = KT > 0 ? KT : kMaxSlots;
+    const int K = KT > 0 ? KT : slots.K;
+    __shared__ double sh[8];
+    __shared__ bool last;
+    const int v = blockIdx.y;
+    const double* x = V + size_t(v) * n;
+    double sq = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double inv = 1.0 / dia[size_t(slots.centre) * n + i];
-        double g[kO];
+        double z = 0.0;
 #pragma unroll
-        for (int k = 0; k < kO; ++k) g[k] = 0.0;
-        if (pen_w > 0.0) {
-            double m[kMaxSlots];
-            bool has[kMaxSlots];
-            for (int s = 0; s < kMaxSlots; ++s) {
-                m[s] = 0.0;
-                has[s] = false;
-            }
-            for (int p = rp[i]; p < rp[i + 1]; ++p) {
-                const int d = ci[p] - i;
-                for (int s = 0; s < slots.K; ++s)
-                    if (slots.off[s] == d) {
-                        m[s] = mval[p];
-                        has[s] = true;
-                    }
-            }
-            double h[kMaxSlots * kMaxSlots];
-            for (int q = 0; q < slots.npair; ++q) h[q] = 0.0;
-            h[slots.pcentre] = 1.0;
-            for (int s = 0; s < slots.K; ++s) {
-                const int k = i + slots.off[s];
-                if (!has[s] || k < 0 || k >= n) continue;
-                for (int t = 0; t < slots.K; ++t)
-                    h[slots.pair[s][t]] -= m[s] * dia[size_t(t) * n + k];
-            }
-            double W = 0.0;
-            for (int q = 0; q < slots.npair; ++q) W += fabs(h[q]);
-            const double pen = W - pen_c;
-            if (pen > 0.0) {
-                part += pen_w * pen * pen / double(n);
-                const double coef = 2.0 * pen_w * pen / double(n) * inv;
-                for (int s = 0; s < slots.K; ++s) {
-                    const int k = i + slots.off[s];
-                    if (!has[s] || k < 0 || k >= n) continue;
-                    double dW = 0.0;
-                    for (int t = 0; t < slots.K; ++t) {
-                        const double hv = h[slots.pair[s][t]];
-                        const double sg = hv > 0.0 ? 1.0 : (hv < 0.0 ? -1.0 : 0.0);
-                        dW -= sg * dia[size_t(t) * n + k];
-                    }
-                    g[s] += coef * dW;
-                }
-            }
+        for (int s = 0; s < kMax; ++s) {
+            const int j = i + slots.off[s];
+            if (s < K && j >= 0 && j < n) z = fma(dia[size_t(s) * n + i], x[j], z);
         }
-        for (int v = 0; v < nvec; ++v) {
+        Z[size_t(v) * n + i] = z;
+        sq = fma(x[i], x[i], sq);
+    }
+    for (int d = 16; d > 0; d >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, d);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    double* vp = part + size_t(v) * gridDim.x;
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += sh[w];
+        vp[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(&tickets[v], 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (int k = threadIdx.x; k < int(gridDim.x); k += blockDim.x) t += __ldcg(&vp[k]);
+    for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t = 0.0;
+        for (int w = 0; w < 8; ++w) t += sh[w];
+        wv[v] = t > 0.0 ? 1.0 / (double(nvec) * t) : 0.0;
+    }
+}
+
+// The row-sum penalty's part of the loss and of row i's output gradient:
+// pen_w/n * max(0, W_i - pen_c)^2, W_i the row sum of |H| for H = I - M A (the
+// factor by which a forward walk's weight grows at state i), from row i of M
+// and the rows of A at its neighbours.
+__device__ double penalty_row(int n, int i, const double* m, unsigned mask, const double* dia,
+                              const SlotTable& slots, double inv, double pen_w, double pen_c,
+                              double* g) {
+    double h[kMaxSlots * kMaxSlots];
+    for (int q = 0; q < slots.npair; ++q) h[q] = 0.0;
+    h[slots.pcentre] = 1.0;
+    for (int s = 0; s < slots.K; ++s) {
+        const int k = i + slots.off[s];
+        if (!((mask >> s) & 1u) || k < 0 || k >= n) continue;
+        for (int t = 0; t < slots.K; ++t) h[slots.pair[s][t]] -= m[s] * dia[size_t(t) * n + k];
+    }
+    double W = 0.0;
+    for (int q = 0; q < slots.npair; ++q) W += fabs(h[q]);
+    const double pen = W - pen_c;
+    if (!(pen > 0.0)) return 0.0;
+    const double coef = 2.0 * pen_w * pen / double(n) * inv;
+    for (int s = 0; s < slots.K; ++s) {
+        const int k = i + slots.off[s];
+        if (!((mask >> s) & 1u) || k < 0 || k >= n) continue;
+        double dW = 0.0;
+        for (int t = 0; t < slots.K; ++t) {
+            const double hv = h[slots.pair[s][t]];
+            const double sg = hv > 0.0 ? 1.0 : (hv < 0.0 ? -1.0 : 0.0);
+            dW -= sg * dia[size_t(t) * n + k];
+        }
+        g[s] += coef * dW;
+    }
+    return pen_w * pen * pen / double(n);
+}
+
+// e_v = v - M (A v) per row; loss and the output gradient G.  PEN: with the
+// row-sum penalty.  A block is 32 rows by kLossGroups groups of vectors (a
+// 32^3 sample alone has too few rows to fill the chip); the groups' gradients
+// are added in shared memory in group order.
+constexpr int kLossGroups = 8;
+template <int KT, bool PEN>
+__global__ void __launch_bounds__(32 * kLossGroups)
+    k_spai_loss_grad(int n, int nvec, const double* mdia, const unsigned short* mask,
+                     const double* dia, SlotTable slots, const double* V, const double* Z,
+                     const double* wv, double pen_w, double pen_c, float* G, double* loss) {
+    constexpr int kMax = KT > 0 ? KT : kMaxSlots;
+    const int K = KT > 0 ? KT : slots.K;
+    __shared__ double sg[kLossGroups][kMax][32];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    const bool live = i < n;
+    double part = 0.0;
+    double g[kMax];
+#pragma unroll
+    for (int s = 0; s < kMax; ++s) g[s] = 0.0;
+    if (live) {
+        const double inv = 1.0 / dia[size_t(slots.centre) * n + i];
+        const unsigned msk = mask[i];
+        double m[kMax];
+#pragma unroll
+        for (int s = 0; s < kMax; ++s) m[s] = s < K ? mdia[size_t(s) * n + i] : 0.0;
+        if constexpr (PEN)
+            if (grp == 0)
+                part += penalty_row(n, i, m, msk, dia, slots, inv, pen_w, pen_c, g);
+        for (int v = grp; v < nvec; v += kLossGroups) {
             const double* z = Z + size_t(v) * n;
+            double zs[kMax];
             double mz = 0.0;
-            for (int p = rp[i]; p < rp[i + 1]; ++p) mz += mval[p] * z[ci[p]];
+#pragma unroll
+            for (int s = 0; s < kMax; ++s) {
+                // A slot off the row's pattern has no neighbour.
+                zs[s] = s < K && ((msk >> s) & 1u) ? z[i + slots.off[s]] : 0.0;
+                mz += m[s] * zs[s];
+            }
             const double e = V[size_t(v) * n + i] - mz;
             part += e * e * wv[v];
             const double c = -2.0 * e * wv[v] * inv;
-            for (int p = rp[i]; p < rp[i + 1]; ++p) {
-                const int d = ci[p] - i;
-                for (int s = 0; s < slots.K; ++s)
-                    if (slots.off[s] == d) g[s] += c * z[ci[p]];
+#pragma unroll
+            for (int s = 0; s < kMax; ++s) g[s] += c * zs[s];
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < kMax; ++s) sg[grp][s][lane] = g[s];
+    __syncthreads();
+    // Group grp sums slots 2 grp and 2 grp + 1 of the 16 outputs.
+    if (live) {
+        float o[2] = {0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int s = 2 * grp + q;
+            if (s < K) {
+                double t = 0.0;
+                for (int w = 0; w < kLossGroups; ++w) t += sg[w][s][lane];
+                o[q] = float(t);
             }
         }
-        float4* dst = reinterpret_cast<float4*>(G + size_t(i) * kO);
-#pragma unroll
-        for (int k = 0; k < kO; k += 4)
-            dst[k / 4] = make_float4(float(g[k]), float(g[k + 1]), float(g[k + 2]), float(g[k + 3]));
+        *reinterpret_cast<float2*>(G + size_t(i) * kO + 2 * grp) = make_float2(o[0], o[1]);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, part);
-}
-
-// wv[v] = 1 / (nvec * |v|^2) from the per-vector sums of squares.
-__global__ void k_spai_weights(const double* sq, int nvec, double* wv) {
-    const int v = threadIdx.x;
-    if (v < nvec) wv[v] = sq[v] > 0.0 ? 1.0 / (double(nvec) * sq[v]) : 0.0;
+    __shared__ double sl[kLossGroups];
+    if (lane == 0) sl[grp] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < kLossGroups; ++w) t += sl[w];
+        atomicAdd(loss, t);
+    }
 }
 
 __global__ void k_adam(float* p, float* m, float* v, const float* g, int count, float lr,
@@ -812,6 +995,10 @@ struct mclsgpu_spai {
     long long step = 0;
     double pen_w = 0.0;       // row-sum penalty weight (0 = off)
     double pen_c = 1.0;       // row-sum threshold
+    // Scratch of the training gradient, kept between calls up to kScratchKeep
+    // bytes (released with the network).
+    unsigned char* scratch = nullptr;
+    size_t scratch_bytes = 0;
 };
 
 namespace mclsgpu {
@@ -837,7 +1024,7 @@ int slot_table(mclsgpu_context* ctx, const mclsgpu_operator* op, int want, SlotT
         t.off[s] = op->dia_off[s];
         if (op->dia_off[s] == 0) t.centre = s;
     }
-    for (int s = t.K; s < kMaxSlots; ++s) t.off[s] = 0x7fffffff;
+    for (int s = t.K; s < kMaxSlots; ++s) t.off[s] = 0;  // never selected (s < K)
     if (t.centre < 0)
         return set_error(ctx, MCLSGPU_ERR_UNSUPPORTED, "learned SPAI: operator has no diagonal");
     std::vector<int> sums;
@@ -856,6 +1043,18 @@ int slot_table(mclsgpu_context* ctx, const mclsgpu_operator* op, int want, SlotT
     return MCLSGPU_OK;
 }
 
+// Calls f(integral_constant<int, K>) with the operator's slot count when it
+// is one of the unrolled ones (5-, 7- and 9-point stencils), else with 0.
+template <class F>
+void with_slots(int K, F f) {
+    switch (K) {
+        case 5: f(std::integral_constant<int, 5>{}); break;
+        case 7: f(std::integral_constant<int, 7>{}); break;
+        case 9: f(std::integral_constant<int, 9>{}); break;
+        default: f(std::integral_constant<int, 0>{});
+    }
+}
+
 // The kernels' dynamic shared memory exceeds the 48 KB default: opt in once
 // per device (the attribute belongs to the device's context).
 std::mutex g_attr_mutex;
@@ -865,18 +1064,24 @@ int set_smem_attributes(mclsgpu_context* ctx) {
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     const int d = ctx->device;
     if (d >= 0 && d < 64 && g_attr_set[d]) return MCLSGPU_OK;
-    cudaError_t e = cudaFuncSetAttribute(k_spai_forward,
+    cudaError_t e = cudaSuccess;
+    for (int K : {0, 5, 7, 9})
+        with_slots(K, [&](auto k) {
+            constexpr int KT = decltype(k)::value;
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_spai_forward<KT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_spai_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kBwSmem);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_spai_backward<KT>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kBwSmem);
+        });
     if (e != cudaSuccess) return cuda_fail(ctx, e, "spai shared-memory opt-in");
     if (d >= 0 && d < 64) g_attr_set[d] = true;
     return MCLSGPU_OK;
 }
 
 int launch_forward(mclsgpu_spai* net, mclsgpu_operator* op, const SlotTable& t, double* mval,
-                   float* out) {
+                   float* out, double* mdia = nullptr, unsigned short* mask = nullptr) {
     mclsgpu_context* ctx = net->ctx;
     int rc = set_smem_attributes(ctx);
     if (rc) return rc;
@@ -888,37 +1093,61 @@ int launch_forward(mclsgpu_spai* net, mclsgpu_operator* op, const SlotTable& t, 
     a.slots = t;
     a.n = op->A.n;
     a.mval = mval;
+    a.mdia = mdia;
+    a.mask = mask;
     a.out = out;
+    a.out_align32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
     a.status = ctx->d_status;
     const int ntiles = (op->A.n + kTileRows - 1) / kTileRows;
-    // Up to 4 CTAs per SM (4 x 128 TMEM columns).
-    const int grid = ntiles < ctx->num_sms * 4 ? ntiles : ctx->num_sms * 4;
-    k_spai_forward<<<grid, kThreads, kFwdSmem, ctx->stream>>>(a);
+    const int fit = ctx->num_sms * kFwdCtas;
+    const int grid = ntiles < fit ? ntiles : fit;
+    with_slots(t.K, [&](auto k) {
+        k_spai_forward<decltype(k)::value><<<grid, kThreads, kFwdSmem, ctx->stream>>>(a);
+    });
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(ctx, e, "spai forward launch");
 }
 
-// Scratch for the loss/gradient pass.
+// Scratch of one gradient: sub-arrays of one allocation.
+constexpr size_t kScratchKeep = size_t(256) << 20;
 struct GradScratch {
-    double* mval = nullptr;
-    double* Z = nullptr;
-    double* sq = nullptr;
-    double* wv = nullptr;
-    double* part = nullptr;
-    double* loss = nullptr;
-    float* G = nullptr;
-    void release() {
-        dfree(mval);
-        dfree(Z);
-        dfree(sq);
-        dfree(wv);
-        dfree(part);
-        dfree(loss);
-        dfree(G);
-    }
+    double* mdia;
+    double* Z;
+    double* part;
+    double* wv;
+    float* G;
+    unsigned short* mask;
+    double* loss;         // loss, then the tickets: cleared together
+    unsigned* tickets;
+    size_t clear;         // bytes from loss on
 };
 
+size_t grad_layout(unsigned char* base, int n, int nvec, int K, int blocks, GradScratch* g) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        unsigned char* p = base + at;
+        at += (bytes + 255) & ~size_t(255);
+        return p;
+    };
+    g->mdia = reinterpret_cast<double*>(take(sizeof(double) * n * K));
+    g->Z = reinterpret_cast<double*>(take(sizeof(double) * n * nvec));
+    g->part = reinterpret_cast<double*>(take(sizeof(double) * nvec * blocks));
+    g->wv = reinterpret_cast<double*>(take(sizeof(double) * nvec));
+    g->G = reinterpret_cast<float*>(take(sizeof(float) * n * kO));
+    g->mask = reinterpret_cast<unsigned short*>(take(sizeof(unsigned short) * n));
+    g->clear = sizeof(double) + sizeof(unsigned) * nvec;
+    g->loss = reinterpret_cast<double*>(take(g->clear));
+    g->tickets = reinterpret_cast<unsigned*>(g->loss + 1);
+    return at;
+}
+
 // Zero the gradient, then loss + gradient of the parameters on (op, V).
+//
+// A 32^3 sample with 15 vectors took 0.4 ms in 65 launches (A v and |v|^2 one
+// vector at a time, the loss with one thread per row walking the CSR row
+// twice per vector) and 2 to 22 ms in the seven allocations and releases of
+// each call.  Now: one pass over all vectors, the network's pass (M by
+// diagonals), the loss pass, the backward pass, and scratch that is kept.
 int gradient(mclsgpu_spai* net, mclsgpu_operator* op, const double* V, int nvec, double* loss_out) {
     mclsgpu_context* ctx = net->ctx;
     cudaStream_t s = ctx->stream;
@@ -928,30 +1157,28 @@ int gradient(mclsgpu_spai* net, mclsgpu_operator* op, const double* V, int nvec,
     if (nvec < 1 || nvec > 1024)
         return set_error(ctx, MCLSGPU_ERR_INVALID_ARG, "spai gradient: 1..1024 vectors");
     const int n = op->A.n;
+    const int blocks = grid_for(n, 256, 4 * ctx->num_sms);
     GradScratch g;
-    cudaError_t e;
-    if ((e = dmalloc(&g.mval, size_t(op->A.nnz))) != cudaSuccess ||
-        (e = dmalloc(&g.Z, size_t(n) * nvec)) != cudaSuccess ||
-        (e = dmalloc(&g.sq, size_t(nvec))) != cudaSuccess ||
-        (e = dmalloc(&g.wv, size_t(nvec))) != cudaSuccess ||
-        (e = dmalloc(&g.part, size_t(scan_partials_needed(n)))) != cudaSuccess ||
-        (e = dmalloc(&g.loss, 1)) != cudaSuccess ||
-        (e = dmalloc(&g.G, size_t(n) * kO)) != cudaSuccess) {
-        g.release();
-        return cuda_fail(ctx, e, "cudaMalloc");
-    }
-    cudaMemsetAsync(net->grad, 0, sizeof(float) * kParams, s);
-    cudaMemsetAsync(g.loss, 0, sizeof(double), s);
-    rc = launch_forward(net, op, t, g.mval, nullptr);
-    if (!rc) {
-        for (int v = 0; v < nvec; ++v) {
-            spmv(s, op->A, V + size_t(v) * n, g.Z + size_t(v) * n);
-            sum_sq(s, V + size_t(v) * n, n, g.part, g.sq + v);
+    const size_t bytes = grad_layout(nullptr, n, nvec, t.K, blocks, &g);
+    unsigned char* mem = net->scratch;
+    cudaError_t e = cudaSuccess;
+    if (bytes > net->scratch_bytes) {
+        const bool keep = bytes <= kScratchKeep;
+        if (keep) {
+            dfree(net->scratch);
+            net->scratch_bytes = 0;
         }
-        k_spai_weights<<<1, 1024, 0, s>>>(g.sq, nvec, g.wv);
-        k_spai_loss_grad<<<grid_for(n), 256, 0, s>>>(n, nvec, op->A.rp, op->A.ci, g.mval,
-                                                     op->dia_val, t, V, g.Z, g.wv, net->pen_w,
-                                                     net->pen_c, g.G, g.loss);
+        if ((e = dmalloc(&mem, bytes)) != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
+        if (keep) {
+            net->scratch = mem;
+            net->scratch_bytes = bytes;
+        }
+    }
+    grad_layout(mem, n, nvec, t.K, blocks, &g);
+    cudaMemsetAsync(net->grad, 0, sizeof(float) * kParams, s);
+    cudaMemsetAsync(g.loss, 0, g.clear, s);
+    rc = launch_forward(net, op, t, nullptr, nullptr, g.mdia, g.mask);
+    if (!rc) {
         SpaiBwdArgs b{};
         b.params = net->params;
         b.dia = op->dia_val;
@@ -961,8 +1188,19 @@ int gradient(mclsgpu_spai* net, mclsgpu_operator* op, const double* V, int nvec,
         b.grad = net->grad;
         b.status = ctx->d_status;
         const int ntiles = (n + kTileRows - 1) / kTileRows;
-        const int grid = ntiles < ctx->num_sms ? ntiles : ctx->num_sms;
-        k_spai_backward<<<grid, kThreads, kBwSmem, s>>>(b);
+        const int fit = ctx->num_sms * kBwCtas;
+        const int grid = ntiles < fit ? ntiles : fit;
+        with_slots(t.K, [&](auto k) {
+            constexpr int KT = decltype(k)::value;
+            k_spai_vectors<KT><<<dim3(blocks, nvec), 256, 0, s>>>(
+                n, nvec, op->dia_val, t, V, g.Z, g.part, g.tickets, g.wv);
+            auto loss_grad = net->pen_w > 0.0 ? k_spai_loss_grad<KT, true>
+                                              : k_spai_loss_grad<KT, false>;
+            loss_grad<<<(n + 31) / 32, 32 * kLossGroups, 0, s>>>(
+                n, nvec, g.mdia, g.mask, op->dia_val, t, V, g.Z, g.wv, net->pen_w, net->pen_c,
+                g.G, g.loss);
+            k_spai_backward<KT><<<grid, kThreads, kBwSmem, s>>>(b);
+        });
         e = cudaGetLastError();
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "spai backward launch");
     }
@@ -974,7 +1212,7 @@ int gradient(mclsgpu_spai* net, mclsgpu_operator* op, const double* V, int nvec,
         if (!rc) rc = check_device_status(ctx);
         if (loss_out) *loss_out = l;
     }
-    g.release();
+    if (mem != net->scratch) dfree(mem);
     return rc;
 }
 
@@ -1153,6 +1391,7 @@ int mclsgpu_spai_destroy(mclsgpu_spai* net) {
     dfree(net->grad);
     dfree(net->m);
     dfree(net->v);
+    dfree(net->scratch);
     delete net;
     return MCLSGPU_OK;
 }
