@@ -749,9 +749,8 @@ void anderson_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_de
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
     AndersonWork* w = dom->aa;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
+    mcsa_solve_begin(dom);
     cudaMemsetAsync(w->ticket, 0, sizeof(unsigned int), s);
-    mcsa_reset_counters(dom);
     if (b_dev != dom->b)
         cudaMemcpyAsync(dom->b, b_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     if (x_dev != dom->x)
@@ -800,10 +799,7 @@ int anderson_solve(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
         w->graph_key = key;
         w->graph_hist = dom->d_resid;
     }
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
+    cudaEventRecord(ctx->ev[0], s);
     anderson_begin(dom, b_dev, x_dev, p);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e == cudaSuccess && !w->h_st->done) {
@@ -821,18 +817,16 @@ int anderson_solve(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
     if (e == cudaSuccess) {
         if (x_dev != dom->x)
             cudaMemcpyAsync(x_dev, dom->x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
-        cudaEventRecord(e1, s);
+        cudaEventRecord(ctx->ev[1], s);
         cudaMemcpyAsync(w->h_st, w->st, sizeof(AaState), cudaMemcpyDeviceToHost, s);
+        mcsa_enqueue_report(dom);
         e = cudaStreamSynchronize(s);
     }
     float ms = 0.f;
-    if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "anderson solve");
-    if ((rc = check_device_status(ctx))) return rc;
+    if ((rc = mcsa_finish_report(dom, stats))) return rc;
     if (stats) {
-        if ((rc = mcsa_read_stats(dom, stats))) return rc;
         fill_stats(dom, *w->h_st, ms, stats);
     }
     return MCLSGPU_OK;
@@ -925,11 +919,12 @@ int mclsgpu_anderson_finish(mclsgpu_domain* dom, double* x_dev, mclsgpu_stats* s
     if (x_dev != dom->x)
         cudaMemcpyAsync(x_dev, dom->x, size_t(dom->n) * sizeof(double), cudaMemcpyDeviceToDevice,
                         s);
+    mcsa_enqueue_report(dom);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "anderson finish");
     dom->aa_step_ready = 0;
     if (!stats) return MCLSGPU_OK;
-    int rc = mcsa_read_stats(dom, stats);
+    int rc = mcsa_finish_report(dom, stats);
     if (!rc) fill_stats(dom, *dom->aa->h_st, 0.0, stats);
     return rc;
 }

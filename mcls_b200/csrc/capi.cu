@@ -37,7 +37,10 @@ int check_device_status(mclsgpu_context* ctx) {
                                     cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "device status");
-    const int st = *ctx->h_status;
+    return status_error(ctx, *ctx->h_status);
+}
+
+int status_error(mclsgpu_context* ctx, int st) {
     if (!st) return MCLSGPU_OK;
     cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
     if (st & DEV_ERR_DEGENERATE)
@@ -193,6 +196,10 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->d_resid);
     if (d->h_state) cudaFreeHost(d->h_state);
     d->h_state = nullptr;
+    if (d->h_report) cudaFreeHost(d->h_report);
+    d->h_report = nullptr;
+    if (d->h_stage) cudaFreeHost(d->h_stage);
+    d->h_stage = nullptr;
     if (d->graph) cudaGraphExecDestroy(d->graph);
     d->graph = nullptr;
 }
@@ -234,6 +241,8 @@ int mclsgpu_context_create(int device, mclsgpu_context** out) {
     if (e == cudaSuccess) e = dmalloc(&ctx->d_status, 1);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_status), sizeof(int));
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+    for (cudaEvent_t& ev : ctx->ev)
+        if (e == cudaSuccess) e = cudaEventCreate(&ev);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         delete ctx;
@@ -249,6 +258,8 @@ int mclsgpu_context_destroy(mclsgpu_context* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     dfree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    for (cudaEvent_t ev : ctx->ev)
+        if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MCLSGPU_OK;
@@ -544,7 +555,11 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
             (e = dmalloc(&dom->tmp2, n)) != cudaSuccess || (e = dmalloc(&dom->d_state, 1)) != cudaSuccess ||
             (e = dmalloc(&dom->x2, n)) != cudaSuccess || (e = dmalloc(&dom->rp2, n)) != cudaSuccess ||
             (e = dmalloc(&dom->d_ticket, 1)) != cudaSuccess ||
-            (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_state), sizeof(McsaState))) != cudaSuccess)
+            (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_state), sizeof(McsaState))) != cudaSuccess ||
+            (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_report), sizeof(SolveReport))) != cudaSuccess ||
+            (n <= kStageMax &&
+             (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_stage),
+                                 size_t(n) * sizeof(double))) != cudaSuccess))
             rc = cuda_fail(ctx, e, "cudaMalloc domain buffers");
     }
     if (!rc) {

@@ -35,6 +35,7 @@ struct mclsgpu_context {
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;      // device error word
     int* h_status = nullptr;      // pinned mirror
+    cudaEvent_t ev[2] = {nullptr, nullptr};  // start and end of the solve in progress
     std::string err;
 };
 
@@ -145,6 +146,22 @@ struct RowFinish {
     const int* order = nullptr; // position -> row (null: the identity)
 };
 
+// What the host reads at the end of a solve, written by the device into
+// pinned memory: one synchronisation in place of a copy per item.
+struct SolveReport {
+    McsaState st;
+    double src_sumsq;            // |PL b|^2
+    unsigned long long steps;    // walk steps
+    unsigned long long hist;     // histories
+    unsigned long long walk_ns;  // FP32 walk kernels
+    unsigned long long launches;
+    int status;                  // device error word
+    int pad;
+};
+
+// Host vectors up to this many entries are copied out through pinned memory.
+constexpr int kStageMax = 32768;
+
 }  // namespace mclsgpu
 
 struct mclsgpu_domain {
@@ -215,6 +232,8 @@ struct mclsgpu_domain {
     unsigned int* d_ticket = nullptr;  // last-block ticket of the fused residual
     mclsgpu::McsaState* d_state = nullptr;
     mclsgpu::McsaState* h_state = nullptr;  // pinned
+    mclsgpu::SolveReport* h_report = nullptr;  // pinned, written by the device
+    double* h_stage = nullptr;     // pinned, n doubles (n <= kStageMax, else null)
     cudaGraphExec_t graph = nullptr;
     int graph_key = -1;
     int body_kernels = 0;          // kernel nodes in one MCSA iteration
@@ -252,6 +271,8 @@ namespace mclsgpu {
 int set_error(mclsgpu_context* ctx, int code, const char* fmt, ...);
 int cuda_fail(mclsgpu_context* ctx, cudaError_t e, const char* what);
 int check_device_status(mclsgpu_context* ctx);
+// The error of a device status word (0: none); clears the device's.
+int status_error(mclsgpu_context* ctx, int status);
 // Every device allocation and release of the library goes through dmalloc and
 // dfree; the counters behind mclsgpu_debug_device_allocations count them.
 extern std::atomic<long long> g_device_allocs;
@@ -362,9 +383,9 @@ int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchL
 void prec_residual(mclsgpu_domain* dom, const double* x, const double* b, double* rp_out);
 // y = PL A PR x   (LinearProblem::apply); uses dom->tmp and dom->tmp2.
 void composite_apply(mclsgpu_domain* dom, const double* x, double* y);
-// x2 = x + w r; r2 = PL (b - A PR x2) for r = PL (b - A PR x): one fused pass,
-// from r alone, when PL is I, point Jacobi or held on A's diagonals and there
-// is no PR (x2 != x, r2 != r); x2 may then be null.
+// x2 = x + w r (unless x2 is null); r2 = PL (b - A PR x2) for r = PL (b - A PR x),
+// formed as r - w PL A PR r: one fused pass when PL is I or point Jacobi and
+// there is no PR, two when PL is held on A's diagonals (x2 != x, r2 != r).
 void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, double w,
                          double* x2, double* r2);
 // out = the Monte Carlo estimate for the source v (already left
@@ -382,9 +403,13 @@ inline bool walk_finishes(const mclsgpu_domain* dom) {
     return dom->p.precision == MCLSGPU_FP32 && dom->p.direction == MCLSGPU_FORWARD &&
            !(dom->p.weight_cutoff > 0.0);
 }
-// Walk statistics since the last reset (steps, histories, walk time).
-int mcsa_read_stats(mclsgpu_domain* dom, mclsgpu_stats* st);
-void mcsa_reset_counters(mclsgpu_domain* dom);
+// Clears the device status and the walk statistics (one kernel).
+void mcsa_solve_begin(mclsgpu_domain* dom);
+// Enqueues the end-of-solve report; once the stream is synchronised,
+// mcsa_finish_report returns its device error, if any, and fills the walk
+// statistics (steps, histories, walk time).
+void mcsa_enqueue_report(mclsgpu_domain* dom);
+int mcsa_finish_report(mclsgpu_domain* dom, mclsgpu_stats* st);
 
 // ---- Anderson-accelerated MCSA (anderson.cu) ------------------------------------
 void release_anderson(mclsgpu_domain* dom);

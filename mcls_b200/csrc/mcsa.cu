@@ -26,6 +26,7 @@
 #include <array>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "internal.h"
@@ -213,13 +214,50 @@ __device__ __forceinline__ void add_walk_time(unsigned long long* t) {
     t[1] = 0;
 }
 
+// The words a solve's counters and report live in.
+struct Counters {
+    int* status;
+    unsigned long long* steps;
+    unsigned long long* hist;
+    unsigned long long* tim;
+    const McsaState* st;
+    const double* src_sumsq;
+};
+
+__device__ __forceinline__ void write_report(const Counters& c, SolveReport* r) {
+    SolveReport v;
+    v.st = *c.st;
+    v.src_sumsq = *c.src_sumsq;
+    v.steps = *c.steps;
+    v.hist = *c.hist;
+    v.walk_ns = c.tim[2];
+    v.launches = c.tim[3];
+    v.status = *c.status;
+    v.pad = 0;
+    *r = v;
+}
+
+__global__ void k_report(Counters c, SolveReport* r) { write_report(c, r); }
+
+// Start of a solve: the device error word and the walk statistics cleared.
+__global__ void k_solve_begin(Counters c) {
+    *c.status = 0;
+    *c.steps = 0;
+    *c.hist = 0;
+    c.tim[2] = 0;
+    c.tim[3] = 0;
+}
+
 // End of a Monte Carlo solve: the stream epoch, the history count, the walk
-// timing.
-__global__ void k_mc_end(unsigned long long* epoch, unsigned long long* hist, const int* d_nh,
-                         unsigned long long* tim) {
-    *epoch += 1ULL;
-    *hist += (unsigned long long)(*d_nh);
-    add_walk_time(tim);
+// timing, and the host's report (may be null).
+__global__ void k_mc_end(unsigned long long* epoch, const int* d_nh, Counters c,
+                         SolveReport* report) {
+    const unsigned long long e = *epoch, h = *c.hist;
+    const int nh = *d_nh;
+    *epoch = e + 1ULL;
+    *c.hist = h + (unsigned long long)nh;
+    add_walk_time(c.tim);
+    if (report) write_report(c, report);
 }
 
 // Convergence check of one MCSA iteration (src/MCLS_MCSASolverManager_impl.hpp:380-394).
@@ -393,10 +431,10 @@ __global__ void __launch_bounds__(kFusedThreads) k_precond_norm(Op M, ResidArgs 
     norm_and_check(a, acc);
 }
 
-__global__ void k_mcsa_init(McsaState* st, const double* src_sumsq, double tol, int check_freq,
-                            int max_iters, const double* r_sumsq) {
+__device__ __forceinline__ McsaState initial_state(double src_sumsq, double r_sumsq, double tol,
+                                                  int check_freq, int max_iters) {
     McsaState s{};
-    double sn = sqrt(*src_sumsq);
+    double sn = sqrt(src_sumsq);
     s.pad = 0;
     // Homogeneous case (:312-316)
     double crit_norm = fabs(sn) < 10.0 * 2.220446049250313e-16 ? 1.0 : sn;
@@ -405,9 +443,101 @@ __global__ void k_mcsa_init(McsaState* st, const double* src_sumsq, double tol, 
     s.max_iters = max_iters;
     s.iter = 0;
     s.done = 0;
-    s.rnorm = sqrt(*r_sumsq);
+    s.rnorm = sqrt(r_sumsq);
     s.converged = 0;
-    *st = s;
+    return s;
+}
+
+__global__ void k_mcsa_init(McsaState* st, const double* src_sumsq, double tol, int check_freq,
+                            int max_iters, const double* r_sumsq) {
+    *st = initial_state(*src_sumsq, *r_sumsq, tol, check_freq, max_iters);
+}
+
+// The start of an MCSA solve with no left preconditioner or a diagonal one in
+// one pass: b and x copied to the loop's vectors, rp = PL (b - A x), |PL b|^2
+// and |rp|^2, and (last block) the loop state, the counters and the forward
+// walk's history count.  Apart these were twelve launches and copies, 30 us
+// of a small system's solve.
+struct BeginArgs {
+    const double* b_in;
+    const double* x_in;
+    double* b;
+    double* x;
+    double* rp;
+    const double* dinv;
+    double* part;             // 2 per block
+    unsigned int* ticket;
+    double* sc;               // [0] and [2] forward walk, [5] |rp|^2, [6] |PL b|^2
+    McsaState* st;
+    double tol;
+    int check_freq;
+    int max_iters;
+    int forward_nh;           // > 0: the forward walk's histories
+    int* d_nh;
+    int* d_counter;
+    Counters c;
+};
+
+__device__ __forceinline__ double fused_block_sum(double v, double* sh) {
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < kFusedThreads / 32; ++w) t += sh[w];
+    return t;
+}
+
+template <class Op>
+__global__ void __launch_bounds__(kFusedThreads) k_mcsa_begin(Op A, BeginArgs a) {
+    __shared__ double sh[kFusedThreads / 32];
+    __shared__ bool last;
+    double sb = 0.0, sr = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
+        const double s = A.dot(i, [&](int j) { return a.x_in[j]; });
+        const double bi = a.b_in[i];
+        const double di = a.dinv ? a.dinv[i] : 1.0;
+        const double r = a.dinv ? di * (bi - s) : bi - s;
+        const double pb = a.dinv ? di * bi : bi;
+        a.rp[i] = r;
+        if (a.b != a.b_in) a.b[i] = bi;
+        if (a.x != a.x_in) a.x[i] = a.x_in[i];
+        sb = fma(pb, pb, sb);
+        sr = fma(r, r, sr);
+    }
+    const double tb = fused_block_sum(sb, sh), tr = fused_block_sum(sr, sh);
+    if (threadIdx.x == 0) {
+        a.part[2 * blockIdx.x] = tb;
+        a.part[2 * blockIdx.x + 1] = tr;
+        __threadfence();
+        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double ub = 0.0, ur = 0.0;
+    for (int k = threadIdx.x; k < int(gridDim.x); k += blockDim.x) {
+        ub += __ldcg(&a.part[2 * k]);
+        ur += __ldcg(&a.part[2 * k + 1]);
+    }
+    const double src = fused_block_sum(ub, sh), res = fused_block_sum(ur, sh);
+    if (threadIdx.x != 0) return;
+    *a.ticket = 0u;
+    a.sc[5] = res;
+    a.sc[6] = src;
+    *a.st = initial_state(src, res, a.tol, a.check_freq, a.max_iters);
+    if (a.forward_nh > 0) {
+        *a.d_nh = a.forward_nh;
+        a.sc[0] = 1.0;
+        a.sc[2] = 1.0 / double(a.forward_nh);
+    }
+    *a.d_counter = 0;
+    *a.c.status = 0;
+    *a.c.steps = 0;
+    *a.c.hist = 0;
+    a.c.tim[2] = 0;
+    a.c.tim[3] = 0;
 }
 
 }  // namespace
@@ -551,6 +681,31 @@ void composite_apply(mclsgpu_domain* dom, const double* x, double* y) {
     }
 }
 
+static Counters counters(const mclsgpu_domain* dom) {
+    return Counters{dom->ctx->d_status, dom->d_steps,  dom->d_hist,
+                    dom->d_tim,         dom->d_state, dom->d_scalars + 6};
+}
+
+void mcsa_solve_begin(mclsgpu_domain* dom) {
+    k_solve_begin<<<1, 1, 0, dom->ctx->stream>>>(counters(dom));
+}
+
+void mcsa_enqueue_report(mclsgpu_domain* dom) {
+    k_report<<<1, 1, 0, dom->ctx->stream>>>(counters(dom), dom->h_report);
+}
+
+int mcsa_finish_report(mclsgpu_domain* dom, mclsgpu_stats* st) {
+    const SolveReport& r = *dom->h_report;
+    if (int rc = status_error(dom->ctx, r.status)) return rc;
+    if (st) {
+        st->walk_steps = (int64_t)r.steps;
+        st->histories = (int64_t)r.hist;
+        st->walk_ms = double(r.walk_ns) * 1e-6;
+        st->walk_launches = (int64_t)r.launches;
+    }
+    return MCLSGPU_OK;
+}
+
 // One MC solve of the source vector `v` (device, already left preconditioned
 // when required) into out: out = delta, out + delta or x + w rp + delta
 // (`base`; w the smoother's relaxation).  Walks that finish their rows
@@ -559,7 +714,7 @@ void composite_apply(mclsgpu_domain* dom, const double* x, double* y) {
 // and the walk bookkeeping are done by k_residual_norm.
 static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int base, double w,
                        long long max_trace, long long* tr_states, double* tr_w, int* tr_ev,
-                       long long* tr_start, bool fused = false) {
+                       long long* tr_start, bool fused = false, bool report = false) {
     const mclsgpu_mc_params& p = dom->p;
     const double omega = p.neumann_relaxation;
     const int has_omega = p.neumann_relaxation > 0.0;
@@ -608,66 +763,45 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
         f.out = out;
         k_finalize<<<grid_for(dom->n, 256, 148 * 8), 256, 0, s>>>(f);
     }
-    if (!fused) k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_hist, dom->d_nh, dom->d_tim);
+    if (!fused)
+        k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_nh, counters(dom),
+                                 report ? dom->h_report : nullptr);
 }
 
-static int read_stats(mclsgpu_domain* dom, mclsgpu_stats* st) {
-    if (!st) return MCLSGPU_OK;
-    unsigned long long steps = 0, hist = 0, tim[4] = {0, 0, 0, 0};
-    cudaMemcpyAsync(&steps, dom->d_steps, sizeof(steps), cudaMemcpyDeviceToHost, dom->ctx->stream);
-    cudaMemcpyAsync(&hist, dom->d_hist, sizeof(hist), cudaMemcpyDeviceToHost, dom->ctx->stream);
-    cudaMemcpyAsync(tim, dom->d_tim, sizeof(tim), cudaMemcpyDeviceToHost, dom->ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(dom->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "stats");
-    st->walk_steps = (int64_t)steps;
-    st->histories = (int64_t)hist;
-    st->walk_ms = double(tim[2]) * 1e-6;
-    st->walk_launches = (int64_t)tim[3];
-    return MCLSGPU_OK;
-}
-
-static void reset_counters(mclsgpu_domain* dom) {
-    cudaStream_t s = dom->ctx->stream;
-    cudaMemsetAsync(dom->d_steps, 0, sizeof(unsigned long long), s);
-    cudaMemsetAsync(dom->d_hist, 0, sizeof(unsigned long long), s);
-    cudaMemsetAsync(dom->d_tim + 2, 0, 2 * sizeof(unsigned long long), s);
-}
-
-// MC solve with device vectors.
+// MC solve with device vectors.  host_x (may be null): pinned memory that
+// receives x too.
 static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x_dev, int internal,
                            long long max_trace, long long* tr_states, double* tr_w, int* tr_ev,
-                           long long* tr_start, mclsgpu_stats* stats) {
+                           long long* tr_start, mclsgpu_stats* stats, double* host_x = nullptr) {
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
-    reset_counters(dom);
+    mcsa_solve_begin(dom);
     const double* v = rhs_dev;
     if (dom->left && !internal) {
         spmv(s, dom->left->P, rhs_dev, dom->tmp);
         v = dom->tmp;
     }
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
+    cudaEventRecord(ctx->ev[0], s);
+    // The walk's report is the last word of a solve without right recovery.
     if (dom->right && !internal) {
         // v is rhs_dev or tmp, so tmp2 is free for the unrecovered result.
-        enqueue_mc(dom, v, dom->tmp2, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start);
+        enqueue_mc(dom, v, dom->tmp2, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start,
+                   false, true);
         spmv(s, dom->right->P, dom->tmp2, x_dev);
     } else {
-        enqueue_mc(dom, v, x_dev, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start);
+        enqueue_mc(dom, v, x_dev, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start,
+                   false, true);
     }
-    cudaEventRecord(e1, s);
+    cudaEventRecord(ctx->ev[1], s);
+    if (host_x)
+        cudaMemcpyAsync(host_x, x_dev, size_t(dom->n) * sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mc solve");
-    int rc = check_device_status(ctx);
-    if (rc) return rc;
+    if (int rc = mcsa_finish_report(dom, stats)) return rc;
     if (stats) {
-        if ((rc = read_stats(dom, stats))) return rc;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
         stats->solve_ms = ms;
         stats->iterations = 0;
         stats->converged = 1;
@@ -675,14 +809,16 @@ static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x
     return MCLSGPU_OK;
 }
 
-// x2 = x + w r (rounded as the reference's vector update)
-__global__ void k_axpy_to(const double* x, const double* r, double w, double* x2, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
+// The Richardson step from y = PL A PR r in r2: r2 = r - w y and, when x2 is
+// not null, x2 = x + w r (rounded as the reference's vector update).
+__global__ void k_richardson_step(const double* x, const double* r, double w, double* x2,
+                                  double* r2, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double ri = r[i];
+        r2[i] = ri - w * r2[i];
+        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
+    }
 }
-
-int mcsa_read_stats(mclsgpu_domain* dom, mclsgpu_stats* st) { return read_stats(dom, st); }
-void mcsa_reset_counters(mclsgpu_domain* dom) { reset_counters(dom); }
 
 void mc_correction(mclsgpu_domain* dom, const double* v, double* out) {
     enqueue_mc(dom, v, out, kBaseNone, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
@@ -717,8 +853,8 @@ void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, 
         MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_richardson, dom->tmp, x, r, w,
                          x2, r2);
     } else {
-        k_axpy_to<<<grid, kFusedThreads, 0, s>>>(x, r, w, x2, dom->n);
-        update_prec_residual(dom, x2, dom->b, r2);
+        composite_apply(dom, r, r2);
+        k_richardson_step<<<grid, kFusedThreads, 0, s>>>(x, r, w, x2, r2, dom->n);
     }
 }
 
@@ -732,9 +868,15 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
     if (!fused_iteration(dom, mp)) {
-        for (int l = 0; l < mp->smoother_steps; ++l)
-            enqueue_fixed_point_step(dom, mp->fixed_point_type, mp->richardson_omega);
-        enqueue_mc(dom, dom->rp, dom->x, kBaseOut, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
+        if (mp->smoother_steps == 1 && mp->fixed_point_type == MCLSGPU_FIXED_POINT_RICHARDSON) {
+            richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, nullptr, dom->rp2);
+            enqueue_mc(dom, dom->rp2, dom->x, kBaseSmoothed, mp->richardson_omega, 0, nullptr,
+                       nullptr, nullptr, nullptr);
+        } else {
+            for (int l = 0; l < mp->smoother_steps; ++l)
+                enqueue_fixed_point_step(dom, mp->fixed_point_type, mp->richardson_omega);
+            enqueue_mc(dom, dom->rp, dom->x, kBaseOut, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
+        }
         update_prec_residual(dom, dom->x, dom->b, dom->rp);
         sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
         if (use_cond)
@@ -844,28 +986,74 @@ static int build_mcsa_graph(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp) 
     return MCLSGPU_OK;
 }
 
-static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
-                             const mclsgpu_mcsa_params* mp, mclsgpu_stats* stats) {
+// b, x0, the initial residual, the norms and the loop state; counters cleared.
+// Returns the launches made.
+static int mcsa_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_dev,
+                      const mclsgpu_mcsa_params* mp) {
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
-    reset_counters(dom);
-    // The fused iteration expects a zero work-queue counter and ticket on
-    // entry (it resets both itself at the end of every iteration).
+    const mclsgpu_operator* op = dom->op;
+    const mclsgpu_precond* L = dom->left;
+    const bool forward = dom->p.direction == MCLSGPU_FORWARD;
+    if (fused_iteration(dom, mp) && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI)) {
+        BeginArgs a{};
+        a.b_in = b_dev;
+        a.x_in = x_dev;
+        a.b = dom->b;
+        a.x = dom->x;
+        a.rp = dom->rp;
+        a.dinv = L ? L->diag : nullptr;
+        a.part = dom->part;
+        a.ticket = dom->d_ticket;
+        a.sc = dom->d_scalars;
+        a.st = dom->d_state;
+        a.tol = mp->tolerance;
+        a.check_freq = mp->check_freq;
+        a.max_iters = mp->max_iters;
+        const int per = dom->p.sample_ratio > 0.0 ? int(std::ceil(dom->p.sample_ratio)) : 1;
+        a.forward_nh = forward ? n * per : 0;
+        a.d_nh = dom->d_nh;
+        a.d_counter = dom->d_counter;
+        a.c = counters(dom);
+        // Two partial sums per block in dom->part, sized for 8 blocks per SM.
+        const int grid = grid_for(n, kFusedThreads, ctx->num_sms * 4);
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_mcsa_begin, a);
+        return 1;
+    }
+    mcsa_solve_begin(dom);
+    // The fused iteration expects a zero work-queue counter on entry (it
+    // resets it itself at the end of every iteration).
     cudaMemsetAsync(dom->d_counter, 0, sizeof(int), s);
-    cudaMemsetAsync(dom->d_ticket, 0, sizeof(unsigned int), s);
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
+    if (b_dev != dom->b)
+        cudaMemcpyAsync(dom->b, b_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    if (x_dev != dom->x)
+        cudaMemcpyAsync(dom->x, x_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    // Source norm |PL b|_2 (:299-318) and the initial preconditioned residual.
+    const double* pb = dom->b;
+    if (L) {
+        spmv(s, L->P, dom->b, dom->tmp);
+        pb = dom->tmp;
+    }
+    sum_sq(s, pb, n, dom->part, dom->d_scalars + 6);
+    update_prec_residual(dom, dom->x, dom->b, dom->rp);
+    sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
+    k_mcsa_init<<<1, 1, 0, s>>>(dom->d_state, dom->d_scalars + 6, mp->tolerance, mp->check_freq,
+                                mp->max_iters, dom->d_scalars + 5);
+    if (fused_iteration(dom, mp) && forward) launch_forward_setup(dom);
+    return 10;
+}
+
+static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
+                             const mclsgpu_mcsa_params* mp, mclsgpu_stats* stats,
+                             double* host_x = nullptr) {
+    mclsgpu_context* ctx = dom->ctx;
+    cudaStream_t s = ctx->stream;
+    const int n = dom->n;
     if (mp->max_iters > dom->resid_cap) {
         dfree(dom->d_resid);
         cudaError_t e = dmalloc(&dom->d_resid, size_t(mp->max_iters));
-        if (e != cudaSuccess) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            return cuda_fail(ctx, e, "cudaMalloc");
-        }
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
         dom->resid_cap = mp->max_iters;
         if (dom->graph) {
             cudaGraphExecDestroy(dom->graph);
@@ -875,39 +1063,15 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
     // Graph key: everything baked into the captured iteration.
     const int key = (mp->smoother_steps * 1000003 ^ int(mp->richardson_omega * 1e6)) * 4 +
                     mp->fixed_point_type;
-    if (int rc = prepare_fixed_point(dom, mp->fixed_point_type)) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return rc;
-    }
+    if (int rc = prepare_fixed_point(dom, mp->fixed_point_type)) return rc;
     // Variable-length reference-stream walks synchronise with the host.
     const bool host_loop = mp->host_loop || walk_needs_rounds(dom);
     if (!host_loop && (!dom->graph || dom->graph_key != key)) {
-        int rc = build_mcsa_graph(dom, mp);
-        if (rc) {
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            return rc;
-        }
+        if (int rc = build_mcsa_graph(dom, mp)) return rc;
         dom->graph_key = key;
     }
-    cudaEventRecord(e0, s);
-    if (b_dev != dom->b)
-        cudaMemcpyAsync(dom->b, b_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    if (x_dev != dom->x)
-        cudaMemcpyAsync(dom->x, x_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    // Source norm |PL b|_2 (:299-318) and the initial preconditioned residual.
-    const double* pb = dom->b;
-    if (dom->left) {
-        spmv(s, dom->left->P, dom->b, dom->tmp);
-        pb = dom->tmp;
-    }
-    sum_sq(s, pb, n, dom->part, dom->d_scalars + 6);
-    update_prec_residual(dom, dom->x, dom->b, dom->rp);
-    sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
-    k_mcsa_init<<<1, 1, 0, s>>>(dom->d_state, dom->d_scalars + 6, mp->tolerance, mp->check_freq,
-                                mp->max_iters, dom->d_scalars + 5);
-    if (fused_iteration(dom, mp) && dom->p.direction == MCLSGPU_FORWARD) launch_forward_setup(dom);
+    cudaEventRecord(ctx->ev[0], s);
+    const int setup = mcsa_begin(dom, b_dev, x_dev, mp);
     cudaError_t e = cudaSuccess;
     if (!host_loop) {
         e = cudaGraphLaunch(dom->graph, s);
@@ -920,28 +1084,25 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
             if (e == cudaSuccess && dom->h_state->done) break;
         }
     }
-    cudaEventRecord(e1, s);
+    cudaEventRecord(ctx->ev[1], s);
     if (e == cudaSuccess) {
         // Right preconditioner recovery (:410-418).
+        const double* xr = dom->x;
         if (dom->right) {
             spmv(s, dom->right->P, dom->x, dom->tmp);
-            cudaMemcpyAsync(x_dev, dom->tmp, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
-        } else if (x_dev != dom->x) {
-            cudaMemcpyAsync(x_dev, dom->x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+            xr = dom->tmp;
         }
-        cudaMemcpyAsync(dom->h_state, dom->d_state, sizeof(McsaState), cudaMemcpyDeviceToHost, s);
+        const size_t bytes = size_t(n) * sizeof(double);
+        if (x_dev != xr) cudaMemcpyAsync(x_dev, xr, bytes, cudaMemcpyDeviceToDevice, s);
+        if (host_x) cudaMemcpyAsync(host_x, xr, bytes, cudaMemcpyDeviceToHost, s);
+        mcsa_enqueue_report(dom);
         e = cudaStreamSynchronize(s);
     }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa graph");
-    int rc = check_device_status(ctx);
-    if (rc) return rc;
-    double src_sumsq = 0.0;
-    cudaMemcpy(&src_sumsq, dom->d_scalars + 6, sizeof(double), cudaMemcpyDeviceToHost);
-    const McsaState st = *dom->h_state;
+    if (int rc = mcsa_finish_report(dom, stats)) return rc;
+    const double src_sumsq = dom->h_report->src_sumsq;
+    const McsaState st = dom->h_report->st;
     if (mp->verbose) {
         std::vector<double> hist(st.iter < dom->resid_cap ? st.iter : dom->resid_cap);
         if (!hist.empty())
@@ -959,7 +1120,8 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
         std::printf("\n**************************************************\n\n");
     }
     if (stats) {
-        if ((rc = read_stats(dom, stats))) return rc;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
         stats->iterations = st.iter;
         stats->converged = st.converged;
         stats->residual_norm = st.rnorm;
@@ -967,9 +1129,9 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
         stats->achieved_tol = sn > 0.0 ? st.rnorm / sn : st.rnorm;  // achievedTol (:142-173)
         stats->solve_ms = ms;
         stats->fallback_taken = dom->left ? dom->left->fallback : 0;
-        // kernels of the captured iterations plus the set-up launches
-        // (source norm, initial residual and norm, state init)
-        stats->kernel_launches = int64_t(dom->body_kernels) * st.iter + 9;
+        // kernels of the captured iterations plus the set-up launches and the
+        // report
+        stats->kernel_launches = int64_t(dom->body_kernels) * st.iter + setup + 1;
         stats->rho = dom->left ? dom->left->rho : -1.0;
     }
     return MCLSGPU_OK;
@@ -983,8 +1145,7 @@ void mcsa_loop_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_d
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
-    reset_counters(dom);
+    mcsa_solve_begin(dom);
     if (b_dev != dom->b)
         cudaMemcpyAsync(dom->b, b_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     if (x_dev != dom->x)
@@ -1025,16 +1186,13 @@ int mcsa_loop_finish(mclsgpu_domain* dom, double* x_dev, float ms, int kernels_p
     } else if (x_dev != dom->x) {
         cudaMemcpyAsync(x_dev, dom->x, bytes, cudaMemcpyDeviceToDevice, s);
     }
-    cudaMemcpyAsync(dom->h_state, dom->d_state, sizeof(McsaState), cudaMemcpyDeviceToHost, s);
-    double src_sumsq = 0.0;
-    cudaMemcpyAsync(&src_sumsq, dom->d_scalars + 6, sizeof(double), cudaMemcpyDeviceToHost, s);
+    mcsa_enqueue_report(dom);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa loop");
-    int rc = check_device_status(ctx);
-    if (rc) return rc;
-    const McsaState st = *dom->h_state;
+    if (int rc = mcsa_finish_report(dom, stats)) return rc;
+    const McsaState st = dom->h_report->st;
+    const double src_sumsq = dom->h_report->src_sumsq;
     if (stats) {
-        if ((rc = read_stats(dom, stats))) return rc;
         stats->iterations = st.iter;
         stats->converged = st.converged;
         stats->residual_norm = st.rnorm;
@@ -1102,8 +1260,12 @@ int mclsgpu_mc_solve(mclsgpu_domain* dom, const double* rhs, double* x, int inte
     const size_t bytes = size_t(dom->n) * sizeof(double);
     cudaMemcpyAsync(dom->b, rhs, bytes, cudaMemcpyHostToDevice, s);
     int rc = mc_solve_device(dom, dom->b, dom->x, internal, 0, nullptr, nullptr, nullptr, nullptr,
-                             stats);
+                             stats, dom->h_stage);
     if (rc) return rc;
+    if (dom->h_stage) {
+        std::memcpy(x, dom->h_stage, bytes);
+        return MCLSGPU_OK;
+    }
     cudaError_t e = cudaMemcpyAsync(x, dom->x, bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(dom->ctx, e, "mc_solve copy-out");
@@ -1180,9 +1342,8 @@ int mclsgpu_mcsa_begin(mclsgpu_domain* dom, const double* b_dev, const double* x
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
     if ((rc = prepare_fixed_point(dom, p.fixed_point_type))) return rc;
-    cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
+    mcsa_solve_begin(dom);
     cudaMemsetAsync(dom->d_ticket, 0, sizeof(unsigned int), s);
-    reset_counters(dom);
     if (b_dev != dom->b) cudaMemcpyAsync(dom->b, b_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     if (x0_dev != dom->x) cudaMemcpyAsync(dom->x, x0_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     // |PL b|_2 and the initial preconditioned residual
@@ -1258,10 +1419,11 @@ int mclsgpu_mcsa_finish(mclsgpu_domain* dom, double* x_dev, mclsgpu_stats* stats
     } else if (x_dev != dom->x) {
         cudaMemcpyAsync(x_dev, dom->x, bytes, cudaMemcpyDeviceToDevice, s);
     }
+    mcsa_enqueue_report(dom);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa finish");
     dom->step_ready = 0;
-    return stats ? read_stats(dom, stats) : MCLSGPU_OK;
+    return stats ? mcsa_finish_report(dom, stats) : MCLSGPU_OK;
 }
 
 int mclsgpu_domain_residual(mclsgpu_domain* dom, double* rp_dev) {
@@ -1367,8 +1529,12 @@ int mclsgpu_mcsa_solve(mclsgpu_domain* dom, const double* b, double* x,
     const size_t bytes = size_t(dom->n) * sizeof(double);
     cudaMemcpyAsync(dom->b, b, bytes, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dom->x, x, bytes, cudaMemcpyHostToDevice, s);
-    rc = mcsa_solve_device(dom, dom->b, dom->x, &p, stats);
+    rc = mcsa_solve_device(dom, dom->b, dom->x, &p, stats, dom->h_stage);
     if (rc) return rc;
+    if (dom->h_stage) {
+        std::memcpy(x, dom->h_stage, bytes);
+        return MCLSGPU_OK;
+    }
     cudaError_t e = cudaMemcpyAsync(x, dom->x, bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(dom->ctx, e, "mcsa copy-out");
