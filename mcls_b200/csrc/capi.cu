@@ -158,7 +158,6 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->rec);
     dfree(d->walk_order);
     dfree(d->d_jump);
-    dfree(d->d_pos);
     dfree(d->hoff);
     dfree(d->hlen);
     dfree(d->hoff2);
@@ -166,22 +165,13 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->delta);
     if (d->set_graph) cudaGraphExecDestroy(d->set_graph);
     d->set_graph = nullptr;
-    dfree(d->d_epoch);
-    dfree(d->src);
     dfree(d->scdf);
     dfree(d->guide);
     dfree(d->counts);
-    dfree(d->offs);
     dfree(d->start);
     dfree(d->y64);
-    dfree(d->c32);
+    dfree(d->words);
     dfree(d->c64);
-    dfree(d->d_nh);
-    dfree(d->d_counter);
-    dfree(d->d_scalars);
-    dfree(d->d_steps);
-    dfree(d->d_tim);
-    dfree(d->d_hist);
     dfree(d->part);
     dfree(d->ipart);
     dfree(d->x);
@@ -191,15 +181,7 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->tmp2);
     dfree(d->x2);
     dfree(d->rp2);
-    dfree(d->d_ticket);
-    dfree(d->d_state);
     dfree(d->d_resid);
-    if (d->h_state) cudaFreeHost(d->h_state);
-    d->h_state = nullptr;
-    if (d->h_report) cudaFreeHost(d->h_report);
-    d->h_report = nullptr;
-    if (d->h_stage) cudaFreeHost(d->h_stage);
-    d->h_stage = nullptr;
     if (d->graph) cudaGraphExecDestroy(d->graph);
     d->graph = nullptr;
 }
@@ -238,8 +220,12 @@ int mclsgpu_context_create(int device, mclsgpu_context** out) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = dmalloc(&ctx->d_status, 1);
+    if (e == cudaSuccess) e = dmalloc(&ctx->d_status, 2);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_status), sizeof(int));
+    if (e == cudaSuccess)
+        e = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_report),
+                           sizeof(SolveReport) + kStageMax * sizeof(double));
+    if (e == cudaSuccess) ctx->h_stage = reinterpret_cast<double*>(ctx->h_report + 1);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
     for (cudaEvent_t& ev : ctx->ev)
         if (e == cudaSuccess) e = cudaEventCreate(&ev);
@@ -258,6 +244,7 @@ int mclsgpu_context_destroy(mclsgpu_context* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     dfree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->h_report) cudaFreeHost(ctx->h_report);
     for (cudaEvent_t ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -538,39 +525,41 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
     const int scan_parts = scan_partials_needed(n);
     const int parts = (scan_parts > fused_blocks ? scan_parts : fused_blocks) + 8;
     if (!rc) {
-        if ((e = dmalloc(&dom->src, n)) != cudaSuccess || (e = dmalloc(&dom->scdf, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->guide, n)) != cudaSuccess || (e = dmalloc(&dom->counts, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->offs, n)) != cudaSuccess ||
+        if ((e = dmalloc(&dom->scdf, n)) != cudaSuccess ||
+            (e = dmalloc(&dom->guide, size_t(n) / 16 + 2)) != cudaSuccess ||
+            (e = dmalloc(&dom->counts, n)) != cudaSuccess ||
             (e = dmalloc(&dom->start, size_t(dom->nh_cap) + 1)) != cudaSuccess ||
-            (e = dmalloc(&dom->y64, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->c32, n)) != cudaSuccess || (e = dmalloc(&dom->c64, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_nh, 1)) != cudaSuccess || (e = dmalloc(&dom->d_counter, 1)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_scalars, 16)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_steps, 1)) != cudaSuccess || (e = dmalloc(&dom->d_hist, 1)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_tim, 4)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_pos, 1)) != cudaSuccess || (e = dmalloc(&dom->d_epoch, 1)) != cudaSuccess ||
+            (e = dmalloc(&dom->y64, n)) != cudaSuccess || (e = dmalloc(&dom->c64, n)) != cudaSuccess ||
+            (e = dmalloc(&dom->words, kWordBytes)) != cudaSuccess ||
             (e = dmalloc(&dom->part, parts)) != cudaSuccess || (e = dmalloc(&dom->ipart, parts)) != cudaSuccess ||
             (e = dmalloc(&dom->x, n)) != cudaSuccess || (e = dmalloc(&dom->b, n)) != cudaSuccess ||
             (e = dmalloc(&dom->rp, n)) != cudaSuccess || (e = dmalloc(&dom->tmp, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->tmp2, n)) != cudaSuccess || (e = dmalloc(&dom->d_state, 1)) != cudaSuccess ||
-            (e = dmalloc(&dom->x2, n)) != cudaSuccess || (e = dmalloc(&dom->rp2, n)) != cudaSuccess ||
-            (e = dmalloc(&dom->d_ticket, 1)) != cudaSuccess ||
-            (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_state), sizeof(McsaState))) != cudaSuccess ||
-            (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_report), sizeof(SolveReport))) != cudaSuccess ||
-            (n <= kStageMax &&
-             (e = cudaMallocHost(reinterpret_cast<void**>(&dom->h_stage),
-                                 size_t(n) * sizeof(double))) != cudaSuccess))
+            (e = dmalloc(&dom->tmp2, n)) != cudaSuccess ||
+            (e = dmalloc(&dom->x2, n)) != cudaSuccess || (e = dmalloc(&dom->rp2, n)) != cudaSuccess)
             rc = cuda_fail(ctx, e, "cudaMalloc domain buffers");
     }
     if (!rc) {
+        // The solve's counters and scalars share one allocation.
+        unsigned char* w = dom->words;
+        auto take = [&](auto*& p, size_t count) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(w);
+            w += (count * sizeof(*p) + 31) & ~size_t(31);
+        };
+        take(dom->d_scalars, 16);
+        take(dom->d_state, 1);
+        take(dom->d_tim, 4);
+        take(dom->d_nh, 1);
+        take(dom->d_counter, 1);
+        take(dom->d_steps, 1);
+        take(dom->d_hist, 1);
+        take(dom->d_pos, 1);
+        take(dom->d_epoch, 1);
+        take(dom->d_ticket, 1);
+        dom->h_state = &ctx->h_report->st;
+    }
+    if (!rc) {
         dom->part_cap = parts;
-        cudaMemsetAsync(dom->d_pos, 0, sizeof(unsigned long long), ctx->stream);
-        cudaMemsetAsync(dom->d_epoch, 0, sizeof(unsigned long long), ctx->stream);
-        cudaMemsetAsync(dom->d_steps, 0, sizeof(unsigned long long), ctx->stream);
-        cudaMemsetAsync(dom->d_hist, 0, sizeof(unsigned long long), ctx->stream);
-        cudaMemsetAsync(dom->d_ticket, 0, sizeof(unsigned int), ctx->stream);
-        cudaMemsetAsync(dom->d_counter, 0, sizeof(int), ctx->stream);
-        cudaMemsetAsync(dom->d_scalars, 0, 16 * sizeof(double), ctx->stream);
+        cudaMemsetAsync(dom->words, 0, kWordBytes, ctx->stream);
         const unsigned long long tim0[4] = {~0ULL, 0ULL, 0ULL, 0ULL};
         cudaMemcpyAsync(dom->d_tim, tim0, sizeof(tim0), cudaMemcpyHostToDevice, ctx->stream);
         cudaStreamSynchronize(ctx->stream);

@@ -279,14 +279,12 @@ int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
     if ((e = dmalloc(&D.ci, tot + 1)) != cudaSuccess || (e = dmalloc(&D.v, tot + 1)) != cudaSuccess ||
         (e = dmalloc(&dom->cdf, tot + 1)) != cudaSuccess || (e = dmalloc(&dom->w, n + 1)) != cudaSuccess)
         return cuda_fail(ctx, e, "cudaMalloc");
-    int* d_neg = nullptr;
-    if ((e = dmalloc(&d_neg, 1)) != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
+    int* d_neg = ctx->d_status + 1;
     cudaMemsetAsync(d_neg, 0, sizeof(int), s);
     k_domain_fill<<<grid_for(n), 256, 0, s>>>(M.rp, M.ci, M.v, n, row0, relax, D.rp, D.ci, D.v,
                                               dom->cdf, dom->w, ctx->d_status, d_neg);
     cudaMemcpyAsync(&dom->neg_h, d_neg, sizeof(int), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
-    dfree(d_neg);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "domain fill");
     if ((rc = check_device_status(ctx))) return rc;
 

@@ -244,7 +244,6 @@ struct Scratch {
         dfree(d.d_scalars);
         dfree(d.d_state);
         dfree(d.d_resid);
-        if (d.h_state) cudaFreeHost(d.h_state);
     }
     cudaError_t alloc(int n, int parts, int hist) {
         cudaError_t e;
@@ -258,7 +257,7 @@ struct Scratch {
             (e = dmalloc(&d.d_resid, size_t(hist))) != cudaSuccess)
             return e;
         d.resid_cap = hist;
-        return cudaMallocHost(reinterpret_cast<void**>(&d.h_state), sizeof(McsaState));
+        return cudaSuccess;
     }
 };
 
@@ -274,6 +273,7 @@ int fixed_point_solve(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_precon
     d.left = left;
     d.right = right;
     d.n = n;
+    d.h_state = &ctx->h_report->st;
     const int parts = 2 * ctx->num_sms * 8 + 8;
     d.part_cap = parts;
     cudaError_t e = sc.alloc(n, parts, mp->max_iters);

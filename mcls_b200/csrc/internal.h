@@ -27,14 +27,47 @@ struct Status {
     std::string msg;
 };
 
+struct McsaState {
+    int iter;            // iterations completed
+    int done;            // 1 once the loop must stop
+    int check_freq;
+    int max_iters;
+    double crit;         // tolerance * |PL b|
+    double rnorm;        // last |rp|_2
+    int converged;
+    int pad;
+};
+
+// What the host reads at the end of a solve, written by the device into
+// pinned memory: one synchronisation in place of a copy per item.
+struct SolveReport {
+    McsaState st;
+    double src_sumsq;            // |PL b|^2
+    unsigned long long steps;    // walk steps
+    unsigned long long hist;     // histories
+    unsigned long long walk_ns;  // FP32 walk kernels
+    unsigned long long launches;
+    int status;                  // device error word
+    int pad;
+};
+
+// Host vectors up to this many entries are copied out through pinned memory.
+constexpr int kStageMax = 32768;
+constexpr size_t kWordBytes = 1024;  // a domain's counters and scalars
+
 }  // namespace mclsgpu
 
 struct mclsgpu_context {
     int device = 0;
     int num_sms = 148;
     cudaStream_t stream = nullptr;
-    int* d_status = nullptr;      // device error word
+    int* d_status = nullptr;      // device error word; [1]: domain set-up flag
     int* h_status = nullptr;      // pinned mirror
+    // Pinned: the report of the solve in progress (calls on a context are
+    // serialised), written by the device, and kStageMax doubles for small host
+    // vectors.
+    mclsgpu::SolveReport* h_report = nullptr;
+    double* h_stage = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};  // start and end of the solve in progress
     std::string err;
 };
@@ -103,17 +136,6 @@ namespace mclsgpu {
 
 struct AndersonWork;
 
-struct McsaState {
-    int iter;            // iterations completed
-    int done;            // 1 once the loop must stop
-    int check_freq;
-    int max_iters;
-    double crit;         // tolerance * |PL b|
-    double rnorm;        // last |rp|_2
-    int converged;
-    int pad;
-};
-
 // Order in which the forward walk's threads take the rows of a domain on a
 // structured grid (X fastest, then Y, then Z): bricks of bx x by x bz rows, the
 // last ones narrower, x fastest inside a brick; bricks follow each other along
@@ -146,21 +168,6 @@ struct RowFinish {
     const int* order = nullptr; // position -> row (null: the identity)
 };
 
-// What the host reads at the end of a solve, written by the device into
-// pinned memory: one synchronisation in place of a copy per item.
-struct SolveReport {
-    McsaState st;
-    double src_sumsq;            // |PL b|^2
-    unsigned long long steps;    // walk steps
-    unsigned long long hist;     // histories
-    unsigned long long walk_ns;  // FP32 walk kernels
-    unsigned long long launches;
-    int status;                  // device error word
-    int pad;
-};
-
-// Host vectors up to this many entries are copied out through pinned memory.
-constexpr int kStageMax = 32768;
 
 }  // namespace mclsgpu
 
@@ -204,15 +211,13 @@ struct mclsgpu_domain {
     unsigned long long* d_pos = nullptr;  // reference mode: draws consumed
     // Source / tally work buffers.
     int64_t nh_cap = 0;
-    double* src = nullptr;         // scaled source vector (n)
     double* scdf = nullptr;        // source CDF (n)
-    int* guide = nullptr;          // guide table (n)
+    int* guide = nullptr;          // guide table (n / 16 + 2 at most)
     int* counts = nullptr;         // histories per state (n)
-    int* offs = nullptr;           // emission offsets (n)
     int* start = nullptr;          // start state | sign<<31 per history
     double* y64 = nullptr;         // tallies, reduced in FP64 (n)
-    float* c32 = nullptr;          // forward: FP32 tally source (n)
     double* c64 = nullptr;         // forward: FP64 tally source (n)
+    unsigned char* words = nullptr;  // the allocation behind the counters below
     int* d_nh = nullptr;           // histories of the current solve
     int* d_counter = nullptr;      // walk work-queue counter
     double* d_scalars = nullptr;   // [0] |src|_1, [1] cdf total, [2] 1/nh ...
@@ -231,9 +236,7 @@ struct mclsgpu_domain {
     double* rp2 = nullptr;         // fused iteration: residual after smoothing
     unsigned int* d_ticket = nullptr;  // last-block ticket of the fused residual
     mclsgpu::McsaState* d_state = nullptr;
-    mclsgpu::McsaState* h_state = nullptr;  // pinned
-    mclsgpu::SolveReport* h_report = nullptr;  // pinned, written by the device
-    double* h_stage = nullptr;     // pinned, n doubles (n <= kStageMax, else null)
+    mclsgpu::McsaState* h_state = nullptr;  // pinned (the context's report)
     cudaGraphExec_t graph = nullptr;
     int graph_key = -1;
     int body_kernels = 0;          // kernel nodes in one MCSA iteration
@@ -477,20 +480,13 @@ void launch_walk_part(const PartWalk& p, mclsgpu_context* ctx);
 
 // ---- scans and reductions (scan.cu) ------------------------------------------
 int scan_partials_needed(int n);
-// Deterministic FP64 sum of |v[i]*scale| (scale applied when has_scale).
-void abs_sum(cudaStream_t s, const double* v, int n, double scale,
-             int has_scale, double* part, double* out);
-// Source CDF: c[0] = v[0]*sc, c[i] = c[i-1] + |v[i]*sc|, then c /= c[n-1];
-// writes total to *total.  sequential != 0 reproduces the reference's
-// left-to-right order in one thread.
-void source_cdf(cudaStream_t s, const double* v, int n, double scale,
-                int has_scale, int sequential, double* part, double* cdf,
-                double* total);
-// Exclusive suffix sum: out[i] = sum_{j>i} in[j]; *total = sum.
-void suffix_scan_int(cudaStream_t s, const int* in, int n, int* part,
-                     int* out, int* total);
-// Inclusive max-scan in place (guide table).
-void max_scan_int(cudaStream_t s, int* a, int n, int* part);
+// The reference's left-to-right sums (one thread): |v*scale|_1 into *norm1 (the
+// scale applied when has_scale), and the source CDF c[0] = v[0]*sc, c[i] =
+// c[i-1] + |v[i]*sc|, then c /= c[n-1], its unnormalised end into *total.
+void source_sequential(cudaStream_t s, const double* v, int n, double scale, int has_scale,
+                       double* norm1, double* cdf, double* total);
+void abs_sum_sequential(cudaStream_t s, const double* v, int n, double scale, int has_scale,
+                        double* norm1);
 // Sum of squares (deterministic).
 void sum_sq(cudaStream_t s, const double* v, int n, double* part,
             double* out);

@@ -691,11 +691,11 @@ void mcsa_solve_begin(mclsgpu_domain* dom) {
 }
 
 void mcsa_enqueue_report(mclsgpu_domain* dom) {
-    k_report<<<1, 1, 0, dom->ctx->stream>>>(counters(dom), dom->h_report);
+    k_report<<<1, 1, 0, dom->ctx->stream>>>(counters(dom), dom->ctx->h_report);
 }
 
 int mcsa_finish_report(mclsgpu_domain* dom, mclsgpu_stats* st) {
-    const SolveReport& r = *dom->h_report;
+    const SolveReport& r = *dom->ctx->h_report;
     if (int rc = status_error(dom->ctx, r.status)) return rc;
     if (st) {
         st->walk_steps = (int64_t)r.steps;
@@ -765,7 +765,7 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
     }
     if (!fused)
         k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_nh, counters(dom),
-                                 report ? dom->h_report : nullptr);
+                                 report ? dom->ctx->h_report : nullptr);
 }
 
 // MC solve with device vectors.  host_x (may be null): pinned memory that
@@ -1101,8 +1101,8 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa graph");
     if (int rc = mcsa_finish_report(dom, stats)) return rc;
-    const double src_sumsq = dom->h_report->src_sumsq;
-    const McsaState st = dom->h_report->st;
+    const double src_sumsq = dom->ctx->h_report->src_sumsq;
+    const McsaState st = dom->ctx->h_report->st;
     if (mp->verbose) {
         std::vector<double> hist(st.iter < dom->resid_cap ? st.iter : dom->resid_cap);
         if (!hist.empty())
@@ -1190,8 +1190,8 @@ int mcsa_loop_finish(mclsgpu_domain* dom, double* x_dev, float ms, int kernels_p
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa loop");
     if (int rc = mcsa_finish_report(dom, stats)) return rc;
-    const McsaState st = dom->h_report->st;
-    const double src_sumsq = dom->h_report->src_sumsq;
+    const McsaState st = dom->ctx->h_report->st;
+    const double src_sumsq = dom->ctx->h_report->src_sumsq;
     if (stats) {
         stats->iterations = st.iter;
         stats->converged = st.converged;
@@ -1259,11 +1259,12 @@ int mclsgpu_mc_solve(mclsgpu_domain* dom, const double* rhs, double* x, int inte
     cudaStream_t s = dom->ctx->stream;
     const size_t bytes = size_t(dom->n) * sizeof(double);
     cudaMemcpyAsync(dom->b, rhs, bytes, cudaMemcpyHostToDevice, s);
+    double* stage = dom->n <= kStageMax ? dom->ctx->h_stage : nullptr;
     int rc = mc_solve_device(dom, dom->b, dom->x, internal, 0, nullptr, nullptr, nullptr, nullptr,
-                             stats, dom->h_stage);
+                             stats, stage);
     if (rc) return rc;
-    if (dom->h_stage) {
-        std::memcpy(x, dom->h_stage, bytes);
+    if (stage) {
+        std::memcpy(x, stage, bytes);
         return MCLSGPU_OK;
     }
     cudaError_t e = cudaMemcpyAsync(x, dom->x, bytes, cudaMemcpyDeviceToHost, s);
@@ -1529,10 +1530,11 @@ int mclsgpu_mcsa_solve(mclsgpu_domain* dom, const double* b, double* x,
     const size_t bytes = size_t(dom->n) * sizeof(double);
     cudaMemcpyAsync(dom->b, b, bytes, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dom->x, x, bytes, cudaMemcpyHostToDevice, s);
-    rc = mcsa_solve_device(dom, dom->b, dom->x, &p, stats, dom->h_stage);
+    double* stage = dom->n <= kStageMax ? dom->ctx->h_stage : nullptr;
+    rc = mcsa_solve_device(dom, dom->b, dom->x, &p, stats, stage);
     if (rc) return rc;
-    if (dom->h_stage) {
-        std::memcpy(x, dom->h_stage, bytes);
+    if (stage) {
+        std::memcpy(x, stage, bytes);
         return MCLSGPU_OK;
     }
     cudaError_t e = cudaMemcpyAsync(x, dom->x, bytes, cudaMemcpyDeviceToHost, s);

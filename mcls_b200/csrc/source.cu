@@ -11,20 +11,31 @@
 // Forward (UniformForwardSource, src/MCLS_UniformForwardSource_impl.hpp:60-148):
 //   ceil(Sample Ratio) histories per state in state order, weight 1.
 //
-// Sampling uses a guide table over the FP64 CDF: guide[t] is the first state
-// whose floor(cdf*G) reaches t, so the lower_bound of u lies in
-// [guide[t], guide[t+1]] with t = floor(u*G); a short binary search in that
-// window returns exactly std::lower_bound's answer.
+// Sampling uses a guide table over the FP64 CDF, one entry per 16 states:
+// guide[t] is the first state whose cdf*G reaches t, so the lower_bound of u
+// lies in [guide[t], guide[t+1]] with t = floor(u*G); a short binary search in
+// that window returns std::lower_bound's answer.
+//
+// The random adjoint source of a large system is five launches: tile sums and
+// the history count, CDF and guide, draws, tile counts, emission.  Apart (a
+// reduction, a scan of its partials and a copy for each sum, memsets, a
+// separate normalisation, guide marks and a maximum scan) they were nineteen,
+// 80 of the 107 us of an MCSA iteration at 64^3.
 #include <cfloat>
 #include <climits>
+
+#include <cooperative_groups.h>
 
 #include <mutex>
 
 #include "internal.h"
 #include "rng.cuh"
+#include "scan.cuh"
 
 namespace mclsgpu {
 namespace {
+
+using namespace scan;
 
 inline int grid_for(long long work, int threads = 256, int cap = 148 * 16) {
     long long g = (work + threads - 1) / threads;
@@ -36,61 +47,228 @@ __device__ __forceinline__ double load_src(const double* v, int i, double omega,
     return has ? v[i] * omega : v[i];
 }
 
-// nh = int(Nh_total * cdf.back() / norm1)  (:198); weight = norm1 (:67)
-__global__ void k_random_count(int nh_req, double* sc, int* d_nh, int cap, int* status) {
-    const double norm1 = sc[0], total = sc[1];
+// The history count nh = int(Nh_total * cdf.back() / norm1)  (:198); *error is
+// set when the source sums are not finite or, since total <= norm1 in exact
+// arithmetic and so nh <= nh_req <= cap, have lost all precision (a diverging
+// iteration).  A zero source (an exact iterate) gets no histories.
+__device__ __forceinline__ int history_count(int nh_req, double norm1, double total, int cap,
+                                             bool* error) {
     const double r = __ddiv_rn(__dmul_rn(double(nh_req), total), norm1);
     int nh = (r >= 0.0 && r < 2147483647.0) ? int(r) : (r >= 2147483647.0 ? INT_MAX : 0);
-    if (!isfinite(norm1) || !isfinite(total)) {
-        nh = 0;
-        atomicOr(status, DEV_ERR_NONFINITE);
-    } else if (!(norm1 > 0.0)) {
-        nh = 0;  // zero source (an exact iterate): no histories, zero correction
-    }
-    if (nh > cap) {
-        // total <= norm1 in exact arithmetic, so nh <= nh_req <= cap; more
-        // means the source sums lost all precision (a diverging iteration).
-        atomicOr(status, DEV_ERR_NONFINITE);
-        nh = cap;
-    }
-    *d_nh = nh;
+    const bool finite = isfinite(norm1) && isfinite(total);
+    if (!finite || !(norm1 > 0.0)) nh = 0;
+    *error = !finite || nh > cap;
+    return nh > cap ? cap : nh;
+}
+
+// The same with the starting weight norm1 (:67) into the solve's scalars, by
+// one thread.
+__device__ __forceinline__ void random_count(int nh_req, double norm1, double total, int cap,
+                                             double* sc, int* d_nh, int* status) {
+    bool error;
+    const int nh = history_count(nh_req, norm1, total, cap, &error);
+    if (error) atomicOr(status, DEV_ERR_NONFINITE);
+    sc[0] = norm1;
+    sc[1] = total;
     sc[2] = nh > 0 ? 1.0 / double(nh) : 0.0;
+    *d_nh = nh;
 }
 
-__global__ void k_guide_marks(const double* cdf, int n, int* marks) {
-    // marks[t] = max j whose window starts at t = floor(cdf[j-1]*G)+1.
-    const double G = double(n);
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        long long t0 = 0;
-        if (j > 0) {
-            double f = floor(cdf[j - 1] * G);
-            t0 = f < -1.0 ? 0 : (long long)f + 1;
+__global__ void k_random_count(int nh_req, double* sc, int* d_nh, int cap, int* status) {
+    random_count(nh_req, sc[0], sc[1], cap, sc, d_nh, status);
+}
+
+// Stratified: nh_local = ceil(Nh * local_sum / weight) (:241), and the factor
+// nh_local / local_sum of the counts (:246-262) in sc[3].
+__device__ __forceinline__ void strat_factor(int nh_req, double norm1, double* sc) {
+    sc[0] = norm1;
+    if (!(norm1 > 0.0)) {  // zero source: no histories (non-finite sums are flagged elsewhere)
+        sc[3] = 0.0;
+        return;
+    }
+    const double nh_local = ceil(__ddiv_rn(__dmul_rn(double(nh_req), norm1), norm1));
+    sc[3] = __ddiv_rn(double(int(nh_local)), norm1);
+}
+
+__global__ void k_strat_prep(int nh_req, double* sc) { strat_factor(nh_req, sc[0], sc); }
+
+// Sum of the nb tile partials, the first of them replaced by `first`; WRITE:
+// an exclusive scan in place as well.  One block.
+template <class T, bool WRITE>
+__device__ __forceinline__ T scan_tiles(T* part, int nb, T first, T* warp_tot) {
+    T carry = T(0);
+    for (int base = 0; base < nb; base += kThreads) {
+        const int i = base + threadIdx.x;
+        const T v = i == 0 ? first : i < nb ? __ldcg(&part[i]) : T(0);
+        T excl;
+        const T incl = block_scan(v, AddOp(), T(0), warp_tot, &excl);
+        if (WRITE && i < nb) part[i] = carry + excl;
+        __shared__ T chunk;
+        if (threadIdx.x == kThreads - 1) chunk = incl;
+        __syncthreads();
+        carry = carry + chunk;
+        __syncthreads();
+    }
+    return carry;
+}
+
+// True in the block that finishes last, which then sees the others' partials.
+__device__ __forceinline__ bool last_block(unsigned int* ticket) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0u;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// Tile sums of the source CDF's terms (signed first element, :185) and, in the
+// last block, their exclusive scan, |b|_1 (with the CDF's association, so that
+// the two totals agree when b[0] >= 0), the history count or the stratified
+// factor.  part has tiles + 2 entries.
+__global__ void __launch_bounds__(kThreads) k_src_reduce(const double* v, int n, double omega,
+                                                         int has, int strat, int nh_req, int cap,
+                                                         double* part, unsigned int* ticket,
+                                                         double* sc, int* d_nh, int* status) {
+    __shared__ double stage[kTile];
+    __shared__ double warp_tot[32];
+    const int base = blockIdx.x * kTile, nb = gridDim.x;
+    for (int k = threadIdx.x; k < kTile; k += kThreads) {
+        const int i = base + k;
+        const double x = i < n ? load_src(v, i, omega, has) : 0.0;
+        stage[k] = i == 0 ? x : fabs(x);
+    }
+    __syncthreads();
+    const double v0 = stage[0];  // signed in block 0
+    double acc = stage[threadIdx.x * kItems];
+#pragma unroll
+    for (int k = 1; k < kItems; ++k) acc = acc + stage[threadIdx.x * kItems + k];
+    double excl;
+    double incl = block_scan(acc, AddOp(), 0.0, warp_tot, &excl);
+    if (threadIdx.x == kThreads - 1) part[blockIdx.x] = incl;
+    if (blockIdx.x == 0) {
+        // The first tile's sum of magnitudes.
+        if (threadIdx.x == 0) {
+            acc = fabs(v0);
+            for (int k = 1; k < kItems; ++k) acc = acc + stage[k];
         }
-        if (t0 < 0) t0 = 0;
-        if (t0 <= n - 1) atomicMax(&marks[t0], j);
+        incl = block_scan(acc, AddOp(), 0.0, warp_tot, &excl);
+        if (threadIdx.x == kThreads - 1) part[nb + 1] = incl;
+    }
+    __syncthreads();
+    if (!last_block(ticket)) return;
+    const double norm1 = scan_tiles<double, false>(part, nb, __ldcg(&part[nb + 1]), warp_tot);
+    const double total = scan_tiles<double, true>(part, nb, __ldcg(&part[0]), warp_tot);
+    if (threadIdx.x != 0) return;
+    part[nb] = total;
+    if (strat) {
+        strat_factor(nh_req, norm1, sc);
+    } else {
+        random_count(nh_req, norm1, total, cap, sc, d_nh, status);
     }
 }
 
+inline int guide_size(int n) { return (n + 15) / 16; }
+
+// The CDF of a tile (cdf[i] /= cdf.back(), :201-205; the last element is set
+// to exactly 1), its states' counts cleared, and the guide entries that fall
+// into the tile: from the first t its lower boundary reaches to the last one
+// before the next tile's.  RESCAN false: the CDF is there already (the
+// reference's sequential order).
+template <bool RESCAN>
+__global__ void __launch_bounds__(kThreads) k_src_cdf(const double* v, int n, double omega, int has,
+                                                      const double* part, const double* sc,
+                                                      double* cdf, int* counts, int* guide,
+                                                      int G) {
+    __shared__ double stage[kTile];
+    __shared__ double warp_tot[32];
+    const int base = blockIdx.x * kTile;
+    const int len = min(kTile, n - base);
+    double lower, upper;  // the tile's range of the CDF
+    if constexpr (RESCAN) {
+        const double total = sc[1];
+        for (int k = threadIdx.x; k < kTile; k += kThreads) {
+            const int i = base + k;
+            const double x = i < n ? load_src(v, i, omega, has) : 0.0;
+            stage[k] = i == 0 ? x : fabs(x);
+        }
+        __syncthreads();
+        double loc[kItems];
+        loc[0] = stage[threadIdx.x * kItems];
+#pragma unroll
+        for (int k = 1; k < kItems; ++k) loc[k] = loc[k - 1] + stage[threadIdx.x * kItems + k];
+        double excl;
+        block_scan(loc[kItems - 1], AddOp(), 0.0, warp_tot, &excl);
+        const double carry = part[blockIdx.x];
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int i = base + threadIdx.x * kItems + k;
+            stage[threadIdx.x * kItems + k] =
+                i >= n - 1 ? 1.0 : (carry + (excl + loc[k])) / total;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < len; k += kThreads) {
+            cdf[base + k] = stage[k];
+            counts[base + k] = 0;
+        }
+        lower = carry / total;
+        upper = part[blockIdx.x + 1] / total;
+    } else {
+        for (int k = threadIdx.x; k < len; k += kThreads) {
+            stage[k] = cdf[base + k];
+            counts[base + k] = 0;
+        }
+        __syncthreads();
+        lower = base > 0 ? cdf[base - 1] : 0.0;
+        upper = stage[len - 1];
+    }
+    // Guide entries t0..t1 of this tile (0..G over all tiles).
+    const double g = double(G);
+    int t0 = 0, t1 = G;
+    if (blockIdx.x > 0) t0 = min(max(int(floor(lower * g)) + 1, 0), G + 1);
+    if (blockIdx.x + 1 < gridDim.x) t1 = min(max(int(floor(upper * g)), -1), G);
+    // First k in [lo, hi] with stage[k] * G >= t (hi when there is none).
+    auto first = [&](int t, int lo, int hi) {
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (stage[mid] * g < double(t)) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+    };
+    // A warp takes 256 entries at a time; a run of entries inside one state
+    // (a source concentrated in few states) is filled without searching.
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int ta = t0 + 256 * warp; ta <= t1; ta += 256 * (kThreads / 32)) {
+        const int tb = min(ta + 255, t1);
+        const int ka = first(ta, 0, len - 1), kb = first(tb, ka, len - 1);
+        for (int t = ta + lane; t <= tb; t += 32)
+            guide[t] = base + (ka == kb ? ka : first(t, ka, kb));
+    }
+}
+
+// std::lower_bound(cdf, u) through the guide.
 __device__ __forceinline__ int guided_lower_bound(const double* cdf, const int* guide, int n,
-                                                  double u) {
-    long long t = (long long)floor(u * double(n));
-    if (t < 0) t = 0;
-    if (t > n - 1) t = n - 1;
-    int lo = guide[t];
-    int hi = t + 1 < n ? guide[t + 1] : n - 1;
-    if (lo < 0) lo = 0;
+                                                  int G, double u) {
+    int t = int(floor(u * double(G)));
+    t = t < 0 ? 0 : (t > G - 1 ? G - 1 : t);
+    int lo = guide[t], hi = guide[t + 1];
     if (hi < lo) hi = lo;
-    // first j in [lo, hi] with cdf[j] >= u (cdf[hi] >= u by construction)
     while (lo < hi) {
-        int mid = (lo + hi) >> 1;
+        const int mid = (lo + hi) >> 1;
         if (cdf[mid] < u) lo = mid + 1; else hi = mid;
     }
+    // A tile boundary's rounding can put the window one state off.
+    while (lo < n - 1 && cdf[lo] < u) ++lo;
+    while (lo > 0 && cdf[lo - 1] >= u) --lo;
     return lo;
 }
 
 // Random sampling: draw k in [0, nh) -> counts[lower_bound(cdf, u_k)]++.
 // Reference stream: each thread owns a contiguous run of draws and jumps once.
-__global__ void k_sample(const double* cdf, const int* guide, int n, const int* d_nh,
+__global__ void k_sample(const double* cdf, const int* guide, int n, int G, const int* d_nh,
                          int rng_mode, uint64_t seed, const unsigned long long* d_epoch,
                          const uint64_t* jump, const unsigned long long* d_pos, int* counts) {
     const int nh = *d_nh;
@@ -100,7 +278,7 @@ __global__ void k_sample(const double* cdf, const int* guide, int n, const int* 
     if (rng_mode == MCLSGPU_RNG_COUNTER) {
         for (int k = tid; k < nh; k += nthreads) {
             uint64_t x = xs_step(counter_state(ekey, 1, uint64_t(k)));
-            int j = guided_lower_bound(cdf, guide, n, canonical64(x));
+            int j = guided_lower_bound(cdf, guide, n, G, canonical64(x));
             atomicAdd(&counts[j], 1);
         }
     } else {
@@ -111,7 +289,7 @@ __global__ void k_sample(const double* cdf, const int* guide, int n, const int* 
         uint64_t x = xs_jump(jump, seed, *d_pos + uint64_t(k0));
         for (long long k = k0; k < k1; ++k) {
             x = xs_step(x);
-            int j = guided_lower_bound(cdf, guide, n, canonical64(x));
+            int j = guided_lower_bound(cdf, guide, n, G, canonical64(x));
             atomicAdd(&counts[j], 1);
         }
     }
@@ -121,18 +299,7 @@ __global__ void k_advance_pos(unsigned long long* d_pos, const int* d_nh, int mu
     *d_pos += (unsigned long long)(*d_nh) * (unsigned long long)mult;
 }
 
-// Stratified: nh_local = ceil(Nh * local_sum / weight) (:241);
-// counts_i = ceil(|b_i| * (nh_local / local_sum)) (:246-262).
-__global__ void k_strat_prep(int nh_req, double* sc) {
-    const double s = sc[0];
-    if (!(s > 0.0)) {  // zero source: no histories (non-finite sums are flagged elsewhere)
-        sc[3] = 0.0;
-        return;
-    }
-    const double nh_local = ceil(__ddiv_rn(__dmul_rn(double(nh_req), s), s));
-    sc[3] = __ddiv_rn(double(int(nh_local)), s);
-}
-
+// Stratified counts_i = ceil(|b_i| * (nh_local / local_sum)) (:246-262).
 __global__ void k_strat_counts(const double* v, int n, double omega, int has, const double* sc,
                                int* counts) {
     const double num_over_sum = sc[3];
@@ -142,38 +309,83 @@ __global__ void k_strat_counts(const double* v, int n, double omega, int has, co
     }
 }
 
-__global__ void k_strat_total(int* d_nh, double* sc, int cap, int* status) {
-    int nh = *d_nh;
+// Tile sums of the counts in emission order (highest state first, the LIFO
+// stack of :157-175) and, in the last block, their exclusive scan; stratified
+// sampling takes its history count from the total.
+__global__ void __launch_bounds__(kThreads) k_src_count(const int* counts, int n, int strat,
+                                                        int cap, int* part, unsigned int* ticket,
+                                                        double* sc, int* d_nh, int* status) {
+    __shared__ int stage[kTile];
+    __shared__ int warp_tot[32];
+    const int base = blockIdx.x * kTile;
+    for (int k = threadIdx.x; k < kTile; k += kThreads)
+        stage[k] = base + k < n ? counts[n - 1 - (base + k)] : 0;
+    __syncthreads();
+    int acc = 0;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) acc += stage[threadIdx.x * kItems + k];
+    int excl;
+    const int incl = block_scan(acc, AddOp(), 0, warp_tot, &excl);
+    if (threadIdx.x == kThreads - 1) part[blockIdx.x] = incl;
+    __syncthreads();
+    if (!last_block(ticket)) return;
+    int nh = scan_tiles<int, true>(part, gridDim.x, __ldcg(&part[0]), warp_tot);
+    if (threadIdx.x != 0 || !strat) return;
     if (nh > cap) {
         atomicOr(status, DEV_ERR_CAPACITY);
         nh = cap;
-        *d_nh = nh;
     }
+    *d_nh = nh;
     sc[2] = nh > 0 ? 1.0 / double(nh) : 0.0;
 }
 
-// Emission order and step-0 collision tally: start[offs_i + t] = i | sign,
-// y_i = counts_i * w0_i (the tally every history makes at its first state).
-template <class TY>
-__global__ void k_expand(const double* v, int n, double omega, int has, const int* counts,
-                         const int* offs, const double* sc, int cap, int* start, TY* y,
-                         int* status) {
+// Emission order and step-0 collision tally: start[o_i + t] = i | sign with
+// o_i the histories of the higher states, y_i = counts_i * w0_i (the tally
+// every history makes at its first state).
+__global__ void __launch_bounds__(kThreads) k_src_expand(const double* v, int n, double omega,
+                                                         int has, const int* counts,
+                                                         const int* part, const double* sc,
+                                                         int cap, int* start, double* y,
+                                                         int* status) {
+    __shared__ int stage[kTile];
+    __shared__ int warp_tot[32];
+    const int base = blockIdx.x * kTile;
+    for (int k = threadIdx.x; k < kTile; k += kThreads)
+        stage[k] = base + k < n ? counts[n - 1 - (base + k)] : 0;
+    __syncthreads();
+    int acc = 0;
+    int c[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        c[k] = stage[threadIdx.x * kItems + k];
+        acc += c[k];
+    }
+    int excl;
+    block_scan(acc, AddOp(), 0, warp_tot, &excl);
+    int o = part[blockIdx.x] + excl;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        stage[threadIdx.x * kItems + k] = o;
+        o += c[k];
+    }
+    __syncthreads();
     const double weight = sc[0];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int c = counts[i];
+    for (int k = threadIdx.x; k < kTile; k += kThreads) {
+        if (base + k >= n) break;
+        const int i = n - 1 - (base + k);
+        const int ci = counts[i], at = stage[k];
         const double b = load_src(v, i, omega, has);
         const unsigned sign = b > 0.0 ? 0u : 0x80000000u;  // weight_sign (:169)
-        if (c > 0) {
-            const int base = offs[i];
-            if (base + c > cap) {
+        if (ci > 0) {
+            if (at + ci > cap) {
                 atomicOr(status, DEV_ERR_CAPACITY);
             } else {
-                for (int t = 0; t < c; ++t) start[base + t] = int(unsigned(i) | sign);
+                for (int t = 0; t < ci; ++t) start[at + t] = int(unsigned(i) | sign);
             }
-            const double w0 = sign ? -weight : weight;
-            y[i] = TY(double(c) * w0);
+            y[i] = double(ci) * (sign ? -weight : weight);
         } else {
-            y[i] = TY(0);
+            y[i] = 0.0;
         }
     }
 }
@@ -355,177 +567,166 @@ __global__ void k_forward_nh(int* d_nh, int nh, double* sc) {
     sc[2] = 1.0 / double(nh);
 }
 
-// ---- small systems: the whole adjoint source in one CTA ------------------
-// For a few thousand states the multi-kernel source build (reductions,
-// scans, guide table, sampling, expansion: about 19 launches) is all launch
-// latency.  One block of 1024 threads does the same steps in shared memory
-// and registers: |v|_1 and the CDF with the reference's signed first element
-// (both sums with one association, so that they agree when v[0] >= 0), the
-// history count, the normalised CDF, the counter-stream draws with
-// lower_bound (the guide table only narrows that search), the counts' suffix
-// scan (LIFO emission order) and the expansion into starting states.
+// ---- small systems: the whole adjoint source in one cluster --------------
+// For a few thousand states the multi-kernel source build is all launch
+// latency.  One cluster of 8 CTAs does the same steps: every CTA forms the
+// whole CDF in its shared memory (|v|_1, the reference's signed first element,
+// the history count), the CTAs share the counter-stream draws and search them
+// with lower_bound (the guide table only narrows that search), each CTA owns
+// an eighth of the states, whose counts the others reach through distributed
+// shared memory, and expands it into starting states behind the eighths above
+// it (LIFO emission order).
+//
+// What bounds it: the chain of barriers and shared-memory round trips.  Each
+// thread owns an odd number of consecutive states (no bank conflicts), so each
+// scan is one block scan; the searches' power-of-two probes are spread over
+// the banks by a swizzle.  At 100^2 it takes 13 us of a 42 us MCSA iteration;
+// one CTA with a scan per 1,024 states took 44 of 72 us.  Up to kSmallSlice
+// states one CTA does it all (C = 1): the draws are then few and a cluster of 8
+// costs 4 us more than it saves (a solve of 1,024 states 63 against 67 us).
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallSourceMax = 16384;
+constexpr int kSmallCtas = 8;
+constexpr int kSmallSlice = kSmallSourceMax / kSmallCtas;
 
-// Inclusive block scan of one value per thread (all 1024 threads call it).
-__device__ __forceinline__ double block_scan_incl(double x, double* warp_tot) {
+__device__ __forceinline__ int swizzle(int i) {
+    return i ^ (((i >> 4) ^ (i >> 8) ^ (i >> 12)) & 15);
+}
+
+// Exclusive block scan of one value per thread (all 1024 threads call it);
+// *total receives the sum.
+template <class T>
+__device__ __forceinline__ T block_scan_excl(T x, T* warp_tot, T* total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, x, d);
+        const T y = __shfl_up_sync(0xffffffffu, x, d);
         if (lane >= d) x += y;
     }
     if (lane == 31) warp_tot[w] = x;
     __syncthreads();
     if (w == 0) {
-        double t = warp_tot[lane];
+        T t = warp_tot[lane];
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, t, d);
+            const T y = __shfl_up_sync(0xffffffffu, t, d);
             if (lane >= d) t += y;
         }
         warp_tot[lane] = t;
     }
     __syncthreads();
-    const double r = w > 0 ? x + warp_tot[w - 1] : x;
+    T r = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) r = T(0);
+    if (w > 0) r += warp_tot[w - 1];
+    *total = warp_tot[31];
     __syncthreads();
     return r;
 }
 
-__device__ __forceinline__ int block_scan_incl_int(int x, int* warp_tot) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
-    }
-    if (lane == 31) warp_tot[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int t = warp_tot[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, t, d);
-            if (lane >= d) t += y;
-        }
-        warp_tot[lane] = t;
-    }
-    __syncthreads();
-    const int r = w > 0 ? x + warp_tot[w - 1] : x;
-    __syncthreads();
-    return r;
-}
+// Shared memory: the CDF (n doubles, swizzled) and the counts of the CTA's
+// states (the state's sign in the top bit).
+constexpr int kSmallSmem = kSmallSourceMax * sizeof(double) + kSmallSlice * sizeof(int);
 
-// Shared memory: the CDF (n doubles) and the per-state counts (n ints).
-constexpr int kSmallSmem = kSmallSourceMax * (sizeof(double) + sizeof(int));
-
-__global__ void __launch_bounds__(kSmallThreads) k_small_adjoint_source(
-    const double* v, int n, double omega, int has, int nh_req, int cap, uint64_t seed,
-    const unsigned long long* d_epoch, int* start, double* y, double* sc, int* d_nh,
-    int* status) {
+template <int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kSmallThreads)
+    k_small_adjoint_source(const double* v, int n, double omega, int has, int nh_req, int cap,
+                           uint64_t seed, const unsigned long long* d_epoch, int* start,
+                           double* y, double* sc, int* d_nh, int* status) {
     extern __shared__ __align__(16) unsigned char smem_src[];
     double* cdf = reinterpret_cast<double*>(smem_src);
     int* counts = reinterpret_cast<int*>(smem_src + sizeof(double) * kSmallSourceMax);
     __shared__ double wtot[32];
     __shared__ int wtoti[32];
-    __shared__ double s_carry[2];
-    __shared__ int s_carry_i;
-    __shared__ int s_nh;
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        s_carry[0] = 0.0;
-        s_carry[1] = 0.0;
-        s_carry_i = 0;
-    }
-    __syncthreads();
-    // 1. Raw CDF (signed first element) and |v|_1 with the same association.
-    for (int base = 0; base < n; base += kSmallThreads) {
-        const int i = base + tid;
-        double a = 0.0, sgn = 0.0;
-        if (i < n) {
-            const double b = load_src(v, i, omega, has);
-            a = fabs(b);
-            sgn = i == 0 ? b : a;
-        }
-        const double cs = block_scan_incl(sgn, wtot) + s_carry[0];
-        const double ca = block_scan_incl(a, wtot) + s_carry[1];
-        if (i < n) cdf[i] = cs;
-        __syncthreads();
-        if (tid == kSmallThreads - 1) {
-            s_carry[0] = cs;
-            s_carry[1] = ca;
-        }
-        __syncthreads();
-    }
-    // 2. History count nh = int(Nh * cdf.back() / |v|_1) (:198), weights.
-    if (tid == 0) {
-        const double norm1 = s_carry[1], total = s_carry[0];
-        const double r = __ddiv_rn(__dmul_rn(double(nh_req), total), norm1);
-        int nh = (r >= 0.0 && r < 2147483647.0) ? int(r) : (r >= 2147483647.0 ? INT_MAX : 0);
-        if (!isfinite(norm1) || !isfinite(total)) {
-            nh = 0;
-            atomicOr(status, DEV_ERR_NONFINITE);
-        } else if (!(norm1 > 0.0)) {
-            nh = 0;
-        }
-        if (nh > cap) {
-            atomicOr(status, DEV_ERR_NONFINITE);
-            nh = cap;
-        }
-        sc[0] = norm1;
-        sc[1] = total;
-        sc[2] = nh > 0 ? 1.0 / double(nh) : 0.0;
-        *d_nh = nh;
-        s_nh = nh;
-    }
-    __syncthreads();
-    const int nh = s_nh;
-    // 3. Normalise (cdf[n-1] = 1 exactly) and clear the counts.
-    const double total = s_carry[0];
+    __shared__ int s_slice[C];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, rank = int(cluster.block_rank());
+    const int slice = (n + C - 1) / C;
+    const int j0 = min(rank * slice, n), j1 = min(j0 + slice, n);  // this CTA's states
+    const unsigned long long epoch = *d_epoch;
+    // 1. Terms of the CDF (signed first element) and the states' signs.
     for (int i = tid; i < n; i += kSmallThreads) {
-        cdf[i] = i == n - 1 ? 1.0 : cdf[i] / total;
-        counts[i] = 0;
+        const double b = load_src(v, i, omega, has);
+        cdf[swizzle(i)] = i == 0 ? b : fabs(b);
+        if (i >= j0 && i < j1) counts[i - j0] = b > 0.0 ? 0 : INT_MIN;
     }
     __syncthreads();
-    // 4. Draw the starting states (counter stream, kind 1).
-    const uint64_t ekey = epoch_key(seed, *d_epoch);
-    for (int k = tid; k < nh; k += kSmallThreads) {
-        const double u = canonical64(xs_step(counter_state(ekey, 1, uint64_t(k))));
-        int lo = 0, hi = n - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (cdf[mid] < u) lo = mid + 1; else hi = mid;
+    const int items = ((n + kSmallThreads - 1) / kSmallThreads) | 1;
+    const int i0 = min(tid * items, n), i1 = min(i0 + items, n);
+    double sum = 0.0;
+    for (int i = i0; i < i1; ++i) sum += cdf[swizzle(i)];
+    double total;
+    double run = block_scan_excl(sum, wtot, &total);
+    // 2. |v|_1 -- the CDF's total unless the first element is negative -- and
+    //    the history count.
+    double norm1 = total;
+    if (cdf[0] < 0.0) {
+        if (tid == 0) {
+            sum = 0.0;
+            for (int i = i0; i < i1; ++i) sum += fabs(cdf[swizzle(i)]);
         }
-        atomicAdd(&counts[lo], 1);
+        block_scan_excl(sum, wtot, &norm1);
     }
+    bool error;
+    const int nh = history_count(nh_req, norm1, total, cap, &error);
+    if (rank == 0 && tid == 0) random_count(nh_req, norm1, total, cap, sc, d_nh, status);
+    // 3. Normalise (cdf[n-1] = 1 exactly), once every thread has read cdf[0].
     __syncthreads();
-    // 5. Exclusive suffix sum of the counts (LIFO emission: highest state
-    //    first) and, chunk by chunk, the expansion into starting states and
-    //    step-0 tallies.
-    const double weight = sc[0];
-    for (int base = 0; base < n; base += kSmallThreads) {
-        const int k = base + tid;      // position in reversed order
-        const int i = n - 1 - k;       // state
-        const int c = k < n ? counts[i] : 0;
-        const int incl = block_scan_incl_int(c, wtoti) + s_carry_i;
-        if (k < n) {
-            const int o = incl - c;
-            const double b = load_src(v, i, omega, has);
-            const unsigned sign = b > 0.0 ? 0u : 0x80000000u;
-            if (c > 0) {
-                if (o + c > cap) {
-                    atomicOr(status, DEV_ERR_CAPACITY);
-                } else {
-                    for (int t = 0; t < c; ++t) start[o + t] = int(unsigned(i) | sign);
-                }
-                y[i] = double(c) * (sign ? -weight : weight);
-            } else {
-                y[i] = 0.0;
+    for (int i = i0; i < i1; ++i) {
+        run += cdf[swizzle(i)];
+        cdf[swizzle(i)] = i == n - 1 ? 1.0 : run / total;
+    }
+    cluster.sync();  // every CTA's counts are set
+    // 4. Draw the starting states (counter stream, kind 1), two searches in
+    //    flight per thread.
+    const uint64_t ekey = epoch_key(seed, epoch);
+    const int top = n > 1 ? 1 << (31 - __clz(n - 1)) : 0;
+    constexpr int kDraws = 2, kStride = C * kSmallThreads;
+    for (int k = rank * kSmallThreads + tid; k < nh; k += kDraws * kStride) {
+        double u[kDraws];
+        int lo[kDraws];
+#pragma unroll
+        for (int q = 0; q < kDraws; ++q) {
+            u[q] = canonical64(xs_step(counter_state(ekey, 1, uint64_t(k + q * kStride))));
+            lo[q] = 0;
+        }
+        // lower_bound over [0, n-1]: lo is the count of elements known < u.
+        for (int half = top; half > 0; half >>= 1) {
+#pragma unroll
+            for (int q = 0; q < kDraws; ++q) {
+                const int m = lo[q] + half;
+                if (m <= n - 1 && cdf[swizzle(m - 1)] < u[q]) lo[q] = m;
             }
         }
-        __syncthreads();
-        if (tid == kSmallThreads - 1) s_carry_i = incl;
-        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kDraws; ++q)
+            if (k + q * kStride < nh) {
+                const int owner = lo[q] / slice;
+                atomicAdd(cluster.map_shared_rank(counts, owner) + (lo[q] - owner * slice), 1);
+            }
+    }
+    cluster.sync();
+    // 5. Emission (highest state first): a thread's run of states starts after
+    //    the histories of the runs above it, a CTA's after the CTAs above it.
+    constexpr int kOwn = kSmallSlice / kSmallThreads;
+    const int t0 = min(j0 + tid * kOwn, j1), t1 = min(t0 + kOwn, j1);
+    int mine = 0;
+    for (int i = t0; i < t1; ++i) mine += counts[i - j0] & INT_MAX;
+    int all;
+    const int before = block_scan_excl(mine, wtoti, &all);
+    if (tid < C) *cluster.map_shared_rank(&s_slice[rank], tid) = all;
+    cluster.sync();
+    int o = all - before - mine;
+    for (int q = rank + 1; q < C; ++q) o += s_slice[q];
+    for (int i = t1 - 1; i >= t0; --i) {
+        const int ci = counts[i - j0], c = ci & INT_MAX;
+        if (o + c > cap) {
+            if (c > 0) atomicOr(status, DEV_ERR_CAPACITY);
+        } else {
+            for (int t = 0; t < c; ++t) start[o + t] = i | (ci & INT_MIN);
+        }
+        o += c;
+        // Step-0 tally.
+        y[i] = c > 0 ? double(c) * (ci < 0 ? -norm1 : norm1) : 0.0;
     }
 }
 
@@ -537,7 +738,11 @@ bool small_source_ready(mclsgpu_context* ctx) {
     std::lock_guard<std::mutex> lock(g_small_mutex);
     const int d = ctx->device;
     if (d >= 0 && d < 64 && g_small_set[d]) return true;
-    if (cudaFuncSetAttribute(k_small_adjoint_source, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_small_adjoint_source<kSmallCtas>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSmallSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_small_adjoint_source<1>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmallSmem) != cudaSuccess) {
         cudaGetLastError();
         return false;  // keep the multi-kernel path
@@ -571,37 +776,45 @@ void launch_adjoint_source(mclsgpu_domain* dom, const double* v, double omega, i
     if (!parity && p.rng_mode == MCLSGPU_RNG_COUNTER &&
         p.source_sampling == MCLSGPU_SOURCE_RANDOM && n <= kSmallSourceMax &&
         small_source_ready(ctx)) {
-        k_small_adjoint_source<<<1, kSmallThreads, kSmallSmem, s>>>(
+        const bool one = n <= kSmallSlice;
+        auto kernel = one ? k_small_adjoint_source<1> : k_small_adjoint_source<kSmallCtas>;
+        kernel<<<one ? 1 : kSmallCtas, kSmallThreads, kSmallSmem, s>>>(
             v, n, omega, has_omega, nh_req, cap, dom->seed, dom->d_epoch, dom->start, dom->y64,
             dom->d_scalars, dom->d_nh, ctx->d_status);
         return;
     }
-    // weight = |b|_1
-    abs_sum(s, v, n, omega, has_omega, parity ? nullptr : dom->part, dom->d_scalars + 0);
-    cudaMemsetAsync(dom->counts, 0, size_t(n) * sizeof(int), s);
-    if (p.source_sampling == MCLSGPU_SOURCE_RANDOM) {
-        source_cdf(s, v, n, omega, has_omega, parity ? 1 : 0, dom->part, dom->scdf,
-                   dom->d_scalars + 1);
+    const bool strat = p.source_sampling != MCLSGPU_SOURCE_RANDOM;
+    const int nb = tiles(n), G = guide_size(n);
+    if (!parity) {
+        k_src_reduce<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, strat, nh_req, cap, dom->part,
+                                             dom->d_ticket, dom->d_scalars, dom->d_nh,
+                                             ctx->d_status);
+    } else if (strat) {
+        abs_sum_sequential(s, v, n, omega, has_omega, dom->d_scalars + 0);
+        k_strat_prep<<<1, 1, 0, s>>>(nh_req, dom->d_scalars);
+    } else {
+        source_sequential(s, v, n, omega, has_omega, dom->d_scalars + 0, dom->scdf,
+                          dom->d_scalars + 1);
         k_random_count<<<1, 1, 0, s>>>(nh_req, dom->d_scalars, dom->d_nh, cap, ctx->d_status);
-        cudaMemsetAsync(dom->guide, 0xFF, size_t(n) * sizeof(int), s);
-        k_guide_marks<<<grid_for(n), 256, 0, s>>>(dom->scdf, n, dom->guide);
-        max_scan_int(s, dom->guide, n, dom->ipart);
+    }
+    if (!strat) {
+        auto cdf = parity ? k_src_cdf<false> : k_src_cdf<true>;
+        cdf<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, dom->part, dom->d_scalars, dom->scdf,
+                                    dom->counts, dom->guide, G);
         const int sample_grid = p.rng_mode == MCLSGPU_RNG_COUNTER ? ctx->num_sms * 8 : 64;
-        k_sample<<<sample_grid, 256, 0, s>>>(dom->scdf, dom->guide, n, dom->d_nh, p.rng_mode,
+        k_sample<<<sample_grid, 256, 0, s>>>(dom->scdf, dom->guide, n, G, dom->d_nh, p.rng_mode,
                                              dom->seed, dom->d_epoch, dom->d_jump, dom->d_pos,
                                              dom->counts);
         if (p.rng_mode == MCLSGPU_RNG_REFERENCE) k_advance_pos<<<1, 1, 0, s>>>(dom->d_pos, dom->d_nh, 1);
-        suffix_scan_int(s, dom->counts, n, dom->ipart, dom->offs, nullptr);
     } else {
-        k_strat_prep<<<1, 1, 0, s>>>(nh_req, dom->d_scalars);
         k_strat_counts<<<grid_for(n), 256, 0, s>>>(v, n, omega, has_omega, dom->d_scalars,
                                                    dom->counts);
-        suffix_scan_int(s, dom->counts, n, dom->ipart, dom->offs, dom->d_nh);
-        k_strat_total<<<1, 1, 0, s>>>(dom->d_nh, dom->d_scalars, cap, ctx->d_status);
     }
-    k_expand<double><<<grid_for(n), 256, 0, s>>>(v, n, omega, has_omega, dom->counts, dom->offs,
-                                                 dom->d_scalars, cap, dom->start, dom->y64,
-                                                 ctx->d_status);
+    k_src_count<<<nb, kThreads, 0, s>>>(dom->counts, n, strat, cap, dom->ipart, dom->d_ticket,
+                                        dom->d_scalars, dom->d_nh, ctx->d_status);
+    k_src_expand<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, dom->counts, dom->ipart,
+                                         dom->d_scalars, cap, dom->start, dom->y64,
+                                         ctx->d_status);
 }
 
 void launch_forward_setup(mclsgpu_domain* dom) {

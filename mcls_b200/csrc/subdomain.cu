@@ -82,14 +82,13 @@ __global__ void k_part_finish_forward(const double* y, const double* srcp, int n
 __global__ void k_epoch_next(unsigned long long* e) { *e += 1ULL; }
 
 void release_source(mclsgpu_domain* d) {
-    dfree(d->src);
     dfree(d->scdf);
     dfree(d->guide);
     dfree(d->counts);
-    dfree(d->offs);
     dfree(d->start);
     dfree(d->y64);
     dfree(d->d_nh);
+    dfree(d->d_ticket);
     dfree(d->d_scalars);
     dfree(d->part);
     dfree(d->ipart);
@@ -219,10 +218,10 @@ int mclsgpu_subdomain_build(mclsgpu_context* ctx, int64_t n_global, int32_t npar
             rc = set_error(ctx, MCLSGPU_ERR_UNSUPPORTED, "too many histories per solve");
         const int parts = scan_partials_needed(N) + ctx->num_sms * 8 + 8;
         if (!rc &&
-            ((e = dmalloc(&g.src, N)) != cudaSuccess || (e = dmalloc(&g.scdf, N)) != cudaSuccess ||
-             (e = dmalloc(&g.guide, N)) != cudaSuccess ||
+            ((e = dmalloc(&g.scdf, N)) != cudaSuccess ||
+             (e = dmalloc(&g.guide, size_t(N) / 16 + 2)) != cudaSuccess ||
              (e = dmalloc(&g.counts, N)) != cudaSuccess ||
-             (e = dmalloc(&g.offs, N)) != cudaSuccess ||
+             (e = dmalloc(&g.d_ticket, 1)) != cudaSuccess ||
              (e = dmalloc(&g.start, size_t(g.nh_cap) + 1)) != cudaSuccess ||
              (e = dmalloc(&g.y64, N)) != cudaSuccess || (e = dmalloc(&g.d_nh, 1)) != cudaSuccess ||
              (e = dmalloc(&g.d_scalars, 16)) != cudaSuccess ||
@@ -241,6 +240,7 @@ int mclsgpu_subdomain_build(mclsgpu_context* ctx, int64_t n_global, int32_t npar
             cudaMemsetAsync(g.d_epoch, 0, sizeof(unsigned long long), s);
             cudaMemsetAsync(g.d_pos, 0, sizeof(unsigned long long), s);
             cudaMemsetAsync(g.d_scalars, 0, 16 * sizeof(double), s);
+            cudaMemsetAsync(g.d_ticket, 0, sizeof(unsigned int), s);
             cudaMemsetAsync(sd->d_steps, 0, sizeof(unsigned long long), s);
             std::vector<int> hb(nparts + 1);
             for (int q = 0; q <= nparts; ++q) hb[q] = int(bounds[q]);

@@ -55,7 +55,6 @@ struct WalkArgs {
     const double* W;
     // tallies
     double* y64;
-    const float* c32;
     const double* c64;
     unsigned long long* d_steps;
     unsigned long long* d_tim;  // [0] first warp start, [1] last warp end (ns)
@@ -986,7 +985,6 @@ void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
     a.cdf = dom->cdf;
     a.W = dom->w;
     a.y64 = dom->y64;
-    a.c32 = dom->c32;
     a.c64 = dom->c64;
     a.max_trace = max_trace;
     a.tr_states = tr_states;
