@@ -16,12 +16,24 @@
 // a system whose pairs have all met it stops (its rows and walks are
 // skipped), and the loop ends when every pair has met it or at the iteration
 // limit.  One iteration is four kernels in a CUDA graph whose WHILE node the
-// last one controls: Richardson step + residual, tally source, the shared
-// walk, and correction + residual + per-pair norms, whose last block to
-// finish runs the convergence test.
+// last one controls: the residual after the Richardson step, the tally source,
+// the shared walk -- which adds the step and the correction to the iterate
+// (with several histories per row, a pass of its own does) -- and residual +
+// per-pair norms, whose last block to finish runs the convergence test.
+//
+// The passes over the elements take them in units: one row by two
+// consecutive columns per thread (one 16-byte access), the entries from rows of
+// fixed width.  What bounds them is the chain of dependent loads: with one
+// column per thread and the CSR row walked entry by entry (row bounds, column,
+// value) they ran at a third of the HBM rate (128 systems, 5M elements: 109, 57
+// and 164 us).  Fixed rows need no bounds, the gathers of a row are in flight
+// together, and the next tile's column indices are loaded meanwhile, which
+// leaves one memory latency per tile.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -40,37 +52,44 @@ struct BatchState {
 };
 
 constexpr int kThreads = 256;
+constexpr int kRowBlocks = 3;  // blocks per SM of the row passes (their registers)
+
+// Rows of fixed width for the element passes, entry-major: entry k of row i at
+// k * n + i, columns ascending; padding entries repeat the row's own index with
+// value 0.  The width is the longest row's, rounded up to kRowChunk.
+constexpr int kRowChunk = 8;
+struct BatchRows {
+    int n = 0;
+    int chunks = 0;      // width / kRowChunk
+    int* col = nullptr;
+    double* val = nullptr;
+};
 
 struct BatchArgs {
     int nsys;
     int pw;              // per-pair row width: pair (s, r) is s * pw + r
     int per;             // histories per row
-    const int* rp;       // S (CSR)
-    const int* ci;
-    const double* v;
+    BatchRows S;         // the operator
     const double* dinv;  // D^-1
-    const int* hrp;      // H rows (forward domain, FP64)
-    const int* hci;
-    const double* hv;
+    BatchRows H;         // H rows (forward domain, FP64)
     // Per system: first row, first element, log2 of its width, rows.
     const int* srow0;
     const long long* seoff;
     const int* slog;
     const int* sn;
     const int* sorder;   // the systems in placement order
-    // The systems this launch works on: lsys[k] for k < *lcount, their
-    // elements at [lecum[k], lecum[k+1]) of the launch's element space.
+    // The systems this launch works on: lsys[k] for k < *lcount, their tiles of
+    // kThreads units at [ltcum[k], ltcum[k+1]) of the launch's tiles.
     const int* lsys;
-    const long long* lecum;
+    const int* ltcum;
     const int* lcount;
     // The active list the convergence test rebuilds (the iteration's list).
     int* act_sys;
-    long long* act_ecum;
+    int* act_tcum;
     int* act_hcum;
     int* act_count;
     const double* B;
     double* X;
-    double* X2;
     double* RP;
     double* RP2;
     double* Y;
@@ -92,144 +111,245 @@ struct BatchArgs {
     int* status;
 };
 
-// One element of a launch's element space: system s, row i, column r, log2
-// width c, its index e in the element arrays and the element index of its
-// row's column 0 minus the row times the width (so that the element of row j,
-// column r of the same system is base + (j << c) + r).
-struct Elem {
-    int s, i, r, c;
-    size_t e;
-    long long base;
+// Columns of a unit of width class c, and the units of a row.
+__host__ __device__ constexpr int unit_cols(int c) { return c >= 1 ? 2 : 1; }
+__host__ __device__ constexpr int unit_log(int c) { return c >= 1 ? c - 1 : 0; }
+
+// Tiles of a system: kThreads units each, the last one partial.
+__host__ __device__ constexpr long long system_tiles(int n, int c) {
+    return (((long long)n << unit_log(c)) + kThreads - 1) / kThreads;
+}
+
+// One thread's unit: its system s with log2 width c, first row row0 and first
+// element eoff; its row (in the operator: i, in the system: rl) and the index
+// of its first column inside the system's elements.
+struct Unit {
+    int s, c, row0, i, g;
+    unsigned col0;     // g * unit_cols(c)
+    long long eoff;
+    __device__ __forceinline__ size_t elem() const {
+        return size_t(eoff) + ((size_t(i - row0) << c) + col0);
+    }
 };
 
-// The list entry k with lecum[k] <= t < lecum[k+1] (count >= 1 entries).
-__device__ __forceinline__ int elem_entry(const long long* lecum, int count, long long t) {
+// The list entry k with ltcum[k] <= t < ltcum[k+1] (count >= 1 entries).
+__device__ __forceinline__ int tile_entry(const int* ltcum, int count, int t) {
     int lo = 0, hi = count - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (lecum[mid] <= t) lo = mid; else hi = mid - 1;
+        if (ltcum[mid] <= t) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
 
-// A thread's position in the launch's list: entry k and its system's fields,
-// reloaded only when the thread's element crosses into the next entry (the
-// elements a thread visits only increase).
-struct Cursor {
-    int k, s, c, row0;
-    long long lo, hi, eoff;
-    __device__ __forceinline__ void load(const BatchArgs& a, int kk) {
-        k = kk;
-        s = a.lsys[k];
-        c = a.slog[s];
-        row0 = a.srow0[s];
-        eoff = a.seoff[s];
-        lo = a.lecum[k];
-        hi = a.lecum[k + 1];
+// Loop over the launch's tiles: each block takes one contiguous range.  A tile
+// lies in one system, so the system's fields are uniform in the block and
+// reloaded only when it moves on to the next.  body(live, q, next) runs on every
+// thread of the block for every tile, enter(q, live, row) before the first tile
+// of each system (so both may use warp collectives); next: the thread's row in
+// the next tile if that has one in the same system, else -1.
+template <class Enter, class Body>
+__device__ __forceinline__ void for_tiles(const BatchArgs& a, Enter enter, Body body) {
+    __shared__ int s_k0;
+    const int count = *a.lcount;
+    const int total = count > 0 ? a.ltcum[count] : 0;
+    const int span = (total + int(gridDim.x) - 1) / int(gridDim.x);
+    const int beg = blockIdx.x * span;
+    const int end = min(beg + span, total);
+    if (beg >= end) return;  // the whole block
+    if (threadIdx.x == 0) s_k0 = tile_entry(a.ltcum, count, beg);
+    __syncthreads();
+    int k = s_k0 - 1, lo = 0, hi = -1, units = 0;
+    Unit q;
+#pragma unroll 1
+    for (int t = beg; t < end; ++t) {
+        if (t >= hi) {
+            ++k;
+            q.s = a.lsys[k];
+            q.c = a.slog[q.s];
+            q.row0 = a.srow0[q.s];
+            q.eoff = a.seoff[q.s];
+            units = a.sn[q.s] << unit_log(q.c);
+            lo = a.ltcum[k];
+            hi = a.ltcum[k + 1];
+            q.g = threadIdx.x & ((1 << unit_log(q.c)) - 1);
+            q.col0 = unsigned(q.g * unit_cols(q.c));
+            const int u0 = (t - lo) * kThreads + threadIdx.x;
+            enter(q, u0 < units, q.row0 + (u0 >> unit_log(q.c)));
+        }
+        const int u = (t - lo) * kThreads + threadIdx.x, un = u + kThreads;
+        q.i = q.row0 + (u >> unit_log(q.c));
+        body(u < units, q, t + 1 < hi && un < units ? q.row0 + (un >> unit_log(q.c)) : -1);
     }
-    // Element t (lo <= t after the first call; t < lecum[count]).
-    __device__ __forceinline__ Elem at(const BatchArgs& a, long long t) {
-        while (t >= hi) load(a, k + 1);
-        Elem q;
-        q.s = s;
-        q.c = c;
-        const long long local = t - lo;
-        q.i = row0 + int(local >> c);
-        q.r = int(local & ((1 << c) - 1));
-        q.e = size_t(eoff + local);
-        q.base = eoff - ((long long)row0 << c);
-        return q;
+}
+struct NoEnter {
+    __device__ __forceinline__ void operator()(const Unit&, bool, int) const {}
+};
+
+// N consecutive doubles (one access of 8 or 16 bytes; the element arrays are
+// aligned to 128 bytes and a unit to its own size).
+template <int N>
+struct Cols {
+    double v[N];
+};
+template <int N>
+__device__ __forceinline__ Cols<N> ldn(const double* p) {
+    Cols<N> r;
+    if constexpr (N == 2) {
+        const double2 t = *reinterpret_cast<const double2*>(p);
+        r.v[0] = t.x;
+        r.v[1] = t.y;
+    } else
+        r.v[0] = *p;
+    return r;
+}
+template <int N>
+__device__ __forceinline__ void stn(double* p, const Cols<N>& r) {
+    if constexpr (N == 2)
+        *reinterpret_cast<double2*>(p) = make_double2(r.v[0], r.v[1]);
+    else
+        *p = r.v[0];
+}
+
+// f(integral_constant<int, columns>) for the unit's class.
+template <class F>
+__device__ __forceinline__ void with_cols(int c, F f) {
+    if (c >= 1) f(std::integral_constant<int, 2>{});
+    else f(std::integral_constant<int, 1>{});
+}
+
+// The column indices of the first chunk of a thread's row, loaded one tile
+// ahead (the body of a tile starts the next tile's loads after its gathers).
+struct Ahead {
+    int col[kRowChunk];
+    __device__ __forceinline__ void load(const BatchRows& M, int i) {
+#pragma unroll
+        for (int m = 0; m < kRowChunk; ++m) col[m] = M.col[size_t(m) * M.n + i];
     }
 };
 
-// Loop over the launch's elements: each block takes one contiguous range in
-// tiles of blockDim elements; the block's first thread finds the list entry
-// of the range's first element, and every thread steps its own cursor
-// forward from there.  body(live, q) runs on every thread of the block for
-// every tile (block-uniform trip count, so body may use warp collectives).
-template <class Body>
-__device__ __forceinline__ void for_elements(const BatchArgs& a, Body body) {
-    __shared__ int s_k0;
-    const int count = *a.lcount;
-    const long long total = count > 0 ? a.lecum[count] : 0;
-    const long long T = blockDim.x;
-    const long long span = ((total + gridDim.x - 1) / gridDim.x + T - 1) / T * T;
-    const long long beg = (long long)blockIdx.x * span;
-    const long long end = beg + span < total ? beg + span : total;
-    if (beg >= end) return;  // the whole block
-    if (threadIdx.x == 0) s_k0 = elem_entry(a.lecum, count, beg);
-    __syncthreads();
-    Cursor cur;
-    cur.load(a, s_k0);
-    for (long long base = beg; base < end; base += T) {
-        const long long t = base + threadIdx.x;
-        const bool live = t < end;
-        Elem q{};
-        if (live) q = cur.at(a, t);
-        body(live, q);
+// The unit's row of M times the columns of x, entries in ascending column
+// order; `next`: the row whose indices to load into h meanwhile (or -1).
+template <int N>
+__device__ __forceinline__ Cols<N> row_times(const BatchRows& M, const Unit& q, const double* x,
+                                             Ahead& h, int next) {
+    const double* xs = x + q.eoff + q.col0;
+    Cols<N> acc;
+#pragma unroll
+    for (int n = 0; n < N; ++n) acc.v[n] = 0.0;
+    Cols<N> xv[kRowChunk];
+    double val[kRowChunk];
+#pragma unroll
+    for (int m = 0; m < kRowChunk; ++m) {
+        xv[m] = ldn<N>(xs + (size_t(unsigned(h.col[m] - q.row0)) << q.c));
+        val[m] = M.val[size_t(m) * M.n + q.i];
     }
+    if (next >= 0) h.load(M, next);
+#pragma unroll
+    for (int m = 0; m < kRowChunk; ++m) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc.v[n] = fma(val[m], xv[m].v[n], acc.v[n]);
+    }
+#pragma unroll 1
+    for (int k = kRowChunk; k < M.chunks * kRowChunk; ++k) {
+        const int col = M.col[size_t(k) * M.n + q.i];
+        const Cols<N> xk = ldn<N>(xs + (size_t(unsigned(col - q.row0)) << q.c));
+        const double v = M.val[size_t(k) * M.n + q.i];
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc.v[n] = fma(v, xk.v[n], acc.v[n]);
+    }
+    return acc;
 }
 
-// x2 = x + w rp;  rp2 = D^-1 (b - S x2), with x2 at the neighbours formed on
-// the fly (RichardsonIteration::doOneIteration then updatePrecResidual,
-// src/MCLS_RichardsonIteration_impl.hpp:134-147); the walk tallies Y are
-// cleared for this iteration's walk.
-__global__ void __launch_bounds__(kThreads, 8) k_b_richardson_residual(BatchArgs a) {
-    for_elements(a, [&](bool live, const Elem& q) {
+// The residual after the Richardson step x + w rp, from rp alone: rp2 = rp -
+// w D^-1 S rp (src/MCLS_RichardsonIteration_impl.hpp:134-147); Y (not null:
+// the walk adds into it) is cleared for this iteration's walk.
+__global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_richardson_residual(BatchArgs a) {
+    Ahead h;
+    auto enter = [&](const Unit&, bool live, int i) {
+        if (live) h.load(a.S, i);
+    };
+    for_tiles(a, enter, [&](bool live, const Unit& q, int next) {
         if (!live) return;
-        double acc = 0.0;
-        for (int p = a.rp[q.i]; p < a.rp[q.i + 1]; ++p) {
-            const size_t k = size_t(q.base + ((long long)a.ci[p] << q.c) + q.r);
-            acc = fma(a.v[p], __dadd_rn(a.X[k], __dmul_rn(a.omega, a.RP[k])), acc);
-        }
-        a.X2[q.e] = __dadd_rn(a.X[q.e], __dmul_rn(a.omega, a.RP[q.e]));
-        a.RP2[q.e] = a.dinv[q.i] * (a.B[q.e] - acc);
-        a.Y[q.e] = 0.0;
+        const size_t e = q.elem();
+        with_cols(q.c, [&](auto nt) {
+            constexpr int N = decltype(nt)::value;
+            const Cols<N> r = ldn<N>(a.RP + e);
+            const double di = a.dinv[q.i];
+            Cols<N> t = row_times<N>(a.S, q, a.RP, h, next);
+#pragma unroll
+            for (int n = 0; n < N; ++n) t.v[n] = r.v[n] - a.omega * (di * t.v[n]);
+            stn<N>(a.RP2 + e, t);
+            if (a.Y) {
+#pragma unroll
+                for (int n = 0; n < N; ++n) t.v[n] = 0.0;
+                stn<N>(a.Y + e, t);
+            }
+        });
     });
 }
 
 // Tally source of every right-hand side: expected value c = H (w rp2),
 // collision c = w rp2 (FP32).
-__global__ void __launch_bounds__(kThreads, 8) k_b_source(BatchArgs a) {
-    for_elements(a, [&](bool live, const Elem& q) {
+__global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_source(BatchArgs a) {
+    Ahead h;
+    auto enter = [&](const Unit&, bool live, int i) {
+        if (live && a.ev) h.load(a.H, i);
+    };
+    for_tiles(a, enter, [&](bool live, const Unit& q, int next) {
         if (!live) return;
-        double v;
-        if (a.ev) {
-            v = 0.0;
-            for (int p = a.hrp[q.i]; p < a.hrp[q.i + 1]; ++p)
-                v = fma(a.hv[p], a.RP2[size_t(q.base + ((long long)a.hci[p] << q.c) + q.r)], v);
-        } else {
-            v = a.RP2[q.e];
-        }
-        a.cR[q.e] = __double2float_rn(a.nomega * v);
+        const size_t e = q.elem();
+        with_cols(q.c, [&](auto nt) {
+            constexpr int N = decltype(nt)::value;
+            const Cols<N> t = a.ev ? row_times<N>(a.H, q, a.RP2, h, next)
+                                   : ldn<N>(a.RP2 + e);
+            float f[N];
+#pragma unroll
+            for (int n = 0; n < N; ++n) f[n] = __double2float_rn(a.nomega * t.v[n]);
+            float* c = a.cR + e;
+            if constexpr (N == 2)
+                *reinterpret_cast<float2*>(c) = make_float2(f[0], f[1]);
+            else
+                *c = f[0];
+        });
     });
 }
 
-// The corrected iterate at element k: x2 + Y / per (+ w rp2 for the expected
-// value, the estimator's source term; ForwardTally::finalize,
-// src/MCLS_ForwardTally_impl.hpp:180-209).
-__device__ __forceinline__ double corrected(const BatchArgs& a, size_t k) {
-    double d = a.Y[k] * a.inv_per;
-    if (a.ev) d += a.nomega * a.RP2[k];
-    return a.X2[k] + d;
+// x += w rp + Y / per (+ w rp2 for the expected value, the estimator's source
+// term; ForwardTally::finalize, src/MCLS_ForwardTally_impl.hpp:180-209), when
+// the walk's rows have several histories.
+__global__ void __launch_bounds__(kThreads, 4) k_b_correct(BatchArgs a) {
+    for_tiles(a, NoEnter{}, [&](bool live, const Unit& q, int) {
+        if (!live) return;
+        const size_t e = q.elem();
+        with_cols(q.c, [&](auto nt) {
+            constexpr int N = decltype(nt)::value;
+            Cols<N> x = ldn<N>(a.X + e);
+            const Cols<N> r = ldn<N>(a.RP + e), r2 = ldn<N>(a.RP2 + e), y = ldn<N>(a.Y + e);
+#pragma unroll
+            for (int n = 0; n < N; ++n)
+                x.v[n] = batch_corrected(x.v[n], r.v[n], r2.v[n], y.v[n], a.omega, a.nomega,
+                                         a.inv_per, a.ev);
+            stn<N>(a.X + e, x);
+        });
+    });
 }
 
 // The active list from sys_done, in placement order, by one block: each
 // thread counts a contiguous run of systems, a block scan places the runs.
 __device__ void build_active(const BatchArgs& a) {
     __shared__ int s_cnt[1024];
-    __shared__ long long s_el[1024];
+    __shared__ int s_el[1024];
     __shared__ int s_h[1024];
     const int T = blockDim.x, tid = threadIdx.x;
     const int seg = (a.nsys + T - 1) / T;
     const int j0 = min(tid * seg, a.nsys), j1 = min(j0 + seg, a.nsys);
-    int cnt = 0, hs = 0;
-    long long el = 0;
+    int cnt = 0, hs = 0, el = 0;
     for (int j = j0; j < j1; ++j) {
         const int s = a.sorder[j];
         if (a.sys_done[s]) continue;
         ++cnt;
-        el += (long long)a.sn[s] << a.slog[s];
+        el += int(system_tiles(a.sn[s], a.slog[s]));
         hs += a.sn[s] * a.per;
     }
     s_cnt[tid] = cnt;
@@ -237,8 +357,7 @@ __device__ void build_active(const BatchArgs& a) {
     s_h[tid] = hs;
     __syncthreads();
     for (int d = 1; d < T; d <<= 1) {  // inclusive scan (Hillis-Steele)
-        int c2 = 0, h2 = 0;
-        long long e2 = 0;
+        int c2 = 0, h2 = 0, e2 = 0;
         if (tid >= d) {
             c2 = s_cnt[tid - d];
             e2 = s_el[tid - d];
@@ -251,21 +370,21 @@ __device__ void build_active(const BatchArgs& a) {
         __syncthreads();
     }
     int k = s_cnt[tid] - cnt;
-    long long eo = s_el[tid] - el;
+    int eo = s_el[tid] - el;
     int ho = s_h[tid] - hs;
     for (int j = j0; j < j1; ++j) {
         const int s = a.sorder[j];
         if (a.sys_done[s]) continue;
         a.act_sys[k] = s;
-        a.act_ecum[k] = eo;
+        a.act_tcum[k] = eo;
         a.act_hcum[k] = ho;
-        eo += (long long)a.sn[s] << a.slog[s];
+        eo += int(system_tiles(a.sn[s], a.slog[s]));
         ho += a.sn[s] * a.per;
         ++k;
     }
     if (tid == T - 1) {
         *a.act_count = s_cnt[tid];
-        a.act_ecum[s_cnt[tid]] = s_el[tid];
+        a.act_tcum[s_cnt[tid]] = s_el[tid];
         a.act_hcum[s_cnt[tid]] = s_h[tid];
     }
 }
@@ -277,6 +396,7 @@ __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphCondition
     __shared__ int s_conv;
     if (threadIdx.x == 0) s_conv = 0;
     __syncthreads();
+    int changed = 0;
     BatchState st = *a.st;
     const int it = st.iter + 1;
     const bool check = (it % st.check_freq) == 0 || it >= st.max_iters;
@@ -297,10 +417,13 @@ __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphCondition
     for (int s = threadIdx.x; s < a.nsys; s += blockDim.x) {
         int all = 1;
         for (int r = 0; r < a.nrhs[s]; ++r) all &= a.conv_iter[size_t(s) * a.pw + r] >= 0;
-        a.sys_done[s] = all;
+        if (a.sys_done[s] != all) {
+            a.sys_done[s] = all;
+            changed = 1;
+        }
     }
-    __syncthreads();
-    build_active(a);
+    // The list stands while no system finishes.
+    if (__syncthreads_or(changed)) build_active(a);
     if (threadIdx.x == 0) {
         st.iter = it;
         st.converged = s_conv;
@@ -318,66 +441,63 @@ __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphCondition
     }
 }
 
-// Per-(system, column) sums of squares of one tile: a warp whose 32
-// elements all belong to one system reduces the lanes of each column with
-// shuffles and its lanes r < W keep the column sums in registers (a lane's
-// column stays the same from tile to tile while its system does), adding
-// them into the global sums only when the lane's system changes or the loop
-// ends; a warp that straddles systems adds each lane's square directly.
+// Per-(system, column) sums of squares: a thread's columns stay the same from
+// tile to tile of its system, so it keeps their sums in registers; when the
+// block leaves the system the lanes of each column group add them with
+// shuffles and the first of them adds into the global sums.
 struct PairSums {
     double* sums;   // [nsys][pw]
     int pw;
-    int s = -1, r = 0;
-    double v = 0.0;
-    __device__ __forceinline__ void flush() {
-        if (s >= 0 && v != 0.0) atomicAdd(&sums[size_t(s) * pw + r], v);
-        s = -1;
-        v = 0.0;
-    }
-    __device__ __forceinline__ void add(int sys, int c, int rr, double sq) {
-        const unsigned full = 0xffffffffu;
-        const int s0 = __shfl_sync(full, sys, 0);
-        const int c0 = __shfl_sync(full, c, 0);
-        if (__all_sync(full, sys == s0) && s0 >= 0) {
-            double x = sq;
-            for (int d = 16; d >= (1 << c0); d >>= 1) x += __shfl_xor_sync(full, x, d);
-            if ((threadIdx.x & 31) < (1 << c0)) {
-                if (s != s0 || r != rr) {
-                    flush();
-                    s = s0;
-                    r = rr;
-                }
-                v += x;
+    int s = -1, c = 0, g = 0;
+    double v[2] = {0.0, 0.0};
+    __device__ __forceinline__ void flush() {  // the whole warp
+        if (s >= 0) {
+            const int ul = unit_log(c), cols = unit_cols(c);
+            for (int d = 16; d >= (1 << ul); d >>= 1) {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+                v[1] += __shfl_xor_sync(0xffffffffu, v[1], d);
             }
-        } else if (sys >= 0 && sq != 0.0) {
-            atomicAdd(&sums[size_t(sys) * pw + rr], sq);
+            if ((threadIdx.x & 31) < (1 << ul))
+                for (int n = 0; n < cols; ++n)
+                    if (v[n] != 0.0) atomicAdd(&sums[size_t(s) * pw + g * cols + n], v[n]);
         }
+        v[0] = v[1] = 0.0;
+    }
+    __device__ __forceinline__ void enter(const Unit& q) {
+        flush();
+        s = q.s;
+        c = q.c;
+        g = q.g;
     }
 };
 
-// rp = D^-1 (b - S x) and the per-(system, rhs) sums of squares.  CORR: x is
-// this iteration's corrected iterate (formed on the fly at the neighbours
-// and written to X), otherwise Xin.  CHECK: the last block to finish runs
-// the convergence test (the other blocks' sums are complete and visible by
-// then).
-template <bool CORR, bool CHECK>
-__global__ void __launch_bounds__(kThreads, 6) k_b_update(BatchArgs a, const double* Xin, int use_cond,
-                                                       cudaGraphConditionalHandle handle) {
+// rp = D^-1 (b - S x) and the per-(system, rhs) sums of squares.  CHECK: the
+// last block to finish runs the convergence test (the other blocks' sums are
+// complete and visible by then).
+template <bool CHECK>
+__global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, int use_cond,
+                                                         cudaGraphConditionalHandle handle) {
     PairSums ps{a.norm2, a.pw};
-    for_elements(a, [&](bool live, const Elem& q) {
-        double sq = 0.0;
-        if (live) {
-            double acc = 0.0;
-            for (int p = a.rp[q.i]; p < a.rp[q.i + 1]; ++p) {
-                const size_t k = size_t(q.base + ((long long)a.ci[p] << q.c) + q.r);
-                acc = fma(a.v[p], CORR ? corrected(a, k) : Xin[k], acc);
+    Ahead h;
+    auto enter = [&](const Unit& q, bool live, int i) {
+        ps.enter(q);
+        if (live) h.load(a.S, i);
+    };
+    for_tiles(a, enter, [&](bool live, const Unit& q, int next) {
+        if (!live) return;
+        const size_t e = q.elem();
+        with_cols(q.c, [&](auto nt) {
+            constexpr int N = decltype(nt)::value;
+            const Cols<N> bv = ldn<N>(a.B + e);
+            const double di = a.dinv[q.i];
+            Cols<N> t = row_times<N>(a.S, q, a.X, h, next);
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                t.v[n] = di * (bv.v[n] - t.v[n]);
+                ps.v[n] += t.v[n] * t.v[n];
             }
-            if (CORR) a.X[q.e] = corrected(a, q.e);
-            const double rv = a.dinv[q.i] * (a.B[q.e] - acc);
-            a.RP[q.e] = rv;
-            sq = rv * rv;
-        }
-        ps.add(live ? q.s : -1, q.c, q.r, sq);
+            stn<N>(a.RP + e, t);
+        });
     });
     ps.flush();
     if (CHECK) {
@@ -395,13 +515,35 @@ __global__ void __launch_bounds__(kThreads, 6) k_b_update(BatchArgs a, const dou
 }
 
 // Before the loop: sums of squares of D^-1 b per pair (every system).
-__global__ void k_b_init_norms(BatchArgs a) {
+__global__ void __launch_bounds__(kThreads) k_b_init_norms(BatchArgs a) {
     PairSums ps{a.bnorm2, a.pw};
-    for_elements(a, [&](bool live, const Elem& q) {
-        const double v = live ? a.dinv[q.i] * a.B[q.e] : 0.0;
-        ps.add(live ? q.s : -1, q.c, q.r, v * v);
+    auto enter = [&](const Unit& q, bool, int) { ps.enter(q); };
+    for_tiles(a, enter, [&](bool live, const Unit& q, int) {
+        if (!live) return;
+        const size_t e = q.elem();
+        with_cols(q.c, [&](auto nt) {
+            constexpr int N = decltype(nt)::value;
+            const Cols<N> bv = ldn<N>(a.B + e);
+            const double di = a.dinv[q.i];
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const double v = di * bv.v[n];
+                ps.v[n] += v * v;
+            }
+        });
     });
     ps.flush();
+}
+
+// Fixed-width rows from CSR rows of at most chunks * kRowChunk entries.
+__global__ void k_b_rows(const int* rp, const int* ci, const double* v, BatchRows M) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
+        const int p0 = rp[i], len = rp[i + 1] - p0;
+        for (int k = 0; k < M.chunks * kRowChunk; ++k) {
+            M.col[size_t(k) * M.n + i] = k < len ? ci[p0 + k] : i;
+            M.val[size_t(k) * M.n + i] = k < len ? v[p0 + k] : 0.0;
+        }
+    }
 }
 
 // Loop state, per-pair bookkeeping and the active list (every system), by
@@ -444,6 +586,7 @@ struct mclsgpu_batch {
     mclsgpu_operator* op = nullptr;
     mclsgpu_precond* pc = nullptr;
     mclsgpu_domain* dom = nullptr;
+    mclsgpu::BatchRows S, H;       // the operator and H in rows of fixed width
     int* d_nrhs = nullptr;
     // Per system (device): first row, first element, log2 width, rows, and
     // the systems in placement order.
@@ -454,13 +597,13 @@ struct mclsgpu_batch {
     int* d_sorder = nullptr;
     // The active list (rebuilt every iteration) and the list of every system.
     int* act_sys = nullptr;
-    long long* act_ecum = nullptr;
+    int* act_tcum = nullptr;
     int* act_hcum = nullptr;
     int* act_count = nullptr;
     int* all_sys = nullptr;
-    long long* all_ecum = nullptr;
+    int* all_tcum = nullptr;
     int* all_count = nullptr;
-    double *X = nullptr, *X2 = nullptr, *RP = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
+    double *X = nullptr, *RP = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
     float* cR = nullptr;
     double* norm2 = nullptr;
     double* bnorm2 = nullptr;
@@ -477,7 +620,7 @@ struct mclsgpu_batch {
     int grab = 1;                  // walk work-queue grab, in 32-history chunks
     // Grids of the element kernels: every block resident at once (each block
     // takes one contiguous range, so a second wave would double the time).
-    int g_rich = 1, g_src = 1, g_upd = 1, g_upd0 = 1, g_init = 1;
+    int g_rich = 1, g_src = 1, g_cor = 1, g_upd = 1, g_upd0 = 1, g_init = 1;
 };
 
 namespace mclsgpu {
@@ -488,6 +631,10 @@ void batch_release(mclsgpu_batch* b) {
     if (b->dom) mclsgpu_domain_destroy(b->dom);
     if (b->pc) mclsgpu_precond_destroy(b->pc);
     if (b->op) mclsgpu_operator_destroy(b->op);
+    dfree(b->S.col);
+    dfree(b->S.val);
+    dfree(b->H.col);
+    dfree(b->H.val);
     dfree(b->d_nrhs);
     dfree(b->d_srow0);
     dfree(b->d_seoff);
@@ -495,14 +642,13 @@ void batch_release(mclsgpu_batch* b) {
     dfree(b->d_sn);
     dfree(b->d_sorder);
     dfree(b->act_sys);
-    dfree(b->act_ecum);
+    dfree(b->act_tcum);
     dfree(b->act_hcum);
     dfree(b->act_count);
     dfree(b->all_sys);
-    dfree(b->all_ecum);
+    dfree(b->all_tcum);
     dfree(b->all_count);
     dfree(b->X);
-    dfree(b->X2);
     dfree(b->RP);
     dfree(b->RP2);
     dfree(b->B);
@@ -518,6 +664,20 @@ void batch_release(mclsgpu_batch* b) {
     delete b;
 }
 
+int fixed_rows(mclsgpu_context* ctx, const DevCsr& A, int longest, BatchRows& M) {
+    M.n = A.n;
+    M.chunks = std::max(1, (longest + kRowChunk - 1) / kRowChunk);
+    const size_t entries = size_t(M.n) * M.chunks * kRowChunk;
+    cudaError_t e;
+    if ((e = dmalloc(&M.col, entries)) != cudaSuccess ||
+        (e = dmalloc(&M.val, entries)) != cudaSuccess)
+        return cuda_fail(ctx, e, "cudaMalloc batch rows");
+    const int grid = std::min((M.n + kThreads - 1) / kThreads, ctx->num_sms * 8);
+    k_b_rows<<<grid, kThreads, 0, ctx->stream>>>(A.rp, A.ci, A.v, M);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(ctx, e, "batch rows");
+}
+
 // Kernel arguments over the active list (all = false) or every system.
 BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) {
     const mclsgpu_mc_params& p = b->dom->p;
@@ -525,28 +685,23 @@ BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) 
     a.nsys = b->nsys;
     a.pw = b->pw;
     a.per = b->per;
-    a.rp = b->op->A.rp;
-    a.ci = b->op->A.ci;
-    a.v = b->op->A.v;
+    a.S = b->S;
     a.dinv = b->pc->diag;
-    a.hrp = b->dom->D.rp;
-    a.hci = b->dom->D.ci;
-    a.hv = b->dom->D.v;
+    a.H = b->H;
     a.srow0 = b->d_srow0;
     a.seoff = b->d_seoff;
     a.slog = b->d_slog;
     a.sn = b->d_sn;
     a.sorder = b->d_sorder;
     a.lsys = all ? b->all_sys : b->act_sys;
-    a.lecum = all ? b->all_ecum : b->act_ecum;
+    a.ltcum = all ? b->all_tcum : b->act_tcum;
     a.lcount = all ? b->all_count : b->act_count;
     a.act_sys = b->act_sys;
-    a.act_ecum = b->act_ecum;
+    a.act_tcum = b->act_tcum;
     a.act_hcum = b->act_hcum;
     a.act_count = b->act_count;
     a.B = b->B;
     a.X = b->X;
-    a.X2 = b->X2;
     a.RP = b->RP;
     a.RP2 = b->RP2;
     a.Y = b->Y;
@@ -576,7 +731,8 @@ int resident_grid(K kernel, int sms) {
     return sms * (b > 0 ? b : 1);
 }
 
-// One batched MCSA iteration (4 kernels) over the active systems.
+// One batched MCSA iteration (4 kernels; 5 with several histories per row)
+// over the active systems.
 int enqueue_batch_iteration(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, int use_cond,
                             cudaGraphConditionalHandle handle) {
     cudaStream_t s = b->ctx->stream;
@@ -584,9 +740,11 @@ int enqueue_batch_iteration(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, int
     k_b_richardson_residual<<<b->g_rich, kThreads, 0, s>>>(a);
     k_b_source<<<b->g_src, kThreads, 0, s>>>(a);
     const BatchList list{b->act_sys, b->act_hcum, b->act_count, b->d_srow0};
-    int rc = launch_walk_batch(b->dom, b->cls, list, b->cR, b->Y, b->grab);
+    const BatchFinish fin{b->X, b->RP, b->RP2, a.omega, a.nomega, a.inv_per, a.ev};
+    int rc = launch_walk_batch(b->dom, b->cls, list, b->cR, b->Y, fin, b->grab);
     if (rc) return rc;
-    k_b_update<true, true><<<b->g_upd, kThreads, 0, s>>>(a, nullptr, use_cond, handle);
+    if (b->Y) k_b_correct<<<b->g_cor, kThreads, 0, s>>>(a);
+    k_b_update<true><<<b->g_upd, kThreads, 0, s>>>(a, use_cond, handle);
     return MCLSGPU_OK;
 }
 
@@ -702,7 +860,8 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
     }
     // Per-system tables and the list of every system (placement order).
     std::vector<int> srow0(nsys), sn(nsys), all_count(1, nsys);
-    std::vector<long long> seoff(nsys), all_ecum(nsys + 1, 0);
+    std::vector<long long> seoff(nsys);
+    std::vector<int> all_tcum(nsys + 1, 0);
     for (int s = 0; s < nsys; ++s) {
         srow0[s] = int(row0[s]);
         seoff[s] = eoff[s];
@@ -710,7 +869,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
     }
     for (int k = 0; k < nsys; ++k) {
         const int s = order[k];
-        all_ecum[k + 1] = all_ecum[k] + ((long long)n[s] << cls_of[s]);
+        all_tcum[k + 1] = all_tcum[k] + int(system_tiles(int(n[s]), cls_of[s]));
     }
     int rc = mclsgpu_operator_upload(ctx, N, rp.data(), ci.data(), v.data(), &b->op);
     mclsgpu_precond_params pp{};
@@ -729,6 +888,11 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
     if (!rc && (b->dom->slots > 16 || b->dom->rec_q16))
         rc = set_error(ctx, MCLSGPU_ERR_UNSUPPORTED,
                        "batched walks: rows of at most 15 retained entries");
+    // The rows of the element passes.
+    int longest = 0;
+    for (int64_t i = 0; i < N; ++i) longest = std::max(longest, int(rp[i + 1] - rp[i]));
+    if (!rc) rc = fixed_rows(ctx, b->op->A, longest, b->S);
+    if (!rc) rc = fixed_rows(ctx, b->dom->D, b->dom->max_row, b->H);
     const size_t PR = size_t(nsys) * pw;
     cudaError_t e = cudaSuccess;
     if (!rc &&
@@ -738,15 +902,16 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
          (e = dmalloc(&b->d_slog, nsys)) != cudaSuccess || (e = dmalloc(&b->d_sn, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->d_sorder, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->act_sys, nsys)) != cudaSuccess ||
-         (e = dmalloc(&b->act_ecum, nsys + 1)) != cudaSuccess ||
+         (e = dmalloc(&b->act_tcum, nsys + 1)) != cudaSuccess ||
          (e = dmalloc(&b->act_hcum, nsys + 1)) != cudaSuccess ||
          (e = dmalloc(&b->act_count, 1)) != cudaSuccess ||
          (e = dmalloc(&b->all_sys, nsys)) != cudaSuccess ||
-         (e = dmalloc(&b->all_ecum, nsys + 1)) != cudaSuccess ||
+         (e = dmalloc(&b->all_tcum, nsys + 1)) != cudaSuccess ||
          (e = dmalloc(&b->all_count, 1)) != cudaSuccess ||
-         (e = dmalloc(&b->X, NE)) != cudaSuccess || (e = dmalloc(&b->X2, NE)) != cudaSuccess ||
+         (e = dmalloc(&b->X, NE)) != cudaSuccess ||
          (e = dmalloc(&b->RP, NE)) != cudaSuccess || (e = dmalloc(&b->RP2, NE)) != cudaSuccess ||
-         (e = dmalloc(&b->B, NE)) != cudaSuccess || (e = dmalloc(&b->Y, NE)) != cudaSuccess ||
+         (e = dmalloc(&b->B, NE)) != cudaSuccess ||
+         (b->per > 1 && (e = dmalloc(&b->Y, NE)) != cudaSuccess) ||
          (e = dmalloc(&b->cR, NE)) != cudaSuccess || (e = dmalloc(&b->norm2, PR)) != cudaSuccess ||
          (e = dmalloc(&b->bnorm2, PR)) != cudaSuccess ||
          (e = dmalloc(&b->conv_iter, PR)) != cudaSuccess || (e = dmalloc(&b->sys_done, nsys)) != cudaSuccess ||
@@ -757,8 +922,9 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         const int sms = ctx->num_sms;
         b->g_rich = resident_grid(k_b_richardson_residual, sms);
         b->g_src = resident_grid(k_b_source, sms);
-        b->g_upd = resident_grid(k_b_update<true, true>, sms);
-        b->g_upd0 = resident_grid(k_b_update<false, false>, sms);
+        b->g_cor = resident_grid(k_b_correct, sms);
+        b->g_upd = resident_grid(k_b_update<true>, sms);
+        b->g_upd0 = resident_grid(k_b_update<false>, sms);
         b->g_init = resident_grid(k_b_init_norms, sms);
         cudaStream_t s = ctx->stream;
         cudaMemcpyAsync(b->d_nrhs, b->nrhs.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
@@ -769,15 +935,14 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         cudaMemcpyAsync(b->d_sn, sn.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->d_sorder, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->all_sys, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(b->all_ecum, all_ecum.data(), sizeof(long long) * (nsys + 1),
+        cudaMemcpyAsync(b->all_tcum, all_tcum.data(), sizeof(int) * (nsys + 1),
                         cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->all_count, all_count.data(), sizeof(int), cudaMemcpyHostToDevice, s);
         // Padding elements are never written by the loop: zero every array once.
         cudaMemsetAsync(b->X, 0, sizeof(double) * NE, s);
-        cudaMemsetAsync(b->X2, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->RP, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->RP2, 0, sizeof(double) * NE, s);
-        cudaMemsetAsync(b->Y, 0, sizeof(double) * NE, s);
+        if (b->Y) cudaMemsetAsync(b->Y, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->cR, 0, sizeof(float) * NE, s);
         cudaMemsetAsync(b->blocks_done, 0, sizeof(unsigned), s);
         e = cudaStreamSynchronize(s);
@@ -904,8 +1069,7 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
     k_b_state_init<<<1, 1024, 0, s>>>(a, params->max_iters, params->check_freq,
                                        params->tolerance, pairs);
     k_b_init_norms<<<b->g_init, kThreads, 0, s>>>(a);
-    k_b_update<false, false><<<b->g_upd0, kThreads, 0, s>>>(a, b->X, 0,
-                                                          cudaGraphConditionalHandle(0));
+    k_b_update<false><<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
     cudaMemsetAsync(b->norm2, 0, sizeof(double) * PR, s);
     cudaError_t e = cudaSuccess;
     int rc = MCLSGPU_OK;
@@ -938,8 +1102,7 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
         std::vector<double> nr(PR), bn(PR);
         std::vector<int> ci(PR);
         cudaMemsetAsync(b->norm2, 0, sizeof(double) * PR, s);
-        k_b_update<false, false><<<b->g_upd0, kThreads, 0, s>>>(a, b->X, 0,
-                                                              cudaGraphConditionalHandle(0));
+        k_b_update<false><<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
         cudaMemcpyAsync(nr.data(), b->norm2, sizeof(double) * PR, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(bn.data(), b->bnorm2, sizeof(double) * PR, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(ci.data(), b->conv_iter, sizeof(int) * PR, cudaMemcpyDeviceToHost, s);

@@ -370,16 +370,36 @@ struct BatchList {
     const int* lcount;
     const int* srow0;   // system -> its first row
 };
+// The iterate after a batched iteration's smoothing step and correction.
+struct BatchFinish {
+    double* X;
+    const double* RP;
+    const double* RP2;
+    double omega;        // Richardson relaxation
+    double nomega;       // Neumann relaxation (1 when absent)
+    double inv_per;      // 1 / histories per row
+    int ev;              // expected-value estimator
+};
+#if defined(__CUDACC__)
+__device__ __forceinline__ double batch_corrected(double x, double rp, double rp2, double y,
+                                                  double omega, double nomega, double inv_per,
+                                                  int ev) {
+    const double x2 = __dadd_rn(x, __dmul_rn(omega, rp));
+    double d = y * inv_per;
+    if (ev) d += nomega * rp2;
+    return x2 + d;
+}
+#endif
 // Forward walks shared by the right-hand sides of a batch: every history
 // carries one Kahan-compensated FP32 tally per column of its start row's
-// class, reading the tally source cR at each state's elements and adding into
-// Y at the start row's elements.  Only the listed systems' histories run;
-// history h of system s is history srow0[s] * per + (h - hcum[k]) of the
-// whole batch, on that history's own random stream, whatever the list.
-// Each warp takes 32 * grab histories per work-queue grab.  The work-queue
-// counter must be zero on entry; the caller resets it afterwards.
+// class, reading the tally source cR at each state's elements.  With one
+// history per row the walk finishes the row (BatchFinish, Y null); otherwise
+// the tallies are added into Y at the start row's elements.  Only the listed
+// systems' histories run; history h of system s is history srow0[s] * per + (h
+// - hcum[k]) of the whole batch, on that history's own random stream, whatever
+// the list.  Each warp takes 32 * grab consecutive histories at a time.
 int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchList& list,
-                      const float* cR, double* Y, int grab);
+                      const float* cR, double* Y, const BatchFinish& fin, int grab);
 
 // ---- MCSA helpers (mcsa.cu) ----------------------------------------------------
 // rp_out = PL (b - A PR x)   (LinearProblem::updatePrecResidual)

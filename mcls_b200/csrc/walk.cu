@@ -690,6 +690,7 @@ namespace {
 struct BatchWalk {
     const float* cR;
     double* Y;
+    BatchFinish fin;
     BatchList list;
     BatchClasses cls;
     int grab;
@@ -709,15 +710,20 @@ __device__ __forceinline__ int list_entry(const int* hcum, int count, int h) {
 // The tally-source row of state s in class c (W = 2^c columns).
 template <int W>
 __device__ __forceinline__ void load_source_row(const float* p, float (&c)[W]) {
-    if constexpr (W >= 4) {
+    if constexpr (W >= 8) {
 #pragma unroll
-        for (int r = 0; r < W; r += 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(p + r));
-            c[r] = q.x;
-            c[r + 1] = q.y;
-            c[r + 2] = q.z;
-            c[r + 3] = q.w;
+        for (int r = 0; r < W; r += 8) {
+            uint32_t q[8];
+            ld_record256_l1(p + r, q);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) c[r + t] = __uint_as_float(q[t]);
         }
+    } else if constexpr (W == 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        c[0] = q.x;
+        c[1] = q.y;
+        c[2] = q.z;
+        c[3] = q.w;
     } else if constexpr (W == 2) {
         const float2 q = __ldg(reinterpret_cast<const float2*>(p));
         c[0] = q.x;
@@ -731,7 +737,7 @@ __device__ __forceinline__ void load_source_row(const float* p, float (&c)[W]) {
 template <int S, bool ST, int C>
 __device__ __forceinline__ unsigned batch_history(const WalkArgs& a, const char* rec,
                                                   const int* soff, const BatchWalk& m, int s,
-                                                  float w, uint64_t x) {
+                                                  float w, uint64_t x, double* stage) {
     constexpr int W = 1 << C;
     const int r0 = m.cls.crow[C];
     const float* cbase = m.cR + m.cls.cel[C];
@@ -754,11 +760,45 @@ __device__ __forceinline__ unsigned batch_history(const WalkArgs& a, const char*
         walk_step<S, MCLSGPU_FORWARD, ST ? kStencil : kPacked, false>(rec, nullptr, soff, s, w, x, da, dc,
                                                                  k);
     }
+    if (!m.Y) {
+        // The row's only history: its sums go to the warp's finishing pass.
+#pragma unroll
+        for (int r = 0; r < W; ++r) stage[r] = double(acc[r]) - double(comp[r]);
+        return unsigned(L);
+    }
     double* y = m.Y + m.cls.cel[C] + size_t(s0 - r0) * W;
 #pragma unroll
     for (int r = 0; r < W; ++r)
         if (acc[r] != 0.f || comp[r] != 0.f) atomicAdd(&y[r], double(acc[r]) - double(comp[r]));
     return unsigned(L);
+}
+
+// Sums of one lane in the warp's stage: 16 columns and a word of padding, so
+// that the lanes' writes spread over the banks.
+constexpr int kBatchStage = 17;
+
+// The iterate of the warp's 32 rows from their staged sums.  The rows of a
+// warp inside one class and one run of rows are consecutive elements, which
+// the lanes take in order (a lane writing its own row's columns would touch 32
+// lines per column: 450 us for a walk of 97); otherwise row by row.
+__device__ __forceinline__ void finish_rows(const BatchWalk& m, const double* stage, int row,
+                                            int c, bool live) {
+    const BatchFinish& f = m.fin;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    const int row0 = __shfl_sync(kFull, row, 0), c0 = __shfl_sync(kFull, c, 0);
+    auto finish = [&](size_t e, double y) {
+        f.X[e] = batch_corrected(f.X[e], f.RP[e], f.RP2[e], y, f.omega, f.nomega, f.inv_per, f.ev);
+    };
+    if (__all_sync(kFull, live && c == c0 && row == row0 + lane)) {
+        const size_t e0 = size_t(m.cls.cel[c0]) + (size_t(row0 - m.cls.crow[c0]) << c0);
+        for (int t = lane; t < (32 << c0); t += 32)
+            finish(e0 + t, stage[(t >> c0) * kBatchStage + (t & ((1 << c0) - 1))]);
+    } else if (live) {
+        const size_t e0 = size_t(m.cls.cel[c]) + (size_t(row - m.cls.crow[c]) << c);
+        for (int r = 0; r < (1 << c); ++r) finish(e0 + r, stage[lane * kBatchStage + r]);
+    }
+    __syncwarp();
 }
 
 template <int S, bool ST>
@@ -767,25 +807,28 @@ __global__ void __launch_bounds__(256, 3) walk32_batch(WalkArgs a, BatchWalk m) 
     __shared__ uint64_t s_ekey;
     __shared__ int s_nh, s_count;
     __shared__ int s_off[32];
+    // One history per row: the warps' sums, kBatchStage doubles per lane.
+    extern __shared__ double s_stage[];
     stage_offsets(a.stoff, s_off);
     const int lane = threadIdx.x & 31;
+    double* warp_stage = s_stage + (threadIdx.x >> 5) * (32 * kBatchStage);
+    double* mine = warp_stage + lane * kBatchStage;
     if (threadIdx.x == 0) {
         s_ekey = epoch_key(a.seed, *a.d_epoch);
         s_count = *m.list.lcount;
         s_nh = s_count > 0 ? m.list.hcum[s_count] : 0;
     }
     __syncthreads();
+    walk_begin_time(a);
     const char* rec = reinterpret_cast<const char*>(a.rec);
-    if (lane == 0) atomicMin(&a.d_tim[0], global_ns());
     unsigned steps = 0;
-    const int chunk = 32 * m.grab;
-    const int count = s_count;
-    while (true) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(a.d_counter, chunk);
-        base = __shfl_sync(kFull, base, 0);
-        const int nh = s_nh;
-        if (base >= nh) break;
+    // Every history takes the same number of steps: the warps take their
+    // chunks statically (a shared counter is one contended atomic per chunk).
+    const int chunk = 32 * m.grab, warps = gridDim.x * (blockDim.x >> 5);
+    const int count = s_count, nh = s_nh;
+    const int w0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (long long first = (long long)w0 * chunk; first < nh; first += (long long)warps * chunk) {
+        const int base = int(first);
         // The list entry of the grab's first history (one search per warp);
         // the lanes step forward from it.
         int k0 = 0;
@@ -793,44 +836,51 @@ __global__ void __launch_bounds__(256, 3) walk32_batch(WalkArgs a, BatchWalk m) 
         k0 = __shfl_sync(kFull, k0, 0);
         for (int g = 0; g < m.grab; ++g) {
             const int h = base + 32 * g + lane;
-            if (h >= nh) break;
+            if (base + 32 * g >= nh) break;  // the whole warp
+            // A lane past the end walks the last history and drops its sums.
+            const bool live = h < nh;
+            const int hh = live ? h : nh - 1;
             int k = k0;
-            while (k + 1 < count && h >= m.list.hcum[k + 1]) ++k;
+            while (k + 1 < count && hh >= m.list.hcum[k + 1]) ++k;
             const int sys = m.list.lsys[k];
-            const int e = m.list.srow0[sys] * m.per + (h - m.list.hcum[k]);
+            const int e = m.list.srow0[sys] * m.per + (hh - m.list.hcum[k]);
             int s;
             float w;
             uint64_t x;
             walk_start<MCLSGPU_FORWARD>(a, e, s_ekey, 1.f, s, w, x);
             int c = 0;
             while (c < 4 && s >= m.cls.crow[c + 1]) ++c;
+            const int row = s;
+            if (!live && m.Y) continue;  // (per > 1: no warp-wide pass follows)
             switch (c) {
-                case 0: steps += batch_history<S, ST, 0>(a, rec, s_off, m, s, w, x); break;
-                case 1: steps += batch_history<S, ST, 1>(a, rec, s_off, m, s, w, x); break;
-                case 2: steps += batch_history<S, ST, 2>(a, rec, s_off, m, s, w, x); break;
-                case 3: steps += batch_history<S, ST, 3>(a, rec, s_off, m, s, w, x); break;
-                default: steps += batch_history<S, ST, 4>(a, rec, s_off, m, s, w, x); break;
+                case 0: steps += batch_history<S, ST, 0>(a, rec, s_off, m, s, w, x, mine); break;
+                case 1: steps += batch_history<S, ST, 1>(a, rec, s_off, m, s, w, x, mine); break;
+                case 2: steps += batch_history<S, ST, 2>(a, rec, s_off, m, s, w, x, mine); break;
+                case 3: steps += batch_history<S, ST, 3>(a, rec, s_off, m, s, w, x, mine); break;
+                default: steps += batch_history<S, ST, 4>(a, rec, s_off, m, s, w, x, mine); break;
             }
+            if (m.Y) continue;
+            if (!live) steps -= unsigned(a.L);
+            finish_rows(m, warp_stage, row, c, live);
         }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) steps += __shfl_down_sync(kFull, steps, d);
-    if (lane == 0) {
-        if (steps) atomicAdd(a.d_steps, (unsigned long long)steps);
-        atomicMax(&a.d_tim[1], global_ns());
-    }
+    if (lane == 0 && steps) atomicAdd(a.d_steps, (unsigned long long)steps);
+    walk_end_time(a);
 }
 
 template <int S, bool ST>
 void launch_batch_s(const WalkArgs& a, const BatchWalk& m, int sms, int block, cudaStream_t st) {
     static int cached[2] = {0, 0};
     const int slot = block == 128 ? 0 : 1;
+    const size_t smem = size_t(block) * kBatchStage * sizeof(double);  // at most 34 KB
     if (!cached[slot]) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32_batch<S, ST>, block, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32_batch<S, ST>, block, smem);
         cached[slot] = b > 0 ? b : 1;
     }
-    walk32_batch<S, ST><<<sms * cached[slot], block, 0, st>>>(a, m);
+    walk32_batch<S, ST><<<sms * cached[slot], block, smem, st>>>(a, m);
 }
 
 }  // namespace
@@ -863,7 +913,7 @@ static void fill_walk_args(mclsgpu_domain* dom, WalkArgs& a) {
 // Batched forward walks over the domain's FP32 records (records of at most
 // 16 slots; see launch_walk_batch in internal.h).
 int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchList& list,
-                      const float* cR, double* Y, int grab) {
+                      const float* cR, double* Y, const BatchFinish& fin, int grab) {
     mclsgpu_context* ctx = dom->ctx;
     if (dom->p.precision != MCLSGPU_FP32 || dom->p.direction != MCLSGPU_FORWARD || !dom->slots ||
         dom->rec_q16)
@@ -876,7 +926,7 @@ int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchL
     const int sms = ctx->num_sms;
     const int block = dom->walk_block;
     cudaStream_t st = ctx->stream;
-    const BatchWalk m{cR, Y, list, cls, grab, a.per};
+    const BatchWalk m{cR, Y, fin, list, cls, grab, a.per};
     bool ok = true;
     if (dom->stencil_k) {
         switch (dom->slots) {
