@@ -407,8 +407,9 @@ void prec_residual(mclsgpu_domain* dom, const double* x, const double* b, double
 // y = PL A PR x   (LinearProblem::apply); uses dom->tmp and dom->tmp2.
 void composite_apply(mclsgpu_domain* dom, const double* x, double* y);
 // x2 = x + w r (unless x2 is null); r2 = PL (b - A PR x2) for r = PL (b - A PR x),
-// formed as r - w PL A PR r: one fused pass when PL is I or point Jacobi and
-// there is no PR, two when PL is held on A's diagonals (x2 != x, r2 != r).
+// formed as r - w PL A PR r for forward domains: one fused pass when PL is I or
+// point Jacobi and there is no PR, two when PL is held on A's diagonals (x2 !=
+// x, r2 != r).  dom->x2 may be overwritten.
 void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, double w,
                          double* x2, double* r2);
 // out = the Monte Carlo estimate for the source v (already left

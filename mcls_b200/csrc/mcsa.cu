@@ -313,6 +313,23 @@ __global__ void __launch_bounds__(kFusedThreads) k_richardson_residual(
     }
 }
 
+// The same residual as b - A x2 with x2 = x + w rp formed at the neighbours on
+// the fly: adjoint domains.  Their history count is a quotient truncated to an
+// integer, int(Nh * |b|_1 / |b|_1) (src/MCLS_UniformAdjointSource_impl.hpp:198),
+// which the last bit of the source's norm moves between Nh and Nh - 1, so the
+// source keeps the reference's own arithmetic.
+template <class Op>
+__global__ void __launch_bounds__(kFusedThreads) k_smoothed_residual(
+    Op A, const double* b, const double* dinv, const double* x, const double* r, double w,
+    double* x2, double* r2) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
+        const double s = A.dot(i, [&](int j) { return __dadd_rn(x[j], __dmul_rn(w, r[j])); });
+        const double res = b[i] - s;
+        r2[i] = dinv ? dinv[i] * res : res;
+        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
+    }
+}
+
 struct ResidArgs {
     int n;
     const double* b;
@@ -404,8 +421,14 @@ __global__ void __launch_bounds__(kFusedThreads) k_residual_norm(Op A, ResidArgs
     norm_and_check(a, acc);
 }
 
-// The same step with a left preconditioner M stored on A's diagonals (learned
-// SPAI): rp2 = rp - w M v with v = A rp.
+// A left preconditioner M stored on A's diagonals (learned SPAI): out = M v.
+template <class Op>
+__global__ void __launch_bounds__(kFusedThreads) k_dia_apply(Op M, const double* v, double* out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x)
+        out[i] = M.dot(i, [&](int j) { return v[j]; });
+}
+
+// The Richardson step with it: rp2 = rp - w M v with v = A rp.
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_dia_richardson(Op M, const double* v,
                                                                  const double* x, const double* r,
@@ -809,6 +832,12 @@ static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x
     return MCLSGPU_OK;
 }
 
+// x2 = x + w r (rounded as the reference's vector update)
+__global__ void k_axpy_to(const double* x, const double* r, double w, double* x2, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
+}
+
 // The Richardson step from y = PL A PR r in r2: r2 = r - w y and, when x2 is
 // not null, x2 = x + w r (rounded as the reference's vector update).
 __global__ void k_richardson_step(const double* x, const double* r, double w, double* x2,
@@ -845,10 +874,25 @@ void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, 
     const mclsgpu_operator* op = dom->op;
     const int grid = fused_grid(dom);
     const mclsgpu_precond* L = dom->left;
-    if (!dom->right && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI)) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual,
-                          L ? L->diag : nullptr, x, r, w, x2, r2);
-    } else if (!dom->right && L->mdia && op->dia_k > 0) {
+    const bool diag = !dom->right && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI);
+    const bool mdia = !diag && !dom->right && L->mdia && op->dia_k > 0;
+    const double* dinv = diag && L ? L->diag : nullptr;
+    if (dom->p.direction == MCLSGPU_ADJOINT) {
+        if (diag) {
+            MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b, dinv, x, r, w,
+                              x2, r2);
+        } else if (mdia) {
+            MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b, nullptr, x,
+                              r, w, x2, dom->tmp);
+            MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, r2);
+        } else {
+            double* xs = x2 ? x2 : dom->x2;
+            k_axpy_to<<<grid, kFusedThreads, 0, s>>>(x, r, w, xs, dom->n);
+            update_prec_residual(dom, xs, dom->b, r2);
+        }
+    } else if (diag) {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dinv, x, r, w, x2, r2);
+    } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_matvec, r, nullptr, dom->tmp);
         MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_richardson, dom->tmp, x, r, w,
                          x2, r2);

@@ -577,10 +577,11 @@ __global__ void k_forward_nh(int* d_nh, int nh, double* sc) {
 // shared memory, and expands it into starting states behind the eighths above
 // it (LIFO emission order).
 //
-// What bounds it: the chain of barriers and shared-memory round trips.  Each
-// thread owns an odd number of consecutive states (no bank conflicts), so each
-// scan is one block scan; the searches' power-of-two probes are spread over
-// the banks by a swizzle.  At 100^2 it takes 13 us of a 42 us MCSA iteration;
+// What bounds it: the chain of barriers and shared-memory round trips.  The
+// warps scan 32 states at a time for all chunks of 1,024 at once and only the
+// chunks' carries are serial; the searches' power-of-two probes are spread
+// over the banks by a swizzle (70 us without).  The sums' association is
+// fixed: it decides the truncated history count.  At 100^2 it takes 13 us of a 42 us MCSA iteration;
 // one CTA with a scan per 1,024 states took 44 of 72 us.  Up to kSmallSlice
 // states one CTA does it all (C = 1): the draws are then few and a cluster of 8
 // costs 4 us more than it saves (a solve of 1,024 states 63 against 67 us).
@@ -623,6 +624,16 @@ __device__ __forceinline__ T block_scan_excl(T x, T* warp_tot, T* total) {
     return r;
 }
 
+// Inclusive scan of one value per lane.
+__device__ __forceinline__ double warp_scan(double x, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    return x;
+}
+
 // Shared memory: the CDF (n doubles, swizzled) and the counts of the CTA's
 // states (the state's sign in the top bit).
 constexpr int kSmallSmem = kSmallSourceMax * sizeof(double) + kSmallSlice * sizeof(int);
@@ -635,48 +646,80 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kSmallThreads)
     extern __shared__ __align__(16) unsigned char smem_src[];
     double* cdf = reinterpret_cast<double*>(smem_src);
     int* counts = reinterpret_cast<int*>(smem_src + sizeof(double) * kSmallSourceMax);
-    __shared__ double wtot[32];
+    constexpr int kChunks = kSmallSourceMax / kSmallThreads;
+    __shared__ double wsum[kChunks][32];   // a chunk's warp sums, then their scan
+    __shared__ double wabs[32];            // chunk 0's with |v[0]|
+    __shared__ double carry[kChunks + 1];
+    __shared__ double s_norm1;
     __shared__ int wtoti[32];
     __shared__ int s_slice[C];
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int tid = threadIdx.x, rank = int(cluster.block_rank());
+    const int lane = tid & 31, wid = tid >> 5;
     const int slice = (n + C - 1) / C;
     const int j0 = min(rank * slice, n), j1 = min(j0 + slice, n);  // this CTA's states
     const unsigned long long epoch = *d_epoch;
-    // 1. Terms of the CDF (signed first element) and the states' signs.
-    for (int i = tid; i < n; i += kSmallThreads) {
-        const double b = load_src(v, i, omega, has);
-        cdf[swizzle(i)] = i == 0 ? b : fabs(b);
-        if (i >= j0 && i < j1) counts[i - j0] = b > 0.0 ? 0 : INT_MIN;
+    const int chunks = (n + kSmallThreads - 1) / kSmallThreads;
+    // 1. Terms of the CDF (signed first element), scanned within each warp of
+    //    32 states, and the states' signs.
+    constexpr int kAhead = 4;
+    for (int c0 = 0; c0 < chunks; c0 += kAhead) {
+        double b[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int i = (c0 + q) * kSmallThreads + tid;
+            b[q] = i < n ? load_src(v, i, omega, has) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int c = c0 + q, i = c * kSmallThreads + tid;
+            if (c >= chunks) break;
+            if (i >= j0 && i < j1) counts[i - j0] = b[q] > 0.0 ? 0 : INT_MIN;
+            const double x = warp_scan(i == 0 ? b[q] : fabs(b[q]), lane);
+            cdf[swizzle(i)] = x;
+            if (lane == 31) wsum[c][wid] = x;
+            if (c == 0) {
+                // The first warp's sum of magnitudes.
+                const double xa = wid == 0 ? warp_scan(fabs(b[q]), lane) : x;
+                if (lane == 31) wabs[wid] = xa;
+            }
+        }
     }
     __syncthreads();
-    const int items = ((n + kSmallThreads - 1) / kSmallThreads) | 1;
-    const int i0 = min(tid * items, n), i1 = min(i0 + items, n);
-    double sum = 0.0;
-    for (int i = i0; i < i1; ++i) sum += cdf[swizzle(i)];
-    double total;
-    double run = block_scan_excl(sum, wtot, &total);
-    // 2. |v|_1 -- the CDF's total unless the first element is negative -- and
-    //    the history count.
-    double norm1 = total;
-    if (cdf[0] < 0.0) {
-        if (tid == 0) {
-            sum = 0.0;
-            for (int i = i0; i < i1; ++i) sum += fabs(cdf[swizzle(i)]);
+    // 2. Scan of each chunk's warp sums, one warp per chunk.
+    if (wid < chunks) wsum[wid][lane] = warp_scan(wsum[wid][lane], lane);
+    if (wid == 31) wabs[lane] = warp_scan(wabs[lane], lane);
+    __syncthreads();
+    // 3. The chunks' carries, |v|_1 with the same association (so that it
+    //    equals the CDF's total when v[0] >= 0), and the history count.
+    if (tid == 0) {
+        double signed_sum = 0.0, abs_sum = 0.0;
+        for (int c = 0; c < chunks; ++c) {
+            const double last = cdf[swizzle(c * kSmallThreads + kSmallThreads - 1)];
+            carry[c] = signed_sum;
+            signed_sum = (last + wsum[c][30]) + signed_sum;
+            abs_sum = (last + (c == 0 ? wabs[30] : wsum[c][30])) + abs_sum;
         }
-        block_scan_excl(sum, wtot, &norm1);
+        carry[chunks] = signed_sum;
+        s_norm1 = abs_sum;
+        if (rank == 0) random_count(nh_req, abs_sum, signed_sum, cap, sc, d_nh, status);
     }
+    __syncthreads();
+    const double total = carry[chunks], norm1 = s_norm1;
     bool error;
     const int nh = history_count(nh_req, norm1, total, cap, &error);
-    if (rank == 0 && tid == 0) random_count(nh_req, norm1, total, cap, sc, d_nh, status);
-    // 3. Normalise (cdf[n-1] = 1 exactly), once every thread has read cdf[0].
-    __syncthreads();
-    for (int i = i0; i < i1; ++i) {
-        run += cdf[swizzle(i)];
-        cdf[swizzle(i)] = i == n - 1 ? 1.0 : run / total;
+    // 4. Normalise (cdf[n-1] = 1 exactly).
+#pragma unroll 4
+    for (int c = 0; c < chunks; ++c) {
+        const int i = c * kSmallThreads + tid;
+        if (i >= n) break;
+        double x = cdf[swizzle(i)];
+        if (wid > 0) x += wsum[c][wid - 1];
+        x += carry[c];
+        cdf[swizzle(i)] = i == n - 1 ? 1.0 : x / total;
     }
     cluster.sync();  // every CTA's counts are set
-    // 4. Draw the starting states (counter stream, kind 1), two searches in
+    // 5. Draw the starting states (counter stream, kind 1), two searches in
     //    flight per thread.
     const uint64_t ekey = epoch_key(seed, epoch);
     const int top = n > 1 ? 1 << (31 - __clz(n - 1)) : 0;
@@ -705,7 +748,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kSmallThreads)
             }
     }
     cluster.sync();
-    // 5. Emission (highest state first): a thread's run of states starts after
+    // 6. Emission (highest state first): a thread's run of states starts after
     //    the histories of the runs above it, a CTA's after the CTAs above it.
     constexpr int kOwn = kSmallSlice / kSmallThreads;
     const int t0 = min(j0 + tid * kOwn, j1), t1 = min(t0 + kOwn, j1);
