@@ -16,10 +16,10 @@
 // a system whose pairs have all met it stops (its rows and walks are
 // skipped), and the loop ends when every pair has met it or at the iteration
 // limit.  One iteration is four kernels in a CUDA graph whose WHILE node the
-// last one controls: the residual after the Richardson step, the tally source,
-// the shared walk -- which adds the step and the correction to the iterate
-// (with several histories per row, a pass of its own does) -- and residual +
-// per-pair norms, whose last block to finish runs the convergence test.
+// last one controls: the residual at the smoothed iterate, the tally source,
+// the shared walk -- which adds the correction to it (with several histories
+// per row, a pass of its own does) -- and residual + per-pair norms + the next
+// smoothed iterate, whose last block to finish runs the convergence test.
 //
 // The passes over the elements take them in units: one row by two
 // consecutive columns per thread (one 16-byte access), the entries from rows of
@@ -90,6 +90,7 @@ struct BatchArgs {
     int* act_count;
     const double* B;
     double* X;
+    double* X2;          // smoothed iterate x + w rp
     double* RP;
     double* RP2;
     double* Y;
@@ -261,10 +262,11 @@ __device__ __forceinline__ Cols<N> row_times(const BatchRows& M, const Unit& q, 
     return acc;
 }
 
-// The residual after the Richardson step x + w rp, from rp alone: rp2 = rp -
-// w D^-1 S rp (src/MCLS_RichardsonIteration_impl.hpp:134-147); Y (not null:
-// the walk adds into it) is cleared for this iteration's walk.
-__global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_richardson_residual(BatchArgs a) {
+// rp2 = D^-1 (b - S x2) at the smoothed iterate x2 = x + w rp (RichardsonIteration::
+// doOneIteration then updatePrecResidual, src/MCLS_RichardsonIteration_impl.hpp:
+// 134-147); Y (not null: the walk adds into it) is cleared for this
+// iteration's walk.
+__global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_smoothed_residual(BatchArgs a) {
     Ahead h;
     auto enter = [&](const Unit&, bool live, int i) {
         if (live) h.load(a.S, i);
@@ -274,11 +276,11 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_richardson_residual(
         const size_t e = q.elem();
         with_cols(q.c, [&](auto nt) {
             constexpr int N = decltype(nt)::value;
-            const Cols<N> r = ldn<N>(a.RP + e);
+            const Cols<N> bv = ldn<N>(a.B + e);
             const double di = a.dinv[q.i];
-            Cols<N> t = row_times<N>(a.S, q, a.RP, h, next);
+            Cols<N> t = row_times<N>(a.S, q, a.X2, h, next);
 #pragma unroll
-            for (int n = 0; n < N; ++n) t.v[n] = r.v[n] - a.omega * (di * t.v[n]);
+            for (int n = 0; n < N; ++n) t.v[n] = di * (bv.v[n] - t.v[n]);
             stn<N>(a.RP2 + e, t);
             if (a.Y) {
 #pragma unroll
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_source(BatchArgs a) 
     });
 }
 
-// x += w rp + Y / per (+ w rp2 for the expected value, the estimator's source
+// x = x2 + Y / per (+ w rp2 for the expected value, the estimator's source
 // term; ForwardTally::finalize, src/MCLS_ForwardTally_impl.hpp:180-209), when
 // the walk's rows have several histories.
 __global__ void __launch_bounds__(kThreads, 4) k_b_correct(BatchArgs a) {
@@ -324,12 +326,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_b_correct(BatchArgs a) {
         const size_t e = q.elem();
         with_cols(q.c, [&](auto nt) {
             constexpr int N = decltype(nt)::value;
-            Cols<N> x = ldn<N>(a.X + e);
-            const Cols<N> r = ldn<N>(a.RP + e), r2 = ldn<N>(a.RP2 + e), y = ldn<N>(a.Y + e);
+            Cols<N> x = ldn<N>(a.X2 + e);
+            const Cols<N> r2 = ldn<N>(a.RP2 + e), y = ldn<N>(a.Y + e);
 #pragma unroll
             for (int n = 0; n < N; ++n)
-                x.v[n] = batch_corrected(x.v[n], r.v[n], r2.v[n], y.v[n], a.omega, a.nomega,
-                                         a.inv_per, a.ev);
+                x.v[n] = batch_corrected(x.v[n], r2.v[n], y.v[n], a.nomega, a.inv_per, a.ev);
             stn<N>(a.X + e, x);
         });
     });
@@ -471,7 +472,8 @@ struct PairSums {
     }
 };
 
-// rp = D^-1 (b - S x) and the per-(system, rhs) sums of squares.  CHECK: the
+// rp = D^-1 (b - S x), the next smoothed iterate x2 = x + w rp and the
+// per-(system, rhs) sums of squares.  CHECK: the
 // last block to finish runs the convergence test (the other blocks' sums are
 // complete and visible by then).
 template <bool CHECK>
@@ -491,12 +493,15 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, 
             const Cols<N> bv = ldn<N>(a.B + e);
             const double di = a.dinv[q.i];
             Cols<N> t = row_times<N>(a.S, q, a.X, h, next);
+            Cols<N> x = ldn<N>(a.X + e);
 #pragma unroll
             for (int n = 0; n < N; ++n) {
                 t.v[n] = di * (bv.v[n] - t.v[n]);
                 ps.v[n] += t.v[n] * t.v[n];
+                x.v[n] = __dadd_rn(x.v[n], __dmul_rn(a.omega, t.v[n]));
             }
             stn<N>(a.RP + e, t);
+            stn<N>(a.X2 + e, x);
         });
     });
     ps.flush();
@@ -603,7 +608,7 @@ struct mclsgpu_batch {
     int* all_sys = nullptr;
     int* all_tcum = nullptr;
     int* all_count = nullptr;
-    double *X = nullptr, *RP = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
+    double *X = nullptr, *X2 = nullptr, *RP = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
     float* cR = nullptr;
     double* norm2 = nullptr;
     double* bnorm2 = nullptr;
@@ -649,6 +654,7 @@ void batch_release(mclsgpu_batch* b) {
     dfree(b->all_tcum);
     dfree(b->all_count);
     dfree(b->X);
+    dfree(b->X2);
     dfree(b->RP);
     dfree(b->RP2);
     dfree(b->B);
@@ -702,6 +708,7 @@ BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) 
     a.act_count = b->act_count;
     a.B = b->B;
     a.X = b->X;
+    a.X2 = b->X2;
     a.RP = b->RP;
     a.RP2 = b->RP2;
     a.Y = b->Y;
@@ -737,10 +744,10 @@ int enqueue_batch_iteration(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, int
                             cudaGraphConditionalHandle handle) {
     cudaStream_t s = b->ctx->stream;
     BatchArgs a = batch_args(b, mp, false);
-    k_b_richardson_residual<<<b->g_rich, kThreads, 0, s>>>(a);
+    k_b_smoothed_residual<<<b->g_rich, kThreads, 0, s>>>(a);
     k_b_source<<<b->g_src, kThreads, 0, s>>>(a);
     const BatchList list{b->act_sys, b->act_hcum, b->act_count, b->d_srow0};
-    const BatchFinish fin{b->X, b->RP, b->RP2, a.omega, a.nomega, a.inv_per, a.ev};
+    const BatchFinish fin{b->X, b->X2, b->RP2, a.nomega, a.inv_per, a.ev};
     int rc = launch_walk_batch(b->dom, b->cls, list, b->cR, b->Y, fin, b->grab);
     if (rc) return rc;
     if (b->Y) k_b_correct<<<b->g_cor, kThreads, 0, s>>>(a);
@@ -908,7 +915,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
          (e = dmalloc(&b->all_sys, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->all_tcum, nsys + 1)) != cudaSuccess ||
          (e = dmalloc(&b->all_count, 1)) != cudaSuccess ||
-         (e = dmalloc(&b->X, NE)) != cudaSuccess ||
+         (e = dmalloc(&b->X, NE)) != cudaSuccess || (e = dmalloc(&b->X2, NE)) != cudaSuccess ||
          (e = dmalloc(&b->RP, NE)) != cudaSuccess || (e = dmalloc(&b->RP2, NE)) != cudaSuccess ||
          (e = dmalloc(&b->B, NE)) != cudaSuccess ||
          (b->per > 1 && (e = dmalloc(&b->Y, NE)) != cudaSuccess) ||
@@ -920,7 +927,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         rc = cuda_fail(ctx, e, "cudaMalloc batch");
     if (!rc) {
         const int sms = ctx->num_sms;
-        b->g_rich = resident_grid(k_b_richardson_residual, sms);
+        b->g_rich = resident_grid(k_b_smoothed_residual, sms);
         b->g_src = resident_grid(k_b_source, sms);
         b->g_cor = resident_grid(k_b_correct, sms);
         b->g_upd = resident_grid(k_b_update<true>, sms);
@@ -940,6 +947,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         cudaMemcpyAsync(b->all_count, all_count.data(), sizeof(int), cudaMemcpyHostToDevice, s);
         // Padding elements are never written by the loop: zero every array once.
         cudaMemsetAsync(b->X, 0, sizeof(double) * NE, s);
+        cudaMemsetAsync(b->X2, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->RP, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->RP2, 0, sizeof(double) * NE, s);
         if (b->Y) cudaMemsetAsync(b->Y, 0, sizeof(double) * NE, s);

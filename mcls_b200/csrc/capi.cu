@@ -519,9 +519,9 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
     if (!rc && p->precision == MCLSGPU_FP32 && dom->slots == 0)
         rc = set_error(ctx, MCLSGPU_ERR_UNSUPPORTED,
                        "domain rows longer than 31 entries need the FP64 walk");
-    // Partials: one per scan tile (scans) and one per block of the fused
+    // Partials: one per scan tile (scans) and two per block of the fused
     // residual kernels, whose grid is at most 8 blocks per SM.
-    const int fused_blocks = ctx->num_sms * 8;
+    const int fused_blocks = 2 * ctx->num_sms * 8;
     const int scan_parts = scan_partials_needed(n);
     const int parts = (scan_parts > fused_blocks ? scan_parts : fused_blocks) + 8;
     if (!rc) {
@@ -558,7 +558,7 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
         dom->h_state = &ctx->h_report->st;
     }
     if (!rc) {
-        dom->part_cap = parts;
+        dom->part_cap = (scan_parts > fused_blocks / 2 ? scan_parts : fused_blocks / 2) + 8;
         cudaMemsetAsync(dom->words, 0, kWordBytes, ctx->stream);
         const unsigned long long tim0[4] = {~0ULL, 0ULL, 0ULL, 0ULL};
         cudaMemcpyAsync(dom->d_tim, tim0, sizeof(tim0), cudaMemcpyHostToDevice, ctx->stream);

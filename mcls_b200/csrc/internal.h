@@ -150,14 +150,12 @@ RowOrder row_order(int n, int K, const int* off, int rows);
 
 // What a forward fixed-length FP32 walk does with a row's sum of `per`
 // histories: d = sum / per [+ source (expected value)], then out = d,
-// out + d, or xin + w rin + d.
-enum : int { kBaseNone = 0, kBaseOut = 1, kBaseSmoothed = 2 };
+// out + d, or xin + d.
+enum : int { kBaseNone = 0, kBaseOut = 1, kBaseIn = 2 };
 struct RowFinish {
     double* out = nullptr;
     const double* src = nullptr;
     const double* xin = nullptr;
-    const double* rin = nullptr;
-    double w = 0.0;
     double omega = 0.0;
     double inv_per = 1.0;
     int has_omega = 0;
@@ -370,21 +368,18 @@ struct BatchList {
     const int* lcount;
     const int* srow0;   // system -> its first row
 };
-// The iterate after a batched iteration's smoothing step and correction.
+// The iterate after a batched iteration's correction of the smoothed iterate.
 struct BatchFinish {
     double* X;
-    const double* RP;
+    const double* X2;
     const double* RP2;
-    double omega;        // Richardson relaxation
     double nomega;       // Neumann relaxation (1 when absent)
     double inv_per;      // 1 / histories per row
     int ev;              // expected-value estimator
 };
 #if defined(__CUDACC__)
-__device__ __forceinline__ double batch_corrected(double x, double rp, double rp2, double y,
-                                                  double omega, double nomega, double inv_per,
-                                                  int ev) {
-    const double x2 = __dadd_rn(x, __dmul_rn(omega, rp));
+__device__ __forceinline__ double batch_corrected(double x2, double rp2, double y, double nomega,
+                                                  double inv_per, int ev) {
     double d = y * inv_per;
     if (ev) d += nomega * rp2;
     return x2 + d;
@@ -406,10 +401,8 @@ int launch_walk_batch(mclsgpu_domain* dom, const BatchClasses& cls, const BatchL
 void prec_residual(mclsgpu_domain* dom, const double* x, const double* b, double* rp_out);
 // y = PL A PR x   (LinearProblem::apply); uses dom->tmp and dom->tmp2.
 void composite_apply(mclsgpu_domain* dom, const double* x, double* y);
-// x2 = x + w r (unless x2 is null); r2 = PL (b - A PR x2) for r = PL (b - A PR x),
-// formed as r - w PL A PR r for forward domains: one fused pass when PL is I or
-// point Jacobi and there is no PR, two when PL is held on A's diagonals (x2 !=
-// x, r2 != r).  dom->x2 may be overwritten.
+// x2 = x + w r; r2 = PL (b - A PR x2): one fused pass when PL is I, point
+// Jacobi or held on A's diagonals and there is no PR (x2 != x, r2 != r).
 void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, double w,
                          double* x2, double* r2);
 // out = the Monte Carlo estimate for the source v (already left

@@ -154,12 +154,10 @@ struct FinalizeArgs {
     int n;
     int mode;            // 0 adjoint collision, 1 adjoint EV, 2 forward
     int ev;
-    int base;            // kBase*: out = delta, out + delta, or xin + w rin + delta
+    int base;            // kBase*: out = delta, out + delta, or xin + delta
     int fp32;
     double per;          // forward histories per state
     const double* xin;
-    const double* rin;
-    double w;
     const double* sc;    // [2] = 1/nh
     const double* src;   // MC source vector before scaling
     double omega;
@@ -197,8 +195,8 @@ __global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
         }
         if (a.base == kBaseOut)
             d = __dadd_rn(a.out[i], d);
-        else if (a.base == kBaseSmoothed)
-            d = __dadd_rn(__dadd_rn(a.xin[i], __dmul_rn(a.w, a.rin[i])), d);
+        else if (a.base == kBaseIn)
+            d = __dadd_rn(a.xin[i], d);
         a.out[i] = d;
     }
 }
@@ -295,29 +293,10 @@ __global__ void k_mcsa_check_host(McsaState* st, const double* sumsq, double* hi
 // ---- fused iteration kernels (smoother_steps == 1, PL in {I, point Jacobi}) ----
 constexpr int kFusedThreads = 256;
 
-// The residual after one Richardson step x2 = x + w rp, from rp alone:
-// rp2 = PL (b - A x2) = rp - w PL A rp (PL = I or a diagonal).  Against the
-// form that subtracts A x2 from b it reads neither x nor b and gathers one
-// vector at the neighbours instead of two: 56 instead of 88 bytes per row of
-// a symmetric 7-point operator, at 128^3 22 instead of 32 us.  x2 is written
-// when the caller needs it (not null).
-template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_richardson_residual(
-    Op A, const double* dinv, const double* x, const double* r, double w, double* x2,
-    double* r2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
-        const double s = A.dot(i, [&](int j) { return r[j]; });
-        const double ri = r[i];
-        r2[i] = ri - w * (dinv ? dinv[i] * s : s);
-        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
-    }
-}
-
-// The same residual as b - A x2 with x2 = x + w rp formed at the neighbours on
-// the fly: adjoint domains.  Their history count is a quotient truncated to an
-// integer, int(Nh * |b|_1 / |b|_1) (src/MCLS_UniformAdjointSource_impl.hpp:198),
-// which the last bit of the source's norm moves between Nh and Nh - 1, so the
-// source keeps the reference's own arithmetic.
+// Richardson smoothing fused with the residual: x2 = x + w rp (rounded as the
+// separate update would be) and rp2 = PL (b - A x2), reading x + w rp at the
+// neighbours on the fly (Anderson steps; the MCSA loop has x2 from the last
+// iteration's k_residual_norm).
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_smoothed_residual(
     Op A, const double* b, const double* dinv, const double* x, const double* r, double w,
@@ -326,7 +305,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_smoothed_residual(
         const double s = A.dot(i, [&](int j) { return __dadd_rn(x[j], __dmul_rn(w, r[j])); });
         const double res = b[i] - s;
         r2[i] = dinv ? dinv[i] * res : res;
-        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
+        x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
     }
 }
 
@@ -336,6 +315,8 @@ struct ResidArgs {
     const double* dinv;       // null: no left preconditioner
     const double* x;          // the corrected iterate
     double* rout;
+    double* x2;               // x + w rp: the next iteration's smoothed iterate
+    double w;
     double* part;
     unsigned int* ticket;
     McsaState* st;
@@ -407,8 +388,11 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     }
 }
 
+// (256, 8): eight blocks an SM, the grid's size, must be resident; with the 46
+// registers that the one thread's check asks for five were, and the pass took
+// 33 us at 128^3 instead of 28.9 us (k_mcsa_begin: 43 and 32.3 us).
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_residual_norm(Op A, ResidArgs a) {
+__global__ void __launch_bounds__(kFusedThreads, 8) k_residual_norm(Op A, ResidArgs a) {
     const double* x = a.x;
     double acc = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
@@ -416,6 +400,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_residual_norm(Op A, ResidArgs
         const double res = a.b[i] - s;
         const double r = a.dinv ? a.dinv[i] * res : res;
         a.rout[i] = r;
+        a.x2[i] = __dadd_rn(x[i], __dmul_rn(a.w, r));
         acc = fma(r, r, acc);
     }
     norm_and_check(a, acc);
@@ -428,27 +413,15 @@ __global__ void __launch_bounds__(kFusedThreads) k_dia_apply(Op M, const double*
         out[i] = M.dot(i, [&](int j) { return v[j]; });
 }
 
-// The Richardson step with it: rp2 = rp - w M v with v = A rp.
-template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_dia_richardson(Op M, const double* v,
-                                                                 const double* x, const double* r,
-                                                                 double w, double* x2,
-                                                                 double* r2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
-        const double ri = r[i];
-        r2[i] = ri - w * M.dot(i, [&](int j) { return v[j]; });
-        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
-    }
-}
-
 // rp = M (b - A x) from the raw residual, its norm and the convergence check.
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_precond_norm(Op M, ResidArgs a,
+__global__ void __launch_bounds__(kFusedThreads, 8) k_precond_norm(Op M, ResidArgs a,
                                                                const double* raw) {
     double acc = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         const double r = M.dot(i, [&](int j) { return raw[j]; });
         a.rout[i] = r;
+        a.x2[i] = __dadd_rn(a.x[i], __dmul_rn(a.w, r));
         acc = fma(r, r, acc);
     }
     norm_and_check(a, acc);
@@ -477,15 +450,17 @@ __global__ void k_mcsa_init(McsaState* st, const double* src_sumsq, double tol, 
 }
 
 // The start of an MCSA solve with no left preconditioner or a diagonal one in
-// one pass: b and x copied to the loop's vectors, rp = PL (b - A x), |PL b|^2
-// and |rp|^2, and (last block) the loop state, the counters and the forward
-// walk's history count.  Apart these were twelve launches and copies, 30 us
-// of a small system's solve.
+// one pass: b and x copied to the loop's vectors, rp = PL (b - A x), the
+// smoothed iterate, |PL b|^2 and |rp|^2, and (last block) the loop state, the
+// counters and the forward walk's history count.  Apart these were twelve
+// launches and copies, 30 us of a small system's solve.
 struct BeginArgs {
     const double* b_in;
     const double* x_in;
     double* b;
     double* x;
+    double* x2;               // x + w rp
+    double w;
     double* rp;
     const double* dinv;
     double* part;             // 2 per block
@@ -513,7 +488,7 @@ __device__ __forceinline__ double fused_block_sum(double v, double* sh) {
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads) k_mcsa_begin(Op A, BeginArgs a) {
+__global__ void __launch_bounds__(kFusedThreads, 8) k_mcsa_begin(Op A, BeginArgs a) {
     __shared__ double sh[kFusedThreads / 32];
     __shared__ bool last;
     double sb = 0.0, sr = 0.0;
@@ -525,7 +500,9 @@ __global__ void __launch_bounds__(kFusedThreads) k_mcsa_begin(Op A, BeginArgs a)
         const double pb = a.dinv ? di * bi : bi;
         a.rp[i] = r;
         if (a.b != a.b_in) a.b[i] = bi;
-        if (a.x != a.x_in) a.x[i] = a.x_in[i];
+        const double xi = a.x_in[i];
+        if (a.x != a.x_in) a.x[i] = xi;
+        a.x2[i] = __dadd_rn(xi, __dmul_rn(a.w, r));
         sb = fma(pb, pb, sb);
         sr = fma(r, r, sr);
     }
@@ -730,12 +707,11 @@ int mcsa_finish_report(mclsgpu_domain* dom, mclsgpu_stats* st) {
 }
 
 // One MC solve of the source vector `v` (device, already left preconditioned
-// when required) into out: out = delta, out + delta or x + w rp + delta
-// (`base`; w the smoother's relaxation).  Walks that finish their rows
-// themselves write out; the others' tallies are normalised and added by
-// k_finalize.  `fused`: inside the fused MCSA iteration the epoch increment
+// when required) into out: out = delta, out + delta or x2 + delta (`base`).
+// Walks that finish their rows themselves write out; the others' tallies are
+// normalised and added by k_finalize.  `fused`: inside the fused MCSA iteration the epoch increment
 // and the walk bookkeeping are done by k_residual_norm.
-static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int base, double w,
+static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int base,
                        long long max_trace, long long* tr_states, double* tr_w, int* tr_ev,
                        long long* tr_start, bool fused = false, bool report = false) {
     const mclsgpu_mc_params& p = dom->p;
@@ -746,9 +722,7 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
     RowFinish fin;
     fin.out = out;
     fin.src = v;
-    fin.xin = dom->x;
-    fin.rin = dom->rp;
-    fin.w = w;
+    fin.xin = dom->x2;
     fin.omega = omega;
     fin.has_omega = has_omega;
     int ex = 0;
@@ -769,9 +743,7 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
         f.mode = p.direction == MCLSGPU_FORWARD ? 2 : (ev ? 1 : 0);
         f.ev = ev;
         f.base = base;
-        f.xin = dom->x;
-        f.rin = dom->rp;
-        f.w = w;
+        f.xin = dom->x2;
         f.fp32 = p.precision == MCLSGPU_FP32;
         f.per = per;
         f.sc = dom->d_scalars;
@@ -808,11 +780,11 @@ static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x
     // The walk's report is the last word of a solve without right recovery.
     if (dom->right && !internal) {
         // v is rhs_dev or tmp, so tmp2 is free for the unrecovered result.
-        enqueue_mc(dom, v, dom->tmp2, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start,
+        enqueue_mc(dom, v, dom->tmp2, kBaseNone, max_trace, tr_states, tr_w, tr_ev, tr_start,
                    false, true);
         spmv(s, dom->right->P, dom->tmp2, x_dev);
     } else {
-        enqueue_mc(dom, v, x_dev, kBaseNone, 0.0, max_trace, tr_states, tr_w, tr_ev, tr_start,
+        enqueue_mc(dom, v, x_dev, kBaseNone, max_trace, tr_states, tr_w, tr_ev, tr_start,
                    false, true);
     }
     cudaEventRecord(ctx->ev[1], s);
@@ -838,19 +810,8 @@ __global__ void k_axpy_to(const double* x, const double* r, double w, double* x2
         x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
 }
 
-// The Richardson step from y = PL A PR r in r2: r2 = r - w y and, when x2 is
-// not null, x2 = x + w r (rounded as the reference's vector update).
-__global__ void k_richardson_step(const double* x, const double* r, double w, double* x2,
-                                  double* r2, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double ri = r[i];
-        r2[i] = ri - w * r2[i];
-        if (x2) x2[i] = __dadd_rn(x[i], __dmul_rn(w, ri));
-    }
-}
-
 void mc_correction(mclsgpu_domain* dom, const double* v, double* out) {
-    enqueue_mc(dom, v, out, kBaseNone, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
+    enqueue_mc(dom, v, out, kBaseNone, 0, nullptr, nullptr, nullptr, nullptr);
 }
 
 // The fused iteration covers one smoothing step, no right preconditioner and
@@ -862,8 +823,8 @@ static bool fused_iteration(const mclsgpu_domain* dom, const mclsgpu_mcsa_params
             (dom->left->mdia && dom->op->dia_k > 0));
 }
 
-// At most 8 blocks per SM: the per-block partial sums of k_residual_norm go to
-// dom->part, sized for that many blocks.
+// At most 8 blocks per SM: the per-block partial sums (two of them in
+// k_mcsa_begin) go to dom->part, sized for that many blocks.
 static int fused_grid(const mclsgpu_domain* dom) {
     return grid_for(dom->n, kFusedThreads, dom->ctx->num_sms * 8);
 }
@@ -874,53 +835,38 @@ void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, 
     const mclsgpu_operator* op = dom->op;
     const int grid = fused_grid(dom);
     const mclsgpu_precond* L = dom->left;
-    const bool diag = !dom->right && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI);
-    const bool mdia = !diag && !dom->right && L->mdia && op->dia_k > 0;
-    const double* dinv = diag && L ? L->diag : nullptr;
-    if (dom->p.direction == MCLSGPU_ADJOINT) {
-        if (diag) {
-            MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b, dinv, x, r, w,
-                              x2, r2);
-        } else if (mdia) {
-            MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b, nullptr, x,
-                              r, w, x2, dom->tmp);
-            MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, r2);
-        } else {
-            double* xs = x2 ? x2 : dom->x2;
-            k_axpy_to<<<grid, kFusedThreads, 0, s>>>(x, r, w, xs, dom->n);
-            update_prec_residual(dom, xs, dom->b, r2);
-        }
-    } else if (diag) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_richardson_residual, dinv, x, r, w, x2, r2);
-    } else if (mdia) {
-        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_matvec, r, nullptr, dom->tmp);
-        MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_richardson, dom->tmp, x, r, w,
-                         x2, r2);
+    if (!dom->right && (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI)) {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b,
+                          L ? L->diag : nullptr, x, r, w, x2, r2);
+    } else if (!dom->right && L->mdia && op->dia_k > 0) {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_smoothed_residual, dom->b, nullptr, x, r, w,
+                          x2, dom->tmp);
+        MCLSGPU_LAUNCH_M(op, L->mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, r2);
     } else {
-        composite_apply(dom, r, r2);
-        k_richardson_step<<<grid, kFusedThreads, 0, s>>>(x, r, w, x2, r2, dom->n);
+        k_axpy_to<<<grid, kFusedThreads, 0, s>>>(x, r, w, x2, dom->n);
+        update_prec_residual(dom, x2, dom->b, r2);
     }
 }
 
 // One MCSA iteration including its convergence check.  The fused form: the
-// residual after the Richardson step, the source build (forward: tally
-// sources into the records), the walk, which adds the step and the correction
-// to x (or k_finalize does), and residual + norm + check.
+// residual rp2 at the smoothed iterate x2, the source build (forward: tally
+// sources into the records), the walk, which makes x = x2 + the correction (or
+// k_finalize does), and residual + norm + check, which also makes the next
+// iteration's x2 = x + w rp where x and rp are at hand: the smoothing pass then
+// gathers one vector at the neighbours, not two, and x2 is read once.  At 128^3
+// the smoothing pass takes 23.6 us (32 us with x + w rp formed at the
+// neighbours) and the last pass, with x2's store, 28.9 us.  A recurrence rp2 =
+// rp - w PL A rp would save 2 us more but rounds rp2 differently, which moves
+// FP32 tally sources and, in adjoint domains, the history count.
 static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp,
                               cudaGraphConditionalHandle handle, int use_cond) {
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
     if (!fused_iteration(dom, mp)) {
-        if (mp->smoother_steps == 1 && mp->fixed_point_type == MCLSGPU_FIXED_POINT_RICHARDSON) {
-            richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, nullptr, dom->rp2);
-            enqueue_mc(dom, dom->rp2, dom->x, kBaseSmoothed, mp->richardson_omega, 0, nullptr,
-                       nullptr, nullptr, nullptr);
-        } else {
-            for (int l = 0; l < mp->smoother_steps; ++l)
-                enqueue_fixed_point_step(dom, mp->fixed_point_type, mp->richardson_omega);
-            enqueue_mc(dom, dom->rp, dom->x, kBaseOut, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
-        }
+        for (int l = 0; l < mp->smoother_steps; ++l)
+            enqueue_fixed_point_step(dom, mp->fixed_point_type, mp->richardson_omega);
+        enqueue_mc(dom, dom->rp, dom->x, kBaseOut, 0, nullptr, nullptr, nullptr, nullptr);
         update_prec_residual(dom, dom->x, dom->b, dom->rp);
         sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
         if (use_cond)
@@ -937,17 +883,22 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     // goes to tmp and a second pass applies M.
     const double* mdia = dom->left ? dom->left->mdia : nullptr;
     const int grid = fused_grid(dom);
-    richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, nullptr, dom->rp2);
-    // x = x + w rp + delta: the smoothing step's iterate is formed where the
-    // correction is added.
-    enqueue_mc(dom, dom->rp2, dom->x, kBaseSmoothed, mp->richardson_omega, 0, nullptr, nullptr,
-               nullptr, nullptr, true);
+    if (mdia) {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, nullptr,
+                          dom->tmp);
+        MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, dom->rp2);
+    } else {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, dinv, dom->rp2);
+    }
+    enqueue_mc(dom, dom->rp2, dom->x, kBaseIn, 0, nullptr, nullptr, nullptr, nullptr, true);
     ResidArgs a{};
     a.n = n;
     a.b = dom->b;
     a.dinv = dinv;
     a.x = dom->x;
     a.rout = dom->rp;
+    a.x2 = dom->x2;
+    a.w = mp->richardson_omega;
     a.part = dom->part;
     a.ticket = dom->d_ticket;
     a.st = dom->d_state;
@@ -1046,6 +997,8 @@ static int mcsa_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_
         a.x_in = x_dev;
         a.b = dom->b;
         a.x = dom->x;
+        a.x2 = dom->x2;
+        a.w = mp->richardson_omega;
         a.rp = dom->rp;
         a.dinv = L ? L->diag : nullptr;
         a.part = dom->part;
@@ -1060,8 +1013,7 @@ static int mcsa_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_
         a.d_nh = dom->d_nh;
         a.d_counter = dom->d_counter;
         a.c = counters(dom);
-        // Two partial sums per block in dom->part, sized for 8 blocks per SM.
-        const int grid = grid_for(n, kFusedThreads, ctx->num_sms * 4);
+        const int grid = fused_grid(dom);  // two partial sums per block
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_mcsa_begin, a);
         return 1;
     }
@@ -1084,8 +1036,12 @@ static int mcsa_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_
     sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
     k_mcsa_init<<<1, 1, 0, s>>>(dom->d_state, dom->d_scalars + 6, mp->tolerance, mp->check_freq,
                                 mp->max_iters, dom->d_scalars + 5);
-    if (fused_iteration(dom, mp) && forward) launch_forward_setup(dom);
-    return 10;
+    if (fused_iteration(dom, mp)) {
+        k_axpy_to<<<fused_grid(dom), kFusedThreads, 0, s>>>(dom->x, dom->rp, mp->richardson_omega,
+                                                            dom->x2, n);
+        if (forward) launch_forward_setup(dom);
+    }
+    return 11;
 }
 
 static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
@@ -1423,7 +1379,7 @@ int mclsgpu_mcsa_correction(mclsgpu_domain* dom, double* delta_dev) {
     for (int l = 0; l < p.smoother_steps; ++l)
         enqueue_fixed_point_step(dom, p.fixed_point_type, p.richardson_omega);
     // The residual problem's source is already left preconditioned.
-    enqueue_mc(dom, dom->rp, delta_dev, kBaseNone, 0.0, 0, nullptr, nullptr, nullptr, nullptr);
+    enqueue_mc(dom, dom->rp, delta_dev, kBaseNone, 0, nullptr, nullptr, nullptr, nullptr);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mcsa correction");
     return check_device_status(ctx);

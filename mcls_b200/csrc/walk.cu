@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S>::kMinBlocks)
         if (f.ev) d = __dadd_rn(d, f.has_omega ? f.src[i] * f.omega : f.src[i]);
         if (f.base == kBaseOut)
             d = __dadd_rn(f.out[i], d);
-        else if (f.base == kBaseSmoothed)
-            d = __dadd_rn(__dadd_rn(f.xin[i], __dmul_rn(f.w, f.rin[i])), d);
+        else if (f.base == kBaseIn)
+            d = __dadd_rn(f.xin[i], d);
         f.out[i] = d;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -788,7 +788,7 @@ __device__ __forceinline__ void finish_rows(const BatchWalk& m, const double* st
     __syncwarp();
     const int row0 = __shfl_sync(kFull, row, 0), c0 = __shfl_sync(kFull, c, 0);
     auto finish = [&](size_t e, double y) {
-        f.X[e] = batch_corrected(f.X[e], f.RP[e], f.RP2[e], y, f.omega, f.nomega, f.inv_per, f.ev);
+        f.X[e] = batch_corrected(f.X2[e], f.RP2[e], y, f.nomega, f.inv_per, f.ev);
     };
     if (__all_sync(kFull, live && c == c0 && row == row0 + lane)) {
         const size_t e0 = size_t(m.cls.cel[c0]) + (size_t(row0 - m.cls.crow[c0]) << c0);
