@@ -173,7 +173,7 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->words);
     dfree(d->c64);
     dfree(d->part);
-    dfree(d->ipart);
+    dfree(d->emitted);
     dfree(d->x);
     dfree(d->b);
     dfree(d->rp);
@@ -531,7 +531,8 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
             (e = dmalloc(&dom->start, size_t(dom->nh_cap) + 1)) != cudaSuccess ||
             (e = dmalloc(&dom->y64, n)) != cudaSuccess || (e = dmalloc(&dom->c64, n)) != cudaSuccess ||
             (e = dmalloc(&dom->words, kWordBytes)) != cudaSuccess ||
-            (e = dmalloc(&dom->part, parts)) != cudaSuccess || (e = dmalloc(&dom->ipart, parts)) != cudaSuccess ||
+            (e = dmalloc(&dom->part, parts)) != cudaSuccess ||
+            (e = dmalloc(&dom->emitted, scan_parts)) != cudaSuccess ||
             (e = dmalloc(&dom->x, n)) != cudaSuccess || (e = dmalloc(&dom->b, n)) != cudaSuccess ||
             (e = dmalloc(&dom->rp, n)) != cudaSuccess || (e = dmalloc(&dom->tmp, n)) != cudaSuccess ||
             (e = dmalloc(&dom->tmp2, n)) != cudaSuccess ||

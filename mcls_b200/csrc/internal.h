@@ -222,7 +222,7 @@ struct mclsgpu_domain {
     unsigned long long* d_steps = nullptr;  // walk steps (running total)
     unsigned long long* d_tim = nullptr;    // FP32 walk timing (see walk.cu)
     double* part = nullptr;        // reduction / scan partials
-    int* ipart = nullptr;
+    unsigned long long* emitted = nullptr;  // adjoint source: histories of each tile (look-back)
     int part_cap = 0;
     // MCSA buffers.
     double* x = nullptr;

@@ -16,11 +16,11 @@
 // lies in [guide[t], guide[t+1]] with t = floor(u*G); a short binary search in
 // that window returns std::lower_bound's answer.
 //
-// The random adjoint source of a large system is five launches: tile sums and
-// the history count, CDF and guide, draws, tile counts, emission.  Apart (a
-// reduction, a scan of its partials and a copy for each sum, memsets, a
-// separate normalisation, guide marks and a maximum scan) they were nineteen,
-// 80 of the 107 us of an MCSA iteration at 64^3.
+// The random adjoint source of a large system is four launches: tile sums and
+// the history count, CDF and guide, draws, emission.  Apart (a reduction, a
+// scan of its partials and a copy for each sum, memsets, a separate
+// normalisation, guide marks and a maximum scan, a pass for the tile counts)
+// they were nineteen, 80 of the 107 us of an MCSA iteration at 64^3.
 #include <cfloat>
 #include <climits>
 
@@ -92,18 +92,18 @@ __device__ __forceinline__ void strat_factor(int nh_req, double norm1, double* s
 
 __global__ void k_strat_prep(int nh_req, double* sc) { strat_factor(nh_req, sc[0], sc); }
 
-// Sum of the nb tile partials, the first of them replaced by `first`; WRITE:
-// an exclusive scan in place as well.  One block.
-template <class T, bool WRITE>
-__device__ __forceinline__ T scan_tiles(T* part, int nb, T first, T* warp_tot) {
-    T carry = T(0);
+// Totals of the nb tile partials with part[0] (a) and with `abs0` in its place
+// (b), and the exclusive scan of the first in place.  One block.
+__device__ __forceinline__ Pair scan_tiles(double* part, int nb, double abs0, Pair* warp_tot) {
+    __shared__ Pair chunk;
+    Pair carry{0.0, 0.0};
     for (int base = 0; base < nb; base += kThreads) {
         const int i = base + threadIdx.x;
-        const T v = i == 0 ? first : i < nb ? __ldcg(&part[i]) : T(0);
-        T excl;
-        const T incl = block_scan(v, AddOp(), T(0), warp_tot, &excl);
-        if (WRITE && i < nb) part[i] = carry + excl;
-        __shared__ T chunk;
+        const double x = i < nb ? __ldcg(&part[i]) : 0.0;
+        Pair excl;
+        const Pair incl =
+            block_scan(Pair{x, i == 0 ? abs0 : x}, AddOp(), Pair{0.0, 0.0}, warp_tot, &excl);
+        if (i < nb) part[i] = carry.a + excl.a;
         if (threadIdx.x == kThreads - 1) chunk = incl;
         __syncthreads();
         carry = carry + chunk;
@@ -128,41 +128,46 @@ __device__ __forceinline__ bool last_block(unsigned int* ticket) {
 // Tile sums of the source CDF's terms (signed first element, :185) and, in the
 // last block, their exclusive scan, |b|_1 (with the CDF's association, so that
 // the two totals agree when b[0] >= 0), the history count or the stratified
-// factor.  part has tiles + 2 entries.
+// factor.  part has tiles + 2 entries.  Bound by latency (one tile a block,
+// two round trips and the last block's scan): 5.9 us at 64^3, 11 us when the
+// threads read their 8 elements from the same banks and the last block made
+// two scans.
 __global__ void __launch_bounds__(kThreads) k_src_reduce(const double* v, int n, double omega,
                                                          int has, int strat, int nh_req, int cap,
                                                          double* part, unsigned int* ticket,
                                                          double* sc, int* d_nh, int* status) {
     __shared__ double stage[kTile];
-    __shared__ double warp_tot[32];
+    __shared__ Pair warp_tot[32];
+    double* const warp_totd = &warp_tot[0].a;
     const int base = blockIdx.x * kTile, nb = gridDim.x;
-    for (int k = threadIdx.x; k < kTile; k += kThreads) {
-        const int i = base + k;
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int k = threadIdx.x + q * kThreads, i = base + k;
         const double x = i < n ? load_src(v, i, omega, has) : 0.0;
-        stage[k] = i == 0 ? x : fabs(x);
+        stage[swz<8>(k)] = i == 0 ? x : fabs(x);
     }
     __syncthreads();
     const double v0 = stage[0];  // signed in block 0
-    double acc = stage[threadIdx.x * kItems];
+    double acc = stage[swz<8>(threadIdx.x * kItems)];
 #pragma unroll
-    for (int k = 1; k < kItems; ++k) acc = acc + stage[threadIdx.x * kItems + k];
+    for (int k = 1; k < kItems; ++k) acc = acc + stage[swz<8>(threadIdx.x * kItems + k)];
     double excl;
-    double incl = block_scan(acc, AddOp(), 0.0, warp_tot, &excl);
+    double incl = block_scan(acc, AddOp(), 0.0, warp_totd, &excl);
     if (threadIdx.x == kThreads - 1) part[blockIdx.x] = incl;
     if (blockIdx.x == 0) {
         // The first tile's sum of magnitudes.
         if (threadIdx.x == 0) {
             acc = fabs(v0);
-            for (int k = 1; k < kItems; ++k) acc = acc + stage[k];
+            for (int k = 1; k < kItems; ++k) acc = acc + stage[swz<8>(k)];
         }
-        incl = block_scan(acc, AddOp(), 0.0, warp_tot, &excl);
+        incl = block_scan(acc, AddOp(), 0.0, warp_totd, &excl);
         if (threadIdx.x == kThreads - 1) part[nb + 1] = incl;
     }
     __syncthreads();
     if (!last_block(ticket)) return;
-    const double norm1 = scan_tiles<double, false>(part, nb, __ldcg(&part[nb + 1]), warp_tot);
-    const double total = scan_tiles<double, true>(part, nb, __ldcg(&part[0]), warp_tot);
+    const Pair t = scan_tiles(part, nb, __ldcg(&part[nb + 1]), warp_tot);
     if (threadIdx.x != 0) return;
+    const double total = t.a, norm1 = t.b;
     part[nb] = total;
     if (strat) {
         strat_factor(nh_req, norm1, sc);
@@ -177,53 +182,57 @@ inline int guide_size(int n) { return (n + 15) / 16; }
 // to exactly 1), its states' counts cleared, and the guide entries that fall
 // into the tile: from the first t its lower boundary reaches to the last one
 // before the next tile's.  RESCAN false: the CDF is there already (the
-// reference's sequential order).
+// reference's sequential order).  6.6 us at 64^3; 13 us with bank conflicts
+// and one warp searching a tile's 128 guide entries.
 template <bool RESCAN>
 __global__ void __launch_bounds__(kThreads) k_src_cdf(const double* v, int n, double omega, int has,
                                                       const double* part, const double* sc,
-                                                      double* cdf, int* counts, int* guide,
-                                                      int G) {
+                                                      double* cdf, int* counts, int* guide, int G,
+                                                      unsigned long long* emitted) {
     __shared__ double stage[kTile];
     __shared__ double warp_tot[32];
     const int base = blockIdx.x * kTile;
     const int len = min(kTile, n - base);
     double lower, upper;  // the tile's range of the CDF
+    if (threadIdx.x == 0) emitted[blockIdx.x] = 0ULL;
     if constexpr (RESCAN) {
         const double total = sc[1];
-        for (int k = threadIdx.x; k < kTile; k += kThreads) {
-            const int i = base + k;
+#pragma unroll
+        for (int q = 0; q < kItems; ++q) {
+            const int k = threadIdx.x + q * kThreads, i = base + k;
             const double x = i < n ? load_src(v, i, omega, has) : 0.0;
-            stage[k] = i == 0 ? x : fabs(x);
+            stage[swz<8>(k)] = i == 0 ? x : fabs(x);
         }
         __syncthreads();
         double loc[kItems];
-        loc[0] = stage[threadIdx.x * kItems];
+        loc[0] = stage[swz<8>(threadIdx.x * kItems)];
 #pragma unroll
-        for (int k = 1; k < kItems; ++k) loc[k] = loc[k - 1] + stage[threadIdx.x * kItems + k];
+        for (int k = 1; k < kItems; ++k)
+            loc[k] = loc[k - 1] + stage[swz<8>(threadIdx.x * kItems + k)];
         double excl;
         block_scan(loc[kItems - 1], AddOp(), 0.0, warp_tot, &excl);
         const double carry = part[blockIdx.x];
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             const int i = base + threadIdx.x * kItems + k;
-            stage[threadIdx.x * kItems + k] =
+            stage[swz<8>(threadIdx.x * kItems + k)] =
                 i >= n - 1 ? 1.0 : (carry + (excl + loc[k])) / total;
         }
         __syncthreads();
         for (int k = threadIdx.x; k < len; k += kThreads) {
-            cdf[base + k] = stage[k];
+            cdf[base + k] = stage[swz<8>(k)];
             counts[base + k] = 0;
         }
         lower = carry / total;
         upper = part[blockIdx.x + 1] / total;
     } else {
         for (int k = threadIdx.x; k < len; k += kThreads) {
-            stage[k] = cdf[base + k];
+            stage[swz<8>(k)] = cdf[base + k];
             counts[base + k] = 0;
         }
         __syncthreads();
         lower = base > 0 ? cdf[base - 1] : 0.0;
-        upper = stage[len - 1];
+        upper = stage[swz<8>(len - 1)];
     }
     // Guide entries t0..t1 of this tile (0..G over all tiles).
     const double g = double(G);
@@ -234,13 +243,19 @@ __global__ void __launch_bounds__(kThreads) k_src_cdf(const double* v, int n, do
     auto first = [&](int t, int lo, int hi) {
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (stage[mid] * g < double(t)) lo = mid + 1; else hi = mid;
+            if (stage[swz<8>(mid)] * g < double(t)) lo = mid + 1; else hi = mid;
         }
         return lo;
     };
-    // A warp takes 256 entries at a time; a run of entries inside one state
-    // (a source concentrated in few states) is filled without searching.
+    // One search per entry and thread; where a source is concentrated in few
+    // states and the tile has many entries a warp takes 256, and a run of
+    // entries inside one state is filled without searching.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (t1 - t0 < 8 * kThreads) {
+        for (int t = t0 + threadIdx.x; t <= t1; t += kThreads)
+            guide[t] = base + first(t, 0, len - 1);
+        return;
+    }
     for (int ta = t0 + 256 * warp; ta <= t1; ta += 256 * (kThreads / 32)) {
         const int tb = min(ta + 255, t1);
         const int ka = first(ta, 0, len - 1), kb = first(tb, ka, len - 1);
@@ -301,92 +316,138 @@ __global__ void k_advance_pos(unsigned long long* d_pos, const int* d_nh, int mu
 
 // Stratified counts_i = ceil(|b_i| * (nh_local / local_sum)) (:246-262).
 __global__ void k_strat_counts(const double* v, int n, double omega, int has, const double* sc,
-                               int* counts) {
+                               int* counts, unsigned long long* emitted) {
     const double num_over_sum = sc[3];
+    if (threadIdx.x == 0)
+        for (int t = blockIdx.x; t * kTile < n; t += gridDim.x) emitted[t] = 0ULL;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double c = ceil(__dmul_rn(fabs(load_src(v, i, omega, has)), num_over_sum));
         counts[i] = c > 0.0 ? int(c) : 0;
     }
 }
 
-// Tile sums of the counts in emission order (highest state first, the LIFO
-// stack of :157-175) and, in the last block, their exclusive scan; stratified
-// sampling takes its history count from the total.
-__global__ void __launch_bounds__(kThreads) k_src_count(const int* counts, int n, int strat,
-                                                        int cap, int* part, unsigned int* ticket,
-                                                        double* sc, int* d_nh, int* status) {
-    __shared__ int stage[kTile];
-    __shared__ int warp_tot[32];
-    const int base = blockIdx.x * kTile;
-    for (int k = threadIdx.x; k < kTile; k += kThreads)
-        stage[k] = base + k < n ? counts[n - 1 - (base + k)] : 0;
-    __syncthreads();
-    int acc = 0;
+// The histories of the tiles before `tile` (a warp's look-back): every tile
+// publishes its own count first and, once it knows it, the count up to and
+// including itself.  Tiles are numbered in the order their blocks start, so
+// the ones waited for run or have run; a wait that expires all the same is
+// reported and its tile's histories keep within the buffer.
+constexpr unsigned long long kOwnCount = 1ULL << 62, kUpTo = 2ULL << 62;
+constexpr unsigned long long kCountMask = kOwnCount - 1;
+
+__device__ __forceinline__ long long look_back(const unsigned long long* emitted, int tile,
+                                               int* status) {
+    const int lane = threadIdx.x & 31;
+    long long sum = 0;
+    for (int at = tile - 1; at >= 0; at -= 32) {
+        const int t = at - lane;
+        unsigned long long w = 0ULL;
+        for (int spin = 0; spin < (1 << 20); ++spin) {
+            w = t >= 0 ? *reinterpret_cast<const volatile unsigned long long*>(&emitted[t])
+                       : kUpTo;
+            if (__all_sync(kFull, w != 0ULL)) break;
+        }
+        if (w == 0ULL) atomicOr(status, DEV_ERR_TIMEOUT);
+        const unsigned upto = __ballot_sync(kFull, (w >> 62) == 2ULL);
+        const int last = upto ? __ffs(upto) - 1 : 31;
+        long long x = lane <= last ? (long long)(w & kCountMask) : 0;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) acc += stage[threadIdx.x * kItems + k];
-    int excl;
-    const int incl = block_scan(acc, AddOp(), 0, warp_tot, &excl);
-    if (threadIdx.x == kThreads - 1) part[blockIdx.x] = incl;
-    __syncthreads();
-    if (!last_block(ticket)) return;
-    int nh = scan_tiles<int, true>(part, gridDim.x, __ldcg(&part[0]), warp_tot);
-    if (threadIdx.x != 0 || !strat) return;
-    if (nh > cap) {
-        atomicOr(status, DEV_ERR_CAPACITY);
-        nh = cap;
+        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(kFull, x, d);
+        sum += x;
+        if (upto) break;
     }
-    *d_nh = nh;
-    sc[2] = nh > 0 ? 1.0 / double(nh) : 0.0;
+    return sum;
 }
 
-// Emission order and step-0 collision tally: start[o_i + t] = i | sign with
+// Emission order (highest state first, the LIFO stack of :157-175) and step-0
+// collision tally in one pass over the counts: start[o_i + t] = i | sign with
 // o_i the histories of the higher states, y_i = counts_i * w0_i (the tally
-// every history makes at its first state).
-__global__ void __launch_bounds__(kThreads) k_src_expand(const double* v, int n, double omega,
-                                                         int has, const int* counts,
-                                                         const int* part, const double* sc,
-                                                         int cap, int* start, double* y,
-                                                         int* status) {
+// every history makes at its first state).  Stratified sampling takes its
+// history count from the total.  A tile's counts and sources are loaded before
+// anything is stored.  Bound by the latency of those loads and of the
+// look-back: 10 us at 64^3; a pass for the tile counts and one that read
+// counts and sources one after the other between its stores took 9 and 13 us.
+__global__ void __launch_bounds__(kThreads) k_src_emit(const double* v, int n, double omega,
+                                                       int has, int strat, const int* counts,
+                                                       unsigned long long* emitted,
+                                                       unsigned int* ticket, double* sc, int cap,
+                                                       int* start, double* y, int* d_nh,
+                                                       int* status) {
     __shared__ int stage[kTile];
     __shared__ int warp_tot[32];
-    const int base = blockIdx.x * kTile;
-    for (int k = threadIdx.x; k < kTile; k += kThreads)
-        stage[k] = base + k < n ? counts[n - 1 - (base + k)] : 0;
+    __shared__ int s_tile;
+    __shared__ long long s_before;
+    if (threadIdx.x == 0) {
+        s_tile = int(atomicAdd(ticket, 1u));
+        if (s_tile == int(gridDim.x) - 1) *ticket = 0u;  // the last one to take a number
+    }
     __syncthreads();
-    int acc = 0;
-    int c[kItems];
+    const int tile = s_tile, base = tile * kTile;
+    const double weight = sc[0];
+    int ci[kItems];
+    double b[kItems];
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int i = n - 1 - (base + int(threadIdx.x) + q * kThreads);
+        ci[q] = i >= 0 ? counts[i] : 0;
+        b[q] = i >= 0 ? load_src(v, i, omega, has) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) stage[swz<4>(threadIdx.x + q * kThreads)] = ci[q];
+    __syncthreads();
+    int c[kItems], acc = 0;
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
-        c[k] = stage[threadIdx.x * kItems + k];
+        c[k] = stage[swz<4>(threadIdx.x * kItems + k)];
         acc += c[k];
     }
     int excl;
-    block_scan(acc, AddOp(), 0, warp_tot, &excl);
-    int o = part[blockIdx.x] + excl;
-    __syncthreads();
+    const int incl = block_scan(acc, AddOp(), 0, warp_tot, &excl);
+    if (threadIdx.x == kThreads - 1) {
+        *reinterpret_cast<volatile unsigned long long*>(&emitted[tile]) =
+            (tile == 0 ? kUpTo : kOwnCount) | (unsigned long long)incl;
+        warp_tot[0] = incl;
+    }
+    int o = excl;
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
-        stage[threadIdx.x * kItems + k] = o;
+        stage[swz<4>(threadIdx.x * kItems + k)] = o;
         o += c[k];
     }
     __syncthreads();
-    const double weight = sc[0];
-    for (int k = threadIdx.x; k < kTile; k += kThreads) {
-        if (base + k >= n) break;
-        const int i = n - 1 - (base + k);
-        const int ci = counts[i], at = stage[k];
-        const double b = load_src(v, i, omega, has);
-        const unsigned sign = b > 0.0 ? 0u : 0x80000000u;  // weight_sign (:169)
-        if (ci > 0) {
-            if (at + ci > cap) {
+    if (threadIdx.x < 32) {
+        const long long before = tile > 0 ? look_back(emitted, tile, status) : 0;
+        if (threadIdx.x == 0) {
+            const long long upto = before + warp_tot[0];
+            if (tile > 0)
+                *reinterpret_cast<volatile unsigned long long*>(&emitted[tile]) =
+                    kUpTo | (unsigned long long)upto;
+            s_before = before;
+            if (strat && tile == int(gridDim.x) - 1) {
+                if (upto > cap) atomicOr(status, DEV_ERR_CAPACITY);
+                const int nh = upto > cap ? cap : int(upto);
+                *d_nh = nh;
+                sc[2] = nh > 0 ? 1.0 / double(nh) : 0.0;
+            }
+        }
+    }
+    __syncthreads();
+    const long long before = s_before;
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int k = threadIdx.x + q * kThreads, i = n - 1 - (base + k);
+        if (i < 0) break;
+        const unsigned sign = b[q] > 0.0 ? 0u : 0x80000000u;  // weight_sign (:169)
+        double yi = 0.0;
+        if (ci[q] > 0) {
+            const long long at = before + stage[swz<4>(k)];
+            if (at + ci[q] > cap) {
                 atomicOr(status, DEV_ERR_CAPACITY);
             } else {
-                for (int t = 0; t < ci; ++t) start[at + t] = int(unsigned(i) | sign);
+                for (int t = 0; t < ci[q]; ++t) start[at + t] = int(unsigned(i) | sign);
             }
-            y[i] = double(ci) * (sign ? -weight : weight);
-        } else {
-            y[i] = 0.0;
+            yi = double(ci[q]) * (sign ? -weight : weight);
         }
+        y[i] = yi;
     }
 }
 
@@ -843,7 +904,7 @@ void launch_adjoint_source(mclsgpu_domain* dom, const double* v, double omega, i
     if (!strat) {
         auto cdf = parity ? k_src_cdf<false> : k_src_cdf<true>;
         cdf<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, dom->part, dom->d_scalars, dom->scdf,
-                                    dom->counts, dom->guide, G);
+                                    dom->counts, dom->guide, G, dom->emitted);
         const int sample_grid = p.rng_mode == MCLSGPU_RNG_COUNTER ? ctx->num_sms * 8 : 64;
         k_sample<<<sample_grid, 256, 0, s>>>(dom->scdf, dom->guide, n, G, dom->d_nh, p.rng_mode,
                                              dom->seed, dom->d_epoch, dom->d_jump, dom->d_pos,
@@ -851,13 +912,11 @@ void launch_adjoint_source(mclsgpu_domain* dom, const double* v, double omega, i
         if (p.rng_mode == MCLSGPU_RNG_REFERENCE) k_advance_pos<<<1, 1, 0, s>>>(dom->d_pos, dom->d_nh, 1);
     } else {
         k_strat_counts<<<grid_for(n), 256, 0, s>>>(v, n, omega, has_omega, dom->d_scalars,
-                                                   dom->counts);
+                                                   dom->counts, dom->emitted);
     }
-    k_src_count<<<nb, kThreads, 0, s>>>(dom->counts, n, strat, cap, dom->ipart, dom->d_ticket,
-                                        dom->d_scalars, dom->d_nh, ctx->d_status);
-    k_src_expand<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, dom->counts, dom->ipart,
-                                         dom->d_scalars, cap, dom->start, dom->y64,
-                                         ctx->d_status);
+    k_src_emit<<<nb, kThreads, 0, s>>>(v, n, omega, has_omega, strat, dom->counts, dom->emitted,
+                                       dom->d_ticket, dom->d_scalars, cap, dom->start, dom->y64,
+                                       dom->d_nh, ctx->d_status);
 }
 
 void launch_forward_setup(mclsgpu_domain* dom) {

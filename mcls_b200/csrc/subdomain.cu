@@ -91,7 +91,7 @@ void release_source(mclsgpu_domain* d) {
     dfree(d->d_ticket);
     dfree(d->d_scalars);
     dfree(d->part);
-    dfree(d->ipart);
+    dfree(d->emitted);
     dfree(d->d_epoch);
     dfree(d->d_pos);
 }
@@ -226,7 +226,7 @@ int mclsgpu_subdomain_build(mclsgpu_context* ctx, int64_t n_global, int32_t npar
              (e = dmalloc(&g.y64, N)) != cudaSuccess || (e = dmalloc(&g.d_nh, 1)) != cudaSuccess ||
              (e = dmalloc(&g.d_scalars, 16)) != cudaSuccess ||
              (e = dmalloc(&g.part, parts)) != cudaSuccess ||
-             (e = dmalloc(&g.ipart, parts)) != cudaSuccess ||
+             (e = dmalloc(&g.emitted, parts)) != cudaSuccess ||
              (e = dmalloc(&g.d_epoch, 1)) != cudaSuccess || (e = dmalloc(&g.d_pos, 1)) != cudaSuccess ||
              (e = dmalloc(&sd->y, sd->n)) != cudaSuccess ||
              (e = dmalloc(&sd->srcp, sd->n)) != cudaSuccess ||

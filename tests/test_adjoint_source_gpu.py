@@ -99,3 +99,23 @@ def test_stratified_counts(ctx, n):
     near = np.abs(f - np.round(f)) < 1e-9
     assert nh == got.sum() and np.array_equal(got[~near], want[~near])
     assert np.all(np.diff(tr["start"]) <= 0)
+
+
+# More tiles than one look-back reads (32 at a time) and than run at once.
+@pytest.mark.parametrize("n", [32 * 2048, 33 * 2048 + 1, 3_000_001])
+@pytest.mark.parametrize("stratified", [False, True])
+def test_emission_over_many_tiles(ctx, n, stratified):
+    gen = np.random.default_rng(n)
+    A = sp.csr_matrix(0.7 * sp.eye(n))
+    dom = capi.Domain(ctx, capi.Operator(ctx, A), None, precision=capi.FP64,
+                      rng_mode=capi.RNG_COUNTER, seed=9, history_length=1, sample_ratio=1.0,
+                      source_sampling=capi.SOURCE_STRATIFIED if stratified
+                      else capi.SOURCE_RANDOM)
+    v = source("positive_first", n, gen)
+    x, nh, tr = dom.mc_trace(v, 4 * n + 4, internal=True)
+    got = tr["start"]
+    assert got.size == nh and np.all(np.diff(got) <= 0)
+    # x = counts * (+-|v|_1) / nh: the counts of the states, from the tally.
+    counts = np.bincount(got, minlength=n)
+    w0 = np.abs(v).sum() * np.where(v > 0, 1.0, -1.0)
+    np.testing.assert_allclose(x, counts * w0 / nh, rtol=1e-10, atol=0)
