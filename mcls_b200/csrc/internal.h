@@ -151,7 +151,8 @@ RowOrder row_order(int n, int K, const int* off, int rows);
 // What a forward fixed-length FP32 walk does with a row's sum of `per`
 // histories: d = sum / per [+ source (expected value)], then out = d,
 // out + d, or xin + d.
-enum : int { kBaseNone = 0, kBaseOut = 1, kBaseIn = 2 };
+// kBaseTally: nothing, the caller's next pass reads the tallies (adjoint).
+enum : int { kBaseNone = 0, kBaseOut = 1, kBaseIn = 2, kBaseTally = 3 };
 struct RowFinish {
     double* out = nullptr;
     const double* src = nullptr;

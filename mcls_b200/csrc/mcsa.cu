@@ -295,8 +295,8 @@ constexpr int kFusedThreads = 256;
 
 // Richardson smoothing fused with the residual: x2 = x + w rp (rounded as the
 // separate update would be) and rp2 = PL (b - A x2), reading x + w rp at the
-// neighbours on the fly (Anderson steps; the MCSA loop has x2 from the last
-// iteration's k_residual_norm).
+// neighbours on the fly (Anderson steps and adjoint domains; a forward MCSA
+// loop has x2 from the last iteration's k_residual_norm).
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_smoothed_residual(
     Op A, const double* b, const double* dinv, const double* x, const double* r, double w,
@@ -313,10 +313,12 @@ struct ResidArgs {
     int n;
     const double* b;
     const double* dinv;       // null: no left preconditioner
-    const double* x;          // the corrected iterate
+    double* x;                // the corrected iterate
     double* rout;
-    double* x2;               // x + w rp: the next iteration's smoothed iterate
+    double* x2;               // the smoothed iterate: read (FOLD) or the next x + w rp
     double w;
+    const double* y;          // FOLD: the walk's tallies and 1 / histories
+    const double* inv_nh;
     double* part;
     unsigned int* ticket;
     McsaState* st;
@@ -391,19 +393,38 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
 // (256, 8): eight blocks an SM, the grid's size, must be resident; with the 46
 // registers that the one thread's check asks for five were, and the pass took
 // 33 us at 128^3 instead of 28.9 us (k_mcsa_begin: 43 and 32.3 us).
-template <class Op>
-__global__ void __launch_bounds__(kFusedThreads, 8) k_residual_norm(Op A, ResidArgs a) {
-    const double* x = a.x;
+//
+// FOLD: the collision tallies of adjoint walks are normalised and added here
+// (x = x2 + y / nh, formed at the neighbours as well), which saves the pass
+// that did it (5 us at 64^3, 3 us at 10^4 states); the next smoothed iterate is
+// then left to the next smoothing pass, since x2 is read at the neighbours.
+template <bool FOLD, class Op>
+__device__ __forceinline__ void residual_norm(const Op& A, const ResidArgs& a) {
+    const double inv = FOLD ? *a.inv_nh : 0.0;
+    auto x = [&](int j) {
+        // AdjointTally::normalize: x *= 1/nh  (src/MCLS_AdjointTally_impl.hpp:68-72)
+        if constexpr (FOLD) return __dadd_rn(a.x2[j], __dmul_rn(a.y[j], inv));
+        else return a.x[j];
+    };
     double acc = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
-        const double s = A.dot(i, [&](int j) { return x[j]; });
+        const double s = A.dot(i, x);
         const double res = a.b[i] - s;
         const double r = a.dinv ? a.dinv[i] * res : res;
         a.rout[i] = r;
-        a.x2[i] = __dadd_rn(x[i], __dmul_rn(a.w, r));
+        if constexpr (FOLD) a.x[i] = x(i);
+        else a.x2[i] = __dadd_rn(x(i), __dmul_rn(a.w, r));
         acc = fma(r, r, acc);
     }
     norm_and_check(a, acc);
+}
+template <class Op>
+__global__ void __launch_bounds__(kFusedThreads, 8) k_residual_norm(Op A, ResidArgs a) {
+    residual_norm<false>(A, a);
+}
+template <class Op>
+__global__ void __launch_bounds__(kFusedThreads, 8) k_finalize_norm(Op A, ResidArgs a) {
+    residual_norm<true>(A, a);
 }
 
 // A left preconditioner M stored on A's diagonals (learned SPAI): out = M v.
@@ -709,8 +730,9 @@ int mcsa_finish_report(mclsgpu_domain* dom, mclsgpu_stats* st) {
 // One MC solve of the source vector `v` (device, already left preconditioned
 // when required) into out: out = delta, out + delta or x2 + delta (`base`).
 // Walks that finish their rows themselves write out; the others' tallies are
-// normalised and added by k_finalize.  `fused`: inside the fused MCSA iteration the epoch increment
-// and the walk bookkeeping are done by k_residual_norm.
+// normalised and added by k_finalize (base kBaseTally: by the caller's next
+// pass).  `fused`: inside the fused MCSA iteration the epoch increment and the
+// walk bookkeeping are done by k_residual_norm.
 static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int base,
                        long long max_trace, long long* tr_states, double* tr_w, int* tr_ev,
                        long long* tr_start, bool fused = false, bool report = false) {
@@ -737,7 +759,7 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
     launch_walk(dom, fin, max_trace, tr_states, tr_w, tr_ev, tr_start, fused);
     launch_advance_walk_pos(dom);
     cudaStream_t s = dom->ctx->stream;
-    if (!walk_finishes(dom)) {
+    if (!walk_finishes(dom) && base != kBaseTally) {
         FinalizeArgs f{};
         f.n = dom->n;
         f.mode = p.direction == MCLSGPU_FORWARD ? 2 : (ev ? 1 : 0);
@@ -883,14 +905,20 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     // goes to tmp and a second pass applies M.
     const double* mdia = dom->left ? dom->left->mdia : nullptr;
     const int grid = fused_grid(dom);
-    if (mdia) {
+    // The last pass can add the tallies itself when it needs nothing but them.
+    const bool fold = !mdia && dom->p.direction == MCLSGPU_ADJOINT &&
+                      dom->p.estimator == MCLSGPU_COLLISION;
+    if (fold) {
+        richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, dom->x2, dom->rp2);
+    } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, nullptr,
                           dom->tmp);
         MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_dia_apply, dom->tmp, dom->rp2);
     } else {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, dinv, dom->rp2);
     }
-    enqueue_mc(dom, dom->rp2, dom->x, kBaseIn, 0, nullptr, nullptr, nullptr, nullptr, true);
+    enqueue_mc(dom, dom->rp2, dom->x, fold ? kBaseTally : kBaseIn, 0, nullptr, nullptr, nullptr,
+               nullptr, true);
     ResidArgs a{};
     a.n = n;
     a.b = dom->b;
@@ -899,6 +927,8 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     a.rout = dom->rp;
     a.x2 = dom->x2;
     a.w = mp->richardson_omega;
+    a.y = dom->y64;
+    a.inv_nh = dom->d_scalars + 2;
     a.part = dom->part;
     a.ticket = dom->d_ticket;
     a.st = dom->d_state;
@@ -916,6 +946,8 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x, dom->b, nullptr,
                           dom->tmp);
         MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_precond_norm, a, dom->tmp);
+    } else if (fold) {
+        MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_finalize_norm, a);
     } else {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual_norm, a);
     }
