@@ -156,6 +156,7 @@ void release_domain(mclsgpu_domain* d) {
     dfree(d->w);
     dfree(d->dt_h32);
     dfree(d->rec);
+    dfree(d->rec64);
     dfree(d->walk_order);
     dfree(d->d_jump);
     dfree(d->hoff);

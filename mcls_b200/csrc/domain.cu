@@ -16,6 +16,8 @@
 #include <climits>
 #include <vector>
 
+#include <math_constants.h>
+
 #include "internal.h"
 
 namespace mclsgpu {
@@ -94,6 +96,27 @@ __global__ void k_pack_records(const int* drp, const int* dcol, const double* dh
                 r[1 + t] = make_uint2(__float_as_uint(2.0f), 0u);
             }
         }
+    }
+}
+
+// FP64 records of rows with at most 7 entries: W, the CDF (padding +inf),
+// columns, and a word with the length and (bit 8 + j) the entries whose weight
+// is negative.
+__global__ void k_pack_records64(const int* drp, const int* dcol, const double* dh,
+                                 const double* dcdf, const double* dw, int n, Record64* rec) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int a = drp[i], len = drp[i + 1] - a;
+        Record64 r;
+        r.W = dw[i];
+        unsigned meta = unsigned(len);
+#pragma unroll
+        for (int t = 0; t < Record64::kEntries; ++t) {
+            r.cdf[t] = t < len ? dcdf[a + t] : CUDART_INF;
+            r.col[t] = t < len ? dcol[a + t] : 0;
+            if (t < len && !(dh[a + t] > 0.0)) meta |= 1u << (8 + t);
+        }
+        r.meta = meta;
+        rec[i] = r;
     }
 }
 
@@ -287,6 +310,15 @@ int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "domain fill");
     if ((rc = check_device_status(ctx))) return rc;
+
+    if (dom->p.precision == MCLSGPU_FP64 && hmax <= Record64::kEntries) {
+        // Without the memory for them the walk reads the CSR domain.
+        if (dmalloc(&dom->rec64, n) == cudaSuccess)
+            k_pack_records64<<<grid_for(n), 256, 0, s>>>(D.rp, D.ci, D.v, dom->cdf, dom->w, n,
+                                                         dom->rec64);
+        else
+            cudaGetLastError();
+    }
 
     // FP32 records, packed format: slot count = 1 + longest row, rounded up to
     // a supported stride.

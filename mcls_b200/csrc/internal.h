@@ -170,6 +170,16 @@ struct RowFinish {
 
 }  // namespace mclsgpu
 
+// One row of an FP64 walk in three 32-byte sectors.
+struct alignas(32) Record64 {
+    static constexpr int kEntries = 7;
+    double W;
+    double cdf[kEntries];
+    int col[kEntries];
+    unsigned meta;  // row length | (negative weights << 8)
+};
+static_assert(sizeof(Record64) == 96, "three sectors");
+
 struct mclsgpu_domain {
     mclsgpu_context* ctx = nullptr;
     mclsgpu_operator* op = nullptr;
@@ -187,6 +197,7 @@ struct mclsgpu_domain {
     float* dt_h32 = nullptr;
     // Packed FP32 walk records: row r at rec + r*slots, slot 0 = {W, len},
     // slots 1..slots-1 = {cdf (float bits), col | sign<<31}.
+    Record64* rec64 = nullptr;     // FP64 walks, rows of at most 7 entries (else null)
     uint2* rec = nullptr;
     int slots = 0;
     int max_row = 0;

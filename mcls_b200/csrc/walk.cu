@@ -19,10 +19,9 @@
 // * w0), so walks tally from step 1; histories ended by a weight cutoff
 // (walk32_cutoff) are pulled from a work queue.
 //
-// walk64: the parity kernel.  FP64 CSR domain, binary search with
-// std::lower_bound semantics, FP64 weights and tallies, optional trajectory
-// trace.  With the reference stream it reproduces the reference's
-// trajectories bit for bit.
+// walk64: the parity kernel.  FP64 domain, std::lower_bound's selection, FP64
+// weights and tallies, optional trajectory trace.  With the reference stream it
+// reproduces the reference's trajectories bit for bit.
 #include <climits>
 
 #include "internal.h"
@@ -47,7 +46,8 @@ struct WalkArgs {
     const unsigned long long* d_pos;
     // FP32 records
     const uint2* rec;
-    // FP64 domain
+    // FP64 records (walk64, PACKED) and domain
+    const Record64* rec64;
     const int* rp;
     const int* col;
     const double* h;
@@ -195,6 +195,30 @@ __device__ __forceinline__ int select64(const WalkArgs& a, int s, double u, int&
         if (a.cdf[r0 + mid] < u) lo = mid + 1; else hi = mid;
     }
     return lo;
+}
+
+// The same transition from a packed record: the CDF does not fall along a row,
+// so std::lower_bound's position is the number of values below u.
+__device__ __forceinline__ void select_record64(const Record64* rec, int s, double u, double& Ws,
+                                                int& col, int* status) {
+    uint32_t q[24];
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+        ld_record256(reinterpret_cast<const char*>(rec + s) + 32 * t, q + 8 * t);
+    int lo = 0;
+#pragma unroll
+    for (int j = 0; j < Record64::kEntries; ++j)
+        lo += __hiloint2double(int(q[3 + 2 * j]), int(q[2 + 2 * j])) < u;
+    const int len = int(q[23] & 0xffu);
+    if (lo >= len) {
+        atomicOr(status, DEV_ERR_BOUNDS);
+        lo = len - 1;
+    }
+    col = int(q[16]);
+#pragma unroll
+    for (int j = 1; j < Record64::kEntries; ++j) col = lo == j ? int(q[16 + j]) : col;
+    const double W = __hiloint2double(int(q[1]), int(q[0]));
+    Ws = (q[23] >> (8 + lo)) & 1u ? -W : W;
 }
 
 // One transition of a history at state s (DomainTransporter::transport's
@@ -461,7 +485,11 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S>::kMinBlocks) walk32_cuto
     walk_end_time(a);
 }
 
-template <int DIR>
+// Bound by the latency of a step's loads.  PACKED: rows of at most 7 entries, one
+// record of three sectors per step, 12.3 us for 10^4 histories; the
+// general form follows row pointers, CDF (a binary search), weight and column
+// one after the other, 18.7 us there.
+template <int DIR, bool PACKED>
 __global__ void __launch_bounds__(128) walk64(WalkArgs a) {
     const int nh = *a.d_nh;
     const double weight = a.sc[0];
@@ -498,15 +526,20 @@ __global__ void __launch_bounds__(128) walk64(WalkArgs a) {
             }
             x = xs_step(x);
             const double u = canonical64(x);
-            int r0, len;
-            int lo = select64(a, s, u, r0, len);
-            if (lo >= len) {
-                atomicOr(a.status, DEV_ERR_BOUNDS);
-                lo = len - 1;
+            double Ws;
+            if constexpr (PACKED) {
+                select_record64(a.rec64, s, u, Ws, s, a.status);
+            } else {
+                int r0, len;
+                int lo = select64(a, s, u, r0, len);
+                if (lo >= len) {
+                    atomicOr(a.status, DEV_ERR_BOUNDS);
+                    lo = len - 1;
+                }
+                Ws = a.h[r0 + lo] > 0.0 ? a.W[s] : -a.W[s];
+                s = a.col[r0 + lo];
             }
-            const double Ws = a.h[r0 + lo] > 0.0 ? a.W[s] : -a.W[s];
             w = __dmul_rn(w, Ws);
-            s = a.col[r0 + lo];
             ++k;
             ++steps;
             if (tr) a.tr_states[e * (L + 1) + k] = s;
@@ -903,6 +936,7 @@ static void fill_walk_args(mclsgpu_domain* dom, WalkArgs& a) {
     a.jump = dom->d_jump;
     a.d_pos = dom->d_pos;
     a.rec = dom->rec;
+    a.rec64 = dom->rec64;
     a.d_steps = dom->d_steps;
     a.d_tim = dom->d_tim;
     a.status = ctx->d_status;
@@ -971,6 +1005,15 @@ __global__ void k_update_offsets(int* hoff, const int* hoff2, const int* d_nh, i
 
 __global__ void k_advance_pos_by(unsigned long long* d_pos, long long draws) { *d_pos += draws; }
 
+static void launch_walk64(const mclsgpu_domain* dom, const WalkArgs& a, int grid) {
+    cudaStream_t st = dom->ctx->stream;
+    const bool adjoint = dom->p.direction == MCLSGPU_ADJOINT;
+    auto kernel = dom->rec64 ? (adjoint ? walk64<MCLSGPU_ADJOINT, true> : walk64<MCLSGPU_FORWARD, true>)
+                             : (adjoint ? walk64<MCLSGPU_ADJOINT, false>
+                                        : walk64<MCLSGPU_FORWARD, false>);
+    kernel<<<grid, 128, 0, st>>>(a);
+}
+
 // Variable-length histories on the reference stream (a Weight Cutoff with
 // "Reproducible MC Mode"): the reference draws history e's uniforms right
 // after history e-1's, so e's first draw depends on every earlier length.
@@ -999,10 +1042,7 @@ static void walk_reference_rounds(mclsgpu_domain* dom, WalkArgs a, int grid) {
     int rounds = 0;
     for (;;) {
         ++rounds;
-        if (dom->p.direction == MCLSGPU_ADJOINT)
-            walk64<MCLSGPU_ADJOINT><<<grid, 128, 0, st>>>(a);
-        else
-            walk64<MCLSGPU_FORWARD><<<grid, 128, 0, st>>>(a);
+        launch_walk64(dom, a, grid);
         if (nh == 0 || exclusive_scan_counts_dev(ctx, dom->hlen, nh, dom->hoff2, &total)) break;
         cudaMemsetAsync(changed, 0, sizeof(int), st);
         k_update_offsets<<<grid, 128, 0, st>>>(dom->hoff, dom->hoff2, dom->d_nh, changed);
@@ -1057,10 +1097,8 @@ void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
         const int grid = int(g < ctx->num_sms * 8 ? g : ctx->num_sms * 8);
         if (walk_needs_rounds(dom))
             walk_reference_rounds(dom, a, grid);
-        else if (p.direction == MCLSGPU_ADJOINT)
-            walk64<MCLSGPU_ADJOINT><<<grid, 128, 0, st>>>(a);
         else
-            walk64<MCLSGPU_FORWARD><<<grid, 128, 0, st>>>(a);
+            launch_walk64(dom, a, grid);
     }
 }
 
