@@ -16,8 +16,9 @@
 //                  the drop's rotations on Q, v = F - F_old, dX = x - x_old
 //                  and r = <q_0, v> (|v|^2 for an empty store)
 //   MGS passes     one per further stored column: v -= r q_{j-1},
-//                  r = <q_j, v> (|v|^2 after the last)
-//   control        R's new diagonal; optional drops for the condition number
+//                  r = <q_j, v> (|v|^2 after the last); the last one's last
+//                  block then sets R's new diagonal and makes the optional
+//                  drops for the condition number
 //   RHS pass       q_new = v / |v|, post-add rotations, <F, q_j>; the last
 //                  block back-solves R gamma = Q^T F
 //   update pass    x = x + beta F - sum (gamma_j dX_j + beta (R gamma)_j q_j)
@@ -32,6 +33,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "ops.cuh"
 
 namespace mclsgpu {
 
@@ -91,6 +93,15 @@ struct Args {
     double* hist;
     int hist_cap;
     int* status;
+    int depth;             // storage depth (0: no acceleration)
+    const double* b;       // residual pass: b and PL's diagonal (null: PL = I)
+    const double* dinv;
+    double* r;
+    // The Monte Carlo solve's bookkeeping (null d_nh: its own launch did it).
+    const int* d_nh;
+    unsigned long long* d_epoch;
+    unsigned long long* d_hist;
+    unsigned long long* d_tim;
     cudaGraphConditionalHandle handle;
     int use_cond;
 };
@@ -137,48 +148,75 @@ __device__ __forceinline__ void for_elements(int n, Body body) {
         body(std::integral_constant<int, 1>{}, n - 1);
 }
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+// The block's sums of v[0..m) into sums[0..m): warps by shuffles, then the warps
+// in order.
+template <int M>
+__device__ __forceinline__ void block_sums(const double (&v)[M], int m,
+                                           double (*sh)[kThreads / 32], double* sums) {
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        if (j < m) {
+            double x = v[j];
+            for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
+            if ((threadIdx.x & 31) == 0) sh[j][threadIdx.x >> 5] = x;
+        }
+    }
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    if (int(threadIdx.x) < m) {
+        double t = 0.0;
+        for (int w = 0; w < kThreads / 32; ++w) t += sh[threadIdx.x][w];
+        sums[threadIdx.x] = t;
+    }
     __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < kThreads / 32; ++w) t += sh[w];
-    return t;
 }
 
-// Publish this block's sums of v0 and v1; true in the block that finishes
-// last, whose thread 0 then holds the grid totals (block order, fixed for a
-// fixed launch).
-__device__ __forceinline__ bool grid_sum2(double v0, double v1, const Args& a, double* t0,
-                                          double* t1) {
-    __shared__ double sh[kThreads / 32];
+// Publish this block's sums of v[0..m); true in the block that finishes last,
+// which then holds the grid totals (block order, fixed for a fixed launch) in
+// sums.
+template <int M>
+__device__ __forceinline__ bool grid_sums(const double (&v)[M], int m, const Args& a,
+                                          double* sums) {
+    __shared__ double sh[M][kThreads / 32];
     __shared__ bool last;
-    const double s0 = block_sum(v0, sh);
-    const double s1 = block_sum(v1, sh);
+    block_sums<M>(v, m, sh, sums);
+    if (int(threadIdx.x) < m) {
+        a.part[size_t(blockIdx.x) * M + threadIdx.x] = sums[threadIdx.x];
+        __threadfence();
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        a.part[2 * blockIdx.x] = s0;
-        a.part[2 * blockIdx.x + 1] = s1;
         __threadfence();
         last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        if (last) *a.ticket = 0u;
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    double u0 = 0.0, u1 = 0.0;
+    double u[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) u[j] = 0.0;
+#pragma unroll 4
     for (int k = threadIdx.x; k < int(gridDim.x); k += blockDim.x) {
-        u0 += a.part[2 * k];
-        u1 += a.part[2 * k + 1];
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+            if (j < m) u[j] += __ldcg(&a.part[size_t(k) * M + j]);
     }
-    const double r0 = block_sum(u0, sh);
-    const double r1 = block_sum(u1, sh);
-    if (threadIdx.x == 0) {
-        *t0 = r0;
-        *t1 = r1;
-        *a.ticket = 0u;
-    }
+    block_sums<M>(u, m, sh, sums);
     return true;
+}
+
+// The state in shared memory while one thread works on it (the last block of a
+// pass): word after word in global memory that work took 4 to 14 us a step.
+__device__ __forceinline__ void load_state(AaState* sh, const AaState* st) {
+    static_assert(sizeof(AaState) % sizeof(double) == 0, "copied in words");
+    for (int k = threadIdx.x; k < int(sizeof(AaState) / sizeof(double)); k += blockDim.x)
+        reinterpret_cast<double*>(sh)[k] = __ldcg(reinterpret_cast<const double*>(st) + k);
+    __syncthreads();
+}
+__device__ __forceinline__ void store_state(AaState* st, const AaState* sh) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < int(sizeof(AaState) / sizeof(double)); k += blockDim.x)
+        reinterpret_cast<double*>(st)[k] = reinterpret_cast<const double*>(sh)[k];
 }
 
 // Drop the oldest column (one thread): rotations that restore R's triangle
@@ -209,10 +247,9 @@ __device__ void qr_delete(AaState* st) {
     st->dx_head = (st->dx_head + 1) % st->m;
 }
 
-// Reciprocal 1-norm condition number of the stored R (one thread).
-__device__ double rcond(const AaState* st) {
+// Reciprocal 1-norm condition number of the stored R (one thread; Ri: scratch).
+__device__ double rcond(const AaState* st, double (*Ri)[kMaxDepth]) {
     const int N = st->nstore;
-    double Ri[kMaxDepth][kMaxDepth];
     for (int j = 0; j < N; ++j)
         for (int i = j; i >= 0; --i) {
             double s = i == j ? 1.0 : 0.0;
@@ -250,24 +287,77 @@ __device__ void plan(AaState* st) {
     }
 }
 
-// Apply the recorded rotations to elements i..i+W-1 of the Q columns.
+// New diagonal entry of R, then the drops for the condition number (one thread).
+__device__ void control(AaState* st, double (*Ri)[kMaxDepth]) {
+    st->nrot = 0;
+    st->ok = 0;
+    if (st->add) {
+        const int nc = st->newcol;
+        const double rn = sqrt(st->vnorm2);
+        if (rn > 0.0 && isfinite(rn)) {
+            st->R[nc][nc] = rn;
+            st->inv_rnn = 1.0 / rn;
+            st->nstore = nc + 1;
+            st->ok = 1;
+        } else {
+            for (int j = 0; j < nc; ++j) st->R[j][nc] = 0.0;
+        }
+    }
+    if (st->adjust)
+        while (st->nstore > 1 && rcond(st, Ri) < st->droptol) qr_delete(st);
+}
+
+// The end of a Gram-Schmidt pass (the last block): its total t is R(j, new), or
+// |v|^2 after the last stored column, when the control follows.  fnorm2 (not
+// null): |F|^2.
+__device__ __forceinline__ void end_pass(const Args& a, int j, bool add, int nc, const double* t,
+                                         const double* fnorm2) {
+    const bool finished = !add || j >= nc;
+    if (!finished || a.depth == 0) {
+        if (threadIdx.x == 0) {
+            if (fnorm2) a.st->fnorm2 = *fnorm2;
+            if (add && !finished) a.st->R[j][nc] = *t;
+        }
+        return;
+    }
+    __shared__ AaState sh;
+    __shared__ double Ri[kMaxDepth][kMaxDepth];
+    load_state(&sh, a.st);
+    if (threadIdx.x == 0) {
+        if (fnorm2) sh.fnorm2 = *fnorm2;
+        if (add) sh.vnorm2 = *t;
+        control(&sh, Ri);
+    }
+    store_state(a.st, &sh);
+}
+
+// Apply the recorded rotations to elements i..i+W-1 of the Q columns.  A drop's
+// rotations run down adjacent columns (0,1), (1,2), ..: the column that two of
+// them share stays in registers, so each is read and written once.
 template <int W>
 __device__ __forceinline__ void rotate_q(const Args& a, const AaState* st, int nrot, int i) {
+    int held = -1;  // the column in u
+    Vec<W> u;
     for (int r = 0; r < nrot; ++r) {
         const int c0 = st->ri[r];
         const double c = st->rc[r], s = st->rs[r];
         double* qa = a.Q + size_t(c0) * a.ld;
         double* qb = qa + a.ld;
-        const Vec<W> u = ldv<W>(qa, i), v = ldv<W>(qb, i);
-        Vec<W> ua, vb;
+        if (c0 != held) {
+            if (held >= 0) stv<W>(a.Q + size_t(held) * a.ld, i, u);
+            u = ldv<W>(qa, i);
+        }
+        const Vec<W> v = ldv<W>(qb, i);
+        Vec<W> ua;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             ua.v[w] = __dadd_rn(__dmul_rn(c, u.v[w]), __dmul_rn(s, v.v[w]));
-            vb.v[w] = __dadd_rn(__dmul_rn(-s, u.v[w]), __dmul_rn(c, v.v[w]));
+            u.v[w] = __dadd_rn(__dmul_rn(-s, u.v[w]), __dmul_rn(c, v.v[w]));
         }
         stv<W>(qa, i, ua);
-        stv<W>(qb, i, vb);
+        held = c0 + 1;
     }
+    if (held >= 0) stv<W>(a.Q + size_t(held) * a.ld, i, u);
 }
 
 __global__ void k_aa_init(AaState* st, int max_iters, int m, int start, int adjust, double beta,
@@ -300,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) k_aa_first(Args a) {
     double* dxn = add ? a.DX + size_t((st->dx_head + nc) % st->m) * a.ld : nullptr;
     const double* __restrict__ f = a.f;
     const double* __restrict__ dl = a.delta;
-    double accF = 0.0, accV = 0.0;
+    double acc[2] = {0.0, 0.0};  // |F|^2, <q_0, v> or |v|^2
     for_elements(a.n, [&](auto wt, int i) {
         constexpr int W = decltype(wt)::value;
         const Vec<W> fv = ldv<W>(f, i), dv = ldv<W>(dl, i), xv = ldv<W>(a.x, i);
@@ -308,7 +398,7 @@ __global__ void __launch_bounds__(kThreads) k_aa_first(Args a) {
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             Fv.v[w] = __dadd_rn(__dadd_rn(fv.v[w], __dmul_rn(a.dscale, dv.v[w])), -xv.v[w]);
-            accF = fma(Fv.v[w], Fv.v[w], accF);
+            acc[0] = fma(Fv.v[w], Fv.v[w], acc[0]);
         }
         stv<W>(a.F, i, Fv);
         if (!add) return;
@@ -325,28 +415,20 @@ __global__ void __launch_bounds__(kThreads) k_aa_first(Args a) {
         if (nc > 0) {
             const Vec<W> q = ldv<W>(a.Q, i);
 #pragma unroll
-            for (int w = 0; w < W; ++w) accV = fma(q.v[w], v.v[w], accV);
+            for (int w = 0; w < W; ++w) acc[1] = fma(q.v[w], v.v[w], acc[1]);
         } else {
 #pragma unroll
-            for (int w = 0; w < W; ++w) accV = fma(v.v[w], v.v[w], accV);
+            for (int w = 0; w < W; ++w) acc[1] = fma(v.v[w], v.v[w], acc[1]);
         }
     });
-    double tF, tV;
-    if (!grid_sum2(accF, accV, a, &tF, &tV) || threadIdx.x != 0) return;
-    AaState* sw = a.st;
-    sw->fnorm2 = tF;
-    if (add) {
-        if (nc > 0)
-            sw->R[0][nc] = tV;
-        else
-            sw->vnorm2 = tV;
-    }
+    __shared__ double sums[2];
+    if (grid_sums<2>(acc, add ? 2 : 1, a, sums)) end_pass(a, 0, add, nc, &sums[1], &sums[0]);
 }
 
 // Gram-Schmidt pass j >= 1 of the new column (modified Gram-Schmidt: one
 // stored column per pass): v -= R(j-1, new) q_{j-1}; R(j, new) = <q_j, v>,
 // or |v|^2 after the last stored column.
-__global__ void __launch_bounds__(kThreads) k_aa_mgs(Args a, int j) {
+__global__ void __launch_bounds__(kThreads, 8) k_aa_mgs(Args a, int j) {
     const AaState* st = a.st;
     const int add = st->add, nc = st->newcol;
     if (!add || j > nc) return;  // the same in every block
@@ -354,7 +436,7 @@ __global__ void __launch_bounds__(kThreads) k_aa_mgs(Args a, int j) {
     const double* __restrict__ qprev = a.Q + size_t(j - 1) * a.ld;
     const double* __restrict__ qj = j < nc ? a.Q + size_t(j) * a.ld : nullptr;
     double* __restrict__ V = a.V;
-    double acc = 0.0;
+    double acc[1] = {0.0};
     for_elements(a.n, [&](auto wt, int i) {
         constexpr int W = decltype(wt)::value;
         const Vec<W> vo = ldv<W>(V, i), qp = ldv<W>(qprev, i);
@@ -365,38 +447,14 @@ __global__ void __launch_bounds__(kThreads) k_aa_mgs(Args a, int j) {
         if (qj) {
             const Vec<W> q = ldv<W>(qj, i);
 #pragma unroll
-            for (int w = 0; w < W; ++w) acc = fma(q.v[w], v.v[w], acc);
+            for (int w = 0; w < W; ++w) acc[0] = fma(q.v[w], v.v[w], acc[0]);
         } else {
 #pragma unroll
-            for (int w = 0; w < W; ++w) acc = fma(v.v[w], v.v[w], acc);
+            for (int w = 0; w < W; ++w) acc[0] = fma(v.v[w], v.v[w], acc[0]);
         }
     });
-    double t, unused;
-    if (!grid_sum2(acc, 0.0, a, &t, &unused) || threadIdx.x != 0) return;
-    if (j < nc)
-        a.st->R[j][nc] = t;
-    else
-        a.st->vnorm2 = t;
-}
-
-// New diagonal entry of R, then the drops for the condition number.
-__global__ void k_aa_ctrl(AaState* st) {
-    st->nrot = 0;
-    st->ok = 0;
-    if (st->add) {
-        const int nc = st->newcol;
-        const double rn = sqrt(st->vnorm2);
-        if (rn > 0.0 && isfinite(rn)) {
-            st->R[nc][nc] = rn;
-            st->inv_rnn = 1.0 / rn;
-            st->nstore = nc + 1;
-            st->ok = 1;
-        } else {
-            for (int j = 0; j < nc; ++j) st->R[j][nc] = 0.0;
-        }
-    }
-    if (st->adjust)
-        while (st->nstore > 1 && rcond(st) < st->droptol) qr_delete(st);
+    __shared__ double sums[1];
+    if (grid_sums<1>(acc, 1, a, sums)) end_pass(a, j, true, nc, sums, nullptr);
 }
 
 // q_new = v / |v|, the post-add rotations, <F, q_j>; the last block solves
@@ -404,12 +462,10 @@ __global__ void k_aa_ctrl(AaState* st) {
 // per-thread accumulators (registers, hence occupancy).
 template <int MD>
 __global__ void __launch_bounds__(kThreads) k_aa_rhs(Args a) {
-    __shared__ double sh[kThreads / 32];
-    __shared__ bool last;
-    __shared__ double rhs[kMaxDepth];
+    __shared__ double rhs[MD];
     AaState* st = a.st;
     const int N = st->nstore, ok = st->ok, nc = st->newcol, nrot = st->nrot;
-    const double inv = st->inv_rnn;
+    const double inv = st->inv_rnn, beta = st->beta;
     double acc[MD];
 #pragma unroll
     for (int j = 0; j < MD; ++j) acc[j] = 0.0;
@@ -433,38 +489,23 @@ __global__ void __launch_bounds__(kThreads) k_aa_rhs(Args a) {
                 for (int w = 0; w < W; ++w) acc[j] = fma(F.v[w], q.v[w], acc[j]);
             }
     });
-#pragma unroll
-    for (int j = 0; j < MD; ++j) {
-        if (j < N) {  // N is the same in every thread of the block
-            const double t = block_sum(acc[j], sh);
-            if (threadIdx.x == 0) a.part[size_t(blockIdx.x) * kMaxDepth + j] = t;
-        }
-    }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
-    }
+    if (!grid_sums<MD>(acc, N, a, rhs)) return;
+    __shared__ double R[MD][MD];
+    for (int k = threadIdx.x; k < N * N; k += blockDim.x)
+        R[k / N][k % N] = __ldcg(&st->R[k / N][k % N]);
     __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int j = 0; j < N; ++j) {
-        double u = 0.0;
-        for (int k = threadIdx.x; k < int(gridDim.x); k += blockDim.x)
-            u += a.part[size_t(k) * kMaxDepth + j];
-        const double t = block_sum(u, sh);
-        if (threadIdx.x == 0) rhs[j] = t;
-    }
     if (threadIdx.x != 0) return;
-    *a.ticket = 0u;
+    // R gamma = Q^T F from the last row up; rhs becomes gamma.
     for (int j = N - 1; j >= 0; --j) {
         double g = rhs[j];
-        for (int i = j + 1; i < N; ++i) g = __dadd_rn(g, -__dmul_rn(st->R[j][i], st->gamma[i]));
-        st->gamma[j] = g / st->R[j][j];
+        for (int i = j + 1; i < N; ++i) g = __dadd_rn(g, -__dmul_rn(R[j][i], rhs[i]));
+        rhs[j] = g / R[j][j];
     }
     for (int i = 0; i < N; ++i) {
         double s = 0.0;
-        for (int j = i; j < N; ++j) s = __dadd_rn(s, __dmul_rn(st->R[i][j], st->gamma[j]));
-        st->rgamma[i] = __dmul_rn(st->beta, s);
+        for (int j = i; j < N; ++j) s = __dadd_rn(s, __dmul_rn(R[i][j], rhs[j]));
+        st->gamma[i] = rhs[i];
+        st->rgamma[i] = __dmul_rn(beta, s);
     }
     st->nrot = 0;
 }
@@ -509,8 +550,34 @@ __global__ void __launch_bounds__(kThreads) k_aa_update(Args a) {
     });
 }
 
-// |rp|_2 and the status tests (MCSAStatusTest, MaxIters, FiniteValue); the
-// last block also plans the next step.
+// The sum of squares acc of the residual and (last block) the status tests
+// (MCSAStatusTest, MaxIters, FiniteValue), the Monte Carlo bookkeeping and the
+// plan of the next step.
+__device__ __forceinline__ void check_step(const Args& a, double acc) {
+    __shared__ double sums[1];
+    const double v[1] = {acc};
+    if (!grid_sums<1>(v, 1, a, sums)) return;
+    __shared__ AaState sh;
+    load_state(&sh, a.st);
+    if (threadIdx.x == 32 && a.d_nh) {
+        *a.d_epoch += 1ULL;
+        *a.d_hist += (unsigned long long)*a.d_nh;
+        add_walk_time(a.d_tim);
+    }
+    if (threadIdx.x == 0) {
+        sh.k += 1;
+        sh.rnorm = sqrt(sums[0]);
+        if (a.hist && sh.k <= a.hist_cap) a.hist[sh.k - 1] = sh.rnorm;
+        sh.converged = sh.rnorm < sh.crit;
+        if (!isfinite(sh.rnorm) || !isfinite(sh.fnorm2)) atomicOr(a.status, DEV_ERR_NONFINITE);
+        const int keep = !sh.converged && sh.k < sh.max_iters && !*a.status;
+        sh.done = !keep;
+        plan(&sh);
+        if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
+    }
+    store_state(a.st, &sh);
+}
+
 __global__ void __launch_bounds__(kThreads) k_aa_check(Args a) {
     double acc = 0.0;
     const double* __restrict__ rp = a.rp;
@@ -520,18 +587,23 @@ __global__ void __launch_bounds__(kThreads) k_aa_check(Args a) {
 #pragma unroll
         for (int w = 0; w < W; ++w) acc = fma(r.v[w], r.v[w], acc);
     });
-    double total, unused;
-    if (!grid_sum2(acc, 0.0, a, &total, &unused) || threadIdx.x != 0) return;
-    AaState* st = a.st;
-    st->k += 1;
-    st->rnorm = sqrt(total);
-    if (a.hist && st->k <= a.hist_cap) a.hist[st->k - 1] = st->rnorm;
-    st->converged = st->rnorm < st->crit;
-    if (!isfinite(st->rnorm) || !isfinite(st->fnorm2)) atomicOr(a.status, DEV_ERR_NONFINITE);
-    const int keep = !st->converged && st->k < st->max_iters && !*a.status;
-    st->done = !keep;
-    plan(st);
-    if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
+    check_step(a, acc);
+}
+
+// The residual rp = PL (b - A x) (PL = I or point Jacobi) with its norm and the
+// tests: at 96^3 the separate norm pass took 11 us.
+template <class Op>
+__global__ void __launch_bounds__(kThreads, 8) k_aa_residual_check(Op A, Args a) {
+    double acc = 0.0;
+    const double* x = a.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+        const double s = A.dot(i, [&](int j) { return x[j]; });
+        const double res = a.b[i] - s;
+        const double r = a.dinv ? a.dinv[i] * res : res;
+        a.r[i] = r;
+        acc = fma(r, r, acc);
+    }
+    check_step(a, acc);
 }
 
 __global__ void k_axpy1(double* x, const double* r, int n) {
@@ -642,7 +714,7 @@ int ensure_work(mclsgpu_domain* dom, int m) {
 // f = x, "Smoother Steps" steps f += r, r = PL (b - A f), then this set's
 // Monte Carlo correction of the residual problem into delta.  Returns f.
 const double* enqueue_eval(mclsgpu_domain* dom, const mclsgpu_anderson_params* p,
-                           double* delta) {
+                           double* delta, bool fused) {
     cudaStream_t s = dom->ctx->stream;
     AndersonWork* w = dom->aa;
     const int n = dom->n;
@@ -663,7 +735,7 @@ const double* enqueue_eval(mclsgpu_domain* dom, const mclsgpu_anderson_params* p
         f = dom->x2;
         r = dom->rp2;
     }
-    mc_correction(dom, r, delta);
+    mc_correction(dom, r, delta, fused);
     return f;
 }
 
@@ -671,7 +743,7 @@ const double* enqueue_eval(mclsgpu_domain* dom, const mclsgpu_anderson_params* p
 // and the status test.
 void enqueue_accel(mclsgpu_domain* dom, const mclsgpu_anderson_params* p, const double* f,
                    const double* delta, double dscale, cudaGraphConditionalHandle h,
-                   int use_cond) {
+                   int use_cond, bool fused) {
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
     AndersonWork* w = dom->aa;
@@ -695,12 +767,20 @@ void enqueue_accel(mclsgpu_domain* dom, const mclsgpu_anderson_params* p, const 
     a.hist = dom->d_resid;
     a.hist_cap = dom->resid_cap;
     a.status = ctx->d_status;
+    a.depth = p->storage_depth;
+    a.b = dom->b;
+    a.r = dom->rp;
+    if (fused) {
+        a.d_nh = dom->d_nh;
+        a.d_epoch = dom->d_epoch;
+        a.d_hist = dom->d_hist;
+        a.d_tim = dom->d_tim;
+    }
     a.handle = h;
     a.use_cond = use_cond;
     k_aa_first<<<w->grid, kThreads, 0, s>>>(a);
     if (p->storage_depth > 0) {
         for (int j = 1; j < p->storage_depth; ++j) k_aa_mgs<<<w->grid, kThreads, 0, s>>>(a, j);
-        k_aa_ctrl<<<1, 1, 0, s>>>(w->st);
         if (p->storage_depth <= 4)
             k_aa_rhs<4><<<w->grid, kThreads, 0, s>>>(a);
         else if (p->storage_depth <= 8)
@@ -709,15 +789,23 @@ void enqueue_accel(mclsgpu_domain* dom, const mclsgpu_anderson_params* p, const 
             k_aa_rhs<kMaxDepth><<<w->grid, kThreads, 0, s>>>(a);
     }
     k_aa_update<<<w->grid, kThreads, 0, s>>>(a);
-    prec_residual(dom, dom->x, dom->b, dom->rp);
-    k_aa_check<<<w->grid, kThreads, 0, s>>>(a);
+    const mclsgpu_precond* L = dom->left;
+    if (!L || L->kind == MCLSGPU_PREC_POINT_JACOBI) {
+        if (L) a.dinv = L->diag;
+        MCLSGPU_LAUNCH_OP(dom->op, w->grid, kThreads, s, k_aa_residual_check, a);
+    } else {
+        prec_residual(dom, dom->x, dom->b, dom->rp);
+        k_aa_check<<<w->grid, kThreads, 0, s>>>(a);
+    }
 }
 
 // One Anderson step and its status test (captured into the graph body).
 void enqueue_step(mclsgpu_domain* dom, const mclsgpu_anderson_params* p,
                   cudaGraphConditionalHandle h, int use_cond) {
-    const double* f = enqueue_eval(dom, p, dom->aa->delta);
-    enqueue_accel(dom, p, f, dom->aa->delta, 1.0, h, use_cond);
+    // Forward fixed-length walks need nothing else counted or reset per step.
+    const bool fused = walk_finishes(dom);
+    const double* f = enqueue_eval(dom, p, dom->aa->delta, fused);
+    enqueue_accel(dom, p, f, dom->aa->delta, 1.0, h, use_cond, fused);
 }
 
 // Work space and residual history buffer for a solve with these parameters.
@@ -757,6 +845,7 @@ void anderson_begin(mclsgpu_domain* dom, const double* b_dev, const double* x_de
         cudaMemcpyAsync(dom->x, x_dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     // |b|_2 (MCSAStatusTest uses the unpreconditioned right-hand side) and
     // the residual of the initial guess, tested before the first step.
+    if (walk_finishes(dom)) launch_forward_setup(dom);
     sum_sq(s, dom->b, n, dom->part, dom->d_scalars + 6);
     prec_residual(dom, dom->x, dom->b, dom->rp);
     sum_sq(s, dom->rp, n, dom->part, dom->d_scalars + 5);
@@ -885,7 +974,7 @@ int mclsgpu_anderson_correction(mclsgpu_domain* dom, double* delta_dev) {
     if (!dom->aa_step_ready)
         return set_error(dom->ctx, MCLSGPU_ERR_INVALID_ARG, "mclsgpu_anderson_begin first");
     AndersonWork* w = dom->aa;
-    w->step_f = enqueue_eval(dom, &w->step_p, delta_dev);
+    w->step_f = enqueue_eval(dom, &w->step_p, delta_dev, false);
     cudaError_t e = cudaStreamSynchronize(dom->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "anderson correction");
     return check_device_status(dom->ctx);
@@ -899,7 +988,8 @@ int mclsgpu_anderson_apply(mclsgpu_domain* dom, const double* delta_dev, double 
                          "mclsgpu_anderson_correction first");
     AndersonWork* w = dom->aa;
     cudaStream_t s = dom->ctx->stream;
-    enqueue_accel(dom, &w->step_p, w->step_f, delta_dev, scale, cudaGraphConditionalHandle(0), 0);
+    enqueue_accel(dom, &w->step_p, w->step_f, delta_dev, scale, cudaGraphConditionalHandle(0), 0,
+                  false);
     w->step_f = nullptr;
     cudaMemcpyAsync(w->h_st, w->st, sizeof(AaState), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);

@@ -380,6 +380,19 @@ struct BatchList {
     const int* lcount;
     const int* srow0;   // system -> its first row
 };
+#if defined(__CUDACC__)
+// The duration of the last FP32 walk launch (first block start to last block
+// end) into t[2], the launch count in t[3].
+__device__ __forceinline__ void add_walk_time(unsigned long long* t) {
+    if (t[1] > t[0]) {
+        t[2] += t[1] - t[0];
+        t[3] += 1;
+    }
+    t[0] = ~0ULL;
+    t[1] = 0;
+}
+#endif
+
 // The iterate after a batched iteration's correction of the smoothed iterate.
 struct BatchFinish {
     double* X;
@@ -419,7 +432,10 @@ void richardson_residual(mclsgpu_domain* dom, const double* x, const double* r, 
                          double* x2, double* r2);
 // out = the Monte Carlo estimate for the source v (already left
 // preconditioned): one MC solve, advancing the domain's random stream.
-void mc_correction(mclsgpu_domain* dom, const double* v, double* out);
+// `fused`: forward histories were counted once (launch_forward_setup) and the
+// caller's last pass does the bookkeeping of k_mc_end.
+void mc_correction(mclsgpu_domain* dom, const double* v, double* out, bool fused = false);
+void launch_forward_setup(mclsgpu_domain* dom);
 // True when the domain walks variable-length histories on the reference
 // stream: those walks synchronise with the host (rounds), so the MCSA and
 // Anderson loops run from the host instead of a captured graph.

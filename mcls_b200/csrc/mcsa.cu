@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "ops.cuh"
 #include "rng.cuh"
 
 namespace mclsgpu {
@@ -37,7 +38,6 @@ namespace mclsgpu {
 void launch_adjoint_source(mclsgpu_domain* dom, const double* v, double omega, int has_omega);
 void launch_forward_source(mclsgpu_domain* dom, const double* v, double omega, int has_omega,
                            bool fused);
-void launch_forward_setup(mclsgpu_domain* dom);
 void launch_advance_walk_pos(mclsgpu_domain* dom);
 void prepare_walk(mclsgpu_domain* dom);
 void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
@@ -50,78 +50,6 @@ inline int grid_for(long long work, int threads = 256, int cap = 148 * 16) {
     if (g < 1) g = 1;
     return int(g > cap ? cap : g);
 }
-
-// Row dot products A(r,:) . f(col) over the two operator layouts.  Both visit
-// a row's entries in ascending column order with FMA accumulation, and their
-// padding entries contribute a product with 0 (which adds exactly nothing),
-// so both return the CSR sum bit for bit.
-struct SellView {  // SELL-32
-    const int* off;
-    const int* col;
-    const double* val;
-    int n;
-    template <class F>
-    __device__ __forceinline__ double dot(int r, F f) const {
-        const int a = off[r >> 5];
-        const int o = a + (r & 31), w = (off[(r >> 5) + 1] - a) >> 5;
-        double s = 0.0;
-        for (int k = 0; k < w; ++k) s = fma(val[o + 32 * k], f(col[o + 32 * k]), s);
-        return s;
-    }
-};
-
-// Stencil operator stored by diagonal offset (no indices).  KK > 0 fixes the
-// number of offsets at compile time so the row loop unrolls and every load of
-// the row is issued before the first product.
-template <int KK>
-struct DiaViewT {
-    const double* val;
-    int n;
-    int k;
-    int off[16];
-    template <class F>
-    __device__ __forceinline__ double dot(int r, F f) const {
-        constexpr int kmax = KK > 0 ? KK : 16;
-        const int kk = KK > 0 ? KK : k;
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < kmax; ++j) {
-            if (j >= kk) break;
-            const int c = r + off[j];
-            if (unsigned(c) < unsigned(n)) s = fma(val[size_t(j) * n + r], f(c), s);
-        }
-        return s;
-    }
-};
-using DiaView = DiaViewT<0>;
-
-// Symmetric stencil operator (A(r, r - o) == A(r - o, r)): only the diagonal
-// and the H positive-offset diagonals are read; A(r, r - o_h) is taken as
-// A(r - o_h, r).  The products are the same as DiaViewT's, in the same
-// (ascending column) order, so the sums are bit for bit the same with
-// (1 + H) / (1 + 2H) of the matrix bytes.
-template <int H>
-struct DiaSymView {
-    const double* val;  // [(1 + H) * n]: diagonal, then positive offsets ascending
-    int n;
-    int off[H];
-    template <class F>
-    __device__ __forceinline__ double dot(int r, F f) const {
-        double s = 0.0;
-#pragma unroll
-        for (int h = H - 1; h >= 0; --h) {
-            const int c = r - off[h];
-            if (c >= 0) s = fma(val[size_t(1 + h) * n + c], f(c), s);
-        }
-        s = fma(val[r], f(r), s);
-#pragma unroll
-        for (int h = 0; h < H; ++h) {
-            const int c = r + off[h];
-            if (c < n) s = fma(val[size_t(1 + h) * n + r], f(c), s);
-        }
-        return s;
-    }
-};
 
 // rp = (b - A x) [* dinv]   (LinearProblem::updatePrecResidual, :410-442)
 template <class Op>
@@ -199,17 +127,6 @@ __global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
             d = __dadd_rn(a.xin[i], d);
         a.out[i] = d;
     }
-}
-
-// The duration of the last FP32 walk launch (first block start to last block
-// end) into t[2], the launch count in t[3].
-__device__ __forceinline__ void add_walk_time(unsigned long long* t) {
-    if (t[1] > t[0]) {
-        t[2] += t[1] - t[0];
-        t[3] += 1;
-    }
-    t[0] = ~0ULL;
-    t[1] = 0;
 }
 
 // The words a solve's counters and report live in.
@@ -564,97 +481,6 @@ __global__ void __launch_bounds__(kFusedThreads, 8) k_mcsa_begin(Op A, BeginArgs
 }  // namespace
 
 // ---------------------------------------------------------------------------
-static SellView sell_view(const mclsgpu_operator* op) {
-    return SellView{op->S.off, op->S.col, op->S.val, op->S.n};
-}
-
-template <int H>
-static DiaSymView<H> sym_view(const mclsgpu_operator* op) {
-    DiaSymView<H> v{};
-    v.val = op->sym_val;
-    v.n = op->A.n;
-    for (int h = 0; h < H; ++h) v.off[h] = op->sym_off[h];
-    return v;
-}
-
-template <int KK>
-static DiaViewT<KK> dia_view(const mclsgpu_operator* op) {
-    DiaViewT<KK> v{};
-    v.val = op->dia_val;
-    v.n = op->A.n;
-    v.k = op->dia_k;
-    for (int j = 0; j < 16; ++j) v.off[j] = op->dia_off[j];
-    return v;
-}
-
-// The diagonal-offset view of another matrix on the operator's offsets.
-template <int KK>
-static DiaViewT<KK> dia_view_vals(const mclsgpu_operator* op, const double* vals) {
-    DiaViewT<KK> v = dia_view<KK>(op);
-    v.val = vals;
-    return v;
-}
-
-#define MCLSGPU_LAUNCH_M(op, vals, grid, threads, stream, kern, ...)                         \
-    do {                                                                                     \
-        switch ((op)->dia_k) {                                                               \
-            case 5:                                                                          \
-                kern<DiaViewT<5>><<<grid, threads, 0, stream>>>(dia_view_vals<5>(op, vals),  \
-                                                                __VA_ARGS__);                \
-                break;                                                                       \
-            case 7:                                                                          \
-                kern<DiaViewT<7>><<<grid, threads, 0, stream>>>(dia_view_vals<7>(op, vals),  \
-                                                                __VA_ARGS__);                \
-                break;                                                                       \
-            case 9:                                                                          \
-                kern<DiaViewT<9>><<<grid, threads, 0, stream>>>(dia_view_vals<9>(op, vals),  \
-                                                                __VA_ARGS__);                \
-                break;                                                                       \
-            default:                                                                         \
-                kern<DiaView><<<grid, threads, 0, stream>>>(dia_view_vals<0>(op, vals),      \
-                                                            __VA_ARGS__);                    \
-        }                                                                                    \
-    } while (0)
-
-// Launch `kern<Op>` on the operator's fastest layout: diagonal-offset values
-// for stencil operators (unrolled for the 5-, 7- and 9-point stencils; only
-// the diagonal and upper diagonals when the values are symmetric), SELL-32
-// otherwise.
-#define MCLSGPU_LAUNCH_OP(op, grid, threads, stream, kern, ...)                              \
-    do {                                                                                     \
-        switch ((op)->dia_k) {                                                               \
-            case 0:                                                                          \
-                kern<SellView><<<grid, threads, 0, stream>>>(sell_view(op), __VA_ARGS__);    \
-                break;                                                                       \
-            case 5:                                                                          \
-                if ((op)->sym_h == 2)                                                        \
-                    kern<DiaSymView<2>><<<grid, threads, 0, stream>>>(sym_view<2>(op),        \
-                                                                      __VA_ARGS__);          \
-                else                                                                         \
-                    kern<DiaViewT<5>><<<grid, threads, 0, stream>>>(dia_view<5>(op),          \
-                                                                    __VA_ARGS__);            \
-                break;                                                                       \
-            case 7:                                                                          \
-                if ((op)->sym_h == 3)                                                        \
-                    kern<DiaSymView<3>><<<grid, threads, 0, stream>>>(sym_view<3>(op),        \
-                                                                      __VA_ARGS__);          \
-                else                                                                         \
-                    kern<DiaViewT<7>><<<grid, threads, 0, stream>>>(dia_view<7>(op),          \
-                                                                    __VA_ARGS__);            \
-                break;                                                                       \
-            case 9:                                                                          \
-                if ((op)->sym_h == 4)                                                        \
-                    kern<DiaSymView<4>><<<grid, threads, 0, stream>>>(sym_view<4>(op),        \
-                                                                      __VA_ARGS__);          \
-                else                                                                         \
-                    kern<DiaViewT<9>><<<grid, threads, 0, stream>>>(dia_view<9>(op),          \
-                                                                    __VA_ARGS__);            \
-                break;                                                                       \
-            default:                                                                         \
-                kern<DiaView><<<grid, threads, 0, stream>>>(dia_view<0>(op), __VA_ARGS__);   \
-        }                                                                                    \
-    } while (0)
-
 // rp = PL (b - A PR x)
 static void update_prec_residual(mclsgpu_domain* dom, const double* x, const double* b,
                                  double* rp_out) {
@@ -832,8 +658,8 @@ __global__ void k_axpy_to(const double* x, const double* r, double w, double* x2
         x2[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
 }
 
-void mc_correction(mclsgpu_domain* dom, const double* v, double* out) {
-    enqueue_mc(dom, v, out, kBaseNone, 0, nullptr, nullptr, nullptr, nullptr);
+void mc_correction(mclsgpu_domain* dom, const double* v, double* out, bool fused) {
+    enqueue_mc(dom, v, out, kBaseNone, 0, nullptr, nullptr, nullptr, nullptr, fused);
 }
 
 // The fused iteration covers one smoothing step, no right preconditioner and
