@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kThreads) k_aa_check(Args a) {
 // The residual rp = PL (b - A x) (PL = I or point Jacobi) with its norm and the
 // tests: at 96^3 the separate norm pass took 11 us.
 template <class Op>
-__global__ void __launch_bounds__(kThreads, 8) k_aa_residual_check(Op A, Args a) {
+__global__ void __launch_bounds__(kThreads, Op::kMinBlocks) k_aa_residual_check(Op A, Args a) {
     double acc = 0.0;
     const double* x = a.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {

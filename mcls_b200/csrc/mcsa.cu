@@ -336,11 +336,11 @@ __device__ __forceinline__ void residual_norm(const Op& A, const ResidArgs& a) {
     norm_and_check(a, acc);
 }
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads, 8) k_residual_norm(Op A, ResidArgs a) {
+__global__ void __launch_bounds__(kFusedThreads, Op::kMinBlocks) k_residual_norm(Op A, ResidArgs a) {
     residual_norm<false>(A, a);
 }
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads, 8) k_finalize_norm(Op A, ResidArgs a) {
+__global__ void __launch_bounds__(kFusedThreads, Op::kMinBlocks) k_finalize_norm(Op A, ResidArgs a) {
     residual_norm<true>(A, a);
 }
 
@@ -426,7 +426,7 @@ __device__ __forceinline__ double fused_block_sum(double v, double* sh) {
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kFusedThreads, 8) k_mcsa_begin(Op A, BeginArgs a) {
+__global__ void __launch_bounds__(kFusedThreads, Op::kMinBlocks) k_mcsa_begin(Op A, BeginArgs a) {
     __shared__ double sh[kFusedThreads / 32];
     __shared__ bool last;
     double sb = 0.0, sr = 0.0;
