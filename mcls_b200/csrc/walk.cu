@@ -238,12 +238,24 @@ constexpr int first_slots() {
     return ST == kPacked && S > 8 ? 8 : S;
 }
 
-template <int S, bool L1>
+// Where a step finds the records: global memory past L1 or allocating in it, or
+// the block's copy in shared memory.
+enum : int { kBypass = 0, kCached = 1, kShared = 2 };
+
+template <int S, int MEM>
 __device__ __forceinline__ void load_slots(const char* r, uint32_t* q) {
 #pragma unroll
     for (int t = 0; t < S / 4; ++t) {
-        if constexpr (L1) ld_record256_l1(r + 32 * t, q + 8 * t);
-        else ld_record256(r + 32 * t, q + 8 * t);
+        if constexpr (MEM == kShared) {
+            const uint4 u = *reinterpret_cast<const uint4*>(r + 32 * t);
+            const uint4 v = *reinterpret_cast<const uint4*>(r + 32 * t + 16);
+            q[8 * t] = u.x, q[8 * t + 1] = u.y, q[8 * t + 2] = u.z, q[8 * t + 3] = u.w;
+            q[8 * t + 4] = v.x, q[8 * t + 5] = v.y, q[8 * t + 6] = v.z, q[8 * t + 7] = v.w;
+        } else if constexpr (MEM == kCached) {
+            ld_record256_l1(r + 32 * t, q + 8 * t);
+        } else {
+            ld_record256(r + 32 * t, q + 8 * t);
+        }
     }
 }
 
@@ -252,8 +264,7 @@ __device__ __forceinline__ void load_slots(const char* r, uint32_t* q) {
 // draw u, select the first entry whose CDF value is >= u, update the state
 // and the weight.
 //
-// L1: the record loads allocate in L1 or bypass it.
-template <int S, int DIR, int ST, bool L1, bool POS = false>
+template <int S, int DIR, int ST, int MEM, bool POS = false>
 __device__ __forceinline__ void walk_step(const char* rec, double* y, const int* soff, int& s,
                                           float& w, uint64_t& x, float& acc, float& comp, int k) {
     // One record: S/4 256-bit loads.  rec and y point at global row 0.  Long
@@ -262,7 +273,7 @@ __device__ __forceinline__ void walk_step(const char* rec, double* y, const int*
     constexpr int kFirst = first_slots<S, ST>();
     const char* r = rec + size_t(unsigned(s)) * (S * 8);
     uint32_t q[2 * kFirst];
-    load_slots<kFirst, L1>(r, q);
+    load_slots<kFirst, MEM>(r, q);
     if (DIR == MCLSGPU_ADJOINT) {
         // FP32 weight, FP64 reduction (fire-and-forget RED.ADD.F64).
         if (k > 0) atomicAdd(&y[s], double(w));
@@ -284,7 +295,7 @@ __device__ __forceinline__ void walk_step(const char* rec, double* y, const int*
             sel = select_packed<1, kFirst>(q, u);
         } else {
             uint32_t z[2 * (S - kFirst)];
-            load_slots<S - kFirst, L1>(r + kFirst * 8, z);
+            load_slots<S - kFirst, MEM>(r + kFirst * 8, z);
             sel = select_packed<0, S - kFirst>(z, u);
         }
         neg = sel & 0x80000000u;
@@ -325,6 +336,47 @@ __device__ __forceinline__ void walk_end_time(const WalkArgs& a) {
     if (threadIdx.x == 0) atomicMax(&a.d_tim[1], global_ns());
 }
 
+// All of a small domain's records in the block's shared memory, fetched with
+// bulk copies.
+struct RecordCopy {
+    const char* rec;
+    uint32_t bar;  // mbarrier (shared-memory address)
+
+    // One thread: start the copies (dst: 16-byte aligned shared memory).
+    __device__ __forceinline__ void start(const void* src, int bytes) const {
+        const uint32_t dst = uint32_t(__cvta_generic_to_shared(rec));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"(bytes)
+                     : "memory");
+        constexpr int kChunk = 16 * 1024;
+        for (int at = 0; at < bytes; at += kChunk)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+                "[%3];" ::"r"(dst + at),
+                "l"(reinterpret_cast<const char*>(src) + at), "r"(min(kChunk, bytes - at)), "r"(bar)
+                : "memory");
+    }
+    // True once the records are there; false (and reported) when the wait
+    // expires.
+    __device__ __forceinline__ bool wait(int* status) const {
+        for (int spin = 0; spin < (1 << 22); ++spin) {
+            uint32_t done;
+            asm volatile(
+                "{\n.reg .pred p;\n"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
+                "selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(bar)
+                : "memory");
+            if (done) return true;
+        }
+        atomicOr(status, DEV_ERR_TIMEOUT);
+        return false;
+    }
+};
+
 // What bounds it: 8,850 warp steps per SM for 41.9M steps (128^3, two
 // histories per row), and the loads' L1TEX cycles -- a warp's 32 records lie in
 // up to 32 different lines, one request to L2 each.  So the lanes of a warp
@@ -346,21 +398,46 @@ __device__ __forceinline__ void walk_end_time(const WalkArgs& a) {
 // cleared tally and no pass of its own.  The histories are assigned
 // statically: they all take the same number of steps, and a work queue costs
 // one contended atomic per warp.
-template <int S, int ST, bool POS, bool L1>
+template <int S, int ST, bool POS, int MEM>
 __device__ __forceinline__ double row_histories(const WalkArgs& a, const RowFinish& f,
-                                                const int* soff, uint64_t ekey, int row) {
+                                                const int* soff, uint64_t ekey, int row,
+                                                const RecordCopy& copy) {
     const char* rec = reinterpret_cast<const char*>(a.rec);
     const int L = a.L, H = 1 << f.hlog;
     double sum = 0.0;
     for (int m = threadIdx.x & (H - 1); m < a.per; m += H) {
-        int s = row;
+        int s = row, k = 0;
         float w = 1.f, acc = 0.f, comp = 0.f;
         uint64_t x = history_state(a, ekey, (long long)row * a.per + m);
-        for (int k = 0; k < L; ++k)
-            walk_step<S, MCLSGPU_FORWARD, ST, L1, POS>(rec, nullptr, soff, s, w, x, acc, comp, k);
+        if constexpr (MEM == kShared) {
+            // The first record from memory, while the others are on their way.
+            walk_step<S, MCLSGPU_FORWARD, ST, kBypass, POS>(rec, nullptr, soff, s, w, x, acc, comp,
+                                                            k++);
+            if (!copy.wait(a.status)) return 0.0;
+        }
+        const char* from = MEM == kShared ? copy.rec : rec;
+        for (; k < L; ++k)
+            walk_step<S, MCLSGPU_FORWARD, ST, MEM, POS>(from, nullptr, soff, s, w, x, acc, comp, k);
         sum += double(acc) - double(comp);
     }
     return sum;
+}
+
+// The row's estimate from its histories' sums (one per lane of the row).
+__device__ __forceinline__ void finish_row(const WalkArgs& a, const RowFinish& f, double sum, int i,
+                                           bool live) {
+    for (int d = 1; d < (1 << f.hlog); d <<= 1) sum += __shfl_xor_sync(kFull, sum, d);
+    if (!live || (threadIdx.x & ((1 << f.hlog) - 1)) != 0) return;
+    // sum / count (ForwardTally::finalize, src/MCLS_ForwardTally_impl.hpp:
+    // 194-208); for a power-of-two count the product with its reciprocal
+    // is the same number.
+    double d = f.per_pow2 ? sum * f.inv_per : __ddiv_rn(sum, double(a.per));
+    if (f.ev) d = __dadd_rn(d, f.has_omega ? f.src[i] * f.omega : f.src[i]);
+    if (f.base == kBaseOut)
+        d = __dadd_rn(f.out[i], d);
+    else if (f.base == kBaseIn)
+        d = __dadd_rn(f.xin[i], d);
+    f.out[i] = d;
 }
 
 template <int S, int ST, bool POS>
@@ -379,21 +456,10 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks)
     const bool live = pos < unsigned(a.n);
     const unsigned p = live ? pos : unsigned(a.n) - 1u;
     const int i = f.order ? f.order[p] : int(p);
-    double sum = a.l1 ? row_histories<S, ST, POS, true>(a, f, s_off, s_ekey, i)
-                      : row_histories<S, ST, POS, false>(a, f, s_off, s_ekey, i);
-    for (int d = 1; d < (1 << f.hlog); d <<= 1) sum += __shfl_xor_sync(kFull, sum, d);
-    if (live && (threadIdx.x & ((1 << f.hlog) - 1)) == 0) {
-        // sum / count (ForwardTally::finalize, src/MCLS_ForwardTally_impl.hpp:
-        // 194-208); for a power-of-two count the product with its reciprocal
-        // is the same number.
-        double d = f.per_pow2 ? sum * f.inv_per : __ddiv_rn(sum, double(a.per));
-        if (f.ev) d = __dadd_rn(d, f.has_omega ? f.src[i] * f.omega : f.src[i]);
-        if (f.base == kBaseOut)
-            d = __dadd_rn(f.out[i], d);
-        else if (f.base == kBaseIn)
-            d = __dadd_rn(f.xin[i], d);
-        f.out[i] = d;
-    }
+    const RecordCopy none{};
+    const double sum = a.l1 ? row_histories<S, ST, POS, kCached>(a, f, s_off, s_ekey, i, none)
+                            : row_histories<S, ST, POS, kBypass>(a, f, s_off, s_ekey, i, none);
+    finish_row(a, f, sum, i, live);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(a.d_steps, (unsigned long long)(a.n) * a.per * a.L);
     walk_end_time(a);
@@ -401,10 +467,10 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks)
 
 // Adjoint histories of fixed length, ILP per lane, assigned statically (see
 // walk32_rows); they tally where they stand.
-template <int S, int ST, bool POS, bool L1, int ILP>
+template <int S, int ST, bool POS, int MEM, int ILP>
 __device__ __forceinline__ void adjoint_histories(const WalkArgs& a, const int* soff,
                                                   uint64_t ekey, float wnorm, long long e0,
-                                                  int nh) {
+                                                  int nh, const RecordCopy& copy) {
     const char* rec = reinterpret_cast<const char*>(a.rec);
     const int L = a.L;
     int s[ILP];
@@ -418,13 +484,22 @@ __device__ __forceinline__ void adjoint_histories(const WalkArgs& a, const int* 
         x[m] = 0;
         if (e < nh) walk_start<MCLSGPU_ADJOINT>(a, int(e), ekey, wnorm, s[m], w[m], x[m]);
     }
-    for (int k = 0; k < L; ++k) {
+    int k = 0;
+    if constexpr (MEM == kShared) {
+        static_assert(ILP == 1, "one history per lane");
+        float acc = 0.f, comp = 0.f;
+        walk_step<S, MCLSGPU_ADJOINT, ST, kBypass, POS>(rec, a.y64, soff, s[0], w[0], x[0], acc,
+                                                        comp, k++);
+        if (!copy.wait(a.status)) return;
+        rec = copy.rec;
+    }
+    for (; k < L; ++k) {
 #pragma unroll
         for (int m = 0; m < ILP; ++m) {
             float acc = 0.f, comp = 0.f;
             if (e0 + (long long)m * blockDim.x < nh)
-                walk_step<S, MCLSGPU_ADJOINT, ST, L1, POS>(rec, a.y64, soff, s[m], w[m], x[m],
-                                                           acc, comp, k);
+                walk_step<S, MCLSGPU_ADJOINT, ST, MEM, POS>(rec, a.y64, soff, s[m], w[m], x[m],
+                                                            acc, comp, k);
         }
     }
 }
@@ -448,14 +523,59 @@ __global__ void __launch_bounds__(256, ILP == 1 ? WalkOccupancy<S, ST>::kMinBloc
     __syncthreads();
     // The launch has a thread for every history the domain was sized for.
     const long long e0 = (long long)blockIdx.x * (blockDim.x * ILP) + threadIdx.x;
+    const RecordCopy none{};
     if (e0 < s_nh) {
         if (a.l1)
-            adjoint_histories<S, ST, POS, true, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh);
+            adjoint_histories<S, ST, POS, kCached, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh, none);
         else
-            adjoint_histories<S, ST, POS, false, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh);
+            adjoint_histories<S, ST, POS, kBypass, ILP>(a, s_off, s_ekey, s_wnorm, e0, s_nh, none);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(a.d_steps, (unsigned long long)s_nh * a.L);
+    walk_end_time(a);
+}
+
+// The fixed-length walks of a domain whose records fit a block's shared memory.
+// Their time is a chain of L dependent reads of a record, which the other warps
+// of so few histories cannot hide: every block copies the records once (190 KB
+// take about two microseconds, during which the first step is made) and the
+// other steps read shared memory.  77^2, two histories per row: 6.6 us, 8.9 us
+// from global memory.  Blocks are small, so that all SMs take part.
+constexpr int kSmallBlock = 128;
+constexpr int kSmallRecords = 200 * 1024;  // bytes
+
+template <int S, int ST, bool POS, int DIR>
+__global__ void __launch_bounds__(kSmallBlock) walk32_small(WalkArgs a, RowFinish f) {
+    extern __shared__ __align__(128) char s_rec[];
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ uint64_t s_ekey;
+    __shared__ int s_off[32];
+    RecordCopy copy{s_rec, uint32_t(__cvta_generic_to_shared(&s_bar))};
+    stage_offsets(a.stoff, s_off);
+    if (threadIdx.x == 0) {
+        copy.start(a.rec, a.n * (S * 8));
+        s_ekey = epoch_key(a.seed, *a.d_epoch);
+    }
+    walk_begin_time(a);
+    __syncthreads();
+    const unsigned at = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long histories;
+    if constexpr (DIR == MCLSGPU_FORWARD) {
+        const unsigned pos = at >> f.hlog;
+        const bool live = pos < unsigned(a.n);
+        const int i = int(live ? pos : unsigned(a.n) - 1u);
+        const double sum = row_histories<S, ST, POS, kShared>(a, f, s_off, s_ekey, i, copy);
+        finish_row(a, f, sum, i, live);
+        histories = (unsigned long long)a.n * a.per;
+    } else {
+        const int nh = *a.d_nh;
+        if (at < unsigned(nh))
+            adjoint_histories<S, ST, POS, kShared, 1>(a, s_off, s_ekey, float(a.sc[0]), at, nh,
+                                                      copy);
+        histories = (unsigned long long)nh;
+    }
+    if (at == 0) atomicAdd(a.d_steps, histories * a.L);
+    copy.wait(a.status);  // no block ends with its copies in flight
     walk_end_time(a);
 }
 
@@ -508,7 +628,7 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks) walk32_
         }
         if (!__any_sync(kFull, alive)) break;
         if (alive) {
-            walk_step<S, DIR, ST, false>(rec, a.y64, s_off, s, w, x, acc, comp, k);
+            walk_step<S, DIR, ST, kBypass>(rec, a.y64, s_off, s, w, x, acc, comp, k);
             ++k;
             ++steps;
             if (k >= a.L || fabsf(w) < wcut) {
@@ -636,10 +756,44 @@ void launch_adj(const WalkLaunch& l) {
     walk32_adjoint<S, ST, POS, ILP><<<int(grid), d->walk_block, 0, d->ctx->stream>>>(l.a);
 }
 
+template <int S, int ST, bool POS, int DIR>
+void launch_small(const WalkLaunch& l) {
+    const mclsgpu_domain* d = l.dom;
+    const int bytes = d->n * S * 8;
+    if (!l.launch) {
+        cudaFuncSetAttribute(walk32_small<S, ST, POS, DIR>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallRecords);
+        return;
+    }
+    const long long threads = DIR == MCLSGPU_FORWARD ? (long long)d->n << l.fin.hlog : d->nh_cap;
+    const long long grid = (threads + kSmallBlock - 1) / kSmallBlock;
+    walk32_small<S, ST, POS, DIR><<<int(grid < 1 ? 1 : grid), kSmallBlock, bytes,
+                                    d->ctx->stream>>>(l.a, l.fin);
+}
+
+// Records in shared memory: they must fit, and the blocks must run at once, one
+// per SM.  MCSA solves of 24^2 to 80^2 grids take 5 to 9 % less time than from
+// global memory, adjoint ones 4 to 6 %; nothing on this side of the line is
+// slower.
+template <int S>
+bool small_walk(const mclsgpu_domain* d) {
+    if (S > 16 || (long long)d->n * S * 8 > kSmallRecords) return false;
+    const long long threads = d->p.direction == MCLSGPU_FORWARD
+                                  ? (long long)d->n << d->walk_hlog
+                                  : (long long)d->nh_cap;
+    return threads <= (long long)d->ctx->num_sms * kSmallBlock;
+}
+
 template <int S, int ST, bool POS>
 void launch32_fixed(const WalkLaunch& l) {
-    if (!l.launch) return;
     const mclsgpu_domain* d = l.dom;
+    if constexpr (S <= 16)
+        if (small_walk<S>(d)) {
+            if (d->p.direction == MCLSGPU_ADJOINT)
+                return launch_small<S, ST, POS, MCLSGPU_ADJOINT>(l);
+            return launch_small<S, ST, POS, MCLSGPU_FORWARD>(l);
+        }
+    if (!l.launch) return;
     if (d->p.direction == MCLSGPU_ADJOINT) {
         // Several histories per lane: two on records of at most 64 bytes,
         // four on 32-byte records (the register budget).
@@ -829,7 +983,7 @@ __device__ __forceinline__ unsigned batch_history(const WalkArgs& a, const char*
             acc[r] = t;
         }
         float da = 0.f, dc = 0.f;  // the record header's own tally is unused here
-        walk_step<S, MCLSGPU_FORWARD, ST ? kStencil : kPacked, false>(rec, nullptr, soff, s, w, x, da, dc,
+        walk_step<S, MCLSGPU_FORWARD, ST ? kStencil : kPacked, kBypass>(rec, nullptr, soff, s, w, x, da, dc,
                                                                  k);
     }
     if (!m.Y) {
@@ -1230,7 +1384,7 @@ __global__ void __launch_bounds__(256) walk32_part(PartWalk p) {
             continue;
         }
         while (true) {
-            walk_step<S, DIR, ST, false>(rec, y, s_off, s, w, x, acc, comp, k);
+            walk_step<S, DIR, ST, kBypass>(rec, y, s_off, s, w, x, acc, comp, k);
             ++k;
             ++steps;
             if (k >= p.L || fabsf(w) < wcut) {
