@@ -29,6 +29,8 @@
 #include <cstring>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "internal.h"
 #include "ops.cuh"
 #include "rng.cuh"
@@ -251,12 +253,37 @@ struct ResidArgs {
     int use_cond;
 };
 
-// rp = PL (b - A x), |rp|^2, then (last block) the MCSA convergence check,
-// the stream epoch, the walk timing, the work-queue reset and the loop
-// condition.
-// Block sum of the threads' acc, then (last block to finish) the MCSA
-// convergence check, the stream epoch, the walk timing, the work-queue reset
-// and the loop condition.
+// The words that the end of an iteration reads and updates (one thread), loaded
+// together: one after the other they cost 2 us of a small system's iteration.
+struct IterationWords {
+    McsaState st;
+    int status, nh;
+    unsigned long long epoch, histories, tim[4];
+    __device__ __forceinline__ void load(const ResidArgs& a) {
+        st = *a.st;
+        status = *a.status;
+        nh = *a.d_nh;
+        epoch = *a.d_epoch;
+        histories = *a.d_hist;
+        for (int k = 0; k < 4; ++k) tim[k] = a.d_tim[k];
+    }
+};
+
+// The MCSA convergence check, the stream epoch, the walk timing, the work-queue
+// reset and the loop condition (one thread).
+__device__ __forceinline__ void end_iteration(const ResidArgs& a, IterationWords& w,
+                                              double sumsq) {
+    const int keep = mcsa_check(w.st, w.status, a.st, sumsq, a.hist, a.hist_cap, a.status);
+    *a.d_epoch = w.epoch + 1ULL;
+    *a.d_hist = w.histories + (unsigned long long)w.nh;
+    add_walk_time(w.tim);
+    for (int k = 0; k < 4; ++k) a.d_tim[k] = w.tim[k];
+    *a.d_counter = 0;
+    if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
+}
+
+// Block sum of the threads' acc, then (last block to finish) the end of the
+// iteration.
 __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     __shared__ double warp_sum[kFusedThreads / 32];
     __shared__ bool last;
@@ -273,19 +300,8 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // The bookkeeping's words are loaded together, before the sum they wait
-    // for: one after the other they cost 2 us of a small system's iteration.
-    McsaState st;
-    int status = 0, nh = 0;
-    unsigned long long epoch = 0, histories = 0, tim[4] = {0, 0, 0, 0};
-    if (threadIdx.x == 0) {
-        st = *a.st;
-        status = *a.status;
-        nh = *a.d_nh;
-        epoch = *a.d_epoch;
-        histories = *a.d_hist;
-        for (int k = 0; k < 4; ++k) tim[k] = a.d_tim[k];
-    }
+    IterationWords words;
+    if (threadIdx.x == 0) words.load(a);
     double t = 0.0;
     for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) t += a.part[i];
     for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
@@ -295,16 +311,34 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     if (threadIdx.x == 0) {
         double sumsq = 0.0;
         for (int w = 0; w < kFusedThreads / 32; ++w) sumsq += warp_sum[w];
-        const int keep =
-            mcsa_check(st, status, a.st, sumsq, a.hist, a.hist_cap, a.status);
+        end_iteration(a, words, sumsq);
         *a.ticket = 0u;
-        *a.d_epoch = epoch + 1ULL;
-        *a.d_hist = histories + (unsigned long long)nh;
-        add_walk_time(tim);
-        for (int k = 0; k < 4; ++k) a.d_tim[k] = tim[k];
-        *a.d_counter = 0;
-        if (a.use_cond) cudaGraphSetConditional(a.handle, keep ? 1u : 0u);
     }
+}
+
+// The same for a system whose rows one cluster takes: the blocks' sums meet in
+// the first block's shared memory, and its first thread has loaded the words
+// before the rows.
+constexpr int kClusterCtas = 8, kClusterThreads = 1024;
+__device__ __forceinline__ void norm_and_check_cluster(const ResidArgs& a, IterationWords& words,
+                                                       double acc) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ double warp_sum[kClusterThreads / 32];
+    __shared__ double block_sum[kClusterCtas];
+    for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, d);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double t = warp_sum[threadIdx.x];
+        for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
+        if (threadIdx.x == 0) *cluster.map_shared_rank(&block_sum[blockIdx.x], 0) = t;
+    }
+    cluster.sync();
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    double sumsq = 0.0;
+    for (int r = 0; r < kClusterCtas; ++r) sumsq += block_sum[r];
+    end_iteration(a, words, sumsq);
 }
 
 // (256, 8): eight blocks an SM, the grid's size, must be resident; with the 46
@@ -316,7 +350,7 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
 // that did it (5 us at 64^3, 3 us at 10^4 states); the next smoothed iterate is
 // then left to the next smoothing pass, since x2 is read at the neighbours.
 template <bool FOLD, class Op>
-__device__ __forceinline__ void residual_norm(const Op& A, const ResidArgs& a) {
+__device__ __forceinline__ double residual_rows(const Op& A, const ResidArgs& a) {
     const double inv = FOLD ? *a.inv_nh : 0.0;
     auto x = [&](int j) {
         // AdjointTally::normalize: x *= 1/nh  (src/MCLS_AdjointTally_impl.hpp:68-72)
@@ -333,15 +367,37 @@ __device__ __forceinline__ void residual_norm(const Op& A, const ResidArgs& a) {
         else a.x2[i] = __dadd_rn(x(i), __dmul_rn(a.w, r));
         acc = fma(r, r, acc);
     }
-    norm_and_check(a, acc);
+    return acc;
 }
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads, Op::kMinBlocks) k_residual_norm(Op A, ResidArgs a) {
-    residual_norm<false>(A, a);
+    norm_and_check(a, residual_rows<false>(A, a));
 }
 template <class Op>
 __global__ void __launch_bounds__(kFusedThreads, Op::kMinBlocks) k_finalize_norm(Op A, ResidArgs a) {
-    residual_norm<true>(A, a);
+    norm_and_check(a, residual_rows<true>(A, a));
+}
+
+// Small stencil systems: one cluster of eight 1024-thread CTAs.  The ticket, the
+// partial sums and the words are three trips to L2 after the rows; without them
+// an iteration takes 16.3 instead of 17.7 us at 77^2, 18.2 instead of 20 us at
+// 90^2, 15.9 instead of 16.6 us at 18^3.  At 25^3 (two rows per thread) both
+// take the same, and unstructured rows, whose gathers want more SMs, take
+// longer at any size (21.3 to 22.7 us at 1500 rows).
+constexpr int kClusterRows = 3 * kClusterCtas * kClusterThreads / 2;
+template <class Op>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
+    k_residual_norm_cluster(Op A, ResidArgs a) {
+    IterationWords words;
+    if (blockIdx.x == 0 && threadIdx.x == 0) words.load(a);
+    norm_and_check_cluster(a, words, residual_rows<false>(A, a));
+}
+template <class Op>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
+    k_finalize_norm_cluster(Op A, ResidArgs a) {
+    IterationWords words;
+    if (blockIdx.x == 0 && threadIdx.x == 0) words.load(a);
+    norm_and_check_cluster(a, words, residual_rows<true>(A, a));
 }
 
 // A left preconditioner M stored on A's diagonals (learned SPAI): out = M v.
@@ -772,6 +828,11 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x, dom->b, nullptr,
                           dom->tmp);
         MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_precond_norm, a, dom->tmp);
+    } else if (op->dia_k > 0 && n <= kClusterRows) {
+        if (fold)
+            MCLSGPU_LAUNCH_OP(op, kClusterCtas, kClusterThreads, s, k_finalize_norm_cluster, a);
+        else
+            MCLSGPU_LAUNCH_OP(op, kClusterCtas, kClusterThreads, s, k_residual_norm_cluster, a);
     } else if (fold) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_finalize_norm, a);
     } else {
