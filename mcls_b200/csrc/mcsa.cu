@@ -23,9 +23,11 @@
 // CUDA graph: a WHILE conditional node whose body is one iteration and whose
 // condition is set on the device by the convergence check, so a solve makes
 // no host round trip per iteration.
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -285,14 +287,15 @@ __device__ __forceinline__ void end_iteration(const ResidArgs& a, IterationWords
 // Block sum of the threads' acc, then (last block to finish) the end of the
 // iteration.
 __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
-    __shared__ double warp_sum[kFusedThreads / 32];
+    __shared__ double warp_sum[32];
+    const int warps = int(blockDim.x >> 5);
     __shared__ bool last;
     for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, d);
     if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0;
-        for (int w = 0; w < kFusedThreads / 32; ++w) t += warp_sum[w];
+        for (int w = 0; w < warps; ++w) t += warp_sum[w];
         a.part[blockIdx.x] = t;
         __threadfence();
         last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
@@ -310,7 +313,7 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double sumsq = 0.0;
-        for (int w = 0; w < kFusedThreads / 32; ++w) sumsq += warp_sum[w];
+        for (int w = 0; w < warps; ++w) sumsq += warp_sum[w];
         end_iteration(a, words, sumsq);
         *a.ticket = 0u;
     }
@@ -405,6 +408,52 @@ template <class Op>
 __global__ void __launch_bounds__(kFusedThreads) k_dia_apply(Op M, const double* v, double* out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x)
         out[i] = M.dot(i, [&](int j) { return v[j]; });
+}
+
+// M (b - A x) in one pass, M held on A's diagonals: a block (a row per thread)
+// forms the raw residual of its rows and of a halo of H = max |offset| rows on
+// each side in shared memory and applies M from there.  The halo's rows are
+// formed by two blocks, with the same sums, so the result is that of the two
+// passes, which are launch latency while one wave of blocks holds the system.
+// NORM: with the norm and the end of the iteration.  Learned SPAI on 9-point
+// grids, a solve of 20 iterations: 704 -> 666 us at 128^2, 799 -> 766 at 256^2,
+// 1017 -> 978 at 384^2; with a second wave slower (1271 -> 1323 at 450^2).
+constexpr int kPairRows = 1024, kPairHalo = 512;
+template <bool NORM, class Op>
+__device__ __forceinline__ void residual_pair(const Op& A, const double* mdia, const double* x,
+                                              const double* b, double* out, int halo,
+                                              const ResidArgs& a) {
+    if constexpr (Op::kDiags > 0) {
+        __shared__ double raw[kPairRows + 2 * kPairHalo];
+        const int rows = blockDim.x, r0 = blockIdx.x * rows, r1 = min(r0 + rows, A.n);
+        const int lo = max(r0 - halo, 0), hi = min(r1 + halo, A.n);
+#pragma unroll 2
+        for (int j = lo + int(threadIdx.x); j < hi; j += rows)
+            raw[j - lo] = b[j] - A.dot(j, [&](int c) { return x[c]; });
+        __syncthreads();
+        const int i = r0 + int(threadIdx.x);
+        double acc = 0.0;
+        if (i < r1) {
+            const double r = dot_on_diagonals(A, mdia, i, [&](int c) { return raw[c - lo]; });
+            out[i] = r;
+            if (NORM) {
+                a.x2[i] = __dadd_rn(x[i], __dmul_rn(a.w, r));
+                acc = r * r;
+            }
+        }
+        if (NORM) norm_and_check(a, acc);
+    }
+}
+template <class Op>
+__global__ void __launch_bounds__(kPairRows) k_residual_pair(Op A, const double* mdia,
+                                                                const double* x, const double* b,
+                                                                double* out, int halo) {
+    residual_pair<false>(A, mdia, x, b, out, halo, ResidArgs{});
+}
+template <class Op>
+__global__ void __launch_bounds__(kPairRows) k_residual_pair_norm(Op A, const double* mdia,
+                                                                     int halo, ResidArgs a) {
+    residual_pair<true>(A, mdia, a.x, a.b, a.rout, halo, a);
 }
 
 // rp = M (b - A x) from the raw residual, its norm and the convergence check.
@@ -727,6 +776,17 @@ static bool fused_iteration(const mclsgpu_domain* dom, const mclsgpu_mcsa_params
             (dom->left->mdia && dom->op->dia_k > 0));
 }
 
+// The halo of residual_pair for this domain; 0: two passes.
+static int pair_halo(const mclsgpu_domain* dom) {
+    const mclsgpu_operator* op = dom->op;
+    if (!dom->left || !dom->left->mdia || op->dia_k == 0 ||
+        dom->n > dom->ctx->num_sms * kPairRows)
+        return 0;
+    int h = 1;
+    for (int j = 0; j < op->dia_k; ++j) h = std::max(h, std::abs(op->dia_off[j]));
+    return h <= kPairHalo ? h : 0;
+}
+
 // At most 8 blocks per SM: the per-block partial sums (two of them in
 // k_mcsa_begin) go to dom->part, sized for that many blocks.
 static int fused_grid(const mclsgpu_domain* dom) {
@@ -790,8 +850,17 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     // The last pass can add the tallies itself when it needs nothing but them.
     const bool fold = !mdia && dom->p.direction == MCLSGPU_ADJOINT &&
                       dom->p.estimator == MCLSGPU_COLLISION;
+    const int halo = pair_halo(dom);
+    // Fewer rows per block where there are few, so that most SMs take part.
+    const int pair_rows = n >= 100 * kPairRows  ? kPairRows
+                          : n >= 25 * kPairRows ? kPairRows / 2
+                                                : kPairRows / 4;
+    const int pairs = (n + pair_rows - 1) / pair_rows;
     if (fold) {
         richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, dom->x2, dom->rp2);
+    } else if (halo > 0) {
+        MCLSGPU_LAUNCH_OP(op, pairs, pair_rows, s, k_residual_pair, mdia, dom->x2, dom->b, dom->rp2,
+                          halo);
     } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, nullptr,
                           dom->tmp);
@@ -824,7 +893,9 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     a.d_nh = dom->d_nh;
     a.handle = handle;
     a.use_cond = use_cond;
-    if (mdia) {
+    if (halo > 0) {
+        MCLSGPU_LAUNCH_OP(op, pairs, pair_rows, s, k_residual_pair_norm, mdia, halo, a);
+    } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x, dom->b, nullptr,
                           dom->tmp);
         MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_precond_norm, a, dom->tmp);

@@ -15,6 +15,7 @@ struct SellView {  // SELL-32
     // must overlap (entry by entry 13.5 us for the residual of 10^5 rows of an
     // unstructured operator, 11.5 us so).  The registers cost resident blocks.
     static constexpr int kMinBlocks = 4;
+    static constexpr int kDiags = -1;  // not stored by diagonals
     static constexpr int kBatch = 8;
     const int* off;
     const int* col;
@@ -52,10 +53,13 @@ struct SellView {  // SELL-32
 template <int KK>
 struct DiaViewT {
     static constexpr int kMinBlocks = 8;
+    static constexpr int kDiags = KK > 0 ? KK : 16;  // at most
     const double* val;
     int n;
     int k;
     int off[16];
+    __device__ __forceinline__ int diags() const { return KK > 0 ? KK : k; }
+    __device__ __forceinline__ int offset(int j) const { return off[j]; }
     template <class F>
     __device__ __forceinline__ double dot(int r, F f) const {
         constexpr int kmax = KK > 0 ? KK : 16;
@@ -80,9 +84,15 @@ using DiaView = DiaViewT<0>;
 template <int H>
 struct DiaSymView {
     static constexpr int kMinBlocks = 8;
+    static constexpr int kDiags = 2 * H + 1;
     const double* val;  // [(1 + H) * n]: diagonal, then positive offsets ascending
     int n;
     int off[H];
+    __device__ __forceinline__ int diags() const { return kDiags; }
+    // Diagonal j in ascending order.
+    __device__ __forceinline__ int offset(int j) const {
+        return j < H ? -off[H - 1 - j] : j == H ? 0 : off[j - H - 1];
+    }
     template <class F>
     __device__ __forceinline__ double dot(int r, F f) const {
         double s = 0.0;
@@ -100,6 +110,20 @@ struct DiaSymView {
         return s;
     }
 };
+
+// Row r of another matrix on A's diagonals (values vals) times f: the sum that
+// DiaViewT's dot gives for it.
+template <class Op, class F>
+__device__ __forceinline__ double dot_on_diagonals(const Op& A, const double* vals, int r, F f) {
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < Op::kDiags; ++j) {
+        if (j >= A.diags()) break;
+        const int c = r + A.offset(j);
+        if (unsigned(c) < unsigned(A.n)) s = fma(vals[size_t(j) * A.n + r], f(c), s);
+    }
+    return s;
+}
 
 inline SellView sell_view(const mclsgpu_operator* op) {
     return SellView{op->S.off, op->S.col, op->S.val, op->S.n};
