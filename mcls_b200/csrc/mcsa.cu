@@ -82,57 +82,6 @@ __global__ void k_richardson(double* x, const double* r, int n, double w) {
         x[i] = __dadd_rn(x[i], __dmul_rn(w, r[i]));
 }
 
-struct FinalizeArgs {
-    int n;
-    int mode;            // 0 adjoint collision, 1 adjoint EV, 2 forward
-    int ev;
-    int base;            // kBase*: out = delta, out + delta, or xin + delta
-    int fp32;
-    double per;          // forward histories per state
-    const double* xin;
-    const double* sc;    // [2] = 1/nh
-    const double* src;   // MC source vector before scaling
-    double omega;
-    int has_omega;
-    const double* y64;
-    const int* dtrp;
-    const int* dtci;
-    const float* dth32;
-    const double* dth64;
-    double* out;
-};
-
-__global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
-    const double inv = a.sc[2];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
-        double d;
-        const double srci = a.has_omega ? a.src[i] * a.omega : a.src[i];
-        if (a.mode == 0) {
-            // AdjointTally::normalize: x *= 1/nh  (src/MCLS_AdjointTally_impl.hpp:68-72)
-            d = __dmul_rn(a.y64[i], inv);
-        } else if (a.mode == 1) {
-            double t = 0.0;
-            if (a.fp32) {
-                for (int k = a.dtrp[i]; k < a.dtrp[i + 1]; ++k)
-                    t = fma(double(a.dth32[k]), a.y64[a.dtci[k]], t);
-            } else {
-                for (int k = a.dtrp[i]; k < a.dtrp[i + 1]; ++k)
-                    t = fma(a.dth64[k], a.y64[a.dtci[k]], t);
-            }
-            d = __dadd_rn(__dmul_rn(t, inv), srci);
-        } else {
-            // ForwardTally::finalize: sum / count  (src/MCLS_ForwardTally_impl.hpp:194-208)
-            d = __ddiv_rn(a.y64[i], a.per);
-            if (a.ev) d = __dadd_rn(d, srci);
-        }
-        if (a.base == kBaseOut)
-            d = __dadd_rn(a.out[i], d);
-        else if (a.base == kBaseIn)
-            d = __dadd_rn(a.xin[i], d);
-        a.out[i] = d;
-    }
-}
-
 // The words a solve's counters and report live in.
 struct Counters {
     int* status;
@@ -167,16 +116,88 @@ __global__ void k_solve_begin(Counters c) {
     c.tim[3] = 0;
 }
 
-// End of a Monte Carlo solve: the stream epoch, the history count, the walk
-// timing, and the host's report (may be null).
-__global__ void k_mc_end(unsigned long long* epoch, const int* d_nh, Counters c,
-                         SolveReport* report) {
+// End of a Monte Carlo solve (one thread): the stream epoch, the history count,
+// the walk timing, and the host's report (may be null).
+__device__ __forceinline__ void end_mc(unsigned long long* epoch, const int* d_nh,
+                                       const Counters& c, SolveReport* report) {
     const unsigned long long e = *epoch, h = *c.hist;
     const int nh = *d_nh;
     *epoch = e + 1ULL;
     *c.hist = h + (unsigned long long)nh;
     add_walk_time(c.tim);
     if (report) write_report(c, report);
+}
+
+__global__ void k_mc_end(unsigned long long* epoch, const int* d_nh, Counters c,
+                         SolveReport* report) {
+    end_mc(epoch, d_nh, c, report);
+}
+
+struct FinalizeArgs {
+    int n;
+    int mode;            // 0 adjoint collision, 1 adjoint EV, 2 forward
+    int ev;
+    int base;            // kBase*: out = delta, out + delta, or xin + delta
+    int fp32;
+    double per;          // forward histories per state
+    const double* xin;
+    const double* sc;    // [2] = 1/nh
+    const double* src;   // MC source vector before scaling
+    double omega;
+    int has_omega;
+    const double* y64;
+    const int* dtrp;
+    const int* dtci;
+    const float* dth32;
+    const double* dth64;
+    double* out;
+    // A Monte Carlo solve of its own ends here (null epoch: its caller ends it).
+    unsigned long long* epoch;
+    const int* d_nh;
+    Counters c;
+    SolveReport* report;
+    unsigned int* ticket;
+};
+
+// The walks' tallies into the solution; for a Monte Carlo solve of its own the
+// last block also ends the solve (a launch of its own took 4.2 us of the 66 us of
+// a 32^2 solve with host vectors, the ticket 3).
+__global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
+    const double inv = a.sc[2];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+        double d;
+        const double srci = a.has_omega ? a.src[i] * a.omega : a.src[i];
+        if (a.mode == 0) {
+            // AdjointTally::normalize: x *= 1/nh  (src/MCLS_AdjointTally_impl.hpp:68-72)
+            d = __dmul_rn(a.y64[i], inv);
+        } else if (a.mode == 1) {
+            double t = 0.0;
+            if (a.fp32) {
+                for (int k = a.dtrp[i]; k < a.dtrp[i + 1]; ++k)
+                    t = fma(double(a.dth32[k]), a.y64[a.dtci[k]], t);
+            } else {
+                for (int k = a.dtrp[i]; k < a.dtrp[i + 1]; ++k)
+                    t = fma(a.dth64[k], a.y64[a.dtci[k]], t);
+            }
+            d = __dadd_rn(__dmul_rn(t, inv), srci);
+        } else {
+            // ForwardTally::finalize: sum / count  (src/MCLS_ForwardTally_impl.hpp:194-208)
+            d = __ddiv_rn(a.y64[i], a.per);
+            if (a.ev) d = __dadd_rn(d, srci);
+        }
+        if (a.base == kBaseOut)
+            d = __dadd_rn(a.out[i], d);
+        else if (a.base == kBaseIn)
+            d = __dadd_rn(a.xin[i], d);
+        a.out[i] = d;
+    }
+    if (!a.epoch) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(a.ticket, 1u) != gridDim.x - 1) return;
+    *a.ticket = 0u;
+    end_mc(a.epoch, a.d_nh, a.c, a.report);
 }
 
 // Convergence check of one MCSA iteration (src/MCLS_MCSASolverManager_impl.hpp:380-394).
@@ -690,6 +711,7 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
     launch_walk(dom, fin, max_trace, tr_states, tr_w, tr_ev, tr_start, fused);
     launch_advance_walk_pos(dom);
     cudaStream_t s = dom->ctx->stream;
+    SolveReport* const host = report ? dom->ctx->h_report : nullptr;
     if (!walk_finishes(dom) && base != kBaseTally) {
         FinalizeArgs f{};
         f.n = dom->n;
@@ -709,11 +731,17 @@ static void enqueue_mc(mclsgpu_domain* dom, const double* v, double* out, int ba
         f.dth32 = dom->dt_h32;
         f.dth64 = dom->DT.v;
         f.out = out;
+        if (!fused) {
+            f.epoch = dom->d_epoch;
+            f.d_nh = dom->d_nh;
+            f.c = counters(dom);
+            f.report = host;
+            f.ticket = dom->d_ticket;
+        }
         k_finalize<<<grid_for(dom->n, 256, 148 * 8), 256, 0, s>>>(f);
+    } else if (!fused) {
+        k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_nh, counters(dom), host);
     }
-    if (!fused)
-        k_mc_end<<<1, 1, 0, s>>>(dom->d_epoch, dom->d_nh, counters(dom),
-                                 report ? dom->ctx->h_report : nullptr);
 }
 
 // MC solve with device vectors.  host_x (may be null): pinned memory that
