@@ -91,7 +91,6 @@ struct BatchArgs {
     const double* B;
     double* X;
     double* X2;          // smoothed iterate x + w rp
-    double* RP;
     double* RP2;
     double* Y;
     float* cR;
@@ -401,28 +400,48 @@ __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphCondition
     BatchState st = *a.st;
     const int it = st.iter + 1;
     const bool check = (it % st.check_freq) == 0 || it >= st.max_iters;
+    // The pw lanes of a system are neighbours in a warp (pw is a power of two, at
+    // most 16), so a ballot tells whether all its pairs have converged.  A few
+    // pairs per thread are loaded before the first is stored; pair after pair and
+    // with rp written besides, k_b_update took 74 us on 128 systems, 67 us so.
     int conv = 0;
-    for (int q = threadIdx.x; q < a.nsys * a.pw; q += blockDim.x) {
-        const int s = q / a.pw, r = q % a.pw;
-        if (r >= a.nrhs[s]) continue;
-        const double nr = __ldcg(&a.norm2[q]);
-        if (!isfinite(nr)) atomicOr(a.status, DEV_ERR_NONFINITE);
-        if (a.conv_iter[q] < 0 && check && sqrt(nr) <= st.tol * sqrt(a.bnorm2[q]))
-            a.conv_iter[q] = it;
-        if (a.conv_iter[q] >= 0) ++conv;
-        a.norm2[q] = 0.0;
+    const int total = a.nsys * a.pw;
+    const int lane = threadIdx.x & 31;
+    const unsigned group = ((1u << a.pw) - 1u) << (lane & ~(a.pw - 1));
+    constexpr int kAhead = 4;
+    for (int base = 0; base < total; base += kAhead * int(blockDim.x)) {
+        double nr[kAhead], bn[kAhead];
+        int since[kAhead], done[kAhead];
+        bool pair[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int q = base + u * int(blockDim.x) + int(threadIdx.x), s = q / a.pw;
+            pair[u] = q < total && q % a.pw < a.nrhs[s];
+            done[u] = q < total ? a.sys_done[s] : 1;
+            nr[u] = pair[u] ? __ldcg(&a.norm2[q]) : 0.0;
+            bn[u] = pair[u] ? a.bnorm2[q] : 0.0;
+            since[u] = pair[u] ? a.conv_iter[q] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int q = base + u * int(blockDim.x) + int(threadIdx.x), s = q / a.pw;
+            if (pair[u]) {
+                if (!isfinite(nr[u])) atomicOr(a.status, DEV_ERR_NONFINITE);
+                if (since[u] < 0 && check && sqrt(nr[u]) <= st.tol * sqrt(bn[u]))
+                    a.conv_iter[q] = since[u] = it;
+                if (since[u] >= 0) ++conv;
+                a.norm2[q] = 0.0;
+            }
+            // Systems whose every right-hand side has converged stop iterating.
+            const int all = (__ballot_sync(0xffffffffu, since[u] < 0) & group) == 0u;
+            if (q < total && q % a.pw == 0 && done[u] != all) {
+                a.sys_done[s] = all;
+                changed = 1;
+            }
+        }
     }
     atomicAdd(&s_conv, conv);
     __syncthreads();
-    // Systems whose every right-hand side has converged stop iterating.
-    for (int s = threadIdx.x; s < a.nsys; s += blockDim.x) {
-        int all = 1;
-        for (int r = 0; r < a.nrhs[s]; ++r) all &= a.conv_iter[size_t(s) * a.pw + r] >= 0;
-        if (a.sys_done[s] != all) {
-            a.sys_done[s] = all;
-            changed = 1;
-        }
-    }
     // The list stands while no system finishes.
     if (__syncthreads_or(changed)) build_active(a);
     if (threadIdx.x == 0) {
@@ -472,10 +491,10 @@ struct PairSums {
     }
 };
 
-// rp = D^-1 (b - S x), the next smoothed iterate x2 = x + w rp and the
-// per-(system, rhs) sums of squares.  CHECK: the
-// last block to finish runs the convergence test (the other blocks' sums are
-// complete and visible by then).
+// rp = D^-1 (b - S x): the next smoothed iterate x2 = x + w rp and the
+// per-(system, rhs) sums of squares (rp itself is not kept).  CHECK: the last
+// block to finish runs the convergence test (the other blocks' sums are complete
+// and visible by then).
 template <bool CHECK>
 __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, int use_cond,
                                                          cudaGraphConditionalHandle handle) {
@@ -500,7 +519,6 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, 
                 ps.v[n] += t.v[n] * t.v[n];
                 x.v[n] = __dadd_rn(x.v[n], __dmul_rn(a.omega, t.v[n]));
             }
-            stn<N>(a.RP + e, t);
             stn<N>(a.X2 + e, x);
         });
     });
@@ -608,7 +626,7 @@ struct mclsgpu_batch {
     int* all_sys = nullptr;
     int* all_tcum = nullptr;
     int* all_count = nullptr;
-    double *X = nullptr, *X2 = nullptr, *RP = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
+    double *X = nullptr, *X2 = nullptr, *RP2 = nullptr, *B = nullptr, *Y = nullptr;
     float* cR = nullptr;
     double* norm2 = nullptr;
     double* bnorm2 = nullptr;
@@ -655,7 +673,6 @@ void batch_release(mclsgpu_batch* b) {
     dfree(b->all_count);
     dfree(b->X);
     dfree(b->X2);
-    dfree(b->RP);
     dfree(b->RP2);
     dfree(b->B);
     dfree(b->Y);
@@ -709,7 +726,6 @@ BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) 
     a.B = b->B;
     a.X = b->X;
     a.X2 = b->X2;
-    a.RP = b->RP;
     a.RP2 = b->RP2;
     a.Y = b->Y;
     a.cR = b->cR;
@@ -916,7 +932,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
          (e = dmalloc(&b->all_tcum, nsys + 1)) != cudaSuccess ||
          (e = dmalloc(&b->all_count, 1)) != cudaSuccess ||
          (e = dmalloc(&b->X, NE)) != cudaSuccess || (e = dmalloc(&b->X2, NE)) != cudaSuccess ||
-         (e = dmalloc(&b->RP, NE)) != cudaSuccess || (e = dmalloc(&b->RP2, NE)) != cudaSuccess ||
+         (e = dmalloc(&b->RP2, NE)) != cudaSuccess ||
          (e = dmalloc(&b->B, NE)) != cudaSuccess ||
          (b->per > 1 && (e = dmalloc(&b->Y, NE)) != cudaSuccess) ||
          (e = dmalloc(&b->cR, NE)) != cudaSuccess || (e = dmalloc(&b->norm2, PR)) != cudaSuccess ||
@@ -948,7 +964,6 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         // Padding elements are never written by the loop: zero every array once.
         cudaMemsetAsync(b->X, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->X2, 0, sizeof(double) * NE, s);
-        cudaMemsetAsync(b->RP, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->RP2, 0, sizeof(double) * NE, s);
         if (b->Y) cudaMemsetAsync(b->Y, 0, sizeof(double) * NE, s);
         cudaMemsetAsync(b->cR, 0, sizeof(float) * NE, s);
