@@ -70,19 +70,18 @@ CONFIGS = {
                      max_iters=100000),
 }
 # DRAM bytes (read + write) of one walk launch on each workload: ncu's
-# dram__bytes_read.sum (83.90 MB) + dram__bytes_write.sum (7.82 MB) for the
-# stencil forward expected-value walk32 launch at 128^3.
-WALK_DRAM_BYTES_PER_LAUNCH = {"diffusion128": 91.72e6}
-# The same for one walk32 launch of the 192^3 roofline domain (226 MB of
-# records, more than L2): dram__bytes_read.sum (283.14 MB) +
-# dram__bytes_write.sum (47.17 MB) of the 4-histories-per-lane x 256 launch
-# (python -m mcls_b200.walkprof --n 192 --solves 2 --histories-per-lane 4).
-HBM_WALK_DRAM_BYTES_PER_LAUNCH = 330.31e6
-# The same capture's L2 and DRAM figures: what binds the walk (L2 throughput
-# and latency, the records read from HBM about once per launch).
-HBM_WALK_NCU = {"lts_throughput_pct_of_peak": 64.1, "lts_sector_hit_pct": 87.3,
-                "dram_throughput_pct_of_peak": 8.8, "top_stall": "long scoreboard (L2 loads)",
-                "capture": "ncu --set full, one walk32 launch, 192^3, 4 histories per lane x 256"}
+# dram__bytes_read.sum (109.08 MB) + dram__bytes_write.sum (10.0 MB) for the
+# forward expected-value walk32_rows launch of an MCSA iteration at 128^3.
+WALK_DRAM_BYTES_PER_LAUNCH = {"diffusion128": 119.1e6}
+# The same for the 192^3 roofline domain (226 MB of records, more than L2):
+# 368.1 MB + 51.1 MB in an MCSA iteration; a Monte Carlo solve's walk reads no
+# base iterate, 56.6 MB less.
+HBM_WALK_DRAM_BYTES_PER_LAUNCH = 362.6e6
+# The same capture's L2 and DRAM figures: what binds the walk (requests from
+# L1TEX to L2; each record is read from HBM about once per launch).
+HBM_WALK_NCU = {"l1tex_to_l2_request_pct_of_peak": 79.2, "lts_sectors_pct_of_peak": 32.5,
+                "lts_sector_hit_pct": 84.1, "dram_gbs": 1053.0,
+                "capture": "ncu, walk32_rows of an MCSA iteration, 192^3, two histories per row"}
 # The oracle port's whole MCSA solve of a workload, run once to the end
 # (FP64 forward expected-value walks on the counter stream, the workload's
 # histories per iteration, seed 1234): its iteration count, which the
@@ -564,7 +563,7 @@ def run_batched(args, world, rank, local, pg):
         "gpu_launches": int(sum(s["kernel_launches"] for s in stats)),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if achieved else None, "traffic": None,
-                     "kernel": "walk32_multi", "peak_kind": peak_kind, "bytes_per_step": bstep,
+                     "kernel": "walk32_batch", "peak_kind": peak_kind, "bytes_per_step": bstep,
                      "walk_ms_per_launch": per_launch,
                      "walk_share_of_solve": walk_ms / dev_ms if dev_ms else None},
         "wall_s": wall,
@@ -1157,7 +1156,7 @@ def main():
                                "residual, update and norms" if fp == capi.FP32 else "FP64"}
     roofline_workload = {
         "bound": "l2" if traffic and traffic < 0.5 * bytes_per_launch else "hbm",
-        "kernel": "walk32", "achieved": achieved, "unit": "GB/s",
+        "kernel": "walk32_rows", "achieved": achieved, "unit": "GB/s",
         "frac_of_hbm_peak": achieved / peak if achieved else None, "peak": peak,
         "peak_kind": peak_kind, "traffic": traffic,
         "dram_gbs": traffic / (per_launch_ms * 1e-3) / 1e9 if traffic and per_launch_ms else None,
@@ -1189,7 +1188,7 @@ def main():
         tr = HBM_WALK_DRAM_BYTES_PER_LAUNCH
         line["roofline"] = {
             "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-            "traffic": tr, "kernel": "walk32", "peak_kind": peak_kind,
+            "traffic": tr, "kernel": "walk32_rows", "peak_kind": peak_kind,
             "dram_gbs": tr / (hr["per_launch_ms"] * 1e-3) / 1e9 if tr else None,
             "binding": "L2: the algorithmic bytes exceed the HBM peak because each record is "
                        "read from HBM about once per launch and its later reads hit L2",
