@@ -17,7 +17,8 @@
 // adjoint histories (walk32_adjoint) tally with a fire-and-forget FP64
 // reduction per step, the step-0 tally being made by the source build (counts
 // * w0), so walks tally from step 1; histories ended by a weight cutoff
-// (walk32_cutoff) are pulled from a work queue.
+// (walk32_cutoff) are pulled from a work queue.  Fixed-length walks of domains
+// whose records fit shared memory read them there (walk32_small).
 //
 // walk64: the parity kernel.  FP64 domain, std::lower_bound's selection, FP64
 // weights and tallies, optional trajectory trace.  With the reference stream it
