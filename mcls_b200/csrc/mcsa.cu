@@ -342,8 +342,13 @@ __device__ __forceinline__ void norm_and_check(const ResidArgs& a, double acc) {
 
 // The same for a system whose rows one cluster takes: the blocks' sums meet in
 // the first block's shared memory, and its first thread has loaded the words
-// before the rows.
+// before the rows.  Another block's shared memory may be written only once that
+// block has started: every thread arrives at the cluster's barrier on entry
+// (cluster_enter) and waits before the store, so the rows hide the wait.
 constexpr int kClusterCtas = 8, kClusterThreads = 1024;
+__device__ __forceinline__ void cluster_enter() {
+    cooperative_groups::this_cluster().barrier_arrive();
+}
 __device__ __forceinline__ void norm_and_check_cluster(const ResidArgs& a, IterationWords& words,
                                                        double acc) {
     namespace cg = cooperative_groups;
@@ -353,6 +358,7 @@ __device__ __forceinline__ void norm_and_check_cluster(const ResidArgs& a, Itera
     for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, d);
     if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
     __syncthreads();
+    cluster.barrier_wait();  // of cluster_enter
     if (threadIdx.x < 32) {
         double t = warp_sum[threadIdx.x];
         for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
@@ -412,6 +418,7 @@ constexpr int kClusterRows = 3 * kClusterCtas * kClusterThreads / 2;
 template <class Op>
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
     k_residual_norm_cluster(Op A, ResidArgs a) {
+    cluster_enter();
     IterationWords words;
     if (blockIdx.x == 0 && threadIdx.x == 0) words.load(a);
     norm_and_check_cluster(a, words, residual_rows<false>(A, a));
@@ -419,6 +426,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
 template <class Op>
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
     k_finalize_norm_cluster(Op A, ResidArgs a) {
+    cluster_enter();
     IterationWords words;
     if (blockIdx.x == 0 && threadIdx.x == 0) words.load(a);
     norm_and_check_cluster(a, words, residual_rows<true>(A, a));
