@@ -656,7 +656,6 @@ struct AndersonWork {
     AaState* h_st = nullptr;
     cudaGraphExec_t graph = nullptr;
     long long graph_key = -1;
-    const double* graph_hist = nullptr;  // residual history the graph writes
     int body_kernels = 0;
     // Step-wise solves (mclsgpu_anderson_begin .. _finish).
     mclsgpu_anderson_params step_p{};
@@ -817,17 +816,7 @@ int anderson_prepare(mclsgpu_domain* dom, const mclsgpu_anderson_params* p) {
                          "the Anderson solver applies the left preconditioner only");
     int rc = ensure_work(dom, p->storage_depth);
     if (rc) return rc;
-    if (p->max_iters > dom->resid_cap) {
-        cudaStreamSynchronize(ctx->stream);
-        dfree(dom->d_resid);
-        cudaError_t e = dmalloc(&dom->d_resid, size_t(p->max_iters));
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
-        dom->resid_cap = p->max_iters;
-        // The captured MCSA graph holds the old history pointer.
-        if (dom->graph) cudaGraphExecDestroy(dom->graph);
-        dom->graph = nullptr;
-    }
-    return MCLSGPU_OK;
+    return grow_history(dom, p->max_iters);
 }
 
 // Counters, b and x0, the initial residual and state (the status test on
@@ -879,7 +868,7 @@ int anderson_solve(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
     const long long key = (long long)p->smoother_steps * 64 + p->storage_depth;
     // Variable-length reference-stream walks synchronise with the host.
     const bool host_loop = p->host_loop || walk_needs_rounds(dom);
-    if (!host_loop && (!w->graph || w->graph_key != key || w->graph_hist != dom->d_resid)) {
+    if (!host_loop && (!w->graph || w->graph_key != key)) {
         if (w->graph) cudaGraphExecDestroy(w->graph);
         w->graph = nullptr;
         rc = build_while_graph(
@@ -887,7 +876,6 @@ int anderson_solve(mclsgpu_domain* dom, const double* b_dev, double* x_dev,
             &w->body_kernels);
         if (rc) return rc;
         w->graph_key = key;
-        w->graph_hist = dom->d_resid;
     }
     cudaEventRecord(ctx->ev[0], s);
     anderson_begin(dom, b_dev, x_dev, p);

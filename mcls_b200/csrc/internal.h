@@ -353,6 +353,11 @@ int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
 
 // Releases the domain's captured Anderson loop (rebuilt on the next solve).
 void anderson_drop_graph(mclsgpu_domain* dom);
+// Releases every captured loop of the domain: what they hold has changed.
+void drop_loops(mclsgpu_domain* dom);
+// Room for the norms of `iters` iterations in d_resid.  Every captured loop of
+// the domain writes there, so a new buffer drops them all.
+int grow_history(mclsgpu_domain* dom, int iters);
 
 // FP32 forward walks: the tally source of v into the domain's records (H v
 // for the expected-value estimator, v for collision, with the Neumann

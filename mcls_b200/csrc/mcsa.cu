@@ -947,6 +947,26 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     }
 }
 
+void drop_loops(mclsgpu_domain* dom) {
+    if (dom->graph) cudaGraphExecDestroy(dom->graph);
+    dom->graph = nullptr;
+    if (dom->set_graph) cudaGraphExecDestroy(dom->set_graph);
+    dom->set_graph = nullptr;
+    anderson_drop_graph(dom);
+}
+
+int grow_history(mclsgpu_domain* dom, int iters) {
+    if (iters <= dom->resid_cap) return MCLSGPU_OK;
+    cudaStreamSynchronize(dom->ctx->stream);
+    drop_loops(dom);
+    dom->resid_cap = 0;
+    dfree(dom->d_resid);
+    cudaError_t e = dmalloc(&dom->d_resid, size_t(iters));
+    if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "cudaMalloc residual history");
+    dom->resid_cap = iters;
+    return MCLSGPU_OK;
+}
+
 // Build the CUDA graph of the MCSA loop (WHILE node, one iteration per body).
 static int build_mcsa_graph(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp) {
     mclsgpu_context* ctx = dom->ctx;
@@ -1076,16 +1096,7 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
-    if (mp->max_iters > dom->resid_cap) {
-        dfree(dom->d_resid);
-        cudaError_t e = dmalloc(&dom->d_resid, size_t(mp->max_iters));
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
-        dom->resid_cap = mp->max_iters;
-        if (dom->graph) {
-            cudaGraphExecDestroy(dom->graph);
-            dom->graph = nullptr;
-        }
-    }
+    if (int rc = grow_history(dom, mp->max_iters)) return rc;
     // Graph key: everything baked into the captured iteration.
     const int key = (mp->smoother_steps * 1000003 ^ int(mp->richardson_omega * 1e6)) * 4 +
                     mp->fixed_point_type;

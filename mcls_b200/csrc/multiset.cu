@@ -147,20 +147,7 @@ int solve_sets(mclsgpu_domain* dom, const mclsgpu_set_params* sp, const double* 
         cudaError_t e = dmalloc(&dom->delta, size_t(n));
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
     }
-    if (mp.max_iters > dom->resid_cap) {
-        dfree(dom->d_resid);
-        cudaError_t e = dmalloc(&dom->d_resid, size_t(mp.max_iters));
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
-        dom->resid_cap = mp.max_iters;
-        if (dom->graph) {  // the single-set loop recorded the old history buffer
-            cudaGraphExecDestroy(dom->graph);
-            dom->graph = nullptr;
-        }
-        if (dom->set_graph) {
-            cudaGraphExecDestroy(dom->set_graph);
-            dom->set_graph = nullptr;
-        }
-    }
+    if ((rc = grow_history(dom, mp.max_iters))) return rc;
     // The device-side loop when the reducer can be captured; the graph is kept
     // for the next solve with the same reducer, set count and smoother.
     bool graph = sp->capturable && !mp.host_loop && !walk_needs_rounds(dom);

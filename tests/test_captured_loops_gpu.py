@@ -1,0 +1,54 @@
+"""The captured solver loops of one domain (MCSA, multi-set MCSA, Anderson) share
+its buffers: a solve with more iterations than any before replaces the residual
+history, and the loops captured earlier must not write to the old one."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+from mcls_b200 import capi
+from mcls_b200 import problems as P
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mcls_b200", "csrc")
+
+
+def test_the_history_of_a_live_domain_is_replaced_in_one_place():
+    # release_domain (capi.cu), the fixed-point scratch and grow_history (mcsa.cu).
+    places = {}
+    for f in sorted(os.listdir(CSRC)):
+        hits = len(re.findall(r"dfree\([^)]*d_resid\)", open(os.path.join(CSRC, f)).read()))
+        if hits:
+            places[f] = hits
+    assert places == {"capi.cu": 1, "fixedpoint.cu": 1, "mcsa.cu": 1}
+    body = open(os.path.join(CSRC, "mcsa.cu")).read().split("int grow_history(")[1].split("\n}")[0]
+    assert body.index("drop_loops(dom)") < body.index("dfree(dom->d_resid)")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [("sets", "mcsa", "sets"), ("sets", "anderson", "sets"),
+                                   ("mcsa", "anderson", "mcsa"), ("anderson", "mcsa", "anderson"),
+                                   ("mcsa", "sets", "mcsa"), ("anderson", "sets", "anderson")])
+def test_solvers_in_turn_with_growing_iteration_limits(ctx, order):
+    A = P.poisson2d(12)
+    b = np.linspace(0.5, 1.0, A.shape[0])
+    op = capi.Operator(ctx, A)
+    pc = capi.Precond(ctx, op, capi.PREC_POINT_JACOBI)
+    one = capi.set_params(1, lambda ptr, n, stream: None, capturable=True)
+
+    def solve(dom, what, iters, host):
+        if what == "anderson":
+            return dom.anderson_solve(b, tolerance=0.0, max_iters=iters, host_loop=host)[0]
+        if what == "mcsa":
+            return dom.mcsa_solve(b, tolerance=0.0, max_iters=iters, host_loop=host)[0]
+        return dom.mcsa_solve_sets(one, b, tolerance=0.0, max_iters=iters, host_loop=host)[0]
+
+    out = []
+    for host in (0, 1):
+        # Forward, one history a row: the same bits on every run.
+        dom = capi.Domain(ctx, op, pc, precision=capi.FP64, rng_mode=capi.RNG_COUNTER, seed=4,
+                          estimator=capi.EXPECTED_VALUE, direction=capi.FORWARD,
+                          sample_ratio=1.0)
+        out.append([solve(dom, w, n, host) for w, n in zip(order, (5, 60, 20))])
+    for x, y in zip(*out):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
