@@ -696,6 +696,7 @@ int fixed_rows(mclsgpu_context* ctx, const DevCsr& A, int longest, BatchRows& M)
         (e = dmalloc(&M.val, entries)) != cudaSuccess)
         return cuda_fail(ctx, e, "cudaMalloc batch rows");
     const int grid = std::min((M.n + kThreads - 1) / kThreads, ctx->num_sms * 8);
+    drop_stale_error();
     k_b_rows<<<grid, kThreads, 0, ctx->stream>>>(A.rp, A.ci, A.v, M);
     e = cudaGetLastError();
     return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(ctx, e, "batch rows");

@@ -326,6 +326,7 @@ int mclsgpu_operator_apply(mclsgpu_operator* op, const double* x, double* y) {
     const char* what = "copy x";
     e = cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
+        drop_stale_error();
         spmv(ctx->stream, op->A, dx, dy);
         what = "apply: spmv launch";
         e = cudaGetLastError();

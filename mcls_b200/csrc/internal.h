@@ -286,6 +286,9 @@ int cuda_fail(mclsgpu_context* ctx, cudaError_t e, const char* what);
 int check_device_status(mclsgpu_context* ctx);
 // The error of a device status word (0: none); clears the device's.
 int status_error(mclsgpu_context* ctx, int status);
+// An error that the program left behind in the runtime is not this library's:
+// whatever checks its launches with cudaGetLastError drops it first.
+inline void drop_stale_error() { cudaGetLastError(); }
 // Every device allocation and release of the library goes through dmalloc and
 // dfree; the counters behind mclsgpu_debug_device_allocations count them.
 extern std::atomic<long long> g_device_allocs;

@@ -759,6 +759,7 @@ static int mc_solve_device(mclsgpu_domain* dom, const double* rhs_dev, double* x
                            long long* tr_start, mclsgpu_stats* stats, double* host_x = nullptr) {
     mclsgpu_context* ctx = dom->ctx;
     cudaStream_t s = ctx->stream;
+    drop_stale_error();
     mcsa_solve_begin(dom);
     const double* v = rhs_dev;
     if (dom->left && !internal) {
@@ -1097,6 +1098,7 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
     cudaStream_t s = ctx->stream;
     const int n = dom->n;
     if (int rc = grow_history(dom, mp->max_iters)) return rc;
+    drop_stale_error();
     // Graph key: everything baked into the captured iteration.
     const int key = (mp->smoother_steps * 1000003 ^ int(mp->richardson_omega * 1e6)) * 4 +
                     mp->fixed_point_type;

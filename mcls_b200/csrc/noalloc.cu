@@ -107,6 +107,7 @@ extern "C" int mclsgpu_operator_apply_static(mclsgpu_operator* op, const double*
     // Every y row is written by the kernel, so nothing needs clearing.
     e = cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "copy x");
+    drop_stale_error();
     spmv(ctx->stream, op->A, dx, dy);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "static apply: spmv launch");

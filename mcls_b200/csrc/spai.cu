@@ -1112,6 +1112,7 @@ int launch_forward(mclsgpu_spai* net, mclsgpu_operator* op, const SlotTable& t, 
     const int ntiles = (op->A.n + kTileRows - 1) / kTileRows;
     const int fit = ctx->num_sms * kFwdCtas;
     const int grid = ntiles < fit ? ntiles : fit;
+    drop_stale_error();
     with_slots(t.K, [&](auto k) {
         k_spai_forward<decltype(k)::value><<<grid, kThreads, kFwdSmem, ctx->stream>>>(a);
     });

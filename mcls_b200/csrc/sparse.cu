@@ -493,6 +493,7 @@ void spmv(cudaStream_t s, const DevCsr& A, const double* x, double* y) {
 }
 
 int reciprocal_diagonal(mclsgpu_context* ctx, const DevCsr& A, double* dinv) {
+    drop_stale_error();
     k_recip_diag<<<grid_for(A.n), 256, 0, ctx->stream>>>(A.rp, A.ci, A.v, A.n, dinv);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MCLSGPU_OK : cuda_fail(ctx, e, "reciprocal diagonal");

@@ -1505,6 +1505,7 @@ int walk_agreement(mclsgpu_domain* dom, long long histories, uint64_t seed, long
     const long long g = (histories + 255) / 256;
     const int grid = int(g < ctx->num_sms * 8 ? g : ctx->num_sms * 8);
     const uint64_t ekey = epoch_key(seed, 0);
+    drop_stale_error();
     bool ok = true;
 #define MCLSGPU_AGREE(SL, STV) k_walk_agreement<SL, STV><<<grid, 256, 0, st>>>(a, histories, ekey, d_out)
     if (dom->stencil_k && dom->rec_q16) {
