@@ -636,7 +636,7 @@ struct mclsgpu_batch {
     mclsgpu::BatchState* d_state = nullptr;
     mclsgpu::BatchState* h_state = nullptr;
     cudaGraphExec_t graph = nullptr;
-    long long graph_key = -1;
+    mclsgpu::LoopKey graph_key;
     uint64_t graph_seed = 0;       // the domain seed the captured walks carry
     int body_kernels = 0;
     int per = 1;
@@ -1009,7 +1009,6 @@ int mclsgpu_batch_set_launch(mclsgpu_batch* b, int block_size, int grab) {
         return MCLSGPU_ERR_INVALID_ARG;
     b->dom->walk_block = block_size;
     b->grab = grab;
-    b->graph_key = -1;  // the captured loop bakes the launch shape in
     return MCLSGPU_OK;
 }
 
@@ -1046,7 +1045,6 @@ int mclsgpu_batch_autotune(mclsgpu_batch* b, const double* b_dev, double* x_dev,
         }
     b->dom->walk_block = best_b;
     b->grab = best_g;
-    b->graph_key = -1;
     if (block_size) *block_size = best_b;
     if (grab) *grab = best_g;
     if (walk_ms) *walk_ms = best_ms;
@@ -1066,8 +1064,7 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
     const size_t NE = size_t(b->ne), PR = size_t(b->nsys) * b->pw;
     int pairs = 0;
     for (int q = 0; q < b->nsys; ++q) pairs += b->nrhs[q];
-    const long long key = (long long)(params->richardson_omega * 1e6) * 64 +
-                          (long long)b->grab * 2 + (b->dom->walk_block == 128 ? 1 : 0);
+    const LoopKey key{params->richardson_omega, b->grab, b->dom->walk_block};
     if (!params->host_loop && (!b->graph || b->graph_key != key || b->graph_seed != b->dom->seed)) {
         int rc = build_batch_graph(b, params);
         if (rc) return rc;

@@ -51,6 +51,15 @@ struct SolveReport {
     int pad;
 };
 
+// The parameters that are baked into a captured loop, compared exactly: a loop
+// kept for another relaxation, however close, would go on with that one.
+struct LoopKey {
+    double omega = 0.0;
+    int a = -1, b = -1;   // smoother steps and type; batches: grab and block size
+    bool operator==(const LoopKey& o) const { return omega == o.omega && a == o.a && b == o.b; }
+    bool operator!=(const LoopKey& o) const { return !(*this == o); }
+};
+
 // Host vectors up to this many entries are copied out through pinned memory.
 constexpr int kStageMax = 32768;
 constexpr size_t kWordBytes = 1024;  // a domain's counters and scalars
@@ -248,7 +257,7 @@ struct mclsgpu_domain {
     mclsgpu::McsaState* d_state = nullptr;
     mclsgpu::McsaState* h_state = nullptr;  // pinned (the context's report)
     cudaGraphExec_t graph = nullptr;
-    int graph_key = -1;
+    mclsgpu::LoopKey graph_key;
     int body_kernels = 0;          // kernel nodes in one MCSA iteration
     unsigned long long* d_hist = nullptr;   // histories transported (total)
     double* d_resid = nullptr;     // per-iteration |rp|_2 history
@@ -271,7 +280,7 @@ struct mclsgpu_domain {
     void* set_graph_reduce = nullptr;
     void* set_graph_user = nullptr;
     int set_graph_sets = 0;
-    long long set_graph_key = -1;
+    mclsgpu::LoopKey set_graph_key;
     int set_body_kernels = 0;
     // Anderson-accelerated MCSA work space (anderson.cu), built on first use.
     mclsgpu::AndersonWork* aa = nullptr;

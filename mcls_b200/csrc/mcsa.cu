@@ -1099,9 +1099,7 @@ static int mcsa_solve_device(mclsgpu_domain* dom, const double* b_dev, double* x
     const int n = dom->n;
     if (int rc = grow_history(dom, mp->max_iters)) return rc;
     drop_stale_error();
-    // Graph key: everything baked into the captured iteration.
-    const int key = (mp->smoother_steps * 1000003 ^ int(mp->richardson_omega * 1e6)) * 4 +
-                    mp->fixed_point_type;
+    const LoopKey key{mp->richardson_omega, mp->smoother_steps, mp->fixed_point_type};
     if (int rc = prepare_fixed_point(dom, mp->fixed_point_type)) return rc;
     // Variable-length reference-stream walks synchronise with the host.
     const bool host_loop = mp->host_loop || walk_needs_rounds(dom);
@@ -1484,14 +1482,14 @@ int mclsgpu_domain_set_launch(mclsgpu_domain* dom, int histories_per_lane, int b
     dom->walk_ilp = histories_per_lane;
     dom->walk_block = block_size;
     prepare_walk(dom);
-    dom->graph_key = -1;  // the launch shape is baked into the captured loop
+    dom->graph_key = LoopKey{};  // the launch shape is baked into the captured loop
     return MCLSGPU_OK;
 }
 
 int mclsgpu_domain_set_record_cache(mclsgpu_domain* dom, int allocate_l1) {
     if (!dom || (allocate_l1 != 0 && allocate_l1 != 1)) return MCLSGPU_ERR_INVALID_ARG;
     dom->walk_l1 = allocate_l1;
-    dom->graph_key = -1;  // baked into the captured loop
+    dom->graph_key = LoopKey{};  // baked into the captured loop
     if (dom->set_graph) {
         cudaGraphExecDestroy(dom->set_graph);
         dom->set_graph = nullptr;

@@ -152,8 +152,7 @@ int solve_sets(mclsgpu_domain* dom, const mclsgpu_set_params* sp, const double* 
     // for the next solve with the same reducer, set count and smoother.
     bool graph = sp->capturable && !mp.host_loop && !walk_needs_rounds(dom);
     if (graph) {
-        const long long key = (long long)mp.smoother_steps * 1000003LL + mp.fixed_point_type * 7 +
-                              (long long)(mp.richardson_omega * 1e6);
+        const LoopKey key{mp.richardson_omega, mp.smoother_steps, mp.fixed_point_type};
         if (!dom->set_graph || dom->set_graph_reduce != reinterpret_cast<void*>(sp->reduce) ||
             dom->set_graph_user != sp->user || dom->set_graph_sets != sp->num_sets ||
             dom->set_graph_key != key) {

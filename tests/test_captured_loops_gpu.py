@@ -52,3 +52,40 @@ def test_solvers_in_turn_with_growing_iteration_limits(ctx, order):
         out.append([solve(dom, w, n, host) for w, n in zip(order, (5, 60, 20))])
     for x, y in zip(*out):
         assert np.isfinite(x).all() and np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["mcsa", "sets", "batch"])
+def test_a_kept_loop_has_the_relaxation_asked_for(ctx, solver):
+    """The relaxation is baked into the captured loop: one that agrees with the
+    last to six decimals gives what a loop captured for it gives."""
+    A, b = P.diffusion3d_varcoef(9, seed=1)
+    op = capi.Operator(ctx, A)
+    pc = capi.Precond(ctx, op, capi.PREC_POINT_JACOBI)
+    one = capi.set_params(1, lambda ptr, n, stream: None, capturable=True)
+    kw = dict(precision=capi.FP32, direction=capi.FORWARD, estimator=capi.EXPECTED_VALUE,
+              sample_ratio=1.0, seed=2)
+    near = 0.9 + 4e-7
+    out = []
+    for first in (0.9, 0.5, 1.25):
+        if solver == "batch":
+            import torch
+
+            bt = capi.Batch(ctx, [A], [1], **kw)
+            B = torch.tensor(bt.pack([b[:, None]]), device="cuda:0")
+
+            def solve(w):
+                X = torch.zeros_like(B)
+                bt.mcsa_solve_dev(B.data_ptr(), X.data_ptr(), tolerance=0.0, max_iters=5,
+                                  richardson_omega=w)
+                return X.cpu().numpy()
+        else:
+            dom = capi.Domain(ctx, op, pc, **kw)
+
+            def solve(w):
+                p = dict(tolerance=0.0, max_iters=5, richardson_omega=w)
+                return (dom.mcsa_solve(b, **p) if solver == "mcsa" else
+                        dom.mcsa_solve_sets(one, b, **p))[0]
+        solve(first)  # every domain is then at the same histories
+        out.append(solve(near))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[2], out[1])
