@@ -1482,18 +1482,14 @@ int mclsgpu_domain_set_launch(mclsgpu_domain* dom, int histories_per_lane, int b
     dom->walk_ilp = histories_per_lane;
     dom->walk_block = block_size;
     prepare_walk(dom);
-    dom->graph_key = LoopKey{};  // the launch shape is baked into the captured loop
+    drop_loops(dom);  // the launch shape is baked into them
     return MCLSGPU_OK;
 }
 
 int mclsgpu_domain_set_record_cache(mclsgpu_domain* dom, int allocate_l1) {
     if (!dom || (allocate_l1 != 0 && allocate_l1 != 1)) return MCLSGPU_ERR_INVALID_ARG;
     dom->walk_l1 = allocate_l1;
-    dom->graph_key = LoopKey{};  // baked into the captured loop
-    if (dom->set_graph) {
-        cudaGraphExecDestroy(dom->set_graph);
-        dom->set_graph = nullptr;
-    }
+    drop_loops(dom);  // baked into them
     return MCLSGPU_OK;
 }
 

@@ -25,6 +25,16 @@ def test_the_history_of_a_live_domain_is_replaced_in_one_place():
     assert body.index("drop_loops(dom)") < body.index("dfree(dom->d_resid)")
 
 
+@pytest.mark.parametrize("function", ["mcsa.cu:mclsgpu_domain_set_launch",
+                                      "mcsa.cu:mclsgpu_domain_set_record_cache",
+                                      "capi.cu:mclsgpu_domain_reseed"])
+def test_a_setting_baked_into_the_walks_drops_every_loop(function):
+    # The launch shape changes no result, so the loops themselves cannot show it.
+    name, fn = function.split(":")
+    body = open(os.path.join(CSRC, name)).read().split("int " + fn + "(")[1].split("\n}")[0]
+    assert "drop_loops(dom)" in body
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("order", [("sets", "mcsa", "sets"), ("sets", "anderson", "sets"),
                                    ("mcsa", "anderson", "mcsa"), ("anderson", "mcsa", "anderson"),
@@ -52,6 +62,32 @@ def test_solvers_in_turn_with_growing_iteration_limits(ctx, order):
         out.append([solve(dom, w, n, host) for w, n in zip(order, (5, 60, 20))])
     for x, y in zip(*out):
         assert np.isfinite(x).all() and np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["mcsa", "sets", "anderson"])
+def test_settings_between_solves(ctx, solver):
+    A, b = P.diffusion3d_varcoef(21, seed=3)  # 9261 rows: walks from global memory
+    op = capi.Operator(ctx, A)
+    pc = capi.Precond(ctx, op, capi.PREC_POINT_JACOBI)
+    one = capi.set_params(1, lambda ptr, n, stream: None, capturable=True)
+    out = []
+    for change in (False, True):
+        dom = capi.Domain(ctx, op, pc, precision=capi.FP32, direction=capi.FORWARD,
+                          estimator=capi.EXPECTED_VALUE, sample_ratio=2.0, seed=2)
+        for blk, l1 in ((256, 0), (128, 0), (128, 1), (256, 1)):
+            if change:
+                dom.set_launch(1, blk)
+                dom.set_record_cache(l1)
+            if solver == "anderson":
+                x = dom.anderson_solve(b, tolerance=0.0, max_iters=4)[0]
+            elif solver == "mcsa":
+                x = dom.mcsa_solve(b, tolerance=0.0, max_iters=4)[0]
+            else:
+                x = dom.mcsa_solve_sets(one, b, tolerance=0.0, max_iters=4)[0]
+            out.append(x)
+    for x, y in zip(out[:4], out[4:]):
+        assert np.array_equal(x, y)
 
 
 @pytest.mark.gpu
