@@ -977,6 +977,13 @@ int mclsgpu_anderson_apply(mclsgpu_domain* dom, const double* delta_dev, double 
                          "mclsgpu_anderson_correction first");
     AndersonWork* w = dom->aa;
     cudaStream_t s = dom->ctx->stream;
+    if (reinterpret_cast<uintptr_t>(delta_dev) & 15) {
+        // The passes read pairs of entries: a vector that starts at an odd one
+        // goes through the work space's own.
+        cudaMemcpyAsync(w->delta, delta_dev, size_t(dom->n) * sizeof(double),
+                        cudaMemcpyDeviceToDevice, s);
+        delta_dev = w->delta;
+    }
     enqueue_accel(dom, &w->step_p, w->step_f, delta_dev, scale, cudaGraphConditionalHandle(0), 0,
                   false);
     w->step_f = nullptr;
