@@ -296,7 +296,7 @@ struct SpaiFwdArgs {
     double* mdia;          // M by diagonal offsets, 0 off the pattern (may be null)
     unsigned short* mask;  // with mdia: bit s = slot s is on the pattern
     float* out;            // raw outputs [n][16] (may be null)
-    int out_align32;       // out is 32-byte aligned
+    int out_align;         // alignment of out, bytes: 32, 16 or its elements' 4
     int* status;
 };
 
@@ -512,18 +512,21 @@ __global__ void __launch_bounds__(kThreads, kFwdCtas) k_spai_forward(SpaiFwdArgs
         for (int k = 0; k < kO; ++k) o[k] += bias[2 * kH + k];
         if (a.out && row < a.n) {
             float* dst = a.out + size_t(row) * kO;
-            if (a.out_align32) {
+            if (a.out_align == 32) {
 #pragma unroll
                 for (int k = 0; k < kO; k += 8)
                     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + k),
                                  "f"(o[k]), "f"(o[k + 1]), "f"(o[k + 2]), "f"(o[k + 3]),
                                  "f"(o[k + 4]), "f"(o[k + 5]), "f"(o[k + 6]), "f"(o[k + 7])
                                  : "memory");
-            } else {
+            } else if (a.out_align == 16) {
 #pragma unroll
                 for (int k = 0; k < kO; k += 4)
                     *reinterpret_cast<float4*>(dst + k) =
                         make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < kO; ++k) dst[k] = o[k];
             }
         }
         if (a.mval) {
@@ -1107,7 +1110,8 @@ int launch_forward(mclsgpu_spai* net, mclsgpu_operator* op, const SlotTable& t, 
     a.mdia = mdia;
     a.mask = mask;
     a.out = out;
-    a.out_align32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(out);
+    a.out_align = at % 32 == 0 ? 32 : at % 16 == 0 ? 16 : 4;
     a.status = ctx->d_status;
     const int ntiles = (op->A.n + kTileRows - 1) / kTileRows;
     const int fit = ctx->num_sms * kFwdCtas;

@@ -39,3 +39,22 @@ def test_anderson_corrections_at_odd_places(ctx, n, depth):
         out.append(x.cpu().numpy())
     for x in out[1:]:
         assert np.isfinite(x).all() and np.array_equal(x, out[0])
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+def test_network_outputs_at_odd_places(ctx, dims):
+    import torch
+
+    A = P.poisson2d(12, 7) if dims == 2 else P.diffusion3d_varcoef(9, seed=1)[0]
+    n = A.shape[0]
+    op = capi.Operator(ctx, A)
+    net = capi.SpaiNet(ctx, 5 if dims == 2 else 7, seed=3)
+    want, m_want = net.infer(op, A.nnz)
+    for at in (0, 1, 2, 4, 8):  # floats: aligned to 32, 4, 8, 16 and 32 bytes
+        buf = torch.zeros(16 * n + 16, dtype=torch.float32, device="cuda:0")
+        mbuf = torch.zeros(A.nnz + 2, dtype=torch.float64, device="cuda:0")
+        out, m = buf[at:at + 16 * n], mbuf[at % 2:at % 2 + A.nnz]
+        net.infer_dev(op, out.data_ptr(), m.data_ptr())
+        assert np.array_equal(out.cpu().numpy().reshape(n, 16), want)
+        assert np.array_equal(m.cpu().numpy(), m_want)
+        assert not buf[:at].any() and not buf[at + 16 * n:].any()
