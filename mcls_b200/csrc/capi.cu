@@ -55,6 +55,7 @@ int status_error(mclsgpu_context* ctx, int st) {
 }
 
 void prepare_walk(mclsgpu_domain* dom);
+void prepare_walk_lanes(mclsgpu_domain* dom);
 int prepare_walk_order(mclsgpu_domain* dom);
 int walk_agreement(mclsgpu_domain* dom, long long histories, uint64_t seed, long long* hist_diff,
                    long long* trans_diff);
@@ -583,6 +584,7 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
         }
     }
     if (!rc) {
+        prepare_walk_lanes(dom);
         prepare_walk(dom);
         rc = prepare_walk_order(dom);
         prepare_source(dom);

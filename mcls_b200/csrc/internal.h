@@ -173,6 +173,7 @@ struct RowFinish {
     int ev = 0;
     int base = kBaseNone;
     int hlog = 0;               // log2 of the lanes that share a row
+    int split = 1;              // such groups of lanes per row; > 1: they tally
     const int* order = nullptr; // position -> row (null: the identity)
 };
 
@@ -214,9 +215,10 @@ struct mclsgpu_domain {
     int walk_ilp = 1;
     int walk_block = 256;
     int walk_l1 = 0;               // record loads allocated in L1
-    // Forward fixed-length walks: log2 of the lanes that share a row, and the
-    // order the rows are taken in (null: ascending).
+    // Forward fixed-length walks: log2 of the lanes that share a row, the groups
+    // of lanes per row, and the order the rows are taken in (null: ascending).
     int walk_hlog = 0;
+    int walk_split = 1;
     int* walk_order = nullptr;
     int neg_h = 1;                 // some entry of H is negative
     // Stencil records (stencil_k > 0): row r's slot j is column r + stencil_off[j].
@@ -459,11 +461,15 @@ void launch_forward_setup(mclsgpu_domain* dom);
 inline bool walk_needs_rounds(const mclsgpu_domain* dom) {
     return dom->p.rng_mode == MCLSGPU_RNG_REFERENCE && dom->p.weight_cutoff > 0.0;
 }
-// True when the walk kernel itself finishes the estimate (RowFinish): forward
-// fixed-length FP32 walks.  The others leave tallies in y64.
-inline bool walk_finishes(const mclsgpu_domain* dom) {
+// Forward fixed-length FP32 walks, one group of lanes or more per row.
+inline bool walks_rows(const mclsgpu_domain* dom) {
     return dom->p.precision == MCLSGPU_FP32 && dom->p.direction == MCLSGPU_FORWARD &&
            !(dom->p.weight_cutoff > 0.0);
+}
+// True when the walk kernel itself finishes the estimate (RowFinish).  The
+// others leave tallies in y64.
+inline bool walk_finishes(const mclsgpu_domain* dom) {
+    return walks_rows(dom) && dom->walk_split == 1;
 }
 // Clears the device status and the walk statistics (one kernel).
 void mcsa_solve_begin(mclsgpu_domain* dom);

@@ -23,6 +23,7 @@
 // walk64: the parity kernel.  FP64 domain, std::lower_bound's selection, FP64
 // weights and tallies, optional trajectory trace.  With the reference stream it
 // reproduces the reference's trajectories bit for bit.
+#include <algorithm>
 #include <climits>
 
 #include "internal.h"
@@ -398,15 +399,15 @@ struct RecordCopy {
 // out = [base +] sum / per [+ source], so a row's sum needs no atomics, no
 // cleared tally and no pass of its own.  The histories are assigned
 // statically: they all take the same number of steps, and a work queue costs
-// one contended atomic per warp.
+// one contended atomic per warp.  The histories from m0 on in steps of `step`.
 template <int S, int ST, bool POS, int MEM>
-__device__ __forceinline__ double row_histories(const WalkArgs& a, const RowFinish& f,
+__device__ __forceinline__ double row_histories(const WalkArgs& a, int m0, int step,
                                                 const int* soff, uint64_t ekey, int row,
                                                 const RecordCopy& copy) {
     const char* rec = reinterpret_cast<const char*>(a.rec);
-    const int L = a.L, H = 1 << f.hlog;
+    const int L = a.L;
     double sum = 0.0;
-    for (int m = threadIdx.x & (H - 1); m < a.per; m += H) {
+    for (int m = m0; m < a.per; m += step) {
         int s = row, k = 0;
         float w = 1.f, acc = 0.f, comp = 0.f;
         uint64_t x = history_state(a, ekey, (long long)row * a.per + m);
@@ -458,9 +459,39 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks)
     const unsigned p = live ? pos : unsigned(a.n) - 1u;
     const int i = f.order ? f.order[p] : int(p);
     const RecordCopy none{};
-    const double sum = a.l1 ? row_histories<S, ST, POS, kCached>(a, f, s_off, s_ekey, i, none)
-                            : row_histories<S, ST, POS, kBypass>(a, f, s_off, s_ekey, i, none);
+    const int H = 1 << f.hlog, m0 = threadIdx.x & (H - 1);
+    const double sum = a.l1 ? row_histories<S, ST, POS, kCached>(a, m0, H, s_off, s_ekey, i, none)
+                            : row_histories<S, ST, POS, kBypass>(a, m0, H, s_off, s_ekey, i, none);
     finish_row(a, f, sum, i, live);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(a.d_steps, (unsigned long long)(a.n) * a.per * a.L);
+    walk_end_time(a);
+}
+
+// The same where a warp per row leaves the chip idle (few rows, many histories
+// each): f.split warps share a row and add their sums into its tally, which
+// the finalizing pass reads.
+template <int S, int ST>
+__global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks)
+    walk32_split(WalkArgs a, RowFinish f) {
+    __shared__ uint64_t s_ekey;
+    __shared__ int s_off[32];
+    stage_offsets(a.stoff, s_off);
+    if (threadIdx.x == 0) s_ekey = epoch_key(a.seed, *a.d_epoch);
+    walk_begin_time(a);
+    __syncthreads();
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int i = int(warp / unsigned(f.split));
+    if (i < a.n) {  // the same in every lane of a warp
+        const RecordCopy none{};
+        const int lane = threadIdx.x & 31, m0 = int(warp % unsigned(f.split)) * 32 + lane;
+        const int step = 32 * f.split;
+        double sum =
+            a.l1 ? row_histories<S, ST, false, kCached>(a, m0, step, s_off, s_ekey, i, none)
+                 : row_histories<S, ST, false, kBypass>(a, m0, step, s_off, s_ekey, i, none);
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
+        if (lane == 0) atomicAdd(&a.y64[i], sum);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(a.d_steps, (unsigned long long)(a.n) * a.per * a.L);
     walk_end_time(a);
@@ -565,7 +596,9 @@ __global__ void __launch_bounds__(kSmallBlock) walk32_small(WalkArgs a, RowFinis
         const unsigned pos = at >> f.hlog;
         const bool live = pos < unsigned(a.n);
         const int i = int(live ? pos : unsigned(a.n) - 1u);
-        const double sum = row_histories<S, ST, POS, kShared>(a, f, s_off, s_ekey, i, copy);
+        const int H = 1 << f.hlog;
+        const double sum = row_histories<S, ST, POS, kShared>(a, int(threadIdx.x) & (H - 1), H,
+                                                              s_off, s_ekey, i, copy);
         finish_row(a, f, sum, i, live);
         histories = (unsigned long long)a.n * a.per;
     } else {
@@ -744,6 +777,11 @@ template <int S, int ST, bool POS>
 void launch_rows(const WalkLaunch& l) {
     const mclsgpu_domain* d = l.dom;
     const int T = d->walk_block;
+    if (l.fin.split > 1) {
+        const long long threads = ((long long)d->n * l.fin.split) << 5;
+        walk32_split<S, ST><<<int((threads + T - 1) / T), T, 0, d->ctx->stream>>>(l.a, l.fin);
+        return;
+    }
     const long long threads = (long long)d->n << l.fin.hlog;
     walk32_rows<S, ST, POS><<<int((threads + T - 1) / T), T, 0, d->ctx->stream>>>(l.a, l.fin);
 }
@@ -778,7 +816,7 @@ void launch_small(const WalkLaunch& l) {
 // slower.
 template <int S>
 bool small_walk(const mclsgpu_domain* d) {
-    if (S > 16 || (long long)d->n * S * 8 > kSmallRecords) return false;
+    if (S > 16 || (long long)d->n * S * 8 > kSmallRecords || d->walk_split > 1) return false;
     const long long threads = d->p.direction == MCLSGPU_FORWARD
                                   ? (long long)d->n << d->walk_hlog
                                   : (long long)d->nh_cap;
@@ -883,11 +921,27 @@ __global__ void k_fill_order(RowOrder o, int n, int* order) {
 
 }  // namespace
 
+// How a row's histories are shared out (set-up time).  Up to four lanes when
+// they get the same number; where the chip would not be full, as many as there
+// are histories, up to a warp, then several warps that tally.  A lane's
+// histories follow one another: 8 iterations on 32^2 rows with 1,000 histories
+// each take 439 us, with four lanes a row at most 2,430; 101 on the same rows 233
+// and 1,127; 33 on 100^2 rows 310 and 890; 4,000 on 10^2 rows 563 and 8,900.
+void prepare_walk_lanes(mclsgpu_domain* dom) {
+    if (!walks_rows(dom)) return;
+    const int per = dom->p.sample_ratio > 0.0 ? int(ceil(dom->p.sample_ratio)) : 1;
+    int hlog = per % 4 == 0 ? 2 : per % 2 == 0 ? 1 : 0;
+    const long long fit = (long long)dom->ctx->num_sms * 2048, n = dom->n;
+    while (hlog < 5 && (1 << hlog) < per && (n << (hlog + 1)) <= fit) ++hlog;
+    dom->walk_hlog = hlog;
+    const long long most = std::min(fit / (n << 5), (long long)(per + 31) / 32);
+    dom->walk_split = hlog == 5 && most > 1 ? int(most) : 1;
+}
+
 // The row order of the forward walk (set-up time).
 int prepare_walk_order(mclsgpu_domain* dom) {
-    if (!walk_finishes(dom)) return MCLSGPU_OK;
-    const int per = dom->p.sample_ratio > 0.0 ? int(ceil(dom->p.sample_ratio)) : 1;
-    dom->walk_hlog = per % 4 == 0 ? 2 : per % 2 == 0 ? 1 : 0;
+    // More lanes than four share a row only where there are few of them.
+    if (!walk_finishes(dom) || dom->walk_hlog > 2) return MCLSGPU_OK;
     const RowOrder o = row_order(dom->n, dom->op->dia_k, dom->op->dia_off, 32 >> dom->walk_hlog);
     if (o.X <= 1) return MCLSGPU_OK;
     cudaError_t e = dmalloc(&dom->walk_order, size_t(dom->n));
@@ -1281,6 +1335,7 @@ void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
             cudaMemsetAsync(dom->d_counter, 0, sizeof(int), st);
         WalkLaunch l{dom, a, fin, true};
         l.fin.hlog = dom->walk_hlog;
+        l.fin.split = dom->walk_split;
         l.fin.order = dom->walk_order;
         dispatch_walk32(l);
     } else {
