@@ -56,7 +56,7 @@ int status_error(mclsgpu_context* ctx, int st) {
 
 void prepare_walk(mclsgpu_domain* dom);
 void prepare_walk_lanes(mclsgpu_domain* dom);
-int prepare_walk_order(mclsgpu_domain* dom);
+void prepare_walk_order(mclsgpu_domain* dom);
 int walk_agreement(mclsgpu_domain* dom, long long histories, uint64_t seed, long long* hist_diff,
                    long long* trans_diff);
 void prepare_source(mclsgpu_domain* dom);
@@ -586,10 +586,10 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
     if (!rc) {
         prepare_walk_lanes(dom);
         prepare_walk(dom);
-        rc = prepare_walk_order(dom);
+        prepare_walk_order(dom);
         prepare_source(dom);
         e = cudaStreamSynchronize(ctx->stream);
-        if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "domain build");
+        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "domain build");
     }
     if (rc) {
         release_domain(dom);

@@ -814,9 +814,10 @@ void launch_small(const WalkLaunch& l) {
 // per SM.  MCSA solves of 24^2 to 80^2 grids take 5 to 9 % less time than from
 // global memory, adjoint ones 4 to 6 %; nothing on this side of the line is
 // slower.
-template <int S>
 bool small_walk(const mclsgpu_domain* d) {
-    if (S > 16 || (long long)d->n * S * 8 > kSmallRecords || d->walk_split > 1) return false;
+    if (d->p.weight_cutoff > 0.0 || d->slots > 16 || d->walk_split > 1 ||
+        (long long)d->n * d->slots * 8 > kSmallRecords)
+        return false;
     const long long threads = d->p.direction == MCLSGPU_FORWARD
                                   ? (long long)d->n << d->walk_hlog
                                   : (long long)d->nh_cap;
@@ -827,7 +828,7 @@ template <int S, int ST, bool POS>
 void launch32_fixed(const WalkLaunch& l) {
     const mclsgpu_domain* d = l.dom;
     if constexpr (S <= 16)
-        if (small_walk<S>(d)) {
+        if (small_walk(d)) {
             if (d->p.direction == MCLSGPU_ADJOINT)
                 return launch_small<S, ST, POS, MCLSGPU_ADJOINT>(l);
             return launch_small<S, ST, POS, MCLSGPU_FORWARD>(l);
@@ -938,18 +939,21 @@ void prepare_walk_lanes(mclsgpu_domain* dom) {
     dom->walk_split = hlog == 5 && most > 1 ? int(most) : 1;
 }
 
-// The row order of the forward walk (set-up time).
-int prepare_walk_order(mclsgpu_domain* dom) {
-    // More lanes than four share a row only where there are few of them.
-    if (!walk_finishes(dom) || dom->walk_hlog > 2) return MCLSGPU_OK;
+// The row order of the forward walk (set-up time).  Records in shared memory are
+// walked in any order, and more lanes than four share a row only where there are
+// few rows.  Without the memory for it the walk takes the rows as they come.
+void prepare_walk_order(mclsgpu_domain* dom) {
+    if (!walk_finishes(dom) || dom->walk_hlog > 2 || small_walk(dom)) return;
     const RowOrder o = row_order(dom->n, dom->op->dia_k, dom->op->dia_off, 32 >> dom->walk_hlog);
-    if (o.X <= 1) return MCLSGPU_OK;
-    cudaError_t e = dmalloc(&dom->walk_order, size_t(dom->n));
-    if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "cudaMalloc walk order");
+    if (o.X <= 1) return;
+    if (dmalloc(&dom->walk_order, size_t(dom->n)) != cudaSuccess) {
+        cudaGetLastError();
+        dom->walk_order = nullptr;
+        return;
+    }
     const int grid = (dom->n + 255) / 256;
     k_fill_order<<<grid < 2368 ? grid : 2368, 256, 0, dom->ctx->stream>>>(o, dom->n,
                                                                         dom->walk_order);
-    return MCLSGPU_OK;
 }
 
 // Cache the occupancy of the walk kernel this domain will launch (set-up time,

@@ -69,3 +69,19 @@ def test_loops_with_many_histories(ctx, n, per):
             r = (b - A @ x) / A.diagonal()
             assert np.linalg.norm(r) <= 1.0001e-9 * np.linalg.norm(b) * max(
                 1.0, (1 / A.diagonal()).max())
+
+
+@pytest.mark.parametrize("n,order", [(24, 0), (80, 0), (90, 1), (200, 1)])
+def test_small_domains_hold_no_row_order(ctx, n, order):
+    # 80^2 records of 32 bytes are the last to fit a block's shared memory, where
+    # rows are taken as they come.  A domain of histories ended by a weight
+    # cutoff never has an order and allocates the same otherwise.
+    op = capi.Operator(ctx, P.poisson2d(n) / 4.0)
+    count = []
+    for cutoff in (0.0, 1e-3):
+        before = capi.device_allocations()[0]
+        dom = capi.Domain(ctx, op, None, precision=capi.FP32, direction=capi.FORWARD,
+                          estimator=capi.COLLISION, sample_ratio=1.0, weight_cutoff=cutoff)
+        count.append(capi.device_allocations()[0] - before)
+        dom.close()
+    assert count[0] - count[1] == order
