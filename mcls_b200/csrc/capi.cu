@@ -584,6 +584,7 @@ int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op, mclsgpu_pre
         }
     }
     if (!rc) {
+        pack_records64(dom);
         prepare_walk_lanes(dom);
         prepare_walk(dom);
         prepare_walk_order(dom);

@@ -264,6 +264,21 @@ RowOrder row_order(int n, int K, const int* off, int rows) {
     return o;
 }
 
+// FP64 records where the rows are short enough.  The walk can do without them
+// (it then reads the CSR domain), so they are allocated after everything that a
+// domain must have, and a domain that fits memory without them is built.
+void pack_records64(mclsgpu_domain* dom) {
+    const int n = dom->n;
+    if (dom->p.precision != MCLSGPU_FP64 || dom->max_row > Record64::kEntries) return;
+    if (dmalloc(&dom->rec64, size_t(n)) != cudaSuccess) {
+        cudaGetLastError();
+        dom->rec64 = nullptr;
+        return;
+    }
+    k_pack_records64<<<grid_for(n), 256, 0, dom->ctx->stream>>>(
+        dom->D.rp, dom->D.ci, dom->D.v, dom->cdf, dom->w, n, dom->rec64);
+}
+
 // Build the FP64 domain arrays and FP32 records from the composite M.
 int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
                         mclsgpu_domain* dom, int row0) {
@@ -310,15 +325,6 @@ int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "domain fill");
     if ((rc = check_device_status(ctx))) return rc;
-
-    if (dom->p.precision == MCLSGPU_FP64 && hmax <= Record64::kEntries) {
-        // Without the memory for them the walk reads the CSR domain.
-        if (dmalloc(&dom->rec64, n) == cudaSuccess)
-            k_pack_records64<<<grid_for(n), 256, 0, s>>>(D.rp, D.ci, D.v, dom->cdf, dom->w, n,
-                                                         dom->rec64);
-        else
-            cudaGetLastError();
-    }
 
     // FP32 records, packed format: slot count = 1 + longest row, rounded up to
     // a supported stride.

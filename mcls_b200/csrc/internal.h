@@ -364,6 +364,7 @@ int exclusive_scan_counts_dev(mclsgpu_context* ctx, const int* d_cnt, int n, int
 // domain; its columns are global).
 int build_domain_arrays(mclsgpu_context* ctx, const DevCsr& M, double relax,
                         mclsgpu_domain* dom, int row0 = 0);
+void pack_records64(mclsgpu_domain* dom);
 
 // Releases the domain's captured Anderson loop (rebuilt on the next solve).
 void anderson_drop_graph(mclsgpu_domain* dom);
