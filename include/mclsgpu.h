@@ -335,12 +335,14 @@ int mclsgpu_domain_query(mclsgpu_domain* dom, mclsgpu_domain_info* info);
 /* FP32 walk launch shape: histories carried per lane (1, 2, 4 or 8) and threads
  * per block (128 or 256).  Adjoint fixed-length histories use up to 2 per lane
  * on records of at most 64 bytes and up to 4 on 32-byte records; forward
- * histories and those ended by a weight cutoff walk one per lane (the latter
- * in blocks of 256).  No counterpart in the reference. */
+ * histories and those ended by a weight cutoff walk one per lane.  Fixed-length
+ * walks of a domain whose records fit a block's shared memory (200 KB, no more
+ * than 128 histories per SM) have one shape.  No counterpart in the reference. */
 int mclsgpu_domain_set_launch(mclsgpu_domain* dom, int histories_per_lane,
                               int block_size);
 /* Record loads of the FP32 walk allocated in L1 (1) or bypassing it (0, the
- * default).  No counterpart in the reference. */
+ * default); walks from shared memory (see above) and batched walks have no such
+ * loads.  No counterpart in the reference. */
 int mclsgpu_domain_set_record_cache(mclsgpu_domain* dom, int allocate_l1);
 /* Autotuner: times the domain's launch shapes on `reps` Monte Carlo solves of the
  * device vector rhs_dev (n entries), with the record loads bypassing and

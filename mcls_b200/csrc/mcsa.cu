@@ -44,6 +44,7 @@ void launch_forward_source(mclsgpu_domain* dom, const double* v, double omega, i
                            bool fused);
 void launch_advance_walk_pos(mclsgpu_domain* dom);
 void prepare_walk(mclsgpu_domain* dom);
+bool walks_from_shared(const mclsgpu_domain* dom);
 void launch_walk(mclsgpu_domain* dom, const RowFinish& fin, long long max_trace,
                  long long* tr_states, double* tr_w, int* tr_ev, long long* tr_start, bool fused);
 
@@ -1489,6 +1490,7 @@ int mclsgpu_domain_set_launch(mclsgpu_domain* dom, int histories_per_lane, int b
 int mclsgpu_domain_set_record_cache(mclsgpu_domain* dom, int allocate_l1) {
     if (!dom || (allocate_l1 != 0 && allocate_l1 != 1)) return MCLSGPU_ERR_INVALID_ARG;
     dom->walk_l1 = allocate_l1;
+    prepare_walk(dom);
     drop_loops(dom);  // baked into them
     return MCLSGPU_OK;
 }
@@ -1504,19 +1506,18 @@ int mclsgpu_domain_autotune(mclsgpu_domain* dom, const double* rhs_dev, int reps
     cudaMemcpyAsync(&saved[1], dom->d_pos, sizeof(saved[1]), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(dom->ctx, e, "autotune");
-    // The shapes that differ for this domain: forward fixed-length histories
-    // walk one per lane, those ended by a cutoff have one shape, and four per
-    // lane apply to 32-byte records only.  Each with the record loads
+    // The shapes that differ for this domain: records in shared memory have one;
+    // forward histories and those ended by a cutoff walk one per lane, and four
+    // per lane apply to 32-byte records only.  Each with the record loads
     // bypassing L1 and allocated in it.
     const bool fixed = !(dom->p.weight_cutoff > 0.0);
     const bool adjoint = dom->p.direction == MCLSGPU_ADJOINT;
     const int most = !fixed || !adjoint ? 1 : dom->slots == 4 ? 4 : dom->slots == 8 ? 2 : 1;
     std::vector<std::array<int, 3>> shapes;
-    for (int l1 = 0; l1 < (fixed ? 2 : 1); ++l1)
-        for (int h = 1; h <= most; h *= 2) {
-            shapes.push_back({h, 256, l1});
-            if (fixed) shapes.push_back({h, 128, l1});
-        }
+    for (int l1 = 0; l1 < 2; ++l1)
+        for (int h = 1; h <= most; h *= 2)
+            for (int block : {256, 128}) shapes.push_back({h, block, l1});
+    if (walks_from_shared(dom)) shapes.resize(1);
     double best = 1e300;
     int bh = 1, bb = 256, bl = 0;
     for (const auto& sh : shapes) {

@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(kSmallBlock) walk32_small(WalkArgs a, RowFinis
 
 // Histories ended by the weight cutoff: persistent warps whose lanes refill
 // one by one from the work queue as their histories terminate.
-template <int S, int DIR, int ST>
+template <int S, int DIR, int ST, int MEM>
 __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks) walk32_cutoff(WalkArgs a) {
     static_assert(S % 4 == 0, "records are whole 32-byte halves");
     __shared__ uint64_t s_ekey;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(256, WalkOccupancy<S, ST>::kMinBlocks) walk32_
         }
         if (!__any_sync(kFull, alive)) break;
         if (alive) {
-            walk_step<S, DIR, ST, kBypass>(rec, a.y64, s_off, s, w, x, acc, comp, k);
+            walk_step<S, DIR, ST, MEM>(rec, a.y64, s_off, s, w, x, acc, comp, k);
             ++k;
             ++steps;
             if (k >= a.L || fabsf(w) < wcut) {
@@ -754,16 +754,17 @@ __global__ void __launch_bounds__(128) walk64(WalkArgs a) {
     if ((threadIdx.x & 31) == 0 && steps) atomicAdd(a.d_steps, steps);
 }
 
-// Resident 256-thread blocks per SM of a cutoff walk (a persistent grid).
-template <int S, int DIR, int ST>
-int cutoff_blocks_per_sm() {
-    static int cached = 0;
-    if (!cached) {
+// Resident blocks per SM of a cutoff walk (a persistent grid).
+template <int S, int DIR, int ST, int MEM>
+int cutoff_blocks_per_sm(int block) {
+    static int cached[2] = {0, 0};
+    int& c = cached[block == 128 ? 0 : 1];
+    if (!c) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32_cutoff<S, DIR, ST>, 256, 0);
-        cached = b > 0 ? b : 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, walk32_cutoff<S, DIR, ST, MEM>, block, 0);
+        c = b > 0 ? b : 1;
     }
-    return cached;
+    return c;
 }
 
 struct WalkLaunch {
@@ -847,24 +848,27 @@ void launch32_fixed(const WalkLaunch& l) {
     launch_rows<S, ST, POS>(l);
 }
 
+template <int S, int DIR, int ST, int MEM>
+void launch_cutoff(const WalkLaunch& l) {
+    const mclsgpu_domain* d = l.dom;
+    const int T = d->walk_block;
+    const long long fit =
+        (long long)d->ctx->num_sms * cutoff_blocks_per_sm<S, DIR, ST, MEM>(T);
+    if (!l.launch) return;
+    // No more blocks than the histories need, at most what fits at once.
+    const long long need = std::max((d->nh_cap + T - 1) / T, int64_t(1));
+    walk32_cutoff<S, DIR, ST, MEM><<<int(std::min(need, fit)), T, 0, d->ctx->stream>>>(l.a);
+}
+
 template <int S, int ST>
 void launch32_case(const WalkLaunch& l) {
     const mclsgpu_domain* d = l.dom;
     if (d->p.weight_cutoff > 0.0) {
-        // No more blocks than the histories need, at most what fits at once.
-        long long need = (d->nh_cap + 255) / 256;
-        if (need < 1) need = 1;
-        const bool adj = d->p.direction == MCLSGPU_ADJOINT;
-        const long long fit = (long long)d->ctx->num_sms *
-                              (adj ? cutoff_blocks_per_sm<S, MCLSGPU_ADJOINT, ST>()
-                                   : cutoff_blocks_per_sm<S, MCLSGPU_FORWARD, ST>());
-        if (!l.launch) return;
-        const int grid = int(need < fit ? need : fit);
-        if (adj)
-            walk32_cutoff<S, MCLSGPU_ADJOINT, ST><<<grid, 256, 0, d->ctx->stream>>>(l.a);
-        else
-            walk32_cutoff<S, MCLSGPU_FORWARD, ST><<<grid, 256, 0, d->ctx->stream>>>(l.a);
-        return;
+        if (d->p.direction == MCLSGPU_ADJOINT)
+            return d->walk_l1 ? launch_cutoff<S, MCLSGPU_ADJOINT, ST, kCached>(l)
+                              : launch_cutoff<S, MCLSGPU_ADJOINT, ST, kBypass>(l);
+        return d->walk_l1 ? launch_cutoff<S, MCLSGPU_FORWARD, ST, kCached>(l)
+                          : launch_cutoff<S, MCLSGPU_FORWARD, ST, kBypass>(l);
     }
     if constexpr (ST == kStencil)
         if (!d->neg_h) return launch32_fixed<S, ST, true>(l);
@@ -921,6 +925,8 @@ __global__ void k_fill_order(RowOrder o, int n, int* order) {
 }
 
 }  // namespace
+
+bool walks_from_shared(const mclsgpu_domain* dom) { return small_walk(dom); }
 
 // How a row's histories are shared out (set-up time).  Up to four lanes when
 // they get the same number; where the chip would not be full, as many as there

@@ -85,3 +85,15 @@ def test_small_domains_hold_no_row_order(ctx, n, order):
         count.append(capi.device_allocations()[0] - before)
         dom.close()
     assert count[0] - count[1] == order
+
+
+def test_autotune_of_a_walk_with_one_shape(ctx):
+    import torch
+
+    op = capi.Operator(ctx, matrix(700))
+    dom = capi.Domain(ctx, op, None, precision=capi.FP32, direction=capi.FORWARD,
+                      estimator=capi.COLLISION, sample_ratio=1.0, seed=1)
+    v = torch.ones(700, dtype=torch.float64, device="cuda:0")
+    for _ in range(5):
+        t = dom.autotune(v.data_ptr(), reps=1)
+        assert (t["histories_per_lane"], t["block_size"], t["record_cache_l1"]) == (1, 256, 0)
