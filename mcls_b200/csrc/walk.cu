@@ -229,12 +229,15 @@ __device__ __forceinline__ void select_record64(const Record64* rec, int s, doub
     Ws = (q[23] >> (8 + lo)) & 1u ? -W : W;
 }
 
-// Slots of a record that every step reads.  Packed records longer than 64 bytes:
-// rows of an unstructured operator have 7 entries on average and 16 at most, and
-// the walk is bound by the sectors it requests, so the rest is read only by the
-// lanes whose draw lies past the seventh entry (the CDF does not fall along a
-// row and its padding holds 2.0).  With the registers this frees six blocks are
-// resident instead of four.  2 x 10^5 histories on 10^5 rows: 34.4 -> 22 us.
+// Slots of a record that every step reads.  Packed records longer than 64 bytes
+// are read in two parts: the walk is bound by the sectors it requests, so what
+// lies past the seventh entry is read only by the lanes whose draw lies there (the
+// CDF does not fall along a row and its padding holds 2.0), and with the
+// registers this frees six blocks are resident instead of four.  It gives the
+// more the fewer rows are long, and costs nothing where all are: solves of 8
+// iterations on 60,007 rows of 8, 12, 16, 24 and 30 entries each take 293, 337,
+// 398, 528 and 568 us, with whole records 323, 382, 464, 567 and 572; 2 x 10^5
+// histories on 10^5 rows of 7 entries on average and 16 at most 22 and 34.4 us.
 template <int S, int ST>
 constexpr int first_slots() {
     return ST == kPacked && S > 8 ? 8 : S;
