@@ -54,15 +54,22 @@ struct BatchState {
 constexpr int kThreads = 256;
 constexpr int kRowBlocks = 3;  // blocks per SM of the row passes (their registers)
 
-// Rows of fixed width for the element passes, entry-major: entry k of row i at
-// k * n + i, columns ascending; padding entries repeat the row's own index with
-// value 0.  The width is the longest row's, rounded up to kRowChunk.
+// Rows for the element passes: the first 8 entries at a fixed width, entry-major
+// (entry k of row i at k * n + i, columns ascending; padding entries repeat the
+// row's own index with value 0), the others from the CSR rows they came from.
+// Only systems with longer rows look for those, so neither the time nor the
+// memory of a system depends on the rows of another.  10 iterations on 64
+// systems: 1,545 us on 5- and 7-point ones, 1,733 with a 9-point one among them
+// and 1,952 on 9-point ones; at the width of the longest row of all, read entry
+// by entry past the eighth, 3,348 and 3,385.
 constexpr int kRowChunk = 8;
 struct BatchRows {
     int n = 0;
-    int chunks = 0;      // width / kRowChunk
     int* col = nullptr;
     double* val = nullptr;
+    const int* rp = nullptr;
+    const int* ci = nullptr;
+    const double* v = nullptr;
 };
 
 struct BatchArgs {
@@ -76,6 +83,7 @@ struct BatchArgs {
     const int* srow0;
     const long long* seoff;
     const int* slog;
+    const int* slong;    // some row has more than kRowChunk entries
     const int* sn;
     const int* sorder;   // the systems in placement order
     // The systems this launch works on: lsys[k] for k < *lcount, their tiles of
@@ -125,6 +133,7 @@ __host__ __device__ constexpr long long system_tiles(int n, int c) {
 // of its first column inside the system's elements.
 struct Unit {
     int s, c, row0, i, g;
+    int tail;          // the system's rows may go on past kRowChunk entries
     unsigned col0;     // g * unit_cols(c)
     long long eoff;
     __device__ __forceinline__ size_t elem() const {
@@ -167,6 +176,7 @@ __device__ __forceinline__ void for_tiles(const BatchArgs& a, Enter enter, Body 
             ++k;
             q.s = a.lsys[k];
             q.c = a.slog[q.s];
+            q.tail = a.slong[q.s];
             q.row0 = a.srow0[q.s];
             q.eoff = a.seoff[q.s];
             units = a.sn[q.s] << unit_log(q.c);
@@ -228,15 +238,25 @@ struct Ahead {
     }
 };
 
+// Entries past the fixed width that are loaded at a time.
+constexpr int kTail = 4;
+
 // The unit's row of M times the columns of x, entries in ascending column
-// order; `next`: the row whose indices to load into h meanwhile (or -1).
-template <int N>
+// order; `next`: the row whose indices to load into h meanwhile (or -1).  TAIL:
+// some system has rows that go on past the fixed width (in batches without one the
+// look for them costs 3 %).
+template <int N, bool TAIL>
 __device__ __forceinline__ Cols<N> row_times(const BatchRows& M, const Unit& q, const double* x,
                                              Ahead& h, int next) {
     const double* xs = x + q.eoff + q.col0;
     Cols<N> acc;
 #pragma unroll
     for (int n = 0; n < N; ++n) acc.v[n] = 0.0;
+    int p = 0, end = 0;
+    if (TAIL && q.tail) {
+        p = M.rp[q.i] + kRowChunk;
+        end = M.rp[q.i + 1];
+    }
     Cols<N> xv[kRowChunk];
     double val[kRowChunk];
 #pragma unroll
@@ -251,12 +271,25 @@ __device__ __forceinline__ Cols<N> row_times(const BatchRows& M, const Unit& q, 
         for (int n = 0; n < N; ++n) acc.v[n] = fma(val[m], xv[m].v[n], acc.v[n]);
     }
 #pragma unroll 1
-    for (int k = kRowChunk; k < M.chunks * kRowChunk; ++k) {
-        const int col = M.col[size_t(k) * M.n + q.i];
-        const Cols<N> xk = ldn<N>(xs + (size_t(unsigned(col - q.row0)) << q.c));
-        const double v = M.val[size_t(k) * M.n + q.i];
+    for (; TAIL && p < end; p += kTail) {
+        int col[kTail];
+        double v[kTail];
 #pragma unroll
-        for (int n = 0; n < N; ++n) acc.v[n] = fma(v, xk.v[n], acc.v[n]);
+        for (int t = 0; t < kTail; ++t) {  // past the end: the last entry again, not added
+            const int at = min(p + t, end - 1);
+            col[t] = M.ci[at];
+            v[t] = M.v[at];
+        }
+        Cols<N> xk[kTail];
+#pragma unroll
+        for (int t = 0; t < kTail; ++t)
+            xk[t] = ldn<N>(xs + (size_t(unsigned(col[t] - q.row0)) << q.c));
+#pragma unroll
+        for (int t = 0; t < kTail; ++t)
+            if (p + t < end) {
+#pragma unroll
+                for (int n = 0; n < N; ++n) acc.v[n] = fma(v[t], xk[t].v[n], acc.v[n]);
+            }
     }
     return acc;
 }
@@ -265,6 +298,7 @@ __device__ __forceinline__ Cols<N> row_times(const BatchRows& M, const Unit& q, 
 // doOneIteration then updatePrecResidual, src/MCLS_RichardsonIteration_impl.hpp:
 // 134-147); Y (not null: the walk adds into it) is cleared for this
 // iteration's walk.
+template <bool TAIL>
 __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_smoothed_residual(BatchArgs a) {
     Ahead h;
     auto enter = [&](const Unit&, bool live, int i) {
@@ -277,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_smoothed_residual(Ba
             constexpr int N = decltype(nt)::value;
             const Cols<N> bv = ldn<N>(a.B + e);
             const double di = a.dinv[q.i];
-            Cols<N> t = row_times<N>(a.S, q, a.X2, h, next);
+            Cols<N> t = row_times<N, TAIL>(a.S, q, a.X2, h, next);
 #pragma unroll
             for (int n = 0; n < N; ++n) t.v[n] = di * (bv.v[n] - t.v[n]);
             stn<N>(a.RP2 + e, t);
@@ -292,6 +326,7 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_smoothed_residual(Ba
 
 // Tally source of every right-hand side: expected value c = H (w rp2),
 // collision c = w rp2 (FP32).
+template <bool TAIL>
 __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_source(BatchArgs a) {
     Ahead h;
     auto enter = [&](const Unit&, bool live, int i) {
@@ -302,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_source(BatchArgs a) 
         const size_t e = q.elem();
         with_cols(q.c, [&](auto nt) {
             constexpr int N = decltype(nt)::value;
-            const Cols<N> t = a.ev ? row_times<N>(a.H, q, a.RP2, h, next)
+            const Cols<N> t = a.ev ? row_times<N, TAIL>(a.H, q, a.RP2, h, next)
                                    : ldn<N>(a.RP2 + e);
             float f[N];
 #pragma unroll
@@ -495,7 +530,7 @@ struct PairSums {
 // per-(system, rhs) sums of squares (rp itself is not kept).  CHECK: the last
 // block to finish runs the convergence test (the other blocks' sums are complete
 // and visible by then).
-template <bool CHECK>
+template <bool CHECK, bool TAIL>
 __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, int use_cond,
                                                          cudaGraphConditionalHandle handle) {
     PairSums ps{a.norm2, a.pw};
@@ -511,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, kRowBlocks) k_b_update(BatchArgs a, 
             constexpr int N = decltype(nt)::value;
             const Cols<N> bv = ldn<N>(a.B + e);
             const double di = a.dinv[q.i];
-            Cols<N> t = row_times<N>(a.S, q, a.X, h, next);
+            Cols<N> t = row_times<N, TAIL>(a.S, q, a.X, h, next);
             Cols<N> x = ldn<N>(a.X + e);
 #pragma unroll
             for (int n = 0; n < N; ++n) {
@@ -558,11 +593,11 @@ __global__ void __launch_bounds__(kThreads) k_b_init_norms(BatchArgs a) {
     ps.flush();
 }
 
-// Fixed-width rows from CSR rows of at most chunks * kRowChunk entries.
+// The fixed-width part of CSR rows.
 __global__ void k_b_rows(const int* rp, const int* ci, const double* v, BatchRows M) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
         const int p0 = rp[i], len = rp[i + 1] - p0;
-        for (int k = 0; k < M.chunks * kRowChunk; ++k) {
+        for (int k = 0; k < kRowChunk; ++k) {
             M.col[size_t(k) * M.n + i] = k < len ? ci[p0 + k] : i;
             M.val[size_t(k) * M.n + i] = k < len ? v[p0 + k] : 0.0;
         }
@@ -616,6 +651,8 @@ struct mclsgpu_batch {
     int* d_srow0 = nullptr;
     long long* d_seoff = nullptr;
     int* d_slog = nullptr;
+    int* d_slong = nullptr;
+    bool tail = false;             // some row goes on past the fixed width
     int* d_sn = nullptr;
     int* d_sorder = nullptr;
     // The active list (rebuilt every iteration) and the list of every system.
@@ -662,6 +699,7 @@ void batch_release(mclsgpu_batch* b) {
     dfree(b->d_srow0);
     dfree(b->d_seoff);
     dfree(b->d_slog);
+    dfree(b->d_slong);
     dfree(b->d_sn);
     dfree(b->d_sorder);
     dfree(b->act_sys);
@@ -687,10 +725,12 @@ void batch_release(mclsgpu_batch* b) {
     delete b;
 }
 
-int fixed_rows(mclsgpu_context* ctx, const DevCsr& A, int longest, BatchRows& M) {
+int fixed_rows(mclsgpu_context* ctx, const DevCsr& A, BatchRows& M) {
     M.n = A.n;
-    M.chunks = std::max(1, (longest + kRowChunk - 1) / kRowChunk);
-    const size_t entries = size_t(M.n) * M.chunks * kRowChunk;
+    M.rp = A.rp;
+    M.ci = A.ci;
+    M.v = A.v;
+    const size_t entries = size_t(M.n) * kRowChunk;
     cudaError_t e;
     if ((e = dmalloc(&M.col, entries)) != cudaSuccess ||
         (e = dmalloc(&M.val, entries)) != cudaSuccess)
@@ -715,6 +755,7 @@ BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) 
     a.srow0 = b->d_srow0;
     a.seoff = b->d_seoff;
     a.slog = b->d_slog;
+    a.slong = b->d_slong;
     a.sn = b->d_sn;
     a.sorder = b->d_sorder;
     a.lsys = all ? b->all_sys : b->act_sys;
@@ -761,14 +802,17 @@ int enqueue_batch_iteration(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, int
                             cudaGraphConditionalHandle handle) {
     cudaStream_t s = b->ctx->stream;
     BatchArgs a = batch_args(b, mp, false);
-    k_b_smoothed_residual<<<b->g_rich, kThreads, 0, s>>>(a);
-    k_b_source<<<b->g_src, kThreads, 0, s>>>(a);
+    auto residual = b->tail ? k_b_smoothed_residual<true> : k_b_smoothed_residual<false>;
+    auto source = b->tail ? k_b_source<true> : k_b_source<false>;
+    auto update = b->tail ? k_b_update<true, true> : k_b_update<true, false>;
+    residual<<<b->g_rich, kThreads, 0, s>>>(a);
+    source<<<b->g_src, kThreads, 0, s>>>(a);
     const BatchList list{b->act_sys, b->act_hcum, b->act_count, b->d_srow0};
     const BatchFinish fin{b->X, b->X2, b->RP2, a.nomega, a.inv_per, a.ev};
     int rc = launch_walk_batch(b->dom, b->cls, list, b->cR, b->Y, fin, b->grab);
     if (rc) return rc;
     if (b->Y) k_b_correct<<<b->g_cor, kThreads, 0, s>>>(a);
-    k_b_update<true><<<b->g_upd, kThreads, 0, s>>>(a, use_cond, handle);
+    update<<<b->g_upd, kThreads, 0, s>>>(a, use_cond, handle);
     return MCLSGPU_OK;
 }
 
@@ -913,17 +957,27 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         rc = set_error(ctx, MCLSGPU_ERR_UNSUPPORTED,
                        "batched walks: rows of at most 15 retained entries");
     // The rows of the element passes.
+    std::vector<int> slong(nsys, 0);
     int longest = 0;
-    for (int64_t i = 0; i < N; ++i) longest = std::max(longest, int(rp[i + 1] - rp[i]));
-    if (!rc) rc = fixed_rows(ctx, b->op->A, longest, b->S);
-    if (!rc) rc = fixed_rows(ctx, b->dom->D, b->dom->max_row, b->H);
+    for (int k = 0; k < nsys; ++k)
+        for (int64_t i = 0; i < n[k]; ++i) {
+            const int64_t len = rowptr[k][i + 1] - rowptr[k][i];
+            longest = std::max(longest, int(len));
+            if (len > kRowChunk) slong[k] = 1;
+        }
+    // H's rows are parts of the operator's, unless one lacks its diagonal.
+    if (!rc && b->dom->max_row > longest) std::fill(slong.begin(), slong.end(), 1);
+    b->tail = std::count(slong.begin(), slong.end(), 1) > 0;
+    if (!rc) rc = fixed_rows(ctx, b->op->A, b->S);
+    if (!rc && params->estimator == MCLSGPU_EXPECTED_VALUE) rc = fixed_rows(ctx, b->dom->D, b->H);
     const size_t PR = size_t(nsys) * pw;
     cudaError_t e = cudaSuccess;
     if (!rc &&
         ((e = dmalloc(&b->d_nrhs, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->d_srow0, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->d_seoff, nsys)) != cudaSuccess ||
-         (e = dmalloc(&b->d_slog, nsys)) != cudaSuccess || (e = dmalloc(&b->d_sn, nsys)) != cudaSuccess ||
+         (e = dmalloc(&b->d_slog, nsys)) != cudaSuccess ||
+         (e = dmalloc(&b->d_slong, nsys)) != cudaSuccess || (e = dmalloc(&b->d_sn, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->d_sorder, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->act_sys, nsys)) != cudaSuccess ||
          (e = dmalloc(&b->act_tcum, nsys + 1)) != cudaSuccess ||
@@ -944,11 +998,13 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         rc = cuda_fail(ctx, e, "cudaMalloc batch");
     if (!rc) {
         const int sms = ctx->num_sms;
-        b->g_rich = resident_grid(k_b_smoothed_residual, sms);
-        b->g_src = resident_grid(k_b_source, sms);
+        const bool tail = b->tail;
+        b->g_rich = resident_grid(
+            tail ? k_b_smoothed_residual<true> : k_b_smoothed_residual<false>, sms);
+        b->g_src = resident_grid(tail ? k_b_source<true> : k_b_source<false>, sms);
         b->g_cor = resident_grid(k_b_correct, sms);
-        b->g_upd = resident_grid(k_b_update<true>, sms);
-        b->g_upd0 = resident_grid(k_b_update<false>, sms);
+        b->g_upd = resident_grid(tail ? k_b_update<true, true> : k_b_update<true, false>, sms);
+        b->g_upd0 = resident_grid(tail ? k_b_update<false, true> : k_b_update<false, false>, sms);
         b->g_init = resident_grid(k_b_init_norms, sms);
         cudaStream_t s = ctx->stream;
         cudaMemcpyAsync(b->d_nrhs, b->nrhs.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
@@ -956,6 +1012,7 @@ int mclsgpu_batch_build(mclsgpu_context* ctx, int nsys, const int64_t* n,
         cudaMemcpyAsync(b->d_seoff, seoff.data(), sizeof(long long) * nsys, cudaMemcpyHostToDevice,
                         s);
         cudaMemcpyAsync(b->d_slog, cls_of.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
+        cudaMemcpyAsync(b->d_slong, slong.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->d_sn, sn.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->d_sorder, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b->all_sys, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, s);
@@ -1090,7 +1147,8 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
     k_b_state_init<<<1, 1024, 0, s>>>(a, params->max_iters, params->check_freq,
                                        params->tolerance, pairs);
     k_b_init_norms<<<b->g_init, kThreads, 0, s>>>(a);
-    k_b_update<false><<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
+    auto norms = b->tail ? k_b_update<false, true> : k_b_update<false, false>;
+    norms<<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
     cudaMemsetAsync(b->norm2, 0, sizeof(double) * PR, s);
     cudaError_t e = cudaSuccess;
     int rc = MCLSGPU_OK;
@@ -1123,7 +1181,7 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
         std::vector<double> nr(PR), bn(PR);
         std::vector<int> ci(PR);
         cudaMemsetAsync(b->norm2, 0, sizeof(double) * PR, s);
-        k_b_update<false><<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
+        norms<<<b->g_upd0, kThreads, 0, s>>>(a, 0, cudaGraphConditionalHandle(0));
         cudaMemcpyAsync(nr.data(), b->norm2, sizeof(double) * PR, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(bn.data(), b->bnorm2, sizeof(double) * PR, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(ci.data(), b->conv_iter, sizeof(int) * PR, cudaMemcpyDeviceToHost, s);
