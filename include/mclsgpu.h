@@ -280,7 +280,8 @@ int mclsgpu_spai_infer(mclsgpu_spai* net, mclsgpu_operator* op, float* out, doub
 int mclsgpu_spai_infer_dev(mclsgpu_spai* net, mclsgpu_operator* op, float* out_dev,
                            double* mvals_dev, float* ms);
 /* Loss and parameter gradient (host, may be NULL) for nvec device vectors
- * stored one after another (v_dev[k*n + i]). */
+ * stored one after another (v_dev[k*n + i]).  The network keeps the device
+ * scratch of its largest gradient, up to 256 MB, until it is destroyed. */
 int mclsgpu_spai_gradient(mclsgpu_spai* net, mclsgpu_operator* op, const double* v_dev,
                           int nvec, double* loss, float* grad);
 /* One Adam step on that gradient; *loss receives the loss before the step. */
@@ -303,7 +304,9 @@ int mclsgpu_spai_rho(mclsgpu_spai* net, mclsgpu_operator* op, int iters, double*
  * 308-340, src/MCLS_AlmostOptimalDomain_impl.hpp:70-366): builds the
  * (transposed, for ADJOINT) composite operator PL*A*PR, the iteration matrix
  * H = I - w*M on its pattern, the per-row CDFs and weights, and the packed
- * FP32 walk records.  `right` may be NULL (no right preconditioner). */
+ * FP32 walk records.  `right` may be NULL (no right preconditioner).  Where the
+ * memory allows, FP64 domains with rows of at most 7 entries also hold 96 bytes
+ * a row, and larger forward FP32 domains on a structured grid 4. */
 int mclsgpu_domain_build(mclsgpu_context* ctx, mclsgpu_operator* op,
                          mclsgpu_precond* left, mclsgpu_precond* right,
                          const mclsgpu_mc_params* params,
@@ -606,10 +609,10 @@ int mclsgpu_batch_layout(mclsgpu_batch* b, int64_t* elem_offsets, int32_t* width
                          int64_t* elements, int32_t* max_width);
 /* The batch's block-diagonal domain (for mclsgpu_domain_query/reseed). */
 int mclsgpu_batch_domain(mclsgpu_batch* b, mclsgpu_domain** dom);
-/* Walk launch shape: threads per block (128 or 256) and the work-queue grab
- * (each warp takes 32 * grab histories per grab, 1..8).  The autotuner times
- * block sizes {256, 128} x grabs {1, 2, 4} on `reps` iterations of b_dev
- * (x_dev is overwritten) and keeps the fastest walk. */
+/* Walk launch shape: threads per block (128 or 256) and how many histories a
+ * warp takes at a time (32 * grab, 1..8).  The autotuner times block sizes
+ * {256, 128} x grabs {1, 2, 4} on `reps` iterations of b_dev (x_dev is
+ * overwritten) and keeps the fastest walk. */
 int mclsgpu_batch_set_launch(mclsgpu_batch* b, int block_size, int grab);
 int mclsgpu_batch_autotune(mclsgpu_batch* b, const double* b_dev, double* x_dev, int reps,
                            int* block_size, int* grab, double* walk_ms);

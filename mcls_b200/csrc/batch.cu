@@ -114,7 +114,6 @@ struct BatchArgs {
     double inv_per;      // 1 / histories per state
     int ev;              // expected-value estimator
     unsigned long long* d_epoch;
-    int* d_counter;
     unsigned long long* d_tim;
     int* status;
 };
@@ -425,8 +424,8 @@ __device__ void build_active(const BatchArgs& a) {
 }
 
 // Per-pair convergence, loop control and the per-iteration bookkeeping (new
-// stream epoch, work-queue reset, walk timing, norms cleared, the active
-// list rebuilt), run by one block.
+// stream epoch, walk timing, norms cleared, the active list rebuilt), run by
+// one block.
 __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphConditionalHandle handle) {
     __shared__ int s_conv;
     if (threadIdx.x == 0) s_conv = 0;
@@ -486,7 +485,6 @@ __device__ void batch_check(const BatchArgs& a, int use_cond, cudaGraphCondition
         st.done = !keep;
         *a.st = st;
         *a.d_epoch += 1;
-        *a.d_counter = 0;
         unsigned long long* t = a.d_tim;
         if (t[1] > t[0]) t[2] += t[1] - t[0];
         t[3] += 1;
@@ -677,7 +675,7 @@ struct mclsgpu_batch {
     uint64_t graph_seed = 0;       // the domain seed the captured walks carry
     int body_kernels = 0;
     int per = 1;
-    int grab = 1;                  // walk work-queue grab, in 32-history chunks
+    int grab = 1;                  // 32-history chunks that a walk's warp takes at a time
     // Grids of the element kernels: every block resident at once (each block
     // takes one contiguous range, so a second wave would double the time).
     int g_rich = 1, g_src = 1, g_cor = 1, g_upd = 1, g_upd0 = 1, g_init = 1;
@@ -783,7 +781,6 @@ BatchArgs batch_args(mclsgpu_batch* b, const mclsgpu_mcsa_params* mp, bool all) 
     a.inv_per = 1.0 / double(b->per);
     a.ev = p.estimator == MCLSGPU_EXPECTED_VALUE;
     a.d_epoch = b->dom->d_epoch;
-    a.d_counter = b->dom->d_counter;
     a.d_tim = b->dom->d_tim;
     a.status = b->ctx->d_status;
     return a;
@@ -1132,7 +1129,6 @@ int mclsgpu_batch_mcsa_solve_dev(mclsgpu_batch* b, const double* b_dev, double* 
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaMemsetAsync(ctx->d_status, 0, sizeof(int), s);
-    cudaMemsetAsync(b->dom->d_counter, 0, sizeof(int), s);
     cudaMemsetAsync(b->dom->d_steps, 0, sizeof(unsigned long long), s);
     cudaMemsetAsync(b->blocks_done, 0, sizeof(unsigned), s);
     {

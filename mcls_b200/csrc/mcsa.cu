@@ -453,26 +453,24 @@ template <bool NORM, class Op>
 __device__ __forceinline__ void residual_pair(const Op& A, const double* mdia, const double* x,
                                               const double* b, double* out, int halo,
                                               const ResidArgs& a) {
-    if constexpr (Op::kDiags > 0) {
-        __shared__ double raw[kPairRows + 2 * kPairHalo];
-        const int rows = blockDim.x, r0 = blockIdx.x * rows, r1 = min(r0 + rows, A.n);
-        const int lo = max(r0 - halo, 0), hi = min(r1 + halo, A.n);
+    __shared__ double raw[kPairRows + 2 * kPairHalo];
+    const int rows = blockDim.x, r0 = blockIdx.x * rows, r1 = min(r0 + rows, A.n);
+    const int lo = max(r0 - halo, 0), hi = min(r1 + halo, A.n);
 #pragma unroll 2
-        for (int j = lo + int(threadIdx.x); j < hi; j += rows)
-            raw[j - lo] = b[j] - A.dot(j, [&](int c) { return x[c]; });
-        __syncthreads();
-        const int i = r0 + int(threadIdx.x);
-        double acc = 0.0;
-        if (i < r1) {
-            const double r = dot_on_diagonals(A, mdia, i, [&](int c) { return raw[c - lo]; });
-            out[i] = r;
-            if (NORM) {
-                a.x2[i] = __dadd_rn(x[i], __dmul_rn(a.w, r));
-                acc = r * r;
-            }
+    for (int j = lo + int(threadIdx.x); j < hi; j += rows)
+        raw[j - lo] = b[j] - A.dot(j, [&](int c) { return x[c]; });
+    __syncthreads();
+    const int i = r0 + int(threadIdx.x);
+    double acc = 0.0;
+    if (i < r1) {
+        const double r = dot_on_diagonals(A, mdia, i, [&](int c) { return raw[c - lo]; });
+        out[i] = r;
+        if (NORM) {
+            a.x2[i] = __dadd_rn(x[i], __dmul_rn(a.w, r));
+            acc = r * r;
         }
-        if (NORM) norm_and_check(a, acc);
     }
+    if (NORM) norm_and_check(a, acc);
 }
 template <class Op>
 __global__ void __launch_bounds__(kPairRows) k_residual_pair(Op A, const double* mdia,
@@ -897,7 +895,7 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     if (fold) {
         richardson_residual(dom, dom->x, dom->rp, mp->richardson_omega, dom->x2, dom->rp2);
     } else if (halo > 0) {
-        MCLSGPU_LAUNCH_OP(op, pairs, pair_rows, s, k_residual_pair, mdia, dom->x2, dom->b, dom->rp2,
+        MCLSGPU_LAUNCH_DIA(op, pairs, pair_rows, s, k_residual_pair, mdia, dom->x2, dom->b, dom->rp2,
                           halo);
     } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x2, dom->b, nullptr,
@@ -932,16 +930,16 @@ static void enqueue_iteration(mclsgpu_domain* dom, const mclsgpu_mcsa_params* mp
     a.handle = handle;
     a.use_cond = use_cond;
     if (halo > 0) {
-        MCLSGPU_LAUNCH_OP(op, pairs, pair_rows, s, k_residual_pair_norm, mdia, halo, a);
+        MCLSGPU_LAUNCH_DIA(op, pairs, pair_rows, s, k_residual_pair_norm, mdia, halo, a);
     } else if (mdia) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_residual, dom->x, dom->b, nullptr,
                           dom->tmp);
         MCLSGPU_LAUNCH_M(op, mdia, grid, kFusedThreads, s, k_precond_norm, a, dom->tmp);
     } else if (op->dia_k > 0 && n <= kClusterRows) {
         if (fold)
-            MCLSGPU_LAUNCH_OP(op, kClusterCtas, kClusterThreads, s, k_finalize_norm_cluster, a);
+            MCLSGPU_LAUNCH_DIA(op, kClusterCtas, kClusterThreads, s, k_finalize_norm_cluster, a);
         else
-            MCLSGPU_LAUNCH_OP(op, kClusterCtas, kClusterThreads, s, k_residual_norm_cluster, a);
+            MCLSGPU_LAUNCH_DIA(op, kClusterCtas, kClusterThreads, s, k_residual_norm_cluster, a);
     } else if (fold) {
         MCLSGPU_LAUNCH_OP(op, grid, kFusedThreads, s, k_finalize_norm, a);
     } else {

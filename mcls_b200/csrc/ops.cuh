@@ -15,7 +15,6 @@ struct SellView {  // SELL-32
     // must overlap (entry by entry 13.5 us for the residual of 10^5 rows of an
     // unstructured operator, 11.5 us so).  The registers cost resident blocks.
     static constexpr int kMinBlocks = 4;
-    static constexpr int kDiags = -1;  // not stored by diagonals
     static constexpr int kBatch = 8;
     const int* off;
     const int* col;
@@ -177,43 +176,48 @@ inline DiaViewT<KK> dia_view_vals(const mclsgpu_operator* op, const double* vals
         }                                                                                    \
     } while (0)
 
-// Launch `kern<Op>` on the operator's fastest layout: diagonal-offset values
-// for stencil operators (unrolled for the 5-, 7- and 9-point stencils; only
-// the diagonal and upper diagonals when the values are symmetric), SELL-32
-// otherwise.
-#define MCLSGPU_LAUNCH_OP(op, grid, threads, stream, kern, ...)                              \
+// Launch `kern<Op>` on a stencil operator's fastest layout (dia_k > 0):
+// diagonal-offset values, unrolled for the 5-, 7- and 9-point stencils; only the
+// diagonal and upper diagonals when the values are symmetric.
+#define MCLSGPU_LAUNCH_DIA(op, grid, threads, stream, kern, ...)                             \
     do {                                                                                     \
         switch ((op)->dia_k) {                                                               \
-            case 0:                                                                          \
-                kern<SellView><<<grid, threads, 0, stream>>>(sell_view(op), __VA_ARGS__);    \
-                break;                                                                       \
             case 5:                                                                          \
                 if ((op)->sym_h == 2)                                                        \
-                    kern<DiaSymView<2>><<<grid, threads, 0, stream>>>(sym_view<2>(op),        \
+                    kern<DiaSymView<2>><<<grid, threads, 0, stream>>>(sym_view<2>(op),       \
                                                                       __VA_ARGS__);          \
                 else                                                                         \
-                    kern<DiaViewT<5>><<<grid, threads, 0, stream>>>(dia_view<5>(op),          \
+                    kern<DiaViewT<5>><<<grid, threads, 0, stream>>>(dia_view<5>(op),         \
                                                                     __VA_ARGS__);            \
                 break;                                                                       \
             case 7:                                                                          \
                 if ((op)->sym_h == 3)                                                        \
-                    kern<DiaSymView<3>><<<grid, threads, 0, stream>>>(sym_view<3>(op),        \
+                    kern<DiaSymView<3>><<<grid, threads, 0, stream>>>(sym_view<3>(op),       \
                                                                       __VA_ARGS__);          \
                 else                                                                         \
-                    kern<DiaViewT<7>><<<grid, threads, 0, stream>>>(dia_view<7>(op),          \
+                    kern<DiaViewT<7>><<<grid, threads, 0, stream>>>(dia_view<7>(op),         \
                                                                     __VA_ARGS__);            \
                 break;                                                                       \
             case 9:                                                                          \
                 if ((op)->sym_h == 4)                                                        \
-                    kern<DiaSymView<4>><<<grid, threads, 0, stream>>>(sym_view<4>(op),        \
+                    kern<DiaSymView<4>><<<grid, threads, 0, stream>>>(sym_view<4>(op),       \
                                                                       __VA_ARGS__);          \
                 else                                                                         \
-                    kern<DiaViewT<9>><<<grid, threads, 0, stream>>>(dia_view<9>(op),          \
+                    kern<DiaViewT<9>><<<grid, threads, 0, stream>>>(dia_view<9>(op),         \
                                                                     __VA_ARGS__);            \
                 break;                                                                       \
             default:                                                                         \
                 kern<DiaView><<<grid, threads, 0, stream>>>(dia_view<0>(op), __VA_ARGS__);   \
         }                                                                                    \
+    } while (0)
+
+// The same, or on SELL-32 where the operator is no stencil.
+#define MCLSGPU_LAUNCH_OP(op, grid, threads, stream, kern, ...)                              \
+    do {                                                                                     \
+        if ((op)->dia_k == 0)                                                                \
+            kern<SellView><<<grid, threads, 0, stream>>>(sell_view(op), __VA_ARGS__);        \
+        else                                                                                 \
+            MCLSGPU_LAUNCH_DIA(op, grid, threads, stream, kern, __VA_ARGS__);                \
     } while (0)
 
 }  // namespace mclsgpu
