@@ -74,14 +74,14 @@ CONFIGS = {
 # forward expected-value walk32_rows launch of an MCSA iteration at 128^3.
 WALK_DRAM_BYTES_PER_LAUNCH = {"diffusion128": 119.1e6}
 # The same for the 192^3 roofline domain (226 MB of records, more than L2):
-# 368.1 MB + 51.1 MB in an MCSA iteration; a Monte Carlo solve's walk reads no
-# base iterate, 56.6 MB less.
-HBM_WALK_DRAM_BYTES_PER_LAUNCH = 362.6e6
+# 311.5 MB + 48.3 MB for the walk of a Monte Carlo solve, which is what is timed
+# (python -m mcls_b200.walkprof --n 192 --solves 2 --histories-per-lane 1).
+HBM_WALK_DRAM_BYTES_PER_LAUNCH = 359.8e6
 # The same capture's L2 and DRAM figures: what binds the walk (requests from
 # L1TEX to L2; each record is read from HBM about once per launch).
 HBM_WALK_NCU = {"l1tex_to_l2_request_pct_of_peak": 79.2, "lts_sectors_pct_of_peak": 32.5,
-                "lts_sector_hit_pct": 84.1, "dram_gbs": 1053.0,
-                "capture": "ncu, walk32_rows of an MCSA iteration, 192^3, two histories per row"}
+                "lts_sector_hit_pct": 85.8, "dram_gbs": 928.0,
+                "capture": "ncu, walk32_rows of a Monte Carlo solve, 192^3, two histories per row"}
 # The oracle port's whole MCSA solve of a workload, run once to the end
 # (FP64 forward expected-value walks on the counter stream, the workload's
 # histories per iteration, seed 1234): its iteration count, which the
